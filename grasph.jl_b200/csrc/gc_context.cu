@@ -908,8 +908,10 @@ int finalize(gc_ctx* ctx) {
             G.cell = 2.0 * h.H;
             G.cutoff_sq = G.cell * G.cell;
             G.knorm = kernel_norm(h.kk, I.sys[h.a].nd, h.H);
-            G.f_invH = (float)(1.0 / h.H);
-            G.f_knorm = (float)G.knorm;
+            G.inv_cell = 1.0 / G.cell;
+            const bool spline = h.kk == GC_KERNEL_CUBIC_SPLINE;
+            G.f_qs = (float)(spline ? 0.5 / h.H : 1.0 / h.H);
+            G.kq = spline ? -3.0 * G.knorm / h.H : -10.0 * G.knorm / (h.H * h.H);
             if (h.b >= 0) {
                 const HHandle& hh = I.handles[h.b];
                 for (int d = 0; d < 3; ++d) {
@@ -1599,11 +1601,16 @@ int ghost_copy(gc_ctx* ctx, DGhost& G, int stage) {
     return check_launch(ctx, "ghost copy");
 }
 
-// FP32-sweep buffers of a slot or ghost set: N FP64 positions (pos_stride
-// each) followed by N FP32 records (pack_stride floats each).
+// FP32-sweep buffers of a slot or ghost set: the planar FP32 positions
+// (padded to whole quads), N position-only records (pos_quads each), then N
+// sweep records (rec_quads of the mode each).
+float* hpos_of(float* fpk) { return fpk; }
+float4* pos_of(float* fpk, int64_t N, int nd) { return reinterpret_cast<float4*>(fpk) + (N * nd + 3) / 4; }
+float4* rec_of(float* fpk, int64_t N, int nd) { return pos_of(fpk, N, nd) + N * pos_quads(nd); }
+
 template <class T>
-int ensure_fpk(gc_ctx* ctx, T& X, int64_t N, int nd, int ns) {
-    int64_t need = N * (2 * pos_stride(nd) + pack_stride(nd, ns));
+int ensure_fpk(gc_ctx* ctx, T& X, int64_t N, int nd, int mode) {
+    int64_t need = 4 * ((N * nd + 3) / 4 + N * (pos_quads(nd) + rec_quads(nd, mode)));
     if (need > X.cap_fpk) {
         CU(cudaStreamSynchronize(ctx->stream));
         dfree(ctx, X.fpk, X.cap_fpk);
@@ -1613,12 +1620,6 @@ int ensure_fpk(gc_ctx* ctx, T& X, int64_t N, int nd, int ns) {
         X.xpk_static = false;
     }
     return GC_OK;
-}
-
-int aux_mode_for(int pfn) {
-    if (pfn == GC_PFN_FLUID) return AUX_P_OVER_RHO2;
-    if (pfn == GC_PFN_CAUCHY_FLUID) return AUX_INV_RHO2;
-    return AUX_MASS_OVER_RHO;
 }
 
 // The ghosts' side of an XSPH sweep against ghost system_b (`A` holds the
@@ -1672,7 +1673,7 @@ int xsph_ghost_side(gc_ctx* ctx, const ForceArgs& A, int id, int stage) {
     R.a_mass = G.d_mass;
     R.a_cf = nullptr;
     R.a_massf = nullptr;
-    R.afp = nullptr;
+    R.arec = nullptr;
     R.prec = GC_PRECISION_FP64;
     R.nref = 1;
     InterRef& r = R.ref[0];
@@ -1789,7 +1790,7 @@ PackPlan pack_plan(gc_ctx* ctx, int a, const std::vector<int>& ids, int stage, b
     pl.interp = (pl.pk0 == GC_PFN_INTERPOLATE || pl.pk0 == GC_PFN_NEIGHBOR_COUNT) && !count_only;
     // FluidSolidPfn runs the FluidPfn kernel in its fluid-solid mode (PfnInst.fs)
     pl.pfn = pl.pk0 == GC_PFN_FLUID_SOLID ? GC_PFN_FLUID : pl.pk0;
-    pl.mode = aux_mode_for(pl.pfn);
+    pl.mode = aux_mode(pl.pfn);
     pl.xsph = pl.pfn == GC_PFN_XSPH;  // writes v_adjustment; always FP64
     pl.fp32 = ctx->precision == GC_PRECISION_FP32_COMPENSATED && pl.pfn != GC_PFN_COUNT && !pl.xsph && !count_only;
     for (int id : ids)
@@ -1829,22 +1830,16 @@ int sweep_group(gc_ctx* ctx, int a, const std::vector<int>& ids, int stage, bool
     if (pl.interp) return interp_sweeps(ctx, a, ids, stage);
     const int pk0 = pl.pk0, pfn = pl.pfn, mode = pl.mode, pk_ns = pl.pk_ns;
     const bool xsph = pl.xsph, fp32 = pl.fp32;
-    // FP32 sweep buffers: positions, then records (see ensure_fpk)
-    auto xp_of = [](float* fpk) { return (double*)fpk; };
-    auto pk_of = [](float* fpk, int64_t N, int nd) { return fpk + N * 2 * pos_stride(nd); };
     if (pfn != GC_PFN_COUNT && !xsph) {
         if (fp32) {
-            TRY(ensure_fpk(ctx, S, S.N, S.nd, pk_ns));
+            TRY(ensure_fpk(ctx, S, S.N, S.nd, mode));
             // the fused half step of this step may have packed these records
             const bool done = S.pack_done_epoch == ctx->pack_epoch && S.pack_done_stage == stage &&
                               S.pack_done_mode == mode && S.pack_done_ns == pk_ns;
             if (!done) {
-                // positions do not change between the stages of a step
-                const bool pos = S.xpk_epoch != ctx->pack_epoch;
                 launch_pack32(mode, S.N, nullptr, S.nd, pk_ns, S.F(F_X), S.F(F_V), S.F(F_RHO), S.F(F_P),
-                              S.F(F_STRESS), S.inst_of, S.d_mass, pos ? xp_of(S.fpk) : nullptr,
-                              pk_of(S.fpk, S.N, S.nd), ctx->stream);
-                S.xpk_epoch = ctx->pack_epoch;
+                              S.F(F_STRESS), S.inst_of, S.d_mass, hpos_of(S.fpk), nullptr, rec_of(S.fpk, S.N, S.nd),
+                              ctx->stream);
             }
         } else {
             launch_aux(mode, S.N, nullptr, S.F(F_RHO), S.F(F_P), S.inst_of, S.d_mass, S.aux, ctx->stream);
@@ -1874,7 +1869,7 @@ int sweep_group(gc_ctx* ctx, int a, const std::vector<int>& ids, int stage, bool
     A.a_mass = S.d_mass;
     A.a_cf = S.d_cf;
     A.a_massf = S.d_massf;
-    A.afp = fp32 ? pk_of(S.fpk, S.N, S.nd) : nullptr;
+    A.arec = fp32 ? rec_of(S.fpk, S.N, S.nd) : nullptr;
     A.prec = fp32 ? GC_PRECISION_FP32_COMPENSATED : GC_PRECISION_FP64;
     A.err = ctx->d_err;
     A.num_sms = ctx->num_sms;
@@ -1931,17 +1926,15 @@ int sweep_group(gc_ctx* ctx, int a, const std::vector<int>& ids, int stage, bool
             if (pfn != GC_PFN_COUNT && !xsph && !fp32)
                 launch_aux(mode, G.CAP, G.d_count, G.rho, G.p, G.ginst[G.cur], G.d_mass, G.aux, ctx->stream);
             r.baux = G.aux;
-            r.bfp = nullptr;
-            r.bxp = nullptr;
+            r.brec = nullptr;
             if (fp32) {
-                TRY(ensure_fpk(ctx, G, G.CAP, G.nd, pk_ns));
-                const bool pos = G.xpk_epoch != ctx->pack_epoch;
+                TRY(ensure_fpk(ctx, G, G.CAP, G.nd, mode));
                 launch_pack32(mode, G.CAP, G.d_count, G.nd, pk_ns, G.x[G.cur], G.v, G.rho, G.p, G.stress,
-                              G.ginst[G.cur], G.d_mass, pos ? xp_of(G.fpk) : nullptr, pk_of(G.fpk, G.CAP, G.nd),
+                              G.ginst[G.cur], G.d_mass, hpos_of(G.fpk), nullptr, rec_of(G.fpk, G.CAP, G.nd),
                               ctx->stream);
-                G.xpk_epoch = ctx->pack_epoch;
-                r.bfp = pk_of(G.fpk, G.CAP, G.nd);
-                r.bxp = xp_of(G.fpk);
+                r.bh = hpos_of(G.fpk);
+                r.brec = rec_of(G.fpk, G.CAP, G.nd);
+                r.brq = rec_quads(G.nd, mode);
             }
         } else {
             DSlot& B = ctx->slots[D.bslot];
@@ -1952,13 +1945,13 @@ int sweep_group(gc_ctx* ctx, int a, const std::vector<int>& ids, int stage, bool
             r.bp = B.F(F_P);
             r.bstress = B.F(F_STRESS);
             r.bN = B.N;
-            r.bfp = nullptr;
-            r.bxp = nullptr;
+            r.brec = nullptr;
             if (D.btype == BT_SELF) {
                 r.baux = S.aux;
                 if (fp32) {
-                    r.bfp = pk_of(S.fpk, S.N, S.nd);
-                    r.bxp = xp_of(S.fpk);
+                    r.bh = hpos_of(S.fpk);
+                    r.brec = rec_of(S.fpk, S.N, S.nd);
+                    r.brq = rec_quads(S.nd, mode);
                 }
             } else if ((D.btype == BT_SYSTEM || D.btype == BT_VIRTUAL) && pfn != GC_PFN_COUNT && !xsph && !fp32 &&
                        pk0 != GC_PFN_FLUID_SOLID) {
@@ -1968,20 +1961,25 @@ int sweep_group(gc_ctx* ctx, int a, const std::vector<int>& ids, int stage, bool
                 r.baux = B.aux;
             }
             if (fp32 && D.btype != BT_SELF) {
-                // dynamic walls lend only their positions; other systems their records too
+                // dynamic walls lend only their positions; other systems their records
                 const bool rec = D.btype == BT_SYSTEM || D.btype == BT_STATIC || D.btype == BT_VIRTUAL;
-                TRY(ensure_fpk(ctx, B, B.N, B.nd, pk_ns));
+                TRY(ensure_fpk(ctx, B, B.N, B.nd, mode));
                 // positions: once per step, once for good for a system that does not move
-                const bool pos = B.xmoves() ? B.xpk_epoch != ctx->pack_epoch : !B.xpk_static;
+                const bool pos = !rec && (B.xmoves() ? B.xpk_epoch != ctx->pack_epoch : !B.xpk_static);
                 launch_pack32(mode, B.N, nullptr, B.nd, pk_ns, B.F(F_X), B.F(F_V), B.F(F_RHO), B.F(F_P),
                               B.kind >= GC_SYS_STRESS ? B.F(F_STRESS) : nullptr, B.inst_of, B.d_mass,
-                              pos ? xp_of(B.fpk) : nullptr, rec ? pk_of(B.fpk, B.N, B.nd) : nullptr, ctx->stream);
-                B.xpk_epoch = ctx->pack_epoch;
-                if (!B.xmoves()) B.xpk_static = true;
-                r.bxp = xp_of(B.fpk);
+                              hpos_of(B.fpk), pos ? pos_of(B.fpk, B.N, B.nd) : nullptr,
+                              rec ? rec_of(B.fpk, B.N, B.nd) : nullptr, ctx->stream);
+                r.bh = hpos_of(B.fpk);
                 if (rec) {
-                    r.bfp = pk_of(B.fpk, B.N, B.nd);
+                    r.brec = rec_of(B.fpk, B.N, B.nd);
+                    r.brq = rec_quads(B.nd, mode);
                     B.pack_done_epoch = -1;  // packed in this sweep's mode: B's own sweep packs again
+                } else {
+                    B.xpk_epoch = ctx->pack_epoch;
+                    if (!B.xmoves()) B.xpk_static = true;
+                    r.brec = pos_of(B.fpk, B.N, B.nd);
+                    r.brq = pos_quads(B.nd);
                 }
             }
         }
@@ -2041,7 +2039,7 @@ int sweep_group(gc_ctx* ctx, int a, const std::vector<int>& ids, int stage, bool
         R.a_mass = B.d_mass;
         R.a_cf = B.d_cf;
         R.a_massf = B.d_massf;
-        R.afp = fp32 ? pk_of(B.fpk, B.N, B.nd) : nullptr;
+        R.arec = fp32 ? rec_of(B.fpk, B.N, B.nd) : nullptr;
         R.nref = 1;
         InterRef& r = R.ref[0];
         r.btype = BT_SYSTEM;
@@ -2058,8 +2056,9 @@ int sweep_group(gc_ctx* ctx, int a, const std::vector<int>& ids, int stage, bool
         r.bstress = S.F(F_STRESS);
         r.baux = S.aux;
         r.bN = S.N;
-        r.bfp = fp32 ? pk_of(S.fpk, S.N, S.nd) : nullptr;
-        r.bxp = fp32 ? xp_of(S.fpk) : nullptr;
+        r.bh = fp32 ? hpos_of(S.fpk) : nullptr;
+        r.brec = fp32 ? rec_of(S.fpk, S.N, S.nd) : nullptr;
+        r.brq = rec_quads(S.nd, mode);
         st = launch_force_f64(R, false, ctx->stream);
         if (st) return seterr(ctx, st, "two-sided functor not implemented on the device");
         TRY(check_launch(ctx, "sweep (system_b side)"));
@@ -2211,12 +2210,9 @@ int halfstep_stage1(gc_ctx* ctx, int a) {
         if (!groups.empty()) {
             const PackPlan pl = pack_plan(ctx, a, groups[0], 1, false);
             if (pl.fp32 && !pl.interp && !pl.xsph && pl.pfn != GC_PFN_COUNT) {
-                TRY(ensure_fpk(ctx, S, S.N, S.nd, pl.pk_ns));
-                const bool pos = S.xpk_epoch != ctx->pack_epoch;
+                TRY(ensure_fpk(ctx, S, S.N, S.nd, pl.mode));
                 pk = PackArgs{pl.mode, S.nd, pl.pk_ns, S.N, S.F(F_X), S.F(F_V), S.F(F_RHO), S.F(F_P), S.F(F_STRESS),
-                              S.inst_of, S.d_mass, pos ? (double*)S.fpk : nullptr,
-                              S.fpk + S.N * 2 * pos_stride(S.nd)};
-                S.xpk_epoch = ctx->pack_epoch;
+                              S.inst_of, S.d_mass, hpos_of(S.fpk), nullptr, rec_of(S.fpk, S.N, S.nd)};
                 S.pack_done_epoch = ctx->pack_epoch;
                 S.pack_done_stage = 1;
                 S.pack_done_mode = pl.mode;

@@ -9,17 +9,21 @@
 namespace gc {
 
 constexpr int FORCE_TPB = 128;  // threads per block of the sweep
+constexpr int WIN_TPB = 64;     // threads per block of the FP32-compensated sweep
 constexpr int FORCE_BUF = 64;   // staged-neighbour column of the counting sweep (shared memory)
 
 // Launch configurations of the sweep: (min resident blocks, staged
-// neighbours per thread, pair-loop unroll, chunk staging).  Chosen per
+// neighbours per thread, pair-loop unroll, chunk staging) of the FP64 sweep,
+// then the FP32-compensated one's resident blocks and chunk.  Chosen per
 // (system, stage) by the tuner in gc_context.cu.
 struct ForceCfg {
     int minb, buf, unroll;
-    int stg;  // > 0: k_sweep_stg with chunks of stg candidates (policies that stage copies; k_sweep otherwise)
+    int stg;         // > 0: k_sweep_stg with chunks of stg candidates (policies that stage copies; k_sweep otherwise)
+    int wminb, wch;  // k_sweep_win: resident blocks, candidates per chunk
 };
 constexpr int NUM_FORCE_CFG = GC_NUM_SWEEP_CONFIGS;
-constexpr ForceCfg FORCE_CFGS[NUM_FORCE_CFG] = {{4, 64, 1, 0}, {6, 64, 1, 0}, {5, 64, 1, 96}, {6, 64, 1, 96}};
+constexpr ForceCfg FORCE_CFGS[NUM_FORCE_CFG] = {
+    {4, 64, 1, 0, 8, 192}, {6, 64, 1, 0, 7, 224}, {5, 64, 1, 96, 10, 160}, {6, 64, 1, 96, 12, 128}};
 constexpr int MAX_REFS = 8;     // interactions fused into one launch
 
 // system_b kinds as seen by a functor (src/PairwiseFunctors.jl dispatch)
@@ -45,8 +49,9 @@ struct InterRef {
     const int32_t* cs;    // packed CSR over system_b (global b indices)
     int64_t cs_cells;     // cells of cs that are valid (an instance beyond them is skipped)
     const double *bx, *bv, *brho, *bp, *bstress, *baux;
-    const float* bfp;     // FP32 records of system_b (v, rho, aux, 1/rho, stress), pack_stride floats each
-    const double* bxp;    // FP64 positions of system_b, pos_stride doubles each (FP32 sweep), or nullptr
+    const float4* brec;   // FP32 records of system_b (position-only ones of a dynamic boundary), or nullptr
+    int brq;              // their stride in 16-byte quads
+    const float* bh;      // FP32 positions, planar (stride bN), or nullptr
     int64_t bN;           // planar stride of system_b's arrays
     int32_t* counts;      // optional per-particle accepted-pair counts
 };
@@ -61,10 +66,10 @@ struct ForceArgs {
     const double* a_mass;  // per-instance particle mass
     const float* a_cf;     // FP32 copies of the two above
     const float* a_massf;
-    const float* afp;      // FP32 records of system_a (FP32-compensated precision)
+    const float4* arec;    // FP32 records of system_a (FP32-compensated precision)
     int prec;              // GC_PRECISION_*
     int* err;
-    const int2* groups;        // warp groups (start, count) of system_a particles
+    const int2* groups;        // warp groups of system_a particles (group_of)
     const int64_t* ngroups;    // device count of groups
     int num_sms;
     int cfg;                   // index into FORCE_CFGS
@@ -73,6 +78,16 @@ struct ForceArgs {
     InterRef ref[MAX_REFS];
 };
 
+// A warp group: up to 32 consecutive particles of one instance.
+__host__ __device__ inline int2 group_of(int32_t start, int count, int inst) {
+    int2 g;
+    g.x = start;
+    g.y = inst << 6 | count;
+    return g;
+}
+__host__ __device__ inline int group_count(int2 g) { return g.y & 63; }
+__host__ __device__ inline int group_inst(int2 g) { return g.y >> 6; }
+
 int launch_force_f64(const ForceArgs& A, bool count_only, cudaStream_t s);
 void launch_groups_count(const GridInst* gi, int ninst, int nd, const int32_t* cs, int64_t ncols_cap,
                          int64_t cells_cap, int32_t* cnt, cudaStream_t s);
@@ -80,15 +95,35 @@ void launch_groups_fill(const GridInst* gi, int ninst, int nd, const int32_t* cs
                         int64_t ncols_cap, int64_t cells_cap, int2* groups, int64_t* ngroups, cudaStream_t s);
 void launch_aux(int mode, int64_t N, const int64_t* count, const double* rho, const double* p,
                 const int32_t* inst_of, const double* mass, double* aux, cudaStream_t s);
-// Per-particle records of the FP32-compensated sweep, one record per
-// particle so a neighbour costs one or two sectors instead of one per field:
-//   pk:  v[nd], rho, aux(mode), 1/rho, stress[ns], zero padding — pack_stride floats
-//   xpk: x[nd] in FP64, zero padding — pos_stride doubles (the exact neighbour test)
-// Either may be nullptr.  ns may be 0; stress may be nullptr (zeros).
-__host__ __device__ constexpr int pack_stride(int nd, int ns) { return (nd + 3 + ns + 3) / 4 * 4; }
-__host__ __device__ constexpr int pos_stride(int nd) { return nd == 2 ? 2 : 4; }
+// Divisor mode of a functor's records and caches.
+__host__ __device__ constexpr int aux_mode(int pfn) {
+    return pfn == GC_PFN_FLUID || pfn == PFN_FLUID2 ? AUX_P_OVER_RHO2
+           : pfn == GC_PFN_CAUCHY_FLUID             ? AUX_INV_RHO2
+                                                    : AUX_MASS_OVER_RHO;
+}
+// Per-particle records of the FP32-compensated sweep, in 16-byte quads, so a
+// neighbour costs two or three loads.  A position is an FP32 pair x = h + l
+// (h the nearest float, l the rest), whose differences are as good as the
+// FP64 difference rounded to FP32.  σ' is the stress over ρ².
+//   2-D: [hx hy lx ly] then
+//     fluid       [vx vy -p/ρ² 1/ρ] [ρ 0 0 0]
+//     strain rate [vx vy m/ρ 0]
+//     Cauchy      [vx vy 1/ρ ρ] [σ'xx σ'yy σ'xy 0]
+//   3-D: [hx hy hz w0] [lx ly lz w1] [vx vy vz w2], w being
+//     fluid       -p/ρ², 1/ρ, ρ
+//     strain rate m/ρ, 0, 0
+//     Cauchy      1/ρ, ρ, σ'xx, then [σ'yy σ'zz σ'xy σ'xz] [σ'yz 0 0 0]
+// A dynamic boundary lends only positions: its records are the position
+// quads alone (2-D the first, 3-D the first two with w = 0).
+__host__ __device__ constexpr int rec_quads(int nd, int mode) {
+    return mode == AUX_INV_RHO2 ? (nd == 2 ? 3 : 5) : mode == AUX_MASS_OVER_RHO ? (nd == 2 ? 2 : 3) : 3;
+}
+__host__ __device__ constexpr int pos_quads(int nd) { return nd == 2 ? 1 : 2; }
+// hpos: the positions' h alone, planar (the candidate test reads these).
+// Nothing is written without pos or rec, either of which may be nullptr; p
+// and stress may be nullptr (zeros).
 void launch_pack32(int mode, int64_t N, const int64_t* count, int nd, int ns, const double* x, const double* v,
                    const double* rho, const double* p, const double* stress, const int32_t* inst_of,
-                   const double* mass, double* xpk, float* pk, cudaStream_t s);
+                   const double* mass, float* hpos, float4* pos, float4* rec, cudaStream_t s);
 
 }  // namespace gc

@@ -45,11 +45,13 @@ struct SysInst {
 // Per (interaction, instance) grid and system_b parameters.
 struct GridInst {
     double H, cell;                    // h, 2h
-    // (2h)^2, then the FP32 copies of 1/h and of the kernel normalisation:
-    // one 16-byte load in the FP32-compensated pair code
-    alignas(16) double cutoff_sq;
-    float f_invH, f_knorm;
+    double cutoff_sq;                  // (2h)^2
+    double inv_cell;                   // 1/(2h), rounded
     double knorm;                      // kernel normalisation
+    // FP32-compensated sweep: the kernel's gradient and argument factors
+    // (cubic spline −3·knorm/h and 1/2h, Wendland C2 −10·knorm/h² and 1/h)
+    double kq;
+    float f_qs;
     double ming[MAXD];                 // grid origin (src/Interaction.jl:143)
     int64_t ng[MAXD];                  // cells per dimension (:179)
     int64_t ncells, cellbase;          // this instance's cells in the packed grid
@@ -62,27 +64,16 @@ struct GridInst {
     float f_normal[MAXD], f_beta, f_ljcut, f_bmass, f_bc;
     int side_b;                        // 1 in the system_b-side copy of a two-sided interaction
 };
-static_assert(offsetof(GridInst, cutoff_sq) % 16 == 0 && offsetof(GridInst, f_invH) == offsetof(GridInst, cutoff_sq) + 8 &&
-                  offsetof(GridInst, f_knorm) == offsetof(GridInst, cutoff_sq) + 12,
-              "(2h)^2, 1/h and the kernel normalisation are read as one 16-byte load");
-
 // Per (interaction, stage, instance) functor parameters.
 struct PfnInst {
     double alpha, beta, h, delta, eps;
-    // FP32 copies; h2eps = 0.01·h² (the first four 16-byte aligned: the pair
-    // code reads them as one float4)
-    alignas(16) float f_h;
-    float f_h2eps, f_alpha, f_beta;
+    // FP32 copies; h2eps = 0.01·h²
+    float f_h, f_h2eps, f_alpha, f_beta;
     float f_delta, f_eps;
     int S, has_delta, has_eps;
     int two;  // FluidPfn between two fluid systems, or FluidSolidPfn (both sides written)
     int fs;   // FluidSolidPfn: system_a's (the fluid's) pressure on both sides
 };
-static_assert(offsetof(PfnInst, f_h) % 16 == 0 && offsetof(PfnInst, f_h2eps) == offsetof(PfnInst, f_h) + 4 &&
-                  offsetof(PfnInst, f_alpha) == offsetof(PfnInst, f_h) + 8 &&
-                  offsetof(PfnInst, f_beta) == offsetof(PfnInst, f_h) + 12,
-              "h, 0.01·h², α and β are read as one float4");
-
 // Per (virtual system, instance) parameters.
 struct VirtInst {
     double pv[MAXD];  // prescribed_v

@@ -1,6 +1,5 @@
-// gc_pack.cuh — one particle's FP32 sweep record and FP64 position copy
-// (the layout of pack_stride / pos_stride in gc_force.h), shared by the pack
-// kernel and the fused half step.
+// gc_pack.cuh — one particle's FP32 sweep record (the layouts of rec_quads and
+// pos_quads in gc_force.h), shared by the pack kernel and the fused half step.
 #pragma once
 
 #include "gc_force.h"
@@ -8,71 +7,84 @@
 
 namespace gc {
 
-// One FP32 record of ND dimensions and NS stress components: with both
-// known at compile time the record stays in registers.
-template <int ND, int NS>
-__device__ __forceinline__ void pack_rec(const PackArgs& a, int64_t g) {
-    constexpr int R = pack_stride(ND, NS);
+// One record of ND dimensions in mode MODE (NS stress components for the
+// Cauchy functor): with all known at compile time it stays in registers.
+template <int ND, int MODE, int NS>
+__device__ __forceinline__ void pack_rec(const PackArgs& a, int64_t g, const float* h, const float* l) {
     const int64_t N = a.N;
-    float rec[R];
+    constexpr int RQ = rec_quads(ND, MODE);
     const double r = a.rho[g];
+    float v[ND];
 #pragma unroll
-    for (int d = 0; d < ND; ++d) rec[d] = (float)a.v[d * N + g];
-    rec[ND] = (float)r;
-    double aux;
-    if (a.mode == AUX_P_OVER_RHO2) aux = a.p ? a.p[g] / (r * r) : 0.0;  // boundaries may have no pressure
-    else if (a.mode == AUX_INV_RHO2) aux = 1.0 / (r * r);
-    else aux = a.mass[a.inst_of[g]] / r;
-    rec[ND + 1] = (float)aux;
-    rec[ND + 2] = (float)(1.0 / r);
+    for (int d = 0; d < ND; ++d) v[d] = (float)a.v[d * N + g];
+    float w0, w1, w2 = 0.f;
+    if (MODE == AUX_P_OVER_RHO2) {
+        w0 = a.p ? (float)(-(a.p[g] / (r * r))) : 0.f;  // boundaries may have no pressure
+        w1 = (float)(1.0 / r);
+        w2 = (float)r;
+    } else if (MODE == AUX_MASS_OVER_RHO) {
+        w0 = (float)(a.mass[a.inst_of[g]] / r);
+        w1 = 0.f;
+    } else {
+        w0 = (float)(1.0 / r);
+        w1 = (float)r;
+    }
+    float s[6] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
+    if (MODE == AUX_INV_RHO2 && a.stress) {
+        const double i2 = 1.0 / (r * r);
 #pragma unroll
-    for (int q = 0; q < NS; ++q) rec[ND + 3 + q] = a.stress ? (float)a.stress[q * N + g] : 0.0f;
-#pragma unroll
-    for (int q = ND + 3 + NS; q < R; ++q) rec[q] = 0.0f;
-    float4* o = reinterpret_cast<float4*>(a.pk + g * R);
-#pragma unroll
-    for (int q = 0; q < R / 4; ++q) o[q] = make_float4(rec[4 * q], rec[4 * q + 1], rec[4 * q + 2], rec[4 * q + 3]);
-}
-
-// Any other shape (the stress systems' checks admit none): run-time sizes.
-__device__ __forceinline__ void pack_rec_any(const PackArgs& a, int64_t g) {
-    const int64_t N = a.N;
-    const int nd = a.nd, ns = a.ns;
-    const int R = pack_stride(nd, ns);
-    float rec[16];
-    const double r = a.rho[g];
-    for (int d = 0; d < nd; ++d) rec[d] = (float)a.v[d * N + g];
-    rec[nd] = (float)r;
-    double aux;
-    if (a.mode == AUX_P_OVER_RHO2) aux = a.p ? a.p[g] / (r * r) : 0.0;
-    else if (a.mode == AUX_INV_RHO2) aux = 1.0 / (r * r);
-    else aux = a.mass[a.inst_of[g]] / r;
-    rec[nd + 1] = (float)aux;
-    rec[nd + 2] = (float)(1.0 / r);
-    for (int q = 0; q < ns; ++q) rec[nd + 3 + q] = a.stress ? (float)a.stress[q * N + g] : 0.0f;
-    for (int q = nd + 3 + ns; q < R; ++q) rec[q] = 0.0f;
-    float4* o = reinterpret_cast<float4*>(a.pk + g * R);
-    for (int q = 0; q < R / 4; ++q) o[q] = make_float4(rec[4 * q], rec[4 * q + 1], rec[4 * q + 2], rec[4 * q + 3]);
+        for (int q = 0; q < NS; ++q) s[q] = (float)(a.stress[q * N + g] * i2);
+    }
+    float4* o = a.rec + g * RQ;
+    if (ND == 2) {
+        o[0] = make_float4(h[0], h[1], l[0], l[1]);
+        o[1] = make_float4(v[0], v[1], w0, w1);
+        if (MODE == AUX_P_OVER_RHO2) o[2] = make_float4(w2, 0.f, 0.f, 0.f);
+        if (MODE == AUX_INV_RHO2) o[2] = make_float4(s[0], s[1], s[NS == 3 ? 2 : 3], 0.f);
+    } else {
+        o[0] = make_float4(h[0], h[1], h[ND - 1], w0);
+        o[1] = make_float4(l[0], l[1], l[ND - 1], w1);
+        o[2] = make_float4(v[0], v[1], v[ND - 1], MODE == AUX_INV_RHO2 ? s[0] : w2);
+        if (MODE == AUX_INV_RHO2) {
+            o[3] = make_float4(s[1], s[2], s[3], s[4]);
+            o[4] = make_float4(s[5], 0.f, 0.f, 0.f);
+        }
+    }
 }
 
 __device__ __forceinline__ void pack_one(const PackArgs& a, int64_t g) {
     const int64_t N = a.N;
-    const int nd = a.nd, ns = a.ns;
-    if (a.xpk) {
-        // 16-byte stores: (x, y) then (z, 0) in 3-D
-        double2* o = reinterpret_cast<double2*>(a.xpk + g * pos_stride(nd));
-        o[0] = make_double2(a.x[g], a.x[N + g]);
-        if (nd == 3) o[1] = make_double2(a.x[2 * N + g], 0.0);
+    float h[MAXD], l[MAXD];
+#pragma unroll
+    for (int d = 0; d < MAXD; ++d) {
+        const double x = d < a.nd ? a.x[d * N + g] : 0.0;
+        h[d] = (float)x;
+        l[d] = (float)(x - (double)h[d]);
     }
-    if (!a.pk) return;
-    // the records' shapes: no stress, or a Cauchy functor's stress (Voigt
-    // 3 or 4 in 2-D, 6 in 3-D)
-    if (nd == 3 && ns == 6) pack_rec<3, 6>(a, g);
-    else if (nd == 3 && ns == 0) pack_rec<3, 0>(a, g);
-    else if (nd == 2 && ns == 3) pack_rec<2, 3>(a, g);
-    else if (nd == 2 && ns == 4) pack_rec<2, 4>(a, g);
-    else if (nd == 2 && ns == 0) pack_rec<2, 0>(a, g);
-    else pack_rec_any(a, g);
+#pragma unroll
+    for (int d = 0; d < MAXD; ++d)
+        if (d < a.nd) a.hpos[d * N + g] = h[d];
+    if (a.pos) {
+        float4* o = a.pos + g * pos_quads(a.nd);
+        if (a.nd == 2) {
+            o[0] = make_float4(h[0], h[1], l[0], l[1]);
+        } else {
+            o[0] = make_float4(h[0], h[1], h[2], 0.f);
+            o[1] = make_float4(l[0], l[1], l[2], 0.f);
+        }
+    }
+    if (!a.rec) return;
+    // (other shapes of stress have no sweep: the launch refuses them)
+    if (a.nd == 3) {
+        if (a.mode == AUX_P_OVER_RHO2) pack_rec<3, AUX_P_OVER_RHO2, 0>(a, g, h, l);
+        else if (a.mode == AUX_MASS_OVER_RHO) pack_rec<3, AUX_MASS_OVER_RHO, 0>(a, g, h, l);
+        else if (a.ns == 6) pack_rec<3, AUX_INV_RHO2, 6>(a, g, h, l);
+    } else {
+        if (a.mode == AUX_P_OVER_RHO2) pack_rec<2, AUX_P_OVER_RHO2, 0>(a, g, h, l);
+        else if (a.mode == AUX_MASS_OVER_RHO) pack_rec<2, AUX_MASS_OVER_RHO, 0>(a, g, h, l);
+        else if (a.ns == 3) pack_rec<2, AUX_INV_RHO2, 3>(a, g, h, l);
+        else if (a.ns == 4) pack_rec<2, AUX_INV_RHO2, 4>(a, g, h, l);
+    }
 }
 
 }  // namespace gc

@@ -29,7 +29,7 @@ struct UpdArgs {
     double *rho, *p, *stress, *sr, *vort, *strain, *strainp, *dvdt, *drhodt;
 };
 
-// One slot's FP32 sweep records (launch_pack32's arguments; xpk or pk may
+// One slot's FP32 sweep records (launch_pack32's arguments; pos or rec may
 // be nullptr).
 struct PackArgs {
     int mode, nd, ns;
@@ -37,16 +37,15 @@ struct PackArgs {
     const double *x, *v, *rho, *p, *stress;
     const int32_t* inst_of;
     const double* mass;
-    double* xpk;
-    float* pk;
+    float* hpos;
+    float4 *pos, *rec;
 };
-
 
 void launch_halfstep(const StepArgs& a, cudaStream_t s);
 // The half step fused with what follows it for the same particles before
 // the first sweeps (src/TimeIntegration.jl:158, then _sweep_all_stages!'s
 // stage-1 state updater :401-419): per particle the half step, the updater
-// u (u.kind < 0: none; an elementwise kind), then (pk.pk or pk.xpk set) the
+// u (u.kind < 0: none; an elementwise kind), then (pk.pos or pk.rec set) the
 // FP32 records of the stage's first sweep.  One pass over the state instead
 // of three.
 void launch_halfstep_fused(const StepArgs& a, const UpdArgs& u, const PackArgs& pk, cudaStream_t s);

@@ -4,6 +4,6 @@
 
 namespace gc {
 
-GC_DEFINE_FORCE_TU(2, false, launch_force_2d_f64)
+GC_DEFINE_FORCE_TU(2, launch_force_2d_f64)
 
 }  // namespace gc

@@ -1,9 +1,8 @@
-// k_force_2d_f32.cu — 2-D instantiations of the fused pair sweep, FP32-compensated.
-// Compiled with -fmad=false (reference rounding of the FP64 parts).
-#include "k_force_impl.cuh"
+// k_force_2d_f32.cu — 2-D instantiations of the FP32-compensated pair sweep.
+#include "k_sweep_f32.cuh"
 
 namespace gc {
 
-GC_DEFINE_FORCE_TU(2, true, launch_force_2d_f32)
+GC_DEFINE_FORCE_F32_TU(2, launch_force_2d_f32)
 
 }  // namespace gc

@@ -4,6 +4,6 @@
 
 namespace gc {
 
-GC_DEFINE_FORCE_TU(3, false, launch_force_3d_f64)
+GC_DEFINE_FORCE_TU(3, launch_force_3d_f64)
 
 }  // namespace gc

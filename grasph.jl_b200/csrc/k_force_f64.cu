@@ -66,14 +66,15 @@ __global__ void k_groups_fill(const GridInst* __restrict__ gi, int ninst, int nd
     const int64_t T = gi[ninst - 1].colbase + gi[ninst - 1].ncols;
     for (int64_t c = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; c < T && c < ncols_cap;
          c += (int64_t)gridDim.x * blockDim.x) {
-        const GridInst& G = gi[find_inst(gi, ninst, c)];
+        const int k = find_inst(gi, ninst, c);
+        const GridInst& G = gi[k];
         if (G.cellbase + G.ncells > cells_cap) continue;
         const int64_t ngl = G.ng[nd - 1];
         const int64_t local = c - G.colbase;
         const int64_t b = G.cellbase + local * ngl;
         const int32_t s0 = cs[b], n = cs[b + ngl] - s0;
         int32_t o = off[c];
-        for (int32_t q = 0; q < n; q += 32) groups[o++] = make_int2(s0 + q, n - q < 32 ? n - q : 32);
+        for (int32_t q = 0; q < n; q += 32) groups[o++] = group_of(s0 + q, n - q < 32 ? n - q : 32, k);
     }
     if (blockIdx.x == 0 && threadIdx.x == 0) *ngroups = off[ncols_cap];
 }
@@ -118,11 +119,11 @@ __global__ void k_pack32(PackArgs a, const int64_t* count) {
 
 void launch_pack32(int mode, int64_t N, const int64_t* count, int nd, int ns, const double* x, const double* v,
                    const double* rho, const double* p, const double* stress, const int32_t* inst_of,
-                   const double* mass, double* xpk, float* pk, cudaStream_t s) {
-    if (N <= 0 || (!xpk && !pk)) return;
+                   const double* mass, float* hpos, float4* pos, float4* rec, cudaStream_t s) {
+    if (N <= 0 || (!pos && !rec)) return;
     int64_t blocks = (N + 255) / 256;
     if (blocks > 148 * 64) blocks = 148 * 64;
-    PackArgs a{mode, nd, ns, N, x, v, rho, p, stress, inst_of, mass, xpk, pk};
+    PackArgs a{mode, nd, ns, N, x, v, rho, p, stress, inst_of, mass, hpos, pos, rec};
     k_pack32<<<(int)blocks, 256, 0, s>>>(a, count);
     g_launches.fetch_add(1, std::memory_order_relaxed);
 }

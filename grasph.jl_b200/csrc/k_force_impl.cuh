@@ -1,4 +1,5 @@
-// k_force_impl.cuh — the fused pair sweep (FP64 reference arithmetic and FP32-compensated).
+// k_force_impl.cuh — the fused pair sweep in FP64, and what it shares with the
+// FP32-compensated one (k_sweep_f32.cuh).
 //
 // Gather formulation of src/Interaction.jl:393-732: one thread owns one
 // system_a particle and sums its side of every accepted pair of every
@@ -15,8 +16,7 @@
 // column of shared memory and processed in batches: the expensive pair
 // physics runs with every lane busy instead of diverging on rejections.
 //
-// The FP64 policy relies on -fmad=false; the FP32 policy uses explicit
-// __dmul_rn/__dadd_rn for the exact acceptance test.
+// The arithmetic relies on -fmad=false.
 #pragma once
 #include <type_traits>
 #include <cstdio>
@@ -370,29 +370,14 @@ __device__ __forceinline__ int process_pair(const ForceArgs& A, const InterRef& 
     return 1;
 }
 
-// ------------------------------------------------------------ policies
-// The candidate walk below is shared by two physics policies:
-//   PhysF64  the reference's FP64 expression trees (bit-identical pair terms)
-//   PhysF32  FP32 pair physics with Kahan-compensated per-particle sums
-// Both apply the exact FP64 acceptance test, so neighbour sets are identical.
-
+// ------------------------------------------------------------ policy
 template <int ND, int NS, int PFN, int KK>
 struct PhysF64 {
-    static constexpr bool BLOCKED = false;  // plain FP64 sums: nothing to merge at strip ends
     struct Own {
         OwnState<ND> o;
         double sig[NS > 0 ? NS : 1];
     };
     using AccT = Acc<ND, NS>;
-    static constexpr int NSUM = 1;  // (plain FP64 sums live in AccT)
-    template <class Sum>
-    static __device__ __forceinline__ void flush(AccT&, Sum&) {}
-    template <class Sum>
-    static __device__ __forceinline__ void init_sum(Sum&) {}
-    template <class Sum>
-    static __device__ __forceinline__ void store_sum(const ForceArgs& A, int64_t gi, const AccT& acc, Sum&) {
-        store(A, gi, acc);
-    }
     static __device__ __forceinline__ void load(const ForceArgs& A, int64_t gi, Own& w) {
         const int64_t N = A.aN;
 #pragma unroll
@@ -521,423 +506,53 @@ struct PhysF64 {
     }
 };
 
-// ---------------------------------------------------------------- FP32
-__device__ __forceinline__ void kadd(float& s, float& c, float x) {
-    // Kahan (compensated) summation: c carries the rounding error of s.
-    float y = x - c;
-    float t = s + y;
-    c = (t - s) - y;
-    s = t;
-}
-
-// x added to a strip's partial sum when `on`.  An explicit round-to-nearest
-// add: the compiler may not fuse it with the product that made x, which it
-// would otherwise do differently in the two sweeps (and so change bits
-// between launch configurations).
-__device__ __forceinline__ void padd_if(float& p, float x, bool on) {
-    const float t = __fadd_rn(p, x);
-    p = on ? t : p;
-}
-
-// A particle's compensated sums (N components: sum s_j, compensation c_j),
-// in registers or in the warp's shared memory ([2N][32], one column per
-// lane, so a warp's accesses hit 32 different banks).
-template <int N>
-struct SumRegs {
-    float s[N], c[N];
-    __device__ __forceinline__ float& S(int j) { return s[j]; }
-    __device__ __forceinline__ float& C(int j) { return c[j]; }
-};
-template <int N>
-struct SumSmem {
-    float* b;
-    int lane;
-    __device__ __forceinline__ float& S(int j) { return b[j * 32 + lane]; }
-    __device__ __forceinline__ float& C(int j) { return b[(N + j) * 32 + lane]; }
-};
-
-
-template <int ND>
-__device__ __forceinline__ double dot_exact(const double* a, const double* b) {
-    double s = __dmul_rn(a[0], b[0]);
-#pragma unroll
-    for (int d = 1; d < ND; ++d) s = __dadd_rn(s, __dmul_rn(a[d], b[d]));
-    return s;
-}
-
-template <int ND>
-__device__ __forceinline__ float dotf(const float* a, const float* b) {
-    float s = a[0] * b[0];
-#pragma unroll
-    for (int d = 1; d < ND; ++d) s += a[d] * b[d];
-    return s;
-}
-
-template <int KK>
-__device__ __forceinline__ float kernel_dw_dq_f(float norm, float q) {
-    if (KK == GC_KERNEL_CUBIC_SPLINE) {
-        float a = fmaxf(0.f, 2.f - q), b = fmaxf(0.f, 1.f - q);
-        return norm * (-3.f * (0.25f * (a * a) - (b * b)));
-    } else {
-        float a = fmaxf(0.f, 2.f - q);
-        return ((-norm * 10.f) * q) * (a * a * a);
-    }
-}
-
-template <int ND, int NS, int PFN, int KK>
-struct PhysF32 {
-    // record layout of the FP32 pack (pack_stride floats per particle)
-    static constexpr int NSP = PFN == GC_PFN_CAUCHY_FLUID ? NS : 0;
-    static constexpr int R = pack_stride(ND, NSP);
-    static constexpr int XD = pos_stride(ND);
-    struct Own {
-        double x[ND];
-        float v[ND];
-        float rho, aux, irho;
-        float sig[NS > 0 ? NS : 1];
-    };
-    // one record by 16-byte loads
-    static __device__ __forceinline__ void rec_load(const float* __restrict__ pk, int64_t j, float* f) {
-        const float4* p = reinterpret_cast<const float4*>(pk + j * R);
-#pragma unroll
-        for (int q = 0; q < R / 4; ++q) {
-            const float4 t = p[q];
-            f[4 * q] = t.x;
-            f[4 * q + 1] = t.y;
-            f[4 * q + 2] = t.z;
-            f[4 * q + 3] = t.w;
-        }
-    }
-    static __device__ __forceinline__ void pos_load(const InterRef& r, int64_t j, double* x) {
-        if (r.bxp) {
-            const double2* p = reinterpret_cast<const double2*>(r.bxp + j * XD);
-            const double2 a = p[0];
-            x[0] = a.x;
-            x[1] = a.y;
-            if (ND == 3) x[ND - 1] = p[1].x;
-        } else {
-#pragma unroll
-            for (int d = 0; d < ND; ++d) x[d] = r.bx[d * r.bN + j];
-        }
-    }
-    // Per-particle sums s with Kahan compensation c, fed strip by strip: a
-    // pair's term goes into the plain FP32 partial p of its strip (AccT, in
-    // registers), and at the end of each strip p is added to s with
-    // compensation (the sums: registers in k_sweep, shared memory in
-    // k_sweep_stg).  Both sweeps evaluate a particle's pairs of a strip in
-    // the same order and merge at the same strip ends, so every launch
-    // configuration gives the same bits.  Components: dv/dt then dρ/dt
-    // (fluid, Cauchy and counting functors), or the strain rate then the
-    // vorticity.
-    static constexpr bool BLOCKED = true;
-    static constexpr bool FLUIDLIKE = fluid_pfn<PFN>() || PFN == GC_PFN_CAUCHY_FLUID || PFN == GC_PFN_COUNT;
-    static constexpr int NSX = NS > 0 ? NS : 1;
-    static constexpr int NVORT = ND == 2 ? 1 : 3;
-    static constexpr int NSUM = FLUIDLIKE ? ND + 1 : NSX + (PFN == GC_PFN_STRAIN_RATE_VORTICITY ? NVORT : 0);
-    static constexpr int IDR = ND;   // dρ/dt's component (fluid-like)
-    static constexpr int IW = NSX;   // the first vorticity component
-    struct AccT {
-        float p[NSUM];
-    };
-    // A zero partial is skipped (a compensated add of 0 would fold c into
-    // s), so a strip a sweep does not visit merges exactly like an empty one.
-    template <class Sum>
-    static __device__ __forceinline__ void flush(AccT& acc, Sum& sum) {
-#pragma unroll
-        for (int j = 0; j < NSUM; ++j) {
-            if (acc.p[j] != 0.f) kadd(sum.S(j), sum.C(j), acc.p[j]);
-            acc.p[j] = 0.f;
-        }
-    }
-    template <class Sum>
-    static __device__ __forceinline__ void init_sum(Sum& sum) {
-#pragma unroll
-        for (int j = 0; j < NSUM; ++j) sum.S(j) = sum.C(j) = 0.f;
-    }
-    static __device__ __forceinline__ void load(const ForceArgs& A, int64_t gi, Own& w) {
-        const int64_t N = A.aN;
-        float f[R];
-        rec_load(A.afp, gi, f);
-#pragma unroll
-        for (int d = 0; d < ND; ++d) {
-            w.x[d] = A.ax[d * N + gi];
-            w.v[d] = f[d];
-        }
-        w.rho = f[ND];
-        w.aux = f[ND + 1];
-        w.irho = f[ND + 2];
-#pragma unroll
-        for (int q = 0; q < NS; ++q) w.sig[q] = (PFN == GC_PFN_CAUCHY_FLUID) ? f[ND + 3 + q] : 0.f;
-    }
-    static __device__ __forceinline__ const double* xpos(const Own& w) { return w.x; }
-    static __device__ __forceinline__ void init(const ForceArgs&, int64_t, AccT& acc, bool) {
-#pragma unroll
-        for (int j = 0; j < NSUM; ++j) acc.p[j] = 0.f;
-    }
-    // (the sweeps merge every strip's partials before storing)
-    template <class Sum>
-    static __device__ __forceinline__ void store_sum(const ForceArgs& A, int64_t gi, const AccT&, Sum& sum) {
-        // FP64 state += compensated FP32 sum (s − c)
-        const int64_t N = A.aN;
-        if (FLUIDLIKE) {
-#pragma unroll
-            for (int d = 0; d < ND; ++d)
-                A.advdt[d * N + gi] = A.advdt[d * N + gi] + ((double)sum.S(d) - (double)sum.C(d));
-            A.adrhodt[gi] = A.adrhodt[gi] + ((double)sum.S(IDR) - (double)sum.C(IDR));
-        } else {
-#pragma unroll
-            for (int q = 0; q < NS; ++q) A.asr[q * N + gi] = A.asr[q * N + gi] + ((double)sum.S(q) - (double)sum.C(q));
-            if (PFN == GC_PFN_STRAIN_RATE_VORTICITY) {
-#pragma unroll
-                for (int q = 0; q < NVORT; ++q)
-                    A.avort[q * N + gi] = A.avort[q * N + gi] + ((double)sum.S(IW + q) - (double)sum.C(IW + q));
-            }
-        }
-    }
-    static __device__ __forceinline__ double plane_da(const Own& w, const GridInst& G) {
-        double t[ND];
-#pragma unroll
-        for (int d = 0; d < ND; ++d) t[d] = w.x[d] - G.point[d];
-        return dotv<ND>(t, G.normal);
-    }
-    template <int P2>
-    static __device__ __forceinline__ int pair(const ForceArgs& A, const InterRef& r, const GridInst& G,
-                                               const PfnInst& P, int64_t gi, int k, const Own& w, double da,
-                                               int32_t j, AccT& acc) {
-        double xj[ND];
-        pos_load(r, j, xj);
-        return pair_data<P2>(A, r, G, P, gi, k, w, da, xj, SrcGlobal{r.bfp, j}, make_float2(A.a_cf[k], A.a_massf[k]),
-                             acc);
-    }
-
-    // Where a neighbour's record comes from: global memory (k_sweep) or a
-    // staged shared-memory slot (k_sweep_stg).
-    struct SrcGlobal {
-        const float* pk;
-        int64_t j;
-        __device__ __forceinline__ void get(float* f) const { rec_load(pk, j, f); }
-    };
-    struct SrcSlot {
-        const float4* slot;
-        int BT;
-        __device__ __forceinline__ void get(float* f) const {
-#pragma unroll
-            for (int q = 0; q < R / 4; ++q) {
-                const float4 t = slot[(XD / 2 + q) * BT];
-                f[4 * q] = t.x;
-                f[4 * q + 1] = t.y;
-                f[4 * q + 2] = t.z;
-                f[4 * q + 3] = t.w;
-            }
-        }
-    };
-
-    // Copy of a neighbour's position and record into a shared-memory slot
-    // (16-byte asynchronous copies), chunk q at slot[q*BT]; pair_slot reads it.
-    static constexpr int NQP = XD / 2, NQR = R / 4, NQ = NQP + NQR;
-    static __device__ __forceinline__ void issue(const InterRef& r, const PfnInst&, int32_t j, float4* slot,
-                                                 int BT) {
-        const float4* px = reinterpret_cast<const float4*>(r.bxp + (int64_t)j * XD);
-#pragma unroll
-        for (int q = 0; q < NQP; ++q) __pipeline_memcpy_async(&slot[q * BT], &px[q], 16);
-        if (r.btype != BT_DYNAMIC) {
-            const float4* pr = reinterpret_cast<const float4*>(r.bfp + (int64_t)j * R);
-#pragma unroll
-            for (int q = 0; q < NQR; ++q) __pipeline_memcpy_async(&slot[(NQP + q) * BT], &pr[q], 16);
-        }
-    }
-    // system_a's FP32 sound speed and mass of instance k into the warp's slot
-    static __device__ __forceinline__ void stage_cam(const ForceArgs& A, int k, float2* cam) {
-        if (A.a_cf) *cam = make_float2(A.a_cf[k], A.a_massf[k]);
-    }
-    // cam: system_a's (FP32) sound speed and mass of this instance; BTK: the
-    // system_b kind when known at compile time (-1: r.btype)
-    template <int P2, int BTK = -1>
-    static __device__ __forceinline__ int pair_slot(const ForceArgs& A, const InterRef& r, const GridInst& G,
-                                                    const PfnInst& P, int64_t gi, int k, const Own& w, double da,
-                                                    const float4* slot, int BT, const float2* cam, AccT& acc) {
-        double xj[ND];
-#pragma unroll
-        for (int q = 0; q < NQP; ++q) {
-            const double2 t = *reinterpret_cast<const double2*>(&slot[q * BT]);
-            if (2 * q < ND) xj[2 * q] = t.x;
-            if (2 * q + 1 < ND) xj[2 * q + 1] = t.y;
-        }
-        return pair_data<P2, BTK>(A, r, G, P, gi, k, w, da, xj, SrcSlot{slot, BT}, *cam, acc);
-    }
-
-    template <int P2, int BTK = -1, class Src>
-    static __device__ __forceinline__ int pair_data(const ForceArgs& A, const InterRef& r, const GridInst& G,
-                                                    const PfnInst& P, int64_t gi, int k, const Own& w, double da,
-                                                    const double* xj, const Src& src, float2 cam, AccT& acc) {
-        const int bt = BTK >= 0 ? BTK : r.btype;
-        double dx[ND];
-#pragma unroll
-        for (int d = 0; d < ND; ++d) dx[d] = __dsub_rn(w.x[d], xj[d]);
-        const double rr = dot_exact<ND>(dx, dx);
-        // (2h)^2, 1/h and the kernel normalisation: one 16-byte load
-        const int4 gq = *reinterpret_cast<const int4*>(&G.cutoff_sq);
-        // the exact test decides, without a branch, whether the pair's terms
-        // are added (the pair's arithmetic stays one straight-line block)
-        const bool in = rr < __hiloint2double(gq.y, gq.x);
-        if (P2 == GC_PFN_COUNT) {
-            if (!in) return 0;
-            if constexpr (FLUIDLIKE) {
-                acc.p[0] += 1.f;
-                acc.p[IDR] += 1.f;
-            }
-            return 1;
-        }
-        float dxf[ND];
-#pragma unroll
-        for (int d = 0; d < ND; ++d) dxf[d] = (float)dx[d];
-        const float rrf = (float)rr;
-        const float rinv = rsqrtf(rrf);
-        const float rf = rrf * rinv;
-        // h, 0.01·h², α and β: one vector load
-        const float4 pv = *reinterpret_cast<const float4*>(&P.f_h);
-        const float invh = __int_as_float(gq.z);
-        const float q = rf * invh;
-        const float gc = kernel_dw_dq_f<KK>(__int_as_float(gq.w), q) * invh * rinv;
-        float gx[ND];
-#pragma unroll
-        for (int d = 0; d < ND; ++d) gx[d] = gc * dxf[d];
-        const float ca = cam.x, ma = cam.y;
-
-        float vj[ND], rhoj, auxj, irhoj;
-        float fj[R];
-        if (bt == BT_DYNAMIC) {
-            // src/PairwiseFunctors.jl:53,111,222,334: mirrored velocity, own density
-            float db = (float)da;
-#pragma unroll
-            for (int d = 0; d < ND; ++d) db -= dxf[d] * G.f_normal[d];
-            const float m = -fminf(G.f_beta, fabsf(__fdividef(db, (float)da)));
-#pragma unroll
-            for (int d = 0; d < ND; ++d) vj[d] = m * w.v[d];
-            rhoj = w.rho;
-            auxj = w.aux;
-            irhoj = w.irho;
-        } else {
-            src.get(fj);
-#pragma unroll
-            for (int d = 0; d < ND; ++d) vj[d] = fj[d];
-            rhoj = fj[ND];
-            auxj = fj[ND + 1];
-            irhoj = fj[ND + 2];
-        }
-        if constexpr (P2 == GC_PFN_STRAIN_RATE || P2 == GC_PFN_STRAIN_RATE_VORTICITY) {
-            float dv[ND];
-#pragma unroll
-            for (int d = 0; d < ND; ++d) dv[d] = vj[d] - w.v[d];
-            const float f = bt == BT_DYNAMIC ? w.aux : auxj;  // mass / rho
-            float sr[NS > 0 ? NS : 1];
-            if (ND == 2) {
-                sr[0] = dv[0] * gx[0];
-                sr[1] = dv[1] * gx[1];
-                if (NS == 4) {
-                    sr[2] = 0.f;
-                    sr[3] = 0.5f * (dv[0] * gx[1] + dv[1] * gx[0]);
-                } else {
-                    sr[2] = 0.5f * (dv[0] * gx[1] + dv[1] * gx[0]);
-                }
-            } else {
-                sr[0] = dv[0] * gx[0];
-                sr[1] = dv[1] * gx[1];
-                sr[2] = dv[2] * gx[2];
-                sr[3] = 0.5f * (dv[0] * gx[1] + dv[1] * gx[0]);
-                sr[4] = 0.5f * (dv[0] * gx[2] + dv[2] * gx[0]);
-                sr[5] = 0.5f * (dv[1] * gx[2] + dv[2] * gx[1]);
-            }
-            if constexpr (!FLUIDLIKE) {
-#pragma unroll
-                for (int q2 = 0; q2 < NS; ++q2) padd_if(acc.p[q2], sr[q2] * f, in);
-                if constexpr (P2 == GC_PFN_STRAIN_RATE_VORTICITY && PFN == GC_PFN_STRAIN_RATE_VORTICITY) {
-                    padd_if(acc.p[IW], 0.5f * (dv[0] * gx[1] - dv[1] * gx[0]) * f, in);
-                    if (ND == 3) {
-                        padd_if(acc.p[IW + 1], 0.5f * (dv[0] * gx[2] - dv[2] * gx[0]) * f, in);
-                        padd_if(acc.p[IW + 2], 0.5f * (dv[1] * gx[2] - dv[2] * gx[1]) * f, in);
-                    }
-                }
-            }
-            return in ? 1 : 0;
-        } else {
-            // momentum + continuity (FluidPfn, CauchyFluidPfn)
-            float dv[ND];
-#pragma unroll
-            for (int d = 0; d < ND; ++d) dv[d] = w.v[d] - vj[d];
-            const bool self = bt == BT_SELF, dyn = bt == BT_DYNAMIC;
-            const bool two = P2 == PFN_FLUID2 && P.two;  // multiphase / fluid-solid variant only
-            const float cb = ((P2 == GC_PFN_CAUCHY_FLUID && bt == BT_GHOST) || two) ? G.f_bc : ca;
-            float piv = 0.f;
-            const float vr = dotf<ND>(dxf, dv);
-            if (vr < 0.f) {
-                const float muv = __fdividef(pv.x * vr, rrf + pv.y);
-                const float mc = 0.5f * (ca + cb);
-                piv = (pv.w * muv - pv.z * mc) * muv * 2.f * w.irho * irhoj;
-            }
-            if (bt == BT_STATIC) {
-                const float x = G.f_ljcut * rinv, x2 = x * x, x6 = x2 * x2 * x2;
-                const float lj = rf < G.f_ljcut ? (x6 * x6 - x6) / rrf : 0.f;
-                const float rfj = (0.01f * ca) * ca * lj;
-                const float s = -G.f_bmass * piv;
-                if constexpr (FLUIDLIKE)
-#pragma unroll
-                    for (int d = 0; d < ND; ++d) padd_if(acc.p[d], s * gx[d] + rfj * dxf[d], in);
-                return in ? 1 : 0;
-            }
-            const float mj = (self || dyn) ? ma : G.f_bmass;
-            if (fluid_pfn<P2>()) {
-                float dh;
-                if (two && P.fs) {  // the fluid's pressure p = (p/ρ²)·ρ² on both sides
-                    if (G.side_b) dh = -(auxj + (auxj * rhoj * rhoj) * w.irho * w.irho);
-                    else dh = -(w.aux + (w.aux * w.rho * w.rho) * irhoj * irhoj);
-                } else {
-                    dh = -(w.aux + auxj);
-                }
-                // artificial surface tension ε·(−(|p_i| + |p_j|)/(ρ_i ρ_j)), with
-                // |p| = |p/ρ²|·ρ² from the record
-                if (two && P.has_eps) dh -= P.f_eps * (fabsf(w.aux) * w.rho * irhoj + fabsf(auxj) * rhoj * w.irho);
-                const float s = mj * (dh - piv);
-                if constexpr (FLUIDLIKE)
-#pragma unroll
-                    for (int d = 0; d < ND; ++d) padd_if(acc.p[d], s * gx[d], in);
-            } else {
-                // Cauchy stress divergence: stress_j is the own stress on a dynamic boundary
-                float sj[NS > 0 ? NS : 1];
-#pragma unroll
-                for (int q2 = 0; q2 < NS; ++q2) sj[q2] = dyn ? w.sig[q2] : fj[ND + 3 + q2];
-                const float ci = w.aux, cj = auxj;
-                float hv[ND];
-                if (ND == 2) {
-                    constexpr int XY = NS == 3 ? 2 : 3;
-                    hv[0] = (w.sig[0] * gx[0] + w.sig[XY] * gx[1]) * ci + (sj[0] * gx[0] + sj[XY] * gx[1]) * cj;
-                    hv[1] = (w.sig[XY] * gx[0] + w.sig[1] * gx[1]) * ci + (sj[XY] * gx[0] + sj[1] * gx[1]) * cj;
-                } else {
-                    hv[0] = (w.sig[0] * gx[0] + w.sig[3] * gx[1] + w.sig[4] * gx[2]) * ci +
-                            (sj[0] * gx[0] + sj[3] * gx[1] + sj[4] * gx[2]) * cj;
-                    hv[1] = (w.sig[3] * gx[0] + w.sig[1] * gx[1] + w.sig[5] * gx[2]) * ci +
-                            (sj[3] * gx[0] + sj[1] * gx[1] + sj[5] * gx[2]) * cj;
-                    hv[2] = (w.sig[4] * gx[0] + w.sig[5] * gx[1] + w.sig[2] * gx[2]) * ci +
-                            (sj[4] * gx[0] + sj[5] * gx[1] + sj[2] * gx[2]) * cj;
-                }
-                if constexpr (FLUIDLIKE)
-#pragma unroll
-                    for (int d = 0; d < ND; ++d) padd_if(acc.p[d], mj * (hv[d] - piv * gx[d]), in);
-            }
-            float tail = 0.f;
-            if (P.has_delta) {
-                const float cd = two ? 0.5f * (ca + cb) : ca;
-                const float psi = 2.f * P.f_delta * cd * pv.x * (w.rho - rhoj) * dotf<ND>(dxf, gx) / rrf;
-                tail = psi * irhoj;
-            }
-            if constexpr (FLUIDLIKE) padd_if(acc.p[IDR], mj * (dotf<ND>(dv, gx) + tail), in);
-            (void)gi;
-            return in ? 1 : 0;
-        }
-    }
-};
-
 // ------------------------------------------------ shared sweep pieces
+// The divisions of cells_of, out of line (rarely needed).
+template <int ND>
+static __device__ __noinline__ bool cells_divided(const GridInst& G, const double* x, int32_t* c) {
+    bool ok = true;
+    for (int d = 0; d < ND; ++d) {
+        int64_t cd;
+        const bool in = floor_i64(__dsub_rn(x[d], G.ming[d]) / G.cell, &cd) && cd >= 1 && cd < G.ng[d] - 1;
+        c[d] = in ? (int32_t)cd : 1;
+        ok = ok && in;
+    }
+    return ok;
+}
+
+// Cell coordinates floor((x − ming)/cell), and whether all lie inside the
+// grid's border cells (1 where not).  The quotients come from the stored
+// reciprocal, within a few ulps of the divided ones; only where that leaves
+// a floor in doubt (next to an integer, or out of range) are the divisions
+// made (src/Interaction.jl:197-206).
+template <int ND>
+__device__ __forceinline__ bool cells_of(const GridInst& G, const double* x, int32_t* c) {
+    double q[ND];
+    int64_t n[ND];
+#pragma unroll
+    for (int d = 0; d < ND; ++d) {
+        q[d] = __dsub_rn(x[d], G.ming[d]) * G.inv_cell;
+        n[d] = G.ng[d];
+    }
+    bool ok = true, sure = true;
+#pragma unroll
+    for (int d = 0; d < ND; ++d) {
+        c[d] = __double2int_rd(q[d]);
+        const double frac = q[d] - (double)c[d];
+        sure = sure && frac > 1e-9 && frac < 1.0 - 1e-9 && q[d] < 1048576.0;
+        ok = ok && c[d] >= 1 && c[d] < n[d] - 1;
+    }
+    if (sure && ok) return true;
+    double xs[ND];
+    int32_t cs[ND];
+#pragma unroll
+    for (int d = 0; d < ND; ++d) xs[d] = x[d];
+    ok = cells_divided<ND>(G, xs, cs);
+#pragma unroll
+    for (int d = 0; d < ND; ++d) c[d] = cs[d];
+    return ok;
+}
+
 // Per (warp, interaction) set-up of both sweeps.  Returns false when the
 // warp has nothing to do with this interaction: system_b's box is out of
 // reach of every lane (the box test has a 0.1% margin, so no pair is lost)
@@ -967,16 +582,7 @@ __device__ __forceinline__ bool ref_cells(const ForceArgs& A, const InterRef& r,
         return false;
     }
     // cell coordinates (a grid has < 2^31 cells, so they fit int32)
-    ok = true;
-#pragma unroll
-    for (int d = 0; d < ND; ++d) {
-        int64_t cd;
-        if (!floor_i64(__dsub_rn(ox[d], G.ming[d]) / G.cell, &cd) || cd < 1 || cd >= G.ng[d] - 1) {
-            ok = false;
-            cd = 1;
-        }
-        c[d] = (int32_t)cd;
-    }
+    ok = cells_of<ND>(G, ox, c);
     if (active && !ok) atomicOr(A.err, ERR_CAPACITY);
     c0 = __shfl_sync(FULL, c[0], 0);
     c1 = ND == 3 ? __shfl_sync(FULL, c[1], 0) : 0;
@@ -1135,16 +741,14 @@ __global__ void __launch_bounds__(FORCE_TPB, MINB) k_sweep(ForceArgs A) {
     const int64_t nwarps = ((int64_t)gridDim.x * blockDim.x) >> 5;
     for (int64_t wg = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5; wg < ngroups; wg += nwarps) {
         const int2 grp = A.groups[wg];
-        const bool active = lane < grp.y;
+        const bool active = lane < group_count(grp);
         const int32_t gi = grp.x + (active ? lane : 0);  // packed indices fit int32
-        const int k = A.a_inst_of[gi];
+        const int k = group_inst(grp);
         typename Phys::Own w;
         Phys::load(A, gi, w);
         const double* ox = Phys::xpos(w);
         typename Phys::AccT acc;
         Phys::init(A, gi, acc, !COUNT_ONLY);
-        SumRegs<Phys::NSUM> sum;
-        Phys::init_sum(sum);
 
         for (int ri = 0; ri < A.nref; ++ri) {
             const InterRef& r = A.ref[ri];
@@ -1215,14 +819,6 @@ __global__ void __launch_bounds__(FORCE_TPB, MINB) k_sweep(ForceArgs A) {
                         }
                         __syncwarp();
                     }
-                    if (Phys::BLOCKED) {
-                        // the strip's pairs, then its partial sums merged
-                        accepted += flush_all<Phys, COUNT_ONLY, UNROLL, PFN>(A, r, Gs, Ps, gi, k, w, da, nbuf, col,
-                                                                             BT, acc);
-                        nbuf = 0;
-                        __syncwarp();
-                        Phys::flush(acc, sum);
-                    }
                 }
                 accepted += flush_all<Phys, COUNT_ONLY, UNROLL, PFN>(A, r, Gs, Ps, gi, k, w, da, nbuf, col, BT, acc);
                 nbuf = 0;
@@ -1244,12 +840,6 @@ __global__ void __launch_bounds__(FORCE_TPB, MINB) k_sweep(ForceArgs A) {
                             nbuf = 0;
                         }
                     }
-                    if (Phys::BLOCKED) {
-                        accepted += flush_all<Phys, COUNT_ONLY, UNROLL, PFN>(A, r, Gs, Ps, gi, k, w, da, nbuf, col,
-                                                                             BT, acc);
-                        nbuf = 0;
-                        Phys::flush(acc, sum);
-                    }
                 }
                 accepted += flush_all<Phys, COUNT_ONLY, UNROLL, PFN>(A, r, Gs, Ps, gi, k, w, da, nbuf, col, BT, acc);
                 nbuf = 0;
@@ -1257,26 +847,26 @@ __global__ void __launch_bounds__(FORCE_TPB, MINB) k_sweep(ForceArgs A) {
             __syncwarp();
             if (active && r.counts) r.counts[gi] = accepted;
         }
-        if (!COUNT_ONLY && active) Phys::store_sum(A, gi, acc, sum);
+        if (!COUNT_ONLY && active) Phys::store(A, gi, acc);
         __syncwarp();
     }
 }
 
-// ------------------------------------------------- staged FP32 sweep
+// ------------------------------------------------------ staged sweep
 // Shared memory of one warp of k_sweep_stg: the staged copies of a chunk of
-// CH candidates ([NQ][CH] 16-byte chunks: FP64 position, then FP32 record),
+// CH candidates ([NQ][CH] 16-byte chunks: NbSlot's layout),
 // lane 0's position (the origin of the prefilter), the candidates' FP32
 // coordinates relative to it ([ND][CH]), and copies of the interaction's
 // grid and functor parameters for this warp's instance.
 constexpr int STG_GI_BYTES = SWEEP_GI_BYTES;
 constexpr int STG_PI_BYTES = SWEEP_PI_BYTES;
-template <int ND, int NQ, int CH, int NSUM>
+template <int ND, int NQ, int CH>
 __host__ __device__ constexpr int stg_warp_bytes() {
-    return NQ * CH * 16 + 32 + (ND * CH * 4 + 15) / 16 * 16 + STG_GI_BYTES + STG_PI_BYTES + 16 + NSUM * 2 * 32 * 4;
+    return NQ * CH * 16 + 32 + (ND * CH * 4 + 15) / 16 * 16 + STG_GI_BYTES + STG_PI_BYTES + 16;
 }
 
 
-// The FP32-compensated sweep with chunk staging.  The walk is k_sweep's (one
+// The sweep with chunk staging.  The walk is k_sweep's (one
 // warp per group of one grid column, the union of its lanes' candidate
 // ranges strip by strip), but the warp copies each chunk of up to CH
 // consecutive candidates of a strip into its shared memory once (16-byte
@@ -1284,14 +874,14 @@ __host__ __device__ constexpr int stg_warp_bytes() {
 // lane with the FP32 prefilter, and then evaluates each lane's accepted
 // candidates of the chunk from the staged copies.  No pair waits on a
 // global load; the exact cutoff test and the pair arithmetic are the
-// policy's pair_data, as in k_sweep.
+// policy's, as in k_sweep.
 template <class Phys, int ND, int PFN, int MINB, int CH>
 __global__ void __launch_bounds__(FORCE_TPB, MINB) k_sweep_stg(ForceArgs A) {
     pdl_enter();
     static_assert(CH % 32 == 0 && CH >= 32 && CH <= 128, "chunk of 1 to 4 batches of 32");
     constexpr int NB = CH / 32;
     constexpr int NQ = Phys::NQ;
-    constexpr int WB = stg_warp_bytes<ND, NQ, CH, Phys::NSUM>();
+    constexpr int WB = stg_warp_bytes<ND, NQ, CH>();
     extern __shared__ float4 sstg[];
     const unsigned FULL = 0xffffffffu;
     const int lane = threadIdx.x & 31;
@@ -1305,21 +895,18 @@ __global__ void __launch_bounds__(FORCE_TPB, MINB) k_sweep_stg(ForceArgs A) {
     GridInst* gsm = reinterpret_cast<GridInst*>(wbase + NQ * CH * 16 + 32 + (ND * CH * 4 + 15) / 16 * 16);
     PfnInst* psm = reinterpret_cast<PfnInst*>(reinterpret_cast<char*>(gsm) + STG_GI_BYTES);
     float2* camsm = reinterpret_cast<float2*>(reinterpret_cast<char*>(psm) + STG_PI_BYTES);
-    // this lane's compensated sums (touched only at strip ends)
-    SumSmem<Phys::NSUM> sum{reinterpret_cast<float*>(reinterpret_cast<char*>(camsm) + 16), lane};
     const int64_t ngroups = *A.ngroups;
     const int64_t nwarps = ((int64_t)gridDim.x * blockDim.x) >> 5;
     for (int64_t wg = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5; wg < ngroups; wg += nwarps) {
         const int2 grp = A.groups[wg];
-        const bool active = lane < grp.y;
+        const bool active = lane < group_count(grp);
         const int32_t gi = grp.x + (active ? lane : 0);  // packed indices fit int32
-        const int k = A.a_inst_of[gi];
+        const int k = group_inst(grp);
         typename Phys::Own w;
         Phys::load(A, gi, w);
         const double* ox = Phys::xpos(w);
         typename Phys::AccT acc;
         Phys::init(A, gi, acc, true);
-        Phys::init_sum(sum);
 
         for (int ri = 0; ri < A.nref; ++ri) {
             const InterRef& r = A.ref[ri];
@@ -1432,7 +1019,6 @@ __global__ void __launch_bounds__(FORCE_TPB, MINB) k_sweep_stg(ForceArgs A) {
                             }
                             __syncwarp();  // every lane is done with the chunk before the next one lands
                         }
-                        Phys::flush(acc, sum);  // the strip's partial sums
                     }
                 };
                 if (self) strips(std::integral_constant<int, BT_SELF>{});
@@ -1448,13 +1034,12 @@ __global__ void __launch_bounds__(FORCE_TPB, MINB) k_sweep_stg(ForceArgs A) {
                         if (self && j == gi) continue;
                         accepted += Phys::template pair<PFN>(A, r, G, P, gi, k, w, da, j, acc);
                     }
-                    Phys::flush(acc, sum);
                 }
             }
             __syncwarp();
             if (active && r.counts) r.counts[gi] = accepted;
         }
-        if (active) Phys::store_sum(A, gi, acc, sum);
+        if (active) Phys::store(A, gi, acc);
         __syncwarp();
     }
 }
@@ -1468,7 +1053,7 @@ static void launch_c(const ForceArgs& A, cudaStream_t s) {
     if (blocks > (int64_t)A.num_sms * cf.minb * 4) blocks = (int64_t)A.num_sms * cf.minb * 4;
     if (blocks < 1) blocks = 1;
     if constexpr (cf.stg > 0 && Phys::NQ > 0) {
-        constexpr size_t smem = (size_t)(FORCE_TPB / 32) * stg_warp_bytes<ND, Phys::NQ, cf.stg, Phys::NSUM>();
+        constexpr size_t smem = (size_t)(FORCE_TPB / 32) * stg_warp_bytes<ND, Phys::NQ, cf.stg>();
         auto kern = k_sweep_stg<Phys, ND, PFN, cf.minb, cf.stg>;
         if (smem > 48 * 1024) {
             static bool opted = false;
@@ -1503,86 +1088,66 @@ static void launch_cfg(const ForceArgs& A, cudaStream_t s) {
     }
 }
 
-// F32: this translation unit's precision (the FP32-compensated launches and
-// the FP64 ones are compiled separately).
-template <int ND, int NS, int PFN, int KK, bool F32>
+template <int ND, int NS, int PFN, int KK>
 static void launch_t(const ForceArgs& A, bool count_only, cudaStream_t s) {
-    if constexpr (F32) {
-        if constexpr (PFN != GC_PFN_COUNT && PFN != GC_PFN_XSPH && PFN != GC_PFN_INTERPOLATE)
-            launch_cfg<PhysF32<ND, NS, PFN, KK>, ND, PFN>(A, s);
+    using P64 = PhysF64<ND, NS, PFN, KK>;
+    if (count_only) {
+        int64_t blocks = (A.aN * 32 + FORCE_TPB - 1) / FORCE_TPB;
+        if (blocks > (int64_t)A.num_sms * 16) blocks = (int64_t)A.num_sms * 16;
+        if (blocks < 1) blocks = 1;
+        const size_t smem = (size_t)sweep_smem_bytes<ND>(FORCE_BUF);
+        k_sweep<P64, ND, PFN, true, 4, FORCE_BUF, 1><<<(int)blocks, FORCE_TPB, smem, s>>>(A);
     } else {
-        using P64 = PhysF64<ND, NS, PFN, KK>;
-        if (count_only) {
-            int64_t blocks = (A.aN * 32 + FORCE_TPB - 1) / FORCE_TPB;
-            if (blocks > (int64_t)A.num_sms * 16) blocks = (int64_t)A.num_sms * 16;
-            if (blocks < 1) blocks = 1;
-            const size_t smem = (size_t)sweep_smem_bytes<ND>(FORCE_BUF);
-            k_sweep<P64, ND, PFN, true, 4, FORCE_BUF, 1><<<(int)blocks, FORCE_TPB, smem, s>>>(A);
-        } else {
-            launch_cfg<P64, ND, PFN>(A, s);
-        }
+        launch_cfg<P64, ND, PFN>(A, s);
     }
     g_launches.fetch_add(1, std::memory_order_relaxed);
 }
 
-template <int ND, int NS, int KK, bool F32>
+template <int ND, int NS, int KK>
 static int launch_pfn(const ForceArgs& A, bool count_only, cudaStream_t s) {
     switch (A.pfn) {
-        case GC_PFN_FLUID: launch_t<ND, NS, GC_PFN_FLUID, KK, F32>(A, count_only, s); return 0;
-        case PFN_FLUID2: launch_t<ND, NS, PFN_FLUID2, KK, F32>(A, count_only, s); return 0;
-        case GC_PFN_COUNT: launch_t<ND, NS, GC_PFN_COUNT, KK, F32>(A, count_only, s); return 0;
-        case GC_PFN_INTERPOLATE:  // FP64 only
-            if constexpr (F32) {
-                return GC_ERR_UNSUPPORTED;
-            } else {
-                launch_t<ND, NS, GC_PFN_INTERPOLATE, KK, F32>(A, count_only, s);
-                return 0;
-            }
-        case GC_PFN_XSPH:  // FP64 only (a cheap, memory-bound functor)
-            if constexpr (F32) {
-                return GC_ERR_UNSUPPORTED;
-            } else {
-                launch_t<ND, NS, GC_PFN_XSPH, KK, F32>(A, count_only, s);
-                return 0;
-            }
+        case GC_PFN_FLUID: launch_t<ND, NS, GC_PFN_FLUID, KK>(A, count_only, s); return 0;
+        case PFN_FLUID2: launch_t<ND, NS, PFN_FLUID2, KK>(A, count_only, s); return 0;
+        case GC_PFN_COUNT: launch_t<ND, NS, GC_PFN_COUNT, KK>(A, count_only, s); return 0;
+        case GC_PFN_INTERPOLATE: launch_t<ND, NS, GC_PFN_INTERPOLATE, KK>(A, count_only, s); return 0;
+        case GC_PFN_XSPH: launch_t<ND, NS, GC_PFN_XSPH, KK>(A, count_only, s); return 0;
         case GC_PFN_CAUCHY_FLUID:
             if (NS == 0) return GC_ERR_UNSUPPORTED;
-            launch_t<ND, NS, GC_PFN_CAUCHY_FLUID, KK, F32>(A, count_only, s);
+            launch_t<ND, NS, GC_PFN_CAUCHY_FLUID, KK>(A, count_only, s);
             return 0;
         case GC_PFN_STRAIN_RATE:
             if (NS == 0) return GC_ERR_UNSUPPORTED;
-            launch_t<ND, NS, GC_PFN_STRAIN_RATE, KK, F32>(A, count_only, s);
+            launch_t<ND, NS, GC_PFN_STRAIN_RATE, KK>(A, count_only, s);
             return 0;
         case GC_PFN_STRAIN_RATE_VORTICITY:
             if (NS == 0) return GC_ERR_UNSUPPORTED;
-            launch_t<ND, NS, GC_PFN_STRAIN_RATE_VORTICITY, KK, F32>(A, count_only, s);
+            launch_t<ND, NS, GC_PFN_STRAIN_RATE_VORTICITY, KK>(A, count_only, s);
             return 0;
     }
     return GC_ERR_UNSUPPORTED;
 }
 
-template <int ND, int KK, bool F32>
+template <int ND, int KK>
 static int launch_nd(const ForceArgs& A, bool count_only, cudaStream_t s) {
     const bool stress_pfn = A.pfn == GC_PFN_CAUCHY_FLUID || A.pfn == GC_PFN_STRAIN_RATE ||
                             A.pfn == GC_PFN_STRAIN_RATE_VORTICITY ||
                             (A.pfn == GC_PFN_INTERPOLATE && (A.imask & (1 << GC_FIELD_STRESS)));
-    if (!stress_pfn) return launch_pfn<ND, 0, KK, F32>(A, count_only, s);
+    if (!stress_pfn) return launch_pfn<ND, 0, KK>(A, count_only, s);
     if (ND == 2) {
-        if (A.ns == 3) return launch_pfn<ND, 3, KK, F32>(A, count_only, s);
-        if (A.ns == 4) return launch_pfn<ND, 4, KK, F32>(A, count_only, s);
+        if (A.ns == 3) return launch_pfn<ND, 3, KK>(A, count_only, s);
+        if (A.ns == 4) return launch_pfn<ND, 4, KK>(A, count_only, s);
         return GC_ERR_UNSUPPORTED;
     }
-    if (A.ns == 6) return launch_pfn<ND, 6, KK, F32>(A, count_only, s);
+    if (A.ns == 6) return launch_pfn<ND, 6, KK>(A, count_only, s);
     return GC_ERR_UNSUPPORTED;
 }
 
-// One translation unit per (dimension, precision): defines
-// launch_force_<ND>d_<f32|f64>.
-#define GC_DEFINE_FORCE_TU(NDIM, F32, NAME)                                               \
+// One translation unit per dimension: defines launch_force_<ND>d_f64.
+#define GC_DEFINE_FORCE_TU(NDIM, NAME)                                                    \
     int NAME(const ForceArgs& A, bool count_only, cudaStream_t s) {                      \
         if (A.kk == GC_KERNEL_CUBIC_SPLINE)                                               \
-            return launch_nd<NDIM, GC_KERNEL_CUBIC_SPLINE, F32>(A, count_only, s);        \
-        return launch_nd<NDIM, GC_KERNEL_WENDLAND_C2, F32>(A, count_only, s);             \
+            return launch_nd<NDIM, GC_KERNEL_CUBIC_SPLINE>(A, count_only, s);            \
+        return launch_nd<NDIM, GC_KERNEL_WENDLAND_C2>(A, count_only, s);                 \
     }
 
 }  // namespace gc

@@ -61,7 +61,7 @@ __global__ void k_halfstep_fused(StepArgs a, UpdArgs u, PackArgs pk) {
     for (int64_t g = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; g < a.N; g += (int64_t)gridDim.x * blockDim.x) {
         halfstep_one(a, g);
         if (KIND >= 0) update_one<KIND>(u, g);
-        if (pk.pk || pk.xpk) pack_one(pk, g);
+        if (pk.pos || pk.rec) pack_one(pk, g);
     }
 }
 
