@@ -54,7 +54,6 @@ FP32C_TOL = {"rho": 1e-4, "stress": 1e-3}
 # slots that issued an instruction (smsp__issue_active) and the active lanes
 # per warp instruction
 ISSUE_PER_LAUNCH = {("dambreak_3d", "full", "fp32c"): (0.685, 20.94), ("dambreak_3d", "full", "fp64"): (0.625, 17.26)}
-STAGED_CONFIGS = (2, 3)  # launch configurations that run the FP64 sweep chunk-staged
 
 
 def build_workload(name, scale):
@@ -506,16 +505,10 @@ def run_ours(args, rank, world, local_rank):
     flops_per_launch = pairs * FLUID_PAIR_FLOPS[nd]
     achieved_tflops = flops_per_launch / sweep_avg_s / 1e12
     f32 = prec == G.PRECISION_FP32_COMPENSATED
-    # the launch configuration the autotuner kept for most sweeps names the
-    # FP64 kernel: configurations 2 and 3 are the chunk-staged sweep
-    chosen = st1["sweep_cfg_chosen"]
-    staged = f32 or max(range(len(chosen)), key=lambda c: chosen[c]) in STAGED_CONFIGS
-    kname = ("k_sweep_win (fused pair sweep, windows of strips)" if f32
-             else "k_sweep_stg (fused pair sweep, chunk-staged)" if staged
-             else "k_sweep (fused pair sweep, buffered)")
+    kname = "k_sweep_win (fused pair sweep, windows of strips)"
     iss = ISSUE_PER_LAUNCH.get((args.workload, args.scale, args.precision))
     issue = ({"slots_used": iss[0], "lanes_per_instruction": iss[1],
-              "source": "ncu capture of the benched kernel (profiles/)"} if iss and staged else None)
+              "source": "ncu capture of the benched kernel (profiles/)"} if iss else None)
     roof = {"kernel": kname, "bound": "fp32" if f32 else "fp64", "achieved": achieved_tflops,
             "peak": peak.value, "unit": "TFLOP/s", "frac": achieved_tflops / peak.value,
             "peak_source": ("measured FP32 FMA issue rate (gc_measure_fp32_peak)" if f32

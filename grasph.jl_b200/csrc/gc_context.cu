@@ -107,17 +107,18 @@ struct DSlot {
     double* f[2][NF] = {};
     int32_t* id[2] = {};
     int cur = 0;
-    double *q0v = nullptr, *q0rho = nullptr, *aux = nullptr;
+    double *q0v = nullptr, *q0rho = nullptr;
     double *accv = nullptr, *accrho = nullptr;  // RK4 accumulators (allocated on first use)
     int32_t* inst_of = nullptr;
     SysInst* d_inst = nullptr;
     std::vector<SysInst> h_inst;
     double *d_mass = nullptr, *d_c = nullptr;
-    float *d_massf = nullptr, *d_cf = nullptr;
-    float* fpk = nullptr;      // FP32 pack for the FP32-compensated sweep
+    float* d_cf = nullptr;
+    float* fpk = nullptr;      // sweep records (ensure_fpk)
     int64_t cap_fpk = 0;
-    int64_t xpk_epoch = -1;    // pack_epoch the FP64 position copy was made in
-    bool xpk_static = false;   // position copy of a system that does not move is current
+    int64_t xpk_epoch = -1;    // pack_epoch the position records were made in
+    bool xpk_static = false;   // position records of a system that does not move are current
+    bool xpk_fp32 = false;     // their precision
     bool written = false;      // some functor writes this system
     bool moving = true;        // sorted and integrated every step
     bool vsrc = false;         // source of a virtual system: never integrated
@@ -136,6 +137,7 @@ struct DSlot {
     int64_t upd_fused_epoch = -1;
     int64_t pack_done_epoch = -1;
     int pack_done_stage = 0, pack_done_mode = -1, pack_done_ns = -1;
+    bool pack_done_fp32 = false;
     // warp groups of this system's particles (one grid's columns)
     int2* groups = nullptr;
     int64_t* d_ngroups = nullptr;
@@ -160,7 +162,7 @@ struct DGhost {
     double* x[2] = {};
     int32_t *io[2] = {}, *ib[2] = {}, *ginst[2] = {};
     int cur = 0;
-    double *normals = nullptr, *v = nullptr, *rho = nullptr, *p = nullptr, *stress = nullptr, *aux = nullptr;
+    double *normals = nullptr, *v = nullptr, *rho = nullptr, *p = nullptr, *stress = nullptr;
     int32_t *flags = nullptr, *pos = nullptr;
     int64_t* d_count = nullptr;
     GhostInst* d_gh = nullptr;
@@ -702,7 +704,6 @@ int finalize(gc_ctx* ctx) {
         }
         TRY(dalloc(ctx, &D.q0v, (size_t)D.nd * D.N));
         TRY(dalloc(ctx, &D.q0rho, (size_t)D.N));
-        TRY(dalloc(ctx, &D.aux, (size_t)D.N));
         TRY(dalloc(ctx, &D.inst_of, (size_t)D.N));
         TRY(dalloc(ctx, &D.groups, (size_t)D.N + 1));
         TRY(dalloc(ctx, &D.d_ngroups, 1));
@@ -720,14 +721,11 @@ int finalize(gc_ctx* ctx) {
         }
         CU(cudaMemcpyAsync(D.d_mass, m.data(), ninst * 8, cudaMemcpyHostToDevice, ctx->stream));
         CU(cudaMemcpyAsync(D.d_c, c.data(), ninst * 8, cudaMemcpyHostToDevice, ctx->stream));
-        std::vector<float> mf(ninst), cf(ninst);
+        std::vector<float> cf(ninst);
         for (int k = 0; k < ninst; ++k) {
-            mf[k] = (float)m[k];
             cf[k] = (float)c[k];
         }
-        TRY(dalloc(ctx, &D.d_massf, (size_t)ninst));
         TRY(dalloc(ctx, &D.d_cf, (size_t)ninst));
-        CU(cudaMemcpyAsync(D.d_massf, mf.data(), ninst * 4, cudaMemcpyHostToDevice, ctx->stream));
         CU(cudaMemcpyAsync(D.d_cf, cf.data(), ninst * 4, cudaMemcpyHostToDevice, ctx->stream));
         // ids default to 1..n per instance
         std::vector<int32_t> ids(D.N);
@@ -821,7 +819,6 @@ int finalize(gc_ctx* ctx) {
         TRY(dalloc(ctx, &G.normals, (size_t)G.nd * G.CAP));
         TRY(dalloc(ctx, &G.v, (size_t)G.nd * G.CAP));
         TRY(dalloc(ctx, &G.rho, (size_t)G.CAP));
-        TRY(dalloc(ctx, &G.aux, (size_t)G.CAP));
         if (G.ex_p) TRY(dalloc(ctx, &G.p, (size_t)G.CAP));
         if (G.ex_stress) TRY(dalloc(ctx, &G.stress, (size_t)G.ns * G.CAP));
         TRY(dalloc(ctx, &G.flags, (size_t)G.CAP));
@@ -931,7 +928,6 @@ int finalize(gc_ctx* ctx) {
                     G.bmass = I.sys[hh.idx].mass;
                     G.bc = I.sys[hh.idx].c;
                 }
-                G.f_bmass = (float)G.bmass;
                 G.f_bc = (float)G.bc;
             }
         }
@@ -943,7 +939,6 @@ int finalize(gc_ctx* ctx) {
                 const HSys& sa = ctx->inst[k].sys[ctx->inst[k].inters[i].a];
                 gb[k].bmass = sa.mass;
                 gb[k].bc = sa.c;
-                gb[k].f_bmass = (float)sa.mass;
                 gb[k].f_bc = (float)sa.c;
                 gb[k].side_b = 1;
             }
@@ -1601,16 +1596,16 @@ int ghost_copy(gc_ctx* ctx, DGhost& G, int stage) {
     return check_launch(ctx, "ghost copy");
 }
 
-// FP32-sweep buffers of a slot or ghost set: the planar FP32 positions
-// (padded to whole quads), N position-only records (pos_quads each), then N
-// sweep records (rec_quads of the mode each).
+// Sweep buffers of a slot or ghost set: the planar FP32 positions (padded to
+// whole quads), N position-only records (pos_quads each), then N sweep
+// records (rec_quads of the mode and precision each).
 float* hpos_of(float* fpk) { return fpk; }
 float4* pos_of(float* fpk, int64_t N, int nd) { return reinterpret_cast<float4*>(fpk) + (N * nd + 3) / 4; }
-float4* rec_of(float* fpk, int64_t N, int nd) { return pos_of(fpk, N, nd) + N * pos_quads(nd); }
+float4* rec_of(float* fpk, int64_t N, int nd) { return pos_of(fpk, N, nd) + N * pos_quads(nd, true); }
 
 template <class T>
-int ensure_fpk(gc_ctx* ctx, T& X, int64_t N, int nd, int mode) {
-    int64_t need = 4 * ((N * nd + 3) / 4 + N * (pos_quads(nd) + rec_quads(nd, mode)));
+int ensure_fpk(gc_ctx* ctx, T& X, int64_t N, int nd, int mode, bool fp32) {
+    int64_t need = 4 * ((N * nd + 3) / 4 + N * (pos_quads(nd, fp32) + rec_quads(nd, mode, fp32)));
     if (need > X.cap_fpk) {
         CU(cudaStreamSynchronize(ctx->stream));
         dfree(ctx, X.fpk, X.cap_fpk);
@@ -1662,9 +1657,6 @@ int xsph_ghost_side(gc_ctx* ctx, const ForceArgs& A, int id, int stage) {
     R.ax = G.x[G.cur];
     R.av = G.v;
     R.arho = G.rho;
-    R.aaux = nullptr;
-    R.astress = nullptr;
-    R.a_p = nullptr;
     R.advdt = G.gadj;
     R.adrhodt = nullptr;
     R.asr = nullptr;
@@ -1672,7 +1664,6 @@ int xsph_ghost_side(gc_ctx* ctx, const ForceArgs& A, int id, int stage) {
     R.a_c = G.d_c;
     R.a_mass = G.d_mass;
     R.a_cf = nullptr;
-    R.a_massf = nullptr;
     R.arec = nullptr;
     R.prec = GC_PRECISION_FP64;
     R.nref = 1;
@@ -1722,8 +1713,6 @@ int interp_sweeps(gc_ctx* ctx, int a, const std::vector<int>& ids, int stage) {
         R.ax = B.F(F_X);
         R.av = B.F(F_V);
         R.arho = B.F(F_RHO);
-        R.astress = B.F(F_STRESS);
-        R.a_p = B.F(F_P);
         R.advdt = B.F(F_V);        // accumulation targets: v, rho, stress, w_sum
         R.adrhodt = B.F(F_RHO);
         R.asr = B.F(F_STRESS);
@@ -1731,7 +1720,6 @@ int interp_sweeps(gc_ctx* ctx, int a, const std::vector<int>& ids, int stage) {
         R.a_c = B.d_c;
         R.a_mass = B.d_mass;
         R.a_cf = B.d_cf;
-        R.a_massf = B.d_massf;
         R.prec = GC_PRECISION_FP64;
         R.err = ctx->d_err;
         R.groups = B.groups;
@@ -1756,15 +1744,13 @@ int interp_sweeps(gc_ctx* ctx, int a, const std::vector<int>& ids, int stage) {
             r.bx = Gh.x[Gh.cur];
             r.bv = Gh.v;
             r.brho = Gh.rho;
-            r.bp = Gh.p;
             r.bstress = Gh.stress;
             r.bN = Gh.CAP;
         } else {
             r.bx = S.F(F_X);
             r.bv = S.F(F_V);
             r.brho = S.F(F_RHO);
-            r.bp = S.F(F_P);
-            r.bstress = S.F(F_STRESS);
+                r.bstress = S.F(F_STRESS);
             r.bN = S.N;
         }
         int st = launch_force_f64(R, false, ctx->stream);
@@ -1781,6 +1767,7 @@ int interp_sweeps(gc_ctx* ctx, int a, const std::vector<int>& ids, int stage) {
 struct PackPlan {
     int pk0 = GC_PFN_NONE, pfn = GC_PFN_NONE, mode = 0, pk_ns = 0;
     bool interp = false, xsph = false, fp32 = false;
+    bool records = false;  // the functor sweeps records
 };
 
 PackPlan pack_plan(gc_ctx* ctx, int a, const std::vector<int>& ids, int stage, bool count_only) {
@@ -1796,6 +1783,7 @@ PackPlan pack_plan(gc_ctx* ctx, int a, const std::vector<int>& ids, int stage, b
     for (int id : ids)
         if (pl.pfn == GC_PFN_FLUID && ctx->inters[id].h_gi.size() && ctx->inst[0].inters[id].pp[stage - 1][3] == 1.0)
             pl.fp32 = false;  // the S = 1 (multiphase) pressure form stays in FP64
+    pl.records = pl.pfn != GC_PFN_COUNT && !pl.xsph && !pl.interp && !count_only;
     pl.pk_ns = pl.pfn == GC_PFN_CAUCHY_FLUID ? S.ns : 0;
     return pl;
 }
@@ -1830,37 +1818,37 @@ int sweep_group(gc_ctx* ctx, int a, const std::vector<int>& ids, int stage, bool
     if (pl.interp) return interp_sweeps(ctx, a, ids, stage);
     const int pk0 = pl.pk0, pfn = pl.pfn, mode = pl.mode, pk_ns = pl.pk_ns;
     const bool xsph = pl.xsph, fp32 = pl.fp32;
-    if (pfn != GC_PFN_COUNT && !xsph) {
-        if (fp32) {
-            TRY(ensure_fpk(ctx, S, S.N, S.nd, mode));
-            // the fused half step of this step may have packed these records
-            const bool done = S.pack_done_epoch == ctx->pack_epoch && S.pack_done_stage == stage &&
-                              S.pack_done_mode == mode && S.pack_done_ns == pk_ns;
-            if (!done) {
-                launch_pack32(mode, S.N, nullptr, S.nd, pk_ns, S.F(F_X), S.F(F_V), S.F(F_RHO), S.F(F_P),
-                              S.F(F_STRESS), S.inst_of, S.d_mass, hpos_of(S.fpk), nullptr, rec_of(S.fpk, S.N, S.nd),
-                              ctx->stream);
-            }
-        } else {
-            launch_aux(mode, S.N, nullptr, S.F(F_RHO), S.F(F_P), S.inst_of, S.d_mass, S.aux, ctx->stream);
-        }
+    const bool records = pl.records;
+    if (records) {
+        TRY(ensure_fpk(ctx, S, S.N, S.nd, mode, fp32));
+        // the fused half step of this step may have packed these records
+        const bool done = S.pack_done_epoch == ctx->pack_epoch && S.pack_done_stage == stage &&
+                          S.pack_done_mode == mode && S.pack_done_ns == pk_ns && S.pack_done_fp32 == fp32;
+        if (!done)
+            launch_pack(fp32, mode, S.N, nullptr, S.nd, pk_ns, S.F(F_X), S.F(F_V), S.F(F_RHO), S.F(F_P),
+                        S.F(F_STRESS), S.inst_of, S.d_mass, hpos_of(S.fpk), nullptr, rec_of(S.fpk, S.N, S.nd),
+                        ctx->stream);
     }
     ForceArgs A{};
     A.nd = S.nd;
     A.ns = S.ns;
     A.pfn = pfn;
-    if (pfn == GC_PFN_FLUID)  // a two-sided or fluid-solid reference needs the general fluid code
-        for (int id : ids)
+    if (pfn == GC_PFN_FLUID)
+        // a two-sided or fluid-solid reference, the S = 1 pressure form and the
+        // density diffusion need the general fluid code
+        for (int id : ids) {
             if (pk0 == GC_PFN_FLUID_SOLID || ctx->inters[id].two_fluid) A.pfn = PFN_FLUID2;
+            for (auto& I : ctx->inst) {
+                const auto& prm = I.inters[id].pp[stage - 1];
+                if ((int)prm[3] == 1 || !std::isnan(prm[4])) A.pfn = PFN_FLUID2;
+            }
+        }
     A.kk = ctx->inters[ids[0]].kk;
     A.aN = S.N;
     A.a_inst_of = S.inst_of;
     A.ax = S.F(F_X);
     A.av = S.F(F_V);
     A.arho = S.F(F_RHO);
-    A.aaux = S.aux;
-    A.astress = S.F(F_STRESS);
-    A.a_p = S.F(F_P);
     A.advdt = xsph ? S.F(F_VADJ) : S.F(F_DVDT);
     A.adrhodt = S.F(F_DRHODT);
     A.asr = S.F(F_SR);
@@ -1868,8 +1856,7 @@ int sweep_group(gc_ctx* ctx, int a, const std::vector<int>& ids, int stage, bool
     A.a_c = S.d_c;
     A.a_mass = S.d_mass;
     A.a_cf = S.d_cf;
-    A.a_massf = S.d_massf;
-    A.arec = fp32 ? rec_of(S.fpk, S.N, S.nd) : nullptr;
+    A.arec = records ? rec_of(S.fpk, S.N, S.nd) : nullptr;
     A.prec = fp32 ? GC_PRECISION_FP32_COMPENSATED : GC_PRECISION_FP64;
     A.err = ctx->d_err;
     A.num_sms = ctx->num_sms;
@@ -1920,21 +1907,17 @@ int sweep_group(gc_ctx* ctx, int a, const std::vector<int>& ids, int stage, bool
             r.bx = G.x[G.cur];
             r.bv = G.v;
             r.brho = G.rho;
-            r.bp = G.p;
             r.bstress = G.stress;
             r.bN = G.CAP;
-            if (pfn != GC_PFN_COUNT && !xsph && !fp32)
-                launch_aux(mode, G.CAP, G.d_count, G.rho, G.p, G.ginst[G.cur], G.d_mass, G.aux, ctx->stream);
-            r.baux = G.aux;
             r.brec = nullptr;
-            if (fp32) {
-                TRY(ensure_fpk(ctx, G, G.CAP, G.nd, mode));
-                launch_pack32(mode, G.CAP, G.d_count, G.nd, pk_ns, G.x[G.cur], G.v, G.rho, G.p, G.stress,
-                              G.ginst[G.cur], G.d_mass, hpos_of(G.fpk), nullptr, rec_of(G.fpk, G.CAP, G.nd),
-                              ctx->stream);
+            if (records) {
+                TRY(ensure_fpk(ctx, G, G.CAP, G.nd, mode, fp32));
+                launch_pack(fp32, mode, G.CAP, G.d_count, G.nd, pk_ns, G.x[G.cur], G.v, G.rho, G.p, G.stress,
+                            G.ginst[G.cur], G.d_mass, hpos_of(G.fpk), nullptr, rec_of(G.fpk, G.CAP, G.nd),
+                            ctx->stream);
                 r.bh = hpos_of(G.fpk);
                 r.brec = rec_of(G.fpk, G.CAP, G.nd);
-                r.brq = rec_quads(G.nd, mode);
+                r.brq = rec_quads(G.nd, mode, fp32);
             }
         } else {
             DSlot& B = ctx->slots[D.bslot];
@@ -1942,44 +1925,35 @@ int sweep_group(gc_ctx* ctx, int a, const std::vector<int>& ids, int stage, bool
             r.bx = B.F(F_X);
             r.bv = B.F(F_V);
             r.brho = B.F(F_RHO);
-            r.bp = B.F(F_P);
             r.bstress = B.F(F_STRESS);
             r.bN = B.N;
             r.brec = nullptr;
-            if (D.btype == BT_SELF) {
-                r.baux = S.aux;
-                if (fp32) {
-                    r.bh = hpos_of(S.fpk);
-                    r.brec = rec_of(S.fpk, S.N, S.nd);
-                    r.brq = rec_quads(S.nd, mode);
-                }
-            } else if ((D.btype == BT_SYSTEM || D.btype == BT_VIRTUAL) && pfn != GC_PFN_COUNT && !xsph && !fp32 &&
-                       pk0 != GC_PFN_FLUID_SOLID) {
-                launch_aux(mode, B.N, nullptr, B.F(F_RHO), B.F(F_P), B.inst_of, B.d_mass, B.aux, ctx->stream);
-                r.baux = B.aux;
-            } else {
-                r.baux = B.aux;
-            }
-            if (fp32 && D.btype != BT_SELF) {
+            if (records && D.btype == BT_SELF) {
+                r.bh = hpos_of(S.fpk);
+                r.brec = rec_of(S.fpk, S.N, S.nd);
+                r.brq = rec_quads(S.nd, mode, fp32);
+            } else if (records) {
                 // dynamic walls lend only their positions; other systems their records
                 const bool rec = D.btype == BT_SYSTEM || D.btype == BT_STATIC || D.btype == BT_VIRTUAL;
-                TRY(ensure_fpk(ctx, B, B.N, B.nd, mode));
+                TRY(ensure_fpk(ctx, B, B.N, B.nd, mode, fp32));
                 // positions: once per step, once for good for a system that does not move
-                const bool pos = !rec && (B.xmoves() ? B.xpk_epoch != ctx->pack_epoch : !B.xpk_static);
-                launch_pack32(mode, B.N, nullptr, B.nd, pk_ns, B.F(F_X), B.F(F_V), B.F(F_RHO), B.F(F_P),
-                              B.kind >= GC_SYS_STRESS ? B.F(F_STRESS) : nullptr, B.inst_of, B.d_mass,
-                              hpos_of(B.fpk), pos ? pos_of(B.fpk, B.N, B.nd) : nullptr,
-                              rec ? rec_of(B.fpk, B.N, B.nd) : nullptr, ctx->stream);
+                const bool pos = !rec && (B.xpk_fp32 != fp32 ||
+                                          (B.xmoves() ? B.xpk_epoch != ctx->pack_epoch : !B.xpk_static));
+                launch_pack(fp32, mode, B.N, nullptr, B.nd, pk_ns, B.F(F_X), B.F(F_V), B.F(F_RHO), B.F(F_P),
+                            B.kind >= GC_SYS_STRESS ? B.F(F_STRESS) : nullptr, B.inst_of, B.d_mass, hpos_of(B.fpk),
+                            pos ? pos_of(B.fpk, B.N, B.nd) : nullptr, rec ? rec_of(B.fpk, B.N, B.nd) : nullptr,
+                            ctx->stream);
                 r.bh = hpos_of(B.fpk);
                 if (rec) {
                     r.brec = rec_of(B.fpk, B.N, B.nd);
-                    r.brq = rec_quads(B.nd, mode);
+                    r.brq = rec_quads(B.nd, mode, fp32);
                     B.pack_done_epoch = -1;  // packed in this sweep's mode: B's own sweep packs again
                 } else {
                     B.xpk_epoch = ctx->pack_epoch;
+                    B.xpk_fp32 = fp32;
                     if (!B.xmoves()) B.xpk_static = true;
                     r.brec = pos_of(B.fpk, B.N, B.nd);
-                    r.brq = pos_quads(B.nd);
+                    r.brq = pos_quads(B.nd, fp32);
                 }
             }
         }
@@ -2028,9 +2002,6 @@ int sweep_group(gc_ctx* ctx, int a, const std::vector<int>& ids, int stage, bool
         R.ax = B.F(F_X);
         R.av = B.F(F_V);
         R.arho = B.F(F_RHO);
-        R.aaux = B.aux;
-        R.astress = B.F(F_STRESS);
-        R.a_p = B.F(F_P);
         R.advdt = xsph ? B.F(F_VADJ) : B.F(F_DVDT);
         R.adrhodt = B.F(F_DRHODT);
         R.asr = B.F(F_SR);
@@ -2038,8 +2009,7 @@ int sweep_group(gc_ctx* ctx, int a, const std::vector<int>& ids, int stage, bool
         R.a_c = B.d_c;
         R.a_mass = B.d_mass;
         R.a_cf = B.d_cf;
-        R.a_massf = B.d_massf;
-        R.arec = fp32 ? rec_of(B.fpk, B.N, B.nd) : nullptr;
+        R.arec = records ? rec_of(B.fpk, B.N, B.nd) : nullptr;
         R.nref = 1;
         InterRef& r = R.ref[0];
         r.btype = BT_SYSTEM;
@@ -2052,13 +2022,11 @@ int sweep_group(gc_ctx* ctx, int a, const std::vector<int>& ids, int stage, bool
         r.bx = S.F(F_X);
         r.bv = S.F(F_V);
         r.brho = S.F(F_RHO);
-        r.bp = S.F(F_P);
         r.bstress = S.F(F_STRESS);
-        r.baux = S.aux;
         r.bN = S.N;
-        r.bh = fp32 ? hpos_of(S.fpk) : nullptr;
-        r.brec = fp32 ? rec_of(S.fpk, S.N, S.nd) : nullptr;
-        r.brq = rec_quads(S.nd, mode);
+        r.bh = records ? hpos_of(S.fpk) : nullptr;
+        r.brec = records ? rec_of(S.fpk, S.N, S.nd) : nullptr;
+        r.brq = rec_quads(S.nd, mode, fp32);
         st = launch_force_f64(R, false, ctx->stream);
         if (st) return seterr(ctx, st, "two-sided functor not implemented on the device");
         TRY(check_launch(ctx, "sweep (system_b side)"));
@@ -2193,8 +2161,8 @@ int xsph_pass(gc_ctx* ctx) {
 // The LeapFrog half step of slot `a` fused with the stage-1 work that
 // follows it for the same particles: its stage-1 updater when that is one
 // light elementwise kind (moved here from _sweep_all_stages!, :401-419;
-// nothing between the two reads or writes what it touches) and, for an
-// FP32-compensated first sweep after it, that sweep's records
+// nothing between the two reads or writes what it touches) and the records
+// of the first sweep after it
 // (sweep_group then finds them packed).
 int halfstep_stage1(gc_ctx* ctx, int a) {
     DSlot& S = ctx->slots[a];
@@ -2209,14 +2177,16 @@ int halfstep_stage1(gc_ctx* ctx, int a) {
         const auto groups = ctx->nstages >= 1 ? stage_groups(ctx, a, 1) : std::vector<std::vector<int>>{};
         if (!groups.empty()) {
             const PackPlan pl = pack_plan(ctx, a, groups[0], 1, false);
-            if (pl.fp32 && !pl.interp && !pl.xsph && pl.pfn != GC_PFN_COUNT) {
-                TRY(ensure_fpk(ctx, S, S.N, S.nd, pl.mode));
-                pk = PackArgs{pl.mode, S.nd, pl.pk_ns, S.N, S.F(F_X), S.F(F_V), S.F(F_RHO), S.F(F_P), S.F(F_STRESS),
-                              S.inst_of, S.d_mass, hpos_of(S.fpk), nullptr, rec_of(S.fpk, S.N, S.nd)};
+            if (pl.records) {
+                TRY(ensure_fpk(ctx, S, S.N, S.nd, pl.mode, pl.fp32));
+                pk = PackArgs{pl.fp32, pl.mode, S.nd, pl.pk_ns, S.N, S.F(F_X), S.F(F_V), S.F(F_RHO), S.F(F_P),
+                              S.F(F_STRESS), S.inst_of, S.d_mass, hpos_of(S.fpk), nullptr,
+                              rec_of(S.fpk, S.N, S.nd)};
                 S.pack_done_epoch = ctx->pack_epoch;
                 S.pack_done_stage = 1;
                 S.pack_done_mode = pl.mode;
                 S.pack_done_ns = pl.pk_ns;
+                S.pack_done_fp32 = pl.fp32;
             }
         }
     }
@@ -2759,7 +2729,6 @@ int gc_ctx_destroy(gc_ctx* ctx) {
         dev_free(ctx, S.q0rho);
         dev_free(ctx, S.accv);
         dev_free(ctx, S.accrho);
-        dev_free(ctx, S.aux);
         dev_free(ctx, S.inst_of);
         dev_free(ctx, S.groups);
         dev_free(ctx, S.d_ngroups);
@@ -2768,7 +2737,6 @@ int gc_ctx_destroy(gc_ctx* ctx) {
         dev_free(ctx, S.d_inst);
         dev_free(ctx, S.d_mass);
         dev_free(ctx, S.d_c);
-        dev_free(ctx, S.d_massf);
         dev_free(ctx, S.d_cf);
         dev_free(ctx, S.fpk);
         for (auto& ch : S.d_upd)
@@ -2786,7 +2754,6 @@ int gc_ctx_destroy(gc_ctx* ctx) {
         dev_free(ctx, G.rho);
         dev_free(ctx, G.p);
         dev_free(ctx, G.stress);
-        dev_free(ctx, G.aux);
         dev_free(ctx, G.flags);
         dev_free(ctx, G.pos);
         dev_free(ctx, G.d_count);
@@ -4036,6 +4003,10 @@ int64_t ctx_moving_particles(gc_ctx* c, int inst) {
 int64_t ctx_estimate_bytes(gc_ctx* m, int inst) {
     const HInst& I = m->inst[inst];
     int64_t b = 0;
+    auto record_bytes = [](int nd, int ns) {  // a particle's sweep buffers (ensure_fpk), in the wider precision
+        const int mode = ns ? AUX_INV_RHO2 : AUX_P_OVER_RHO2;
+        return 4 * nd + 16 * (pos_quads(nd, false) + rec_quads(nd, mode, false));
+    };
     for (auto& s : I.sys) {
         int comps = 0;
         for (int f = 0; f < GC_NFIELDS; ++f) {
@@ -4043,12 +4014,12 @@ int64_t ctx_estimate_bytes(gc_ctx* m, int inst) {
             const int c = sys_comps(s, f);
             if (c > 0) comps += c;
         }
-        b += s.n * (comps * 8 * 3 + (s.nd + 2) * 8 + 4 * 4 + 8 + 4 * (s.nd + 3 + s.ns) + 8 + 4 * 4);
+        b += s.n * (comps * 8 * 3 + (s.nd + 2) * 8 + 4 * 4 + record_bytes(s.nd, s.ns) + 8 + 4 * 4);
     }
     for (auto& g : I.ghosts) {
         const HSys& src = I.sys[g.src];
         const int64_t cap = src.n * g.nplanes;
-        b += cap * (src.nd * 8 * 4 + 4 * 8 + 8 * 3 + src.ns * 8 + 4 * (src.nd + 3 + src.ns));
+        b += cap * (src.nd * 8 * 4 + 4 * 8 + 8 * 3 + src.ns * 8 + record_bytes(src.nd, src.ns));
     }
     // grid cells from the staged positions' bounding box
     double lo[3] = {1e300, 1e300, 1e300}, hi[3] = {-1e300, -1e300, -1e300};

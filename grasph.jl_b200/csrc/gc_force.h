@@ -12,24 +12,21 @@ constexpr int FORCE_TPB = 128;  // threads per block of the sweep
 constexpr int WIN_TPB = 64;     // threads per block of the FP32-compensated sweep
 constexpr int FORCE_BUF = 64;   // staged-neighbour column of the counting sweep (shared memory)
 
-// Launch configurations of the sweep: (min resident blocks, staged
-// neighbours per thread, pair-loop unroll, chunk staging) of the FP64 sweep,
-// then the FP32-compensated one's resident blocks and chunk.  Chosen per
-// (system, stage) by the tuner in gc_context.cu.
-struct ForceCfg {
-    int minb, buf, unroll;
-    int stg;         // > 0: k_sweep_stg with chunks of stg candidates (policies that stage copies; k_sweep otherwise)
-    int wminb, wch;  // k_sweep_win: resident blocks, candidates per chunk
+// Launch configurations of the window sweep: resident blocks per SM and
+// candidates per chunk, chosen per (system, stage) by the tuner in
+// gc_context.cu.  Every one gives the same bits.
+struct WinCfg {
+    int minb, chunk;
 };
 constexpr int NUM_FORCE_CFG = GC_NUM_SWEEP_CONFIGS;
-constexpr ForceCfg FORCE_CFGS[NUM_FORCE_CFG] = {
-    {4, 64, 1, 0, 8, 192}, {6, 64, 1, 0, 7, 224}, {5, 64, 1, 96, 10, 160}, {6, 64, 1, 96, 12, 128}};
+constexpr WinCfg WIN_CFGS32[NUM_FORCE_CFG] = {{8, 192}, {7, 192}, {6, 224}, {10, 160}};
+constexpr WinCfg WIN_CFGS64[NUM_FORCE_CFG] = {{6, 192}, {5, 192}, {7, 160}, {8, 128}};
 constexpr int MAX_REFS = 8;     // interactions fused into one launch
 
 // system_b kinds as seen by a functor (src/PairwiseFunctors.jl dispatch)
 enum { BT_SELF = 0, BT_DYNAMIC = 1, BT_STATIC = 2, BT_GHOST = 3, BT_SYSTEM = 4 };
 
-// per-particle divisor caches (one per slot, refreshed before each sweep)
+// what a functor's records carry (refreshed before each sweep)
 enum { AUX_P_OVER_RHO2 = 0, AUX_INV_RHO2 = 1, AUX_MASS_OVER_RHO = 2 };
 
 // Device-side functor code: FluidPfn with its two-sided (multiphase),
@@ -48,8 +45,8 @@ struct InterRef {
     const PfnInst* pi;    // per instance, this stage
     const int32_t* cs;    // packed CSR over system_b (global b indices)
     int64_t cs_cells;     // cells of cs that are valid (an instance beyond them is skipped)
-    const double *bx, *bv, *brho, *bp, *bstress, *baux;
-    const float4* brec;   // FP32 records of system_b (position-only ones of a dynamic boundary), or nullptr
+    const double *bx, *bv, *brho, *bstress;
+    const float4* brec;   // sweep records of system_b (position-only ones of a dynamic boundary), or nullptr
     int brq;              // their stride in 16-byte quads
     const float* bh;      // FP32 positions, planar (stride bN), or nullptr
     int64_t bN;           // planar stride of system_b's arrays
@@ -60,19 +57,18 @@ struct ForceArgs {
     int nd, ns, pfn, kk;
     int64_t aN;
     const int32_t* a_inst_of;
-    const double *ax, *av, *arho, *aaux, *astress, *a_p;
+    const double *ax, *av, *arho;
     double *advdt, *adrhodt, *asr, *avort;
     const double* a_c;     // per-instance sound speed
     const double* a_mass;  // per-instance particle mass
-    const float* a_cf;     // FP32 copies of the two above
-    const float* a_massf;
-    const float4* arec;    // FP32 records of system_a (FP32-compensated precision)
+    const float* a_cf;     // FP32 copy of the sound speed
+    const float4* arec;    // sweep records of system_a
     int prec;              // GC_PRECISION_*
     int* err;
     const int2* groups;        // warp groups of system_a particles (group_of)
     const int64_t* ngroups;    // device count of groups
     int num_sms;
-    int cfg;                   // index into FORCE_CFGS
+    int cfg;                   // index into WIN_CFGS32 / WIN_CFGS64
     int imask, iwsum;          // InterpolateFieldFn: fields (1<<GC_FIELD_*), accumulate w_sum into avort
     int nref;
     InterRef ref[MAX_REFS];
@@ -93,18 +89,16 @@ void launch_groups_count(const GridInst* gi, int ninst, int nd, const int32_t* c
                          int64_t cells_cap, int32_t* cnt, cudaStream_t s);
 void launch_groups_fill(const GridInst* gi, int ninst, int nd, const int32_t* cs, const int32_t* off,
                         int64_t ncols_cap, int64_t cells_cap, int2* groups, int64_t* ngroups, cudaStream_t s);
-void launch_aux(int mode, int64_t N, const int64_t* count, const double* rho, const double* p,
-                const int32_t* inst_of, const double* mass, double* aux, cudaStream_t s);
-// Divisor mode of a functor's records and caches.
+// Mode of a functor's records.
 __host__ __device__ constexpr int aux_mode(int pfn) {
     return pfn == GC_PFN_FLUID || pfn == PFN_FLUID2 ? AUX_P_OVER_RHO2
            : pfn == GC_PFN_CAUCHY_FLUID             ? AUX_INV_RHO2
                                                     : AUX_MASS_OVER_RHO;
 }
-// Per-particle records of the FP32-compensated sweep, in 16-byte quads, so a
-// neighbour costs two or three loads.  A position is an FP32 pair x = h + l
-// (h the nearest float, l the rest), whose differences are as good as the
-// FP64 difference rounded to FP32.  σ' is the stress over ρ².
+// Per-particle records of the window sweep, in 16-byte quads, so a neighbour
+// costs a few wide loads.  σ' is the stress over ρ².  FP32-compensated: a
+// position is an FP32 pair x = h + l (h the nearest float, l the rest), whose
+// differences are as good as the FP64 difference rounded to FP32.
 //   2-D: [hx hy lx ly] then
 //     fluid       [vx vy -p/ρ² 1/ρ] [ρ 0 0 0]
 //     strain rate [vx vy m/ρ 0]
@@ -113,17 +107,21 @@ __host__ __device__ constexpr int aux_mode(int pfn) {
 //     fluid       -p/ρ², 1/ρ, ρ
 //     strain rate m/ρ, 0, 0
 //     Cauchy      1/ρ, ρ, σ'xx, then [σ'yy σ'zz σ'xy σ'xz] [σ'yz 0 0 0]
+// FP64, two doubles a quad: x.. v.. then
+//     fluid -p/ρ², 1/ρ, ρ, p; strain rate m/ρ, 0; Cauchy 1/ρ, ρ, σ'.. (0)
+//   (2-D σ': xx yy xy).
 // A dynamic boundary lends only positions: its records are the position
-// quads alone (2-D the first, 3-D the first two with w = 0).
-__host__ __device__ constexpr int rec_quads(int nd, int mode) {
-    return mode == AUX_INV_RHO2 ? (nd == 2 ? 3 : 5) : mode == AUX_MASS_OVER_RHO ? (nd == 2 ? 2 : 3) : 3;
+// quads alone (FP32 3-D with w = 0, FP64 3-D [x y] [z 0]).
+__host__ __device__ constexpr int rec_quads(int nd, int mode, bool fp32) {
+    return fp32 ? (mode == AUX_INV_RHO2 ? (nd == 2 ? 3 : 5) : mode == AUX_MASS_OVER_RHO ? (nd == 2 ? 2 : 3) : 3)
+                : nd + (mode == AUX_INV_RHO2 ? (nd == 2 ? 3 : 4) : mode == AUX_MASS_OVER_RHO ? 1 : 2);
 }
-__host__ __device__ constexpr int pos_quads(int nd) { return nd == 2 ? 1 : 2; }
-// hpos: the positions' h alone, planar (the candidate test reads these).
-// Nothing is written without pos or rec, either of which may be nullptr; p
-// and stress may be nullptr (zeros).
-void launch_pack32(int mode, int64_t N, const int64_t* count, int nd, int ns, const double* x, const double* v,
-                   const double* rho, const double* p, const double* stress, const int32_t* inst_of,
-                   const double* mass, float* hpos, float4* pos, float4* rec, cudaStream_t s);
+__host__ __device__ constexpr int pos_quads(int nd, bool) { return nd == 2 ? 1 : 2; }
+// hpos: the positions rounded to FP32, planar (the candidate test reads
+// these).  Nothing is written without pos or rec, either of which may be
+// nullptr; p and stress may be nullptr (zeros).
+void launch_pack(bool fp32, int mode, int64_t N, const int64_t* count, int nd, int ns, const double* x,
+                 const double* v, const double* rho, const double* p, const double* stress, const int32_t* inst_of,
+                 const double* mass, float* hpos, float4* pos, float4* rec, cudaStream_t s);
 
 }  // namespace gc

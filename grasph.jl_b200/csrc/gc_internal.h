@@ -61,7 +61,7 @@ struct GridInst {
     double normal[MAXD], point[MAXD], beta, ljcut;
     double bmass, bc;                  // system_b mass and sound speed
     // FP32 copies for the FP32-compensated sweep
-    float f_normal[MAXD], f_beta, f_ljcut, f_bmass, f_bc;
+    float f_normal[MAXD], f_beta, f_ljcut, f_bc;
     int side_b;                        // 1 in the system_b-side copy of a two-sided interaction
 };
 // Per (interaction, stage, instance) functor parameters.

@@ -29,9 +29,10 @@ struct UpdArgs {
     double *rho, *p, *stress, *sr, *vort, *strain, *strainp, *dvdt, *drhodt;
 };
 
-// One slot's FP32 sweep records (launch_pack32's arguments; pos or rec may
-// be nullptr).
+// One slot's sweep records (launch_pack's arguments; pos or rec may be
+// nullptr).
 struct PackArgs {
+    bool fp32;
     int mode, nd, ns;
     int64_t N;
     const double *x, *v, *rho, *p, *stress;
@@ -46,7 +47,7 @@ void launch_halfstep(const StepArgs& a, cudaStream_t s);
 // the first sweeps (src/TimeIntegration.jl:158, then _sweep_all_stages!'s
 // stage-1 state updater :401-419): per particle the half step, the updater
 // u (u.kind < 0: none; an elementwise kind), then (pk.pos or pk.rec set) the
-// FP32 records of the stage's first sweep.  One pass over the state instead
+// records of the stage's first sweep.  One pass over the state instead
 // of three.
 void launch_halfstep_fused(const StepArgs& a, const UpdArgs& u, const PackArgs& pk, cudaStream_t s);
 // Whether launch_halfstep_fused takes updater kind `kind` (the light,

@@ -1,5 +1,5 @@
 // k_force_f64.cu — dispatch of the fused pair sweep, warp-group lists and
-// per-particle divisor caches.  Compiled with -fmad=false.
+// sweep records.  Compiled with -fmad=false.
 #include <cstdio>
 
 #include "gc_device.cuh"
@@ -95,44 +95,21 @@ void launch_groups_fill(const GridInst* gi, int ninst, int nd, const int32_t* cs
     g_launches.fetch_add(1, std::memory_order_relaxed);
 }
 
-// Per-particle factors the functors divide by, computed once per stage
-// with the reference's expressions so pair terms stay bit-identical.
-__global__ void k_aux(int mode, int64_t N, const int64_t* count, const double* __restrict__ rho,
-                      const double* __restrict__ p, const int32_t* __restrict__ inst_of, const double* mass,
-                      double* __restrict__ aux) {
-    pdl_enter();
-    int64_t n = count ? *count : N;
-    for (int64_t g = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; g < n; g += (int64_t)gridDim.x * blockDim.x) {
-        double r = rho[g];
-        if (mode == AUX_P_OVER_RHO2) aux[g] = p[g] / (r * r);
-        else if (mode == AUX_INV_RHO2) aux[g] = 1.0 / (r * r);
-        else aux[g] = mass[inst_of[g]] / r;
-    }
-}
-
-__global__ void k_pack32(PackArgs a, const int64_t* count) {
+__global__ void k_pack(PackArgs a, const int64_t* count) {
     pdl_enter();
     const int64_t n = count ? *count : a.N;
     for (int64_t g = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; g < n; g += (int64_t)gridDim.x * blockDim.x)
         pack_one(a, g);
 }
 
-void launch_pack32(int mode, int64_t N, const int64_t* count, int nd, int ns, const double* x, const double* v,
+void launch_pack(bool fp32, int mode, int64_t N, const int64_t* count, int nd, int ns, const double* x, const double* v,
                    const double* rho, const double* p, const double* stress, const int32_t* inst_of,
                    const double* mass, float* hpos, float4* pos, float4* rec, cudaStream_t s) {
     if (N <= 0 || (!pos && !rec)) return;
     int64_t blocks = (N + 255) / 256;
     if (blocks > 148 * 64) blocks = 148 * 64;
-    PackArgs a{mode, nd, ns, N, x, v, rho, p, stress, inst_of, mass, hpos, pos, rec};
-    k_pack32<<<(int)blocks, 256, 0, s>>>(a, count);
-    g_launches.fetch_add(1, std::memory_order_relaxed);
-}
-
-void launch_aux(int mode, int64_t N, const int64_t* count, const double* rho, const double* p,
-                const int32_t* inst_of, const double* mass, double* aux, cudaStream_t s) {
-    if (N <= 0) return;
-    int blocks = (int)((N + 255) / 256);
-    k_aux<<<blocks, 256, 0, s>>>(mode, N, count, rho, p, inst_of, mass, aux);
+    PackArgs a{fp32, mode, nd, ns, N, x, v, rho, p, stress, inst_of, mass, hpos, pos, rec};
+    k_pack<<<(int)blocks, 256, 0, s>>>(a, count);
     g_launches.fetch_add(1, std::memory_order_relaxed);
 }
 

@@ -28,13 +28,6 @@
 
 namespace gc {
 
-// psi / rho for psi == +0 (δ-SPH off): +0 for a positive density, and the
-// literal quotient otherwise.
-__device__ __forceinline__ double zero_over(double r) {
-    if (r > 0.0) return 0.0;
-    return 0.0 / r;
-}
-
 template <int ND>
 struct OwnState {
     double x[ND], v[ND];
@@ -42,62 +35,6 @@ struct OwnState {
 };
 
 // ------------------------------------------------------- pair physics
-// One accepted pair (i owned, j neighbour), returns the i-side increment.
-template <int ND, int NS, int PFN, int KK>
-struct Pair {
-    static __device__ __forceinline__ void geom(const double* dx, double rr, double H, double knorm, double* gx) {
-        double r = sqrt(rr);
-        double q = r / H;
-        double gc = kernel_dw_dq<KK>(knorm, q) / (r * H);
-#pragma unroll
-        for (int d = 0; d < ND; ++d) gx[d] = gc * dx[d];
-    }
-};
-
-template <int ND, int NS>
-__device__ __forceinline__ void cauchy_f(const double* si, const double* sj, double ci, double cj, const double* g,
-                                         double* out) {
-    if (ND == 2) {
-        constexpr int XY = NS == 3 ? 2 : 3;
-        out[0] = (si[0] * g[0] + si[XY] * g[1]) * ci + (sj[0] * g[0] + sj[XY] * g[1]) * cj;
-        out[1] = (si[XY] * g[0] + si[1] * g[1]) * ci + (sj[XY] * g[0] + sj[1] * g[1]) * cj;
-    } else {
-        out[0] = (si[0] * g[0] + si[3] * g[1] + si[4] * g[2]) * ci + (sj[0] * g[0] + sj[3] * g[1] + sj[4] * g[2]) * cj;
-        out[1] = (si[3] * g[0] + si[1] * g[1] + si[5] * g[2]) * ci + (sj[3] * g[0] + sj[1] * g[1] + sj[5] * g[2]) * cj;
-        out[2] = (si[4] * g[0] + si[5] * g[1] + si[2] * g[2]) * ci + (sj[4] * g[0] + sj[5] * g[1] + sj[2] * g[2]) * cj;
-    }
-}
-
-template <int ND, int NS>
-__device__ __forceinline__ void strain_rate_f(const double* dv, const double* g, double* sr) {
-    if (ND == 2) {
-        sr[0] = dv[0] * g[0];
-        sr[1] = dv[1] * g[1];
-        if (NS == 4) {
-            sr[2] = 0.0;
-            sr[3] = 0.5 * (dv[0] * g[1] + dv[1] * g[0]);
-        } else {
-            sr[2] = 0.5 * (dv[0] * g[1] + dv[1] * g[0]);
-        }
-    } else {
-        sr[0] = dv[0] * g[0];
-        sr[1] = dv[1] * g[1];
-        sr[2] = dv[2] * g[2];
-        sr[3] = 0.5 * (dv[0] * g[1] + dv[1] * g[0]);
-        sr[4] = 0.5 * (dv[0] * g[2] + dv[2] * g[0]);
-        sr[5] = 0.5 * (dv[1] * g[2] + dv[2] * g[1]);
-    }
-}
-
-template <int ND>
-__device__ __forceinline__ void vorticity_f(const double* dv, const double* g, double* w) {
-    w[0] = 0.5 * (dv[0] * g[1] - dv[1] * g[0]);
-    if (ND == 3) {
-        w[1] = 0.5 * (dv[0] * g[2] - dv[2] * g[0]);
-        w[2] = 0.5 * (dv[1] * g[2] - dv[2] * g[1]);
-    }
-}
-
 template <int ND, int NS>
 struct Acc {
     double dv[ND];
@@ -106,53 +43,23 @@ struct Acc {
     double w[ND == 2 ? 1 : 3];
 };
 
-// Neighbour j's FP64 state, read from system_b's planar arrays ...
+// Neighbour j's FP64 state, read from system_b's planar arrays.
 struct NbGlobal {
     const InterRef& r;
     int64_t j;
     __device__ __forceinline__ double x(int d) const { return r.bx[d * r.bN + j]; }
     __device__ __forceinline__ double v(int d) const { return r.bv[d * r.bN + j]; }
     __device__ __forceinline__ double rho() const { return r.brho[j]; }
-    __device__ __forceinline__ double aux() const { return r.baux[j]; }
-    __device__ __forceinline__ double p() const { return r.bp[j]; }
     __device__ __forceinline__ double stress(int q) const { return r.bstress[q * r.bN + j]; }
-};
-
-// ... or from its copy staged in shared memory by PhysF64::issue: 16-byte
-// chunks q*BT of the slot, the position's components in pairs, then
-// [v, ρ, aux, p] in pairs (the functors staged there read no stress).
-template <int ND>
-struct NbSlot {
-    static constexpr int XQ = (ND + 1) / 2;
-    const float4* slot;
-    int BT;
-    __device__ __forceinline__ double x(int d) const {
-        return reinterpret_cast<const double*>(&slot[(d >> 1) * BT])[d & 1];
-    }
-    __device__ __forceinline__ double rec(int e) const {
-        return reinterpret_cast<const double*>(&slot[(XQ + (e >> 1)) * BT])[e & 1];
-    }
-    __device__ __forceinline__ double v(int d) const { return rec(d); }
-    __device__ __forceinline__ double rho() const { return rec(ND); }
-    __device__ __forceinline__ double aux() const { return rec(ND + 1); }
-    __device__ __forceinline__ double p() const { return rec(ND + 2); }
-    __device__ __forceinline__ double stress(int) const { return 0.0; }
 };
 
 // One candidate j (source nb) of reference r for owned particle i: the
 // exact reference test r² < (2h)² (src/Interaction.jl:546-548) on the FP64
 // positions, then the functor's i-side term.  Returns 1 when accepted.
-// BTK: the system_b kind when known at compile time (-1: r.btype).
-template <int ND, int NS, int PFN, int KK, int BTK = -1, class Nb>
+template <int ND, int NS, int PFN, int KK>
 __device__ __forceinline__ int process_pair(const ForceArgs& A, const InterRef& r, const GridInst& G,
-                                            const PfnInst& P, int64_t gi, int k, const OwnState<ND>& o,
-                                            const double* osig, double da, const Nb& nb, Acc<ND, NS>& acc,
-                                            const double2* cam = nullptr) {
-    // system_a's sound speed and mass: the warp's shared copy (cam) or the
-    // per-instance arrays
-    auto sound_a = [&]() { return cam ? cam->x : A.a_c[k]; };
-    auto mass_of_a = [&]() { return cam ? cam->y : A.a_mass[k]; };
-    const int btype = BTK >= 0 ? BTK : r.btype;
+                                            const PfnInst& P, int k, const OwnState<ND>& o, const NbGlobal& nb,
+                                            Acc<ND, NS>& acc) {
     double dx[ND];
 #pragma unroll
     for (int d = 0; d < ND; ++d) dx[d] = o.x[d] - nb.x(d);
@@ -190,7 +97,7 @@ __device__ __forceinline__ int process_pair(const ForceArgs& A, const InterRef& 
         const double q = sqrt(rr) / G.H;
         const double wk = kernel_w<KK>(G.knorm, q);
         const double den = o.rho + nb.rho();
-        const double mj = btype == BT_SELF ? mass_of_a() : G.bmass;
+        const double mj = r.btype == BT_SELF ? A.a_mass[k] : G.bmass;
 #pragma unroll
         for (int d = 0; d < ND; ++d) {
             const double du = (((-P.alpha) * (o.v[d] - nb.v(d))) * wk) / den;
@@ -198,184 +105,15 @@ __device__ __forceinline__ int process_pair(const ForceArgs& A, const InterRef& 
         }
         return 1;
     }
-    double gx[ND];
-    Pair<ND, NS, PFN, KK>::geom(dx, rr, G.H, G.knorm, gx);
-    const double ca = sound_a();
-    const double mass_a = mass_of_a();
-
-    if (btype == BT_DYNAMIC) {
-        // src/PairwiseFunctors.jl:53,111,222,334
-        double t[ND];
-#pragma unroll
-        for (int d = 0; d < ND; ++d) t[d] = nb.x(d) - G.point[d];
-        double db = dotv<ND>(t, G.normal);
-        double m = -jmin(G.beta, fabs(db / da));
-        double vj[ND];
-#pragma unroll
-        for (int d = 0; d < ND; ++d) vj[d] = m * o.v[d];
-        if (fluid_pfn<PFN>() || PFN == GC_PFN_CAUCHY_FLUID) {
-            double dv[ND];
-#pragma unroll
-            for (int d = 0; d < ND; ++d) dv[d] = o.v[d] - vj[d];
-            double piv = art_visc<ND>(dx, dv, rr, P.h, o.rho, o.rho, P.alpha, P.beta, ca, ca);
-            if (fluid_pfn<PFN>()) {
-                double dh = P.S == 1 ? -(A.a_p[gi] + A.a_p[gi]) / (o.rho * o.rho) : -(o.aux + o.aux);
-                double s = mass_a * (dh - piv);
-#pragma unroll
-                for (int d = 0; d < ND; ++d) acc.dv[d] = acc.dv[d] + s * gx[d];
-            } else {
-                double hv[ND];
-                cauchy_f<ND, NS>(osig, osig, o.aux, o.aux, gx, hv);
-#pragma unroll
-                for (int d = 0; d < ND; ++d) acc.dv[d] = acc.dv[d] + mass_a * (hv[d] - piv * gx[d]);
-            }
-            double dr = dotv<ND>(dv, gx);
-            double tail;
-            if (P.has_delta) {
-                double psi = diffusion<ND>(dx, rr, o.rho, o.rho, ca, ca, P.h, P.h, gx, P.delta);
-                tail = psi / o.rho;
-            } else {
-                tail = zero_over(o.rho);
-            }
-            double cdc = (fluid_pfn<PFN>() && P.S == 1) ? o.rho / o.rho : 1.0;
-            acc.dr = acc.dr + mass_a * ((fluid_pfn<PFN>() ? dr * cdc : dr) + tail);
-        } else {  // strain rate (+ vorticity)
-            double dv[ND];
-#pragma unroll
-            for (int d = 0; d < ND; ++d) dv[d] = vj[d] - o.v[d];
-            double sr[NS > 0 ? NS : 1];
-            strain_rate_f<ND, NS>(dv, gx, sr);
-            const double f = o.aux;  // mass_a / rho_i
-#pragma unroll
-            for (int q = 0; q < NS; ++q) acc.sr[q] = acc.sr[q] + sr[q] * f;
-            if (PFN == GC_PFN_STRAIN_RATE_VORTICITY) {
-                double w[ND == 2 ? 1 : 3];
-                vorticity_f<ND>(dv, gx, w);
-#pragma unroll
-                for (int q = 0; q < (ND == 2 ? 1 : 3); ++q) acc.w[q] = acc.w[q] + w[q] * f;
-            }
-        }
-        return 1;
-    }
-
-    // neighbour state
-    double vj[ND];
-#pragma unroll
-    for (int d = 0; d < ND; ++d) vj[d] = nb.v(d);
-    const double rhoj = nb.rho();
-
-    if (btype == BT_STATIC && (fluid_pfn<PFN>() || PFN == GC_PFN_CAUCHY_FLUID)) {
-        // src/PairwiseFunctors.jl:210-219, :322-331
-        double dv[ND];
-#pragma unroll
-        for (int d = 0; d < ND; ++d) dv[d] = o.v[d] - vj[d];
-        double piv = art_visc<ND>(dx, dv, rr, P.h, o.rho, rhoj, P.alpha, P.beta, ca, ca);
-        double rf = lennard_jones<ND>(dx, rr, G.ljcut, ca);
-        double s = (-G.bmass) * piv;
-#pragma unroll
-        for (int d = 0; d < ND; ++d) acc.dv[d] = acc.dv[d] + (s * gx[d] + rf * dx[d]);
-        return 1;
-    }
-
-    if (fluid_pfn<PFN>()) {
-        double dv[ND];
-#pragma unroll
-        for (int d = 0; d < ND; ++d) dv[d] = o.v[d] - vj[d];
-        // two-sided fluid x fluid :173 uses both sound speeds, one-sided :193 its own twice
-        const bool two = PFN == PFN_FLUID2 && P.two;  // multiphase / fluid-solid variant only
-        const double cb = two ? G.bc : ca;
-        double piv = art_visc<ND>(dx, dv, rr, P.h, o.rho, rhoj, P.alpha, P.beta, ca, cb);
-        double dh;
-        if (PFN == PFN_FLUID2 && P.fs) {
-            // FluidSolidPfn :494-519: the fluid's pressure on both sides; the
-            // fluid is the neighbour on the system_b side
-            if (G.side_b) {
-                const double pf = nb.p();
-                dh = P.S == 1 ? -(pf + pf) / (o.rho * rhoj) : -(nb.aux() + pf / (o.rho * o.rho));
-            } else {
-                const double pf = A.a_p[gi];
-                dh = P.S == 1 ? -(pf + pf) / (o.rho * rhoj) : -(o.aux + pf / (rhoj * rhoj));
-            }
-        } else {
-            dh = P.S == 1 ? -(A.a_p[gi] + nb.p()) / (o.rho * rhoj) : -(o.aux + nb.aux());
-        }
-        double mj = btype == BT_SELF ? mass_a : G.bmass;
-        if (two) {
-            // dv_tmp = (dh + ast - piv)·gx, then mass_j·dv_tmp; the system_b side
-            // runs this same code with the roles swapped (every factor is
-            // symmetric or flips sign exactly with dx, dv and gx)
-            double c = dh;
-            if (P.has_eps) c = c + P.eps * (-(fabs(A.a_p[gi]) + fabs(nb.p())) / (o.rho * rhoj));
-            c = c - piv;
-#pragma unroll
-            for (int d = 0; d < ND; ++d) acc.dv[d] = acc.dv[d] + mj * (c * gx[d]);
-        } else {
-            double s = mj * (dh - piv);
-#pragma unroll
-            for (int d = 0; d < ND; ++d) acc.dv[d] = acc.dv[d] + s * gx[d];
-        }
-        double dr = dotv<ND>(dv, gx);
-        double tail;
-        if (P.has_delta) {
-            double psi = diffusion<ND>(dx, rr, o.rho, rhoj, ca, cb, P.h, P.h, gx, P.delta);
-            tail = psi / rhoj;
-        } else {
-            tail = zero_over(rhoj);
-        }
-        double cdc = P.S == 1 ? o.rho / rhoj : 1.0;
-        acc.dr = acc.dr + mj * (dr * cdc + tail);
-    } else if (PFN == GC_PFN_CAUCHY_FLUID) {
-        // self :265 / ghost one-sided :286
-        double dv[ND];
-#pragma unroll
-        for (int d = 0; d < ND; ++d) dv[d] = o.v[d] - vj[d];
-        const bool self = btype == BT_SELF;
-        double cb = self ? ca : G.bc;
-        double piv = art_visc<ND>(dx, dv, rr, P.h, o.rho, rhoj, P.alpha, P.beta, ca, cb);
-        double sj[NS > 0 ? NS : 1];
-#pragma unroll
-        for (int q = 0; q < NS; ++q) sj[q] = nb.stress(q);
-        double hv[ND];
-        cauchy_f<ND, NS>(osig, sj, o.aux, nb.aux(), gx, hv);
-        double mj = self ? mass_a : G.bmass;
-#pragma unroll
-        for (int d = 0; d < ND; ++d) acc.dv[d] = acc.dv[d] + mj * (hv[d] - piv * gx[d]);
-        double dr = dotv<ND>(dv, gx);
-        double tail;
-        if (P.has_delta) {
-            double psi = diffusion<ND>(dx, rr, o.rho, rhoj, ca, ca, P.h, P.h, gx, P.delta);
-            tail = psi / rhoj;
-        } else {
-            tail = zero_over(rhoj);
-        }
-        acc.dr = acc.dr + mj * (dr + tail);
-    } else {
-        // strain rate (+vorticity): self :20/:80, generic one-sided :37/:97
-        double dv[ND];
-#pragma unroll
-        for (int d = 0; d < ND; ++d) dv[d] = vj[d] - o.v[d];
-        double sr[NS > 0 ? NS : 1];
-        strain_rate_f<ND, NS>(dv, gx, sr);
-        const double f = nb.aux();  // mass_j / rho_j
-#pragma unroll
-        for (int q = 0; q < NS; ++q) acc.sr[q] = acc.sr[q] + sr[q] * f;
-        if (PFN == GC_PFN_STRAIN_RATE_VORTICITY) {
-            double w[ND == 2 ? 1 : 3];
-            vorticity_f<ND>(dv, gx, w);
-#pragma unroll
-            for (int q = 0; q < (ND == 2 ? 1 : 3); ++q) acc.w[q] = acc.w[q] + w[q] * f;
-        }
-    }
-    (void)gi;
-    return 1;
+    return 0;
 }
 
 // ------------------------------------------------------------ policy
+// The gather policy of the counting, interpolation and velocity-adjust functors.
 template <int ND, int NS, int PFN, int KK>
-struct PhysF64 {
+struct PhysGather {
     struct Own {
         OwnState<ND> o;
-        double sig[NS > 0 ? NS : 1];
     };
     using AccT = Acc<ND, NS>;
     static __device__ __forceinline__ void load(const ForceArgs& A, int64_t gi, Own& w) {
@@ -386,9 +124,6 @@ struct PhysF64 {
             w.o.v[d] = A.av[d * N + gi];
         }
         w.o.rho = A.arho[gi];
-        w.o.aux = A.aaux ? A.aaux[gi] : 0.0;
-#pragma unroll
-        for (int q = 0; q < NS; ++q) w.sig[q] = (PFN == GC_PFN_CAUCHY_FLUID) ? A.astress[q * N + gi] : 0.0;
     }
     static __device__ __forceinline__ const double* xpos(const Own& w) { return w.o.x; }
     static __device__ __forceinline__ void init(const ForceArgs& A, int64_t gi, AccT& acc, bool from_memory) {
@@ -409,20 +144,10 @@ struct PhysF64 {
                 for (int q = 0; q < NS; ++q) acc.sr[q] = A.asr[q * N + gi];
             }
             acc.w[0] = A.iwsum ? A.avort[gi] : 0.0;
-        } else if (PFN == GC_PFN_XSPH) {  // advdt is the v_adjustment array here
+        } else {  // XSPH (advdt is the v_adjustment array here) or counting
 #pragma unroll
             for (int d = 0; d < ND; ++d) acc.dv[d] = A.advdt[d * N + gi];
-        } else if (fluid_pfn<PFN>() || PFN == GC_PFN_CAUCHY_FLUID || PFN == GC_PFN_COUNT) {
-#pragma unroll
-            for (int d = 0; d < ND; ++d) acc.dv[d] = A.advdt[d * N + gi];
-            acc.dr = A.adrhodt[gi];
-        } else {
-#pragma unroll
-            for (int q = 0; q < NS; ++q) acc.sr[q] = A.asr[q * N + gi];
-            if (PFN == GC_PFN_STRAIN_RATE_VORTICITY) {
-#pragma unroll
-                for (int q = 0; q < (ND == 2 ? 1 : 3); ++q) acc.w[q] = A.avort[q * N + gi];
-            }
+            if (PFN == GC_PFN_COUNT) acc.dr = A.adrhodt[gi];
         }
     }
     static __device__ __forceinline__ void store(const ForceArgs& A, int64_t gi, const AccT& acc) {
@@ -438,71 +163,16 @@ struct PhysF64 {
                 for (int q = 0; q < NS; ++q) A.asr[q * N + gi] = acc.sr[q];
             }
             if (A.iwsum) A.avort[gi] = acc.w[0];
-        } else if (PFN == GC_PFN_XSPH) {
-#pragma unroll
-            for (int d = 0; d < ND; ++d) A.advdt[d * N + gi] = acc.dv[d];
-        } else if (fluid_pfn<PFN>() || PFN == GC_PFN_CAUCHY_FLUID || PFN == GC_PFN_COUNT) {
-#pragma unroll
-            for (int d = 0; d < ND; ++d) A.advdt[d * N + gi] = acc.dv[d];
-            A.adrhodt[gi] = acc.dr;
         } else {
 #pragma unroll
-            for (int q = 0; q < NS; ++q) A.asr[q * N + gi] = acc.sr[q];
-            if (PFN == GC_PFN_STRAIN_RATE_VORTICITY) {
-#pragma unroll
-                for (int q = 0; q < (ND == 2 ? 1 : 3); ++q) A.avort[q * N + gi] = acc.w[q];
-            }
+            for (int d = 0; d < ND; ++d) A.advdt[d * N + gi] = acc.dv[d];
+            if (PFN == GC_PFN_COUNT) A.adrhodt[gi] = acc.dr;
         }
-    }
-    static __device__ __forceinline__ double plane_da(const Own& w, const GridInst& G) {
-        double t[ND];
-#pragma unroll
-        for (int d = 0; d < ND; ++d) t[d] = w.o.x[d] - G.point[d];
-        return dotv<ND>(t, G.normal);
     }
     template <int P2>
     static __device__ __forceinline__ int pair(const ForceArgs& A, const InterRef& r, const GridInst& G,
-                                               const PfnInst& P, int64_t gi, int k, const Own& w, double da,
-                                               int32_t j, AccT& acc) {
-        return process_pair<ND, NS, P2, KK>(A, r, G, P, gi, k, w.o, w.sig, da, NbGlobal{r, j}, acc);
-    }
-
-    // Chunk staging (k_sweep_stg) for the fluid functors: a neighbour's FP64
-    // position, then its [v, ρ, aux, p] (NbSlot's layout), copied from the
-    // planar arrays by 8-byte asynchronous copies; a dynamic boundary's
-    // term reads only the position, and p is copied only for the functor
-    // forms that read it.  The pair terms are the same expression trees on
-    // the same values as k_sweep's, so both kernels give the same bits.
-    static constexpr int NQP = (ND + 1) / 2, NQR = 3;
-    static constexpr int NQ = fluid_pfn<PFN>() ? NQP + NQR : 0;
-    static __device__ __forceinline__ void issue(const InterRef& r, const PfnInst& P, int32_t j, float4* slot,
-                                                 int BT) {
-        auto cp = [&](int e, const double* src) {  // double e of the slot
-            __pipeline_memcpy_async(reinterpret_cast<double*>(&slot[(e >> 1) * BT]) + (e & 1), src, 8);
-        };
-        const int64_t N = r.bN;
-#pragma unroll
-        for (int d = 0; d < ND; ++d) cp(d, r.bx + d * N + j);
-        if (r.btype == BT_DYNAMIC) return;
-        constexpr int E = 2 * NQP;  // first double of the record
-#pragma unroll
-        for (int d = 0; d < ND; ++d) cp(E + d, r.bv + d * N + j);
-        cp(E + ND, r.brho + j);
-        if (r.baux) cp(E + ND + 1, r.baux + j);
-        // p: the multiphase pressure form, FluidSolidPfn's fluid side and the
-        // two-sided form's ε term
-        if (P.S == 1 || (PFN == PFN_FLUID2 && (P.fs || P.has_eps))) cp(E + ND + 2, r.bp + j);
-    }
-    template <int P2, int BTK = -1>
-    static __device__ __forceinline__ int pair_slot(const ForceArgs& A, const InterRef& r, const GridInst& G,
-                                                    const PfnInst& P, int64_t gi, int k, const Own& w, double da,
-                                                    const float4* slot, int BT, const float2* cam, AccT& acc) {
-        return process_pair<ND, NS, P2, KK, BTK>(A, r, G, P, gi, k, w.o, w.sig, da, NbSlot<ND>{slot, BT}, acc,
-                                                 reinterpret_cast<const double2*>(cam));
-    }
-    // system_a's sound speed and mass of instance k into the warp's 16-byte slot
-    static __device__ __forceinline__ void stage_cam(const ForceArgs& A, int k, float2* cam) {
-        if (A.a_c && A.a_mass) *reinterpret_cast<double2*>(cam) = make_double2(A.a_c[k], A.a_mass[k]);
+                                               const PfnInst& P, int k, const Own& w, int32_t j, AccT& acc) {
+        return process_pair<ND, NS, P2, KK>(A, r, G, P, k, w.o, NbGlobal{r, j}, acc);
     }
 };
 
@@ -705,19 +375,19 @@ __host__ __device__ constexpr int sweep_smem_bytes(int buf) {
 // converged warps.
 template <class Phys, bool COUNT_ONLY, int UNROLL, int PFN>
 __device__ __forceinline__ int flush_all(const ForceArgs& A, const InterRef& r, const GridInst& G,
-                                         const PfnInst& P, int64_t gi, int k, const typename Phys::Own& w,
-                                         double da, int nbuf, const int32_t* col, int BT, typename Phys::AccT& acc) {
+                                         const PfnInst& P, int k, const typename Phys::Own& w, int nbuf,
+                                         const int32_t* col, int BT, typename Phys::AccT& acc) {
     constexpr int P2 = COUNT_ONLY ? GC_PFN_COUNT : PFN;
     int acc_n = 0;
     int t = 0;
     if (UNROLL == 2) {
         for (; t + 1 < nbuf; t += 2) {
             const int32_t j0 = col[t * BT], j1 = col[(t + 1) * BT];
-            acc_n += Phys::template pair<P2>(A, r, G, P, gi, k, w, da, j0, acc);
-            acc_n += Phys::template pair<P2>(A, r, G, P, gi, k, w, da, j1, acc);
+            acc_n += Phys::template pair<P2>(A, r, G, P, k, w, j0, acc);
+            acc_n += Phys::template pair<P2>(A, r, G, P, k, w, j1, acc);
         }
     }
-    for (; t < nbuf; ++t) acc_n += Phys::template pair<P2>(A, r, G, P, gi, k, w, da, col[t * BT], acc);
+    for (; t < nbuf; ++t) acc_n += Phys::template pair<P2>(A, r, G, P, k, w, col[t * BT], acc);
     return acc_n;
 }
 
@@ -757,7 +427,6 @@ __global__ void __launch_bounds__(FORCE_TPB, MINB) k_sweep(ForceArgs A) {
             int32_t c[ND], c0, c1;
             bool ok, coop;
             if (!ref_cells<ND>(A, r, G, k, ox, active, lane, gi, c, ok, c0, c1, coop)) continue;
-            const double da = r.btype == BT_DYNAMIC ? Phys::plane_da(w, G) : 0.0;
             warp_copy(gsm, G, lane);
             warp_copy(psm, P, lane);
             __syncwarp();
@@ -798,8 +467,7 @@ __global__ void __launch_bounds__(FORCE_TPB, MINB) k_sweep(ForceArgs A) {
                     const int32_t lo = active ? r.cs[base + c[L] - 1] : 0, hi = active ? r.cs[base + c[L] + 2] : 0;
                     for (int32_t ch = u0; ch < u1; ch += 32) {
                         if (__any_sync(FULL, nbuf > BUF - 32)) {
-                            accepted += flush_all<Phys, COUNT_ONLY, UNROLL, PFN>(A, r, Gs, Ps, gi, k, w, da, nbuf, col,
-                                                                                 BT, acc);
+                            accepted += flush_all<Phys, COUNT_ONLY, UNROLL, PFN>(A, r, Gs, Ps, k, w, nbuf, col, BT, acc);
                             nbuf = 0;
                             __syncwarp();
                         }
@@ -820,7 +488,7 @@ __global__ void __launch_bounds__(FORCE_TPB, MINB) k_sweep(ForceArgs A) {
                         __syncwarp();
                     }
                 }
-                accepted += flush_all<Phys, COUNT_ONLY, UNROLL, PFN>(A, r, Gs, Ps, gi, k, w, da, nbuf, col, BT, acc);
+                accepted += flush_all<Phys, COUNT_ONLY, UNROLL, PFN>(A, r, Gs, Ps, k, w, nbuf, col, BT, acc);
                 nbuf = 0;
                 __syncwarp();
             } else if (active && ok) {
@@ -835,13 +503,12 @@ __global__ void __launch_bounds__(FORCE_TPB, MINB) k_sweep(ForceArgs A) {
                         if (self && j == gi) continue;
                         col[(nbuf++) * BT] = j;
                         if (nbuf == BUF) {
-                            accepted += flush_all<Phys, COUNT_ONLY, UNROLL, PFN>(A, r, Gs, Ps, gi, k, w, da, nbuf, col,
-                                                                                 BT, acc);
+                            accepted += flush_all<Phys, COUNT_ONLY, UNROLL, PFN>(A, r, Gs, Ps, k, w, nbuf, col, BT, acc);
                             nbuf = 0;
                         }
                     }
                 }
-                accepted += flush_all<Phys, COUNT_ONLY, UNROLL, PFN>(A, r, Gs, Ps, gi, k, w, da, nbuf, col, BT, acc);
+                accepted += flush_all<Phys, COUNT_ONLY, UNROLL, PFN>(A, r, Gs, Ps, k, w, nbuf, col, BT, acc);
                 nbuf = 0;
             }
             __syncwarp();
@@ -852,302 +519,42 @@ __global__ void __launch_bounds__(FORCE_TPB, MINB) k_sweep(ForceArgs A) {
     }
 }
 
-// ------------------------------------------------------ staged sweep
-// Shared memory of one warp of k_sweep_stg: the staged copies of a chunk of
-// CH candidates ([NQ][CH] 16-byte chunks: NbSlot's layout),
-// lane 0's position (the origin of the prefilter), the candidates' FP32
-// coordinates relative to it ([ND][CH]), and copies of the interaction's
-// grid and functor parameters for this warp's instance.
-constexpr int STG_GI_BYTES = SWEEP_GI_BYTES;
-constexpr int STG_PI_BYTES = SWEEP_PI_BYTES;
-template <int ND, int NQ, int CH>
-__host__ __device__ constexpr int stg_warp_bytes() {
-    return NQ * CH * 16 + 32 + (ND * CH * 4 + 15) / 16 * 16 + STG_GI_BYTES + STG_PI_BYTES + 16;
-}
-
-
-// The sweep with chunk staging.  The walk is k_sweep's (one
-// warp per group of one grid column, the union of its lanes' candidate
-// ranges strip by strip), but the warp copies each chunk of up to CH
-// consecutive candidates of a strip into its shared memory once (16-byte
-// asynchronous copies, one round trip per chunk), tests them against every
-// lane with the FP32 prefilter, and then evaluates each lane's accepted
-// candidates of the chunk from the staged copies.  No pair waits on a
-// global load; the exact cutoff test and the pair arithmetic are the
-// policy's, as in k_sweep.
-template <class Phys, int ND, int PFN, int MINB, int CH>
-__global__ void __launch_bounds__(FORCE_TPB, MINB) k_sweep_stg(ForceArgs A) {
-    pdl_enter();
-    static_assert(CH % 32 == 0 && CH >= 32 && CH <= 128, "chunk of 1 to 4 batches of 32");
-    constexpr int NB = CH / 32;
-    constexpr int NQ = Phys::NQ;
-    constexpr int WB = stg_warp_bytes<ND, NQ, CH>();
-    extern __shared__ float4 sstg[];
-    const unsigned FULL = 0xffffffffu;
-    const int lane = threadIdx.x & 31;
-    char* wbase = reinterpret_cast<char*>(sstg) + (threadIdx.x >> 5) * WB;
-    float4* slots = reinterpret_cast<float4*>(wbase);
-    double* xref = reinterpret_cast<double*>(wbase + NQ * CH * 16);
-    float* cand = reinterpret_cast<float*>(wbase + NQ * CH * 16 + 32);
-    // the pair loop reads the interaction's parameters from these copies
-    // (loop-invariant loads the register budget would otherwise re-issue
-    // from global memory for every pair)
-    GridInst* gsm = reinterpret_cast<GridInst*>(wbase + NQ * CH * 16 + 32 + (ND * CH * 4 + 15) / 16 * 16);
-    PfnInst* psm = reinterpret_cast<PfnInst*>(reinterpret_cast<char*>(gsm) + STG_GI_BYTES);
-    float2* camsm = reinterpret_cast<float2*>(reinterpret_cast<char*>(psm) + STG_PI_BYTES);
-    const int64_t ngroups = *A.ngroups;
-    const int64_t nwarps = ((int64_t)gridDim.x * blockDim.x) >> 5;
-    for (int64_t wg = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5; wg < ngroups; wg += nwarps) {
-        const int2 grp = A.groups[wg];
-        const bool active = lane < group_count(grp);
-        const int32_t gi = grp.x + (active ? lane : 0);  // packed indices fit int32
-        const int k = group_inst(grp);
-        typename Phys::Own w;
-        Phys::load(A, gi, w);
-        const double* ox = Phys::xpos(w);
-        typename Phys::AccT acc;
-        Phys::init(A, gi, acc, true);
-
-        for (int ri = 0; ri < A.nref; ++ri) {
-            const InterRef& r = A.ref[ri];
-            const GridInst& G = r.gi[k];
-            const PfnInst& P = r.pi[k];
-            int32_t c[ND], c0, c1;
-            bool ok, coop;
-            if (!ref_cells<ND>(A, r, G, k, ox, active, lane, gi, c, ok, c0, c1, coop)) continue;
-            const double da = r.btype == BT_DYNAMIC ? Phys::plane_da(w, G) : 0.0;
-            const bool self = r.btype == BT_SELF;
-            int32_t accepted = 0;
-            const int nstrips = ND == 2 ? 3 : 9;
-            warp_copy(gsm, G, lane);
-            warp_copy(psm, P, lane);
-            if (lane == 0) Phys::stage_cam(A, k, camsm);
-            __syncwarp();
-            const GridInst& Gs = *gsm;
-            const PfnInst& Ps = *psm;
-            if (coop) {
-                constexpr int L = ND - 1;
-                int32_t zlo, zhi;
-                warp_zrange<ND>(c, active, zlo, zhi);
-                if (lane == 0) {
-#pragma unroll
-                    for (int d = 0; d < ND; ++d) xref[d] = ox[d];
-                }
-                __syncwarp();
-                // conservative FP32 prefilter relative to lane 0 (k_sweep's);
-                // inactive lanes have an empty own range and accept nothing
-                float xi[ND];
-#pragma unroll
-                for (int d = 0; d < ND; ++d) xi[d] = active ? (float)(ox[d] - xref[d]) : 0.f;
-                const float cut_f = (float)(G.cutoff_sq * 1.001);
-                const int64_t ngl = G.ng[L];
-                auto strip_base = [&](int s2) -> int64_t {
-                    int64_t colflat;
-                    if (ND == 2) colflat = c0 + s2 - 1;
-                    else colflat = (c0 + s2 / 3 - 1) * G.ng[1] + (c1 + s2 % 3 - 1);
-                    return G.cellbase + colflat * ngl;
-                };
-                // every strip's warp-wide candidate range, lane s holding strip s's
-                int32_t su0 = 0, su1 = 0;
-                if (lane < nstrips) {
-                    const int64_t b2 = strip_base(lane);
-                    su0 = r.cs[b2 + zlo - 1];
-                    su1 = r.cs[b2 + zhi + 2];
-                }
-                // the strips, with the pair code specialised for a self
-                // interaction (the dominant kind) and generic otherwise
-                auto strips = [&](auto btk) {
-                    constexpr int BTK = decltype(btk)::value;
-                    for (int sidx = 0; sidx < nstrips; ++sidx) {
-                        const int32_t u0 = __shfl_sync(FULL, su0, sidx), u1 = __shfl_sync(FULL, su1, sidx);
-                        if (u0 >= u1) continue;  // warp-uniform
-                        const int64_t base = strip_base(sidx);
-                        // this lane's own strip range [cs[z-1], cs[z+2]) (empty when inactive)
-                        const int32_t lo = active ? r.cs[base + c[L] - 1] : 0;
-                        const int32_t hi = active ? r.cs[base + c[L] + 2] : 0;
-                        for (int32_t ch = u0; ch < u1; ch += CH) {
-                            const int n = u1 - ch < CH ? (int)(u1 - ch) : CH;
-                            for (int i = lane; i < n; i += 32) Phys::issue(r, Ps, ch + i, slots + i, CH);
-                            __pipeline_commit();
-                            __pipeline_wait_prior(0);
-                            // this lane's staged positions -> relative FP32 coordinates
-#pragma unroll
-                            for (int i0 = 0; i0 < CH; i0 += 32) {
-                                const int i = i0 + lane;
-#pragma unroll
-                                for (int d = 0; d < ND; ++d) {
-                                    float v = 1e30f;  // beyond the chunk: far away
-                                    if (i < n) {
-                                        const double2 t = *reinterpret_cast<const double2*>(&slots[(d >> 1) * CH + i]);
-                                        v = (float)(((d & 1) ? t.y : t.x) - xref[d]);
-                                    }
-                                    cand[d * CH + i] = v;
-                                }
-                            }
-                            __syncwarp();
-                            // accepted candidates of the chunk, one mask per batch of 32
-                            unsigned msk[NB];
-#pragma unroll
-                            for (int b = 0; b < NB; ++b) {
-                                msk[b] = 0u;
-                                if (32 * b < n) {
-                                    const int mb = n - 32 * b < 32 ? n - 32 * b : 32;
-                                    msk[b] = batch_hits<ND, true>(cand + 32 * b, CH, mb, xi, cut_f) &
-                                             own_allow(lo, hi, ch + 32 * b, self, gi);
-                                }
-                            }
-                            // this lane's accepted candidates, from the staged copies, in
-                            // increasing order: msk[0] is the current batch's mask, and an
-                            // empty one shifts the later batches down
-                            int mbase = 0;
-                            while (true) {
-                                if (msk[0] == 0u) {
-#pragma unroll
-                                    for (int s2 = 1; s2 < NB; ++s2) {
-                                        if (msk[0] == 0u) {
-#pragma unroll
-                                            for (int b = 0; b + 1 < NB; ++b) msk[b] = msk[b + 1];
-                                            msk[NB - 1] = 0u;
-                                            mbase += 32;
-                                        }
-                                    }
-                                    if (msk[0] == 0u) break;
-                                }
-                                const int t = mbase + __ffs(msk[0]) - 1;
-                                msk[0] &= msk[0] - 1;
-                                accepted += Phys::template pair_slot<PFN, BTK>(A, r, Gs, Ps, gi, k, w, da, slots + t, CH, camsm, acc);
-                            }
-                            __syncwarp();  // every lane is done with the chunk before the next one lands
-                        }
-                    }
-                };
-                if (self) strips(std::integral_constant<int, BT_SELF>{});
-                else strips(std::integral_constant<int, -1>{});
-            } else if (active && ok) {
-                // rare: lanes disagree on the column in this grid; walk own strips
-                for (int sidx = 0; sidx < nstrips; ++sidx) {
-                    int64_t base;
-                    if (ND == 2) base = G.cellbase + (c[0] + sidx - 1) * G.ng[1] + (c[1] - 1);
-                    else base = G.cellbase + ((c[0] + sidx / 3 - 1) * G.ng[1] + (c[1] + sidx % 3 - 1)) * G.ng[2] + (c[2] - 1);
-                    const int32_t s0 = r.cs[base], e0 = r.cs[base + 3];
-                    for (int32_t j = s0; j < e0; ++j) {
-                        if (self && j == gi) continue;
-                        accepted += Phys::template pair<PFN>(A, r, G, P, gi, k, w, da, j, acc);
-                    }
-                }
-            }
-            __syncwarp();
-            if (active && r.counts) r.counts[gi] = accepted;
-        }
-        if (active) Phys::store(A, gi, acc);
-        __syncwarp();
-    }
-}
-
 // ------------------------------------------------------------ dispatch
-template <class Phys, int ND, int PFN, int C>
-static void launch_c(const ForceArgs& A, cudaStream_t s) {
-    constexpr ForceCfg cf = FORCE_CFGS[C];
-    int64_t warps = A.aN;
-    int64_t blocks = (warps * 32 + FORCE_TPB - 1) / FORCE_TPB;
-    if (blocks > (int64_t)A.num_sms * cf.minb * 4) blocks = (int64_t)A.num_sms * cf.minb * 4;
-    if (blocks < 1) blocks = 1;
-    if constexpr (cf.stg > 0 && Phys::NQ > 0) {
-        constexpr size_t smem = (size_t)(FORCE_TPB / 32) * stg_warp_bytes<ND, Phys::NQ, cf.stg>();
-        auto kern = k_sweep_stg<Phys, ND, PFN, cf.minb, cf.stg>;
-        if (smem > 48 * 1024) {
-            static bool opted = false;
-            if (!opted) {
-                cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-                opted = true;
-            }
-        }
-        kern<<<(int)blocks, FORCE_TPB, smem, s>>>(A);
-    } else {
-        const size_t smem = (size_t)sweep_smem_bytes<ND>(cf.buf);
-        auto kern = k_sweep<Phys, ND, PFN, false, cf.minb, cf.buf, cf.unroll>;
-        if (smem > 48 * 1024) {
-            // beyond the default dynamic shared-memory limit: opt in once per kernel
-            static bool opted = false;
-            if (!opted) {
-                cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-                opted = true;
-            }
-        }
-        kern<<<(int)blocks, FORCE_TPB, smem, s>>>(A);
-    }
-}
-
-template <class Phys, int ND, int PFN>
-static void launch_cfg(const ForceArgs& A, cudaStream_t s) {
-    switch (A.cfg) {
-        case 1: launch_c<Phys, ND, PFN, 1>(A, s); break;
-        case 2: launch_c<Phys, ND, PFN, 2>(A, s); break;
-        case 3: launch_c<Phys, ND, PFN, 3>(A, s); break;
-        default: launch_c<Phys, ND, PFN, 0>(A, s); break;
-    }
-}
-
 template <int ND, int NS, int PFN, int KK>
-static void launch_t(const ForceArgs& A, bool count_only, cudaStream_t s) {
-    using P64 = PhysF64<ND, NS, PFN, KK>;
-    if (count_only) {
-        int64_t blocks = (A.aN * 32 + FORCE_TPB - 1) / FORCE_TPB;
-        if (blocks > (int64_t)A.num_sms * 16) blocks = (int64_t)A.num_sms * 16;
-        if (blocks < 1) blocks = 1;
-        const size_t smem = (size_t)sweep_smem_bytes<ND>(FORCE_BUF);
-        k_sweep<P64, ND, PFN, true, 4, FORCE_BUF, 1><<<(int)blocks, FORCE_TPB, smem, s>>>(A);
-    } else {
-        launch_cfg<P64, ND, PFN>(A, s);
-    }
+static void launch_t(const ForceArgs& A, cudaStream_t s) {
+    constexpr bool COUNT_ONLY = PFN == GC_PFN_NONE;  // counting without sums
+    constexpr int P2 = COUNT_ONLY ? GC_PFN_COUNT : PFN;
+    int64_t blocks = (A.aN * 32 + FORCE_TPB - 1) / FORCE_TPB;
+    if (blocks > (int64_t)A.num_sms * 16) blocks = (int64_t)A.num_sms * 16;
+    if (blocks < 1) blocks = 1;
+    const size_t smem = (size_t)sweep_smem_bytes<ND>(FORCE_BUF);
+    k_sweep<PhysGather<ND, NS, P2, KK>, ND, P2, COUNT_ONLY, 4, FORCE_BUF, 1><<<(int)blocks, FORCE_TPB, smem, s>>>(A);
     g_launches.fetch_add(1, std::memory_order_relaxed);
 }
 
-template <int ND, int NS, int KK>
-static int launch_pfn(const ForceArgs& A, bool count_only, cudaStream_t s) {
-    switch (A.pfn) {
-        case GC_PFN_FLUID: launch_t<ND, NS, GC_PFN_FLUID, KK>(A, count_only, s); return 0;
-        case PFN_FLUID2: launch_t<ND, NS, PFN_FLUID2, KK>(A, count_only, s); return 0;
-        case GC_PFN_COUNT: launch_t<ND, NS, GC_PFN_COUNT, KK>(A, count_only, s); return 0;
-        case GC_PFN_INTERPOLATE: launch_t<ND, NS, GC_PFN_INTERPOLATE, KK>(A, count_only, s); return 0;
-        case GC_PFN_XSPH: launch_t<ND, NS, GC_PFN_XSPH, KK>(A, count_only, s); return 0;
-        case GC_PFN_CAUCHY_FLUID:
-            if (NS == 0) return GC_ERR_UNSUPPORTED;
-            launch_t<ND, NS, GC_PFN_CAUCHY_FLUID, KK>(A, count_only, s);
-            return 0;
-        case GC_PFN_STRAIN_RATE:
-            if (NS == 0) return GC_ERR_UNSUPPORTED;
-            launch_t<ND, NS, GC_PFN_STRAIN_RATE, KK>(A, count_only, s);
-            return 0;
-        case GC_PFN_STRAIN_RATE_VORTICITY:
-            if (NS == 0) return GC_ERR_UNSUPPORTED;
-            launch_t<ND, NS, GC_PFN_STRAIN_RATE_VORTICITY, KK>(A, count_only, s);
-            return 0;
-    }
-    return GC_ERR_UNSUPPORTED;
-}
-
+// The buffered sweep: neighbour counts, InterpolateFieldFn (and
+// NeighborCountFn) and XSPHPfn.
 template <int ND, int KK>
 static int launch_nd(const ForceArgs& A, bool count_only, cudaStream_t s) {
-    const bool stress_pfn = A.pfn == GC_PFN_CAUCHY_FLUID || A.pfn == GC_PFN_STRAIN_RATE ||
-                            A.pfn == GC_PFN_STRAIN_RATE_VORTICITY ||
-                            (A.pfn == GC_PFN_INTERPOLATE && (A.imask & (1 << GC_FIELD_STRESS)));
-    if (!stress_pfn) return launch_pfn<ND, 0, KK>(A, count_only, s);
-    if (ND == 2) {
-        if (A.ns == 3) return launch_pfn<ND, 3, KK>(A, count_only, s);
-        if (A.ns == 4) return launch_pfn<ND, 4, KK>(A, count_only, s);
-        return GC_ERR_UNSUPPORTED;
+    if (count_only) {
+        launch_t<ND, 0, GC_PFN_NONE, KK>(A, s);
+        return 0;
     }
-    if (A.ns == 6) return launch_pfn<ND, 6, KK>(A, count_only, s);
-    return GC_ERR_UNSUPPORTED;
+    if (A.pfn == GC_PFN_COUNT) {
+        launch_t<ND, 0, GC_PFN_COUNT, KK>(A, s);
+        return 0;
+    }
+    if (A.pfn == GC_PFN_XSPH) {
+        launch_t<ND, 0, GC_PFN_XSPH, KK>(A, s);
+        return 0;
+    }
+    if (A.pfn != GC_PFN_INTERPOLATE) return GC_ERR_UNSUPPORTED;
+    if (!(A.imask & (1 << GC_FIELD_STRESS))) launch_t<ND, 0, GC_PFN_INTERPOLATE, KK>(A, s);
+    else if (ND == 2 && A.ns == 3) launch_t<ND, 3, GC_PFN_INTERPOLATE, KK>(A, s);
+    else if (ND == 2 && A.ns == 4) launch_t<ND, 4, GC_PFN_INTERPOLATE, KK>(A, s);
+    else if (ND == 3 && A.ns == 6) launch_t<ND, 6, GC_PFN_INTERPOLATE, KK>(A, s);
+    else return GC_ERR_UNSUPPORTED;
+    return 0;
 }
-
-// One translation unit per dimension: defines launch_force_<ND>d_f64.
-#define GC_DEFINE_FORCE_TU(NDIM, NAME)                                                    \
-    int NAME(const ForceArgs& A, bool count_only, cudaStream_t s) {                      \
-        if (A.kk == GC_KERNEL_CUBIC_SPLINE)                                               \
-            return launch_nd<NDIM, GC_KERNEL_CUBIC_SPLINE>(A, count_only, s);            \
-        return launch_nd<NDIM, GC_KERNEL_WENDLAND_C2>(A, count_only, s);                 \
-    }
 
 }  // namespace gc
