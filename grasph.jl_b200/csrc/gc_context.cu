@@ -141,8 +141,6 @@ struct DSlot {
     // warp groups of this system's particles (one grid's columns)
     int2* groups = nullptr;
     int64_t* d_ngroups = nullptr;
-    int32_t *gcnt = nullptr, *goff = nullptr;
-    int64_t cap_gcols = 0;
     int64_t groups_key = -1, groups_ver = -1;
     double* F(int k) { return f[cur][k]; }
     double* A(int k) { return f[cur ^ 1][k]; }
@@ -155,8 +153,6 @@ struct DGhost {
     // sweep's ghost-indexed sums before they are added to the source
     int2* groups = nullptr;
     int64_t* d_ngroups = nullptr;
-    int32_t *gcnt = nullptr, *goff = nullptr;
-    int64_t cap_gcols = 0;
     int64_t groups_key = -1, groups_ver = -1;
     double* gadj = nullptr;
     double* x[2] = {};
@@ -226,7 +222,7 @@ struct DInter {
     // scan are skipped on the device when the geometry is unchanged
     int* d_keep = nullptr;          // [0] cs is current for d_gi_prev, [1] this step's grid equals it
     GridInst* d_gi_prev = nullptr;  // geometry cs was last counted on, per instance
-    int32_t* hist = nullptr;        // its own histogram (batched still grids): zero between uses
+    int32_t* hist = nullptr;        // its own histogram (batched grids): zero between uses
     int64_t cap_hist = 0;
 };
 
@@ -283,7 +279,6 @@ struct gc_ctx {
     int64_t* d_need = nullptr;
     int64_t* h_need = nullptr;  // pinned
     int nneed = 0;
-    int nplan = 0;  // entries of d_plan_args (the steps' interactions)
     int64_t* d_total_cells = nullptr;  // device copy of the current sort's cell total
     int64_t grid_version = 0;
     int num_sms = 148;
@@ -331,7 +326,8 @@ struct gc_ctx {
     int64_t* d_need_max = nullptr;
     int64_t* h_need_max = nullptr;  // pinned
     int64_t* d_need_cap = nullptr;  // per plan entry, the cells capacity mode sizes for
-    GridPlanArgs* d_plan_args = nullptr;  // grid plan arguments of every interaction
+    PlanItem* d_plans = nullptr;  // the steps' plans, one per entry of d_need
+    unsigned long long* d_gscratch = nullptr;  // launch_groups' scratch
     std::vector<Snapshot> snaps;    // per slot (moving slots only)
     int64_t graph_steps = 0, rollbacks = 0;
     int64_t pack_epoch = 0;  // bumps at the start of every issued step (never rolled back)
@@ -1031,18 +1027,41 @@ int finalize(gc_ctx* ctx) {
     for (size_t i = 0; i < ctx->inters.size(); ++i)
         ctx->inters[i].need_slot = (int64_t)(ctx->slots.size() + ctx->ghosts.size() + i);
     {
-        std::vector<GridPlanArgs> pa;  // the steps' interactions; probe grids are planned at measurement
+        // probe grids are planned at measurement
+        std::vector<PlanItem> items(ctx->nneed);
+        memset(items.data(), 0, items.size() * sizeof(PlanItem));
+        auto bound = [&](PlanItem& it, int g) {
+            DGhost& G = ctx->ghosts[g];
+            it.bound[it.nbound++] = GhostBound{G.d_gh, ctx->slots[G.src].d_inst, G.d_inst, G.nd, G.nplanes};
+        };
+        for (size_t s = 0; s < ctx->slots.size(); ++s) {
+            items[s].kind = PLAN_SORT;
+            items[s].inst = ctx->slots[s].d_inst;
+            items[s].nd = ctx->slots[s].nd;
+        }
+        for (size_t g = 0; g < ctx->ghosts.size(); ++g) {
+            PlanItem& it = items[ctx->ghosts[g].need_slot];
+            it.kind = PLAN_SORT;
+            it.inst = ctx->ghosts[g].d_inst;
+            it.nd = ctx->ghosts[g].nd;
+            bound(it, (int)g);
+        }
         for (auto& D : ctx->inters) {
             if (D.probe) continue;
-            pa.push_back(grid_plan_args(ctx, D));
+            PlanItem& it = items[D.need_slot];
+            it.kind = PLAN_GRID;
+            it.grid = grid_plan_args(ctx, D);
             // the keep check of a still system_b's CSR runs in its plan (the
             // only plan of such an interaction in a step)
-            pa.back().prev = D.d_gi_prev;
-            pa.back().keep = D.d_keep;
+            it.grid.prev = D.d_gi_prev;
+            it.grid.keep = D.d_keep;
+            if (D.ag >= 0) bound(it, D.ag);
+            if (D.btype == BT_GHOST && D.bghost != D.ag) bound(it, D.bghost);
         }
-        ctx->nplan = (int)pa.size();
-        TRY(dalloc(ctx, &ctx->d_plan_args, pa.size()));
-        TRY(hcopy(ctx, ctx->d_plan_args, pa.data(), pa.size() * sizeof(GridPlanArgs), cudaMemcpyHostToDevice));
+        TRY(dalloc(ctx, &ctx->d_plans, items.size()));
+        TRY(hcopy(ctx, ctx->d_plans, items.data(), items.size() * sizeof(PlanItem), cudaMemcpyHostToDevice));
+        TRY(dalloc(ctx, &ctx->d_gscratch, 2));
+        CU(cudaMemsetAsync(ctx->d_gscratch, 0, 2 * sizeof(unsigned long long), ctx->stream));
     }
     ctx->finalized = true;
     return GC_OK;
@@ -1080,15 +1099,16 @@ int ensure_inter_cells(gc_ctx* ctx, DInter& D, int64_t cells) {
         TRY(dalloc(ctx, &D.cs, (size_t)cap));
         if (D.btype != BT_SELF) TRY(dalloc(ctx, &D.cs_a, (size_t)cap));
         D.cap_cells = cap;
-        if (D.d_keep) {
-            // its own histogram for the batched still grids, zero between uses
+        if (!D.probe) {
+            // its own histogram for the batched grids (zero between uses), then
+            // its scan's tile sums
             dfree(ctx, D.hist, D.cap_hist);
-            D.cap_hist = still_hist_elems(cap);
+            D.cap_hist = cap + grid_scan_tiles(cap);
             TRY(dalloc(ctx, &D.hist, (size_t)D.cap_hist));
             CU(cudaMemsetAsync(D.hist, 0, sizeof(int32_t) * D.cap_hist, ctx->stream));
-            // new buffer: nothing counted (the step's plan may already have set keep[1])
-            CU(cudaMemsetAsync(D.d_keep, 0, 2 * sizeof(int), ctx->stream));
         }
+        // new buffer: nothing counted (the step's plan may already have set keep[1])
+        if (D.d_keep) CU(cudaMemsetAsync(D.d_keep, 0, 2 * sizeof(int), ctx->stream));
     }
     return ensure_cells(ctx, cells);
 }
@@ -1106,38 +1126,6 @@ int bbox_slot(gc_ctx* ctx, DSlot& S) {
     launch_bbox_fused(S.F(F_X), S.N, S.nd, S.inst_of, nullptr, S.d_inst, ctx->bbox_scratch, ninst(ctx), ctx->d_err,
                 ctx->stream);
     return check_launch(ctx, "bbox");
-}
-
-// Conservative ghost extent before generation: the reflection of the source
-// bounding box's corners across every plane, padded by one cell.
-__global__ void k_ghost_bound(GhostInst* gh, const SysInst* src, SysInst* gi, int ninst, int nd, int nplanes) {
-    pdl_enter();
-    int k = blockIdx.x * blockDim.x + threadIdx.x;
-    if (k >= ninst) return;
-    const SysInst& S = src[k];
-    double lo[MAXD], hi[MAXD];
-    for (int d = 0; d < nd; ++d) {
-        lo[d] = 1e300;
-        hi[d] = -1e300;
-    }
-    int ncorner = 1 << nd;
-    for (int b = 0; b < nplanes; ++b)
-        for (int cI = 0; cI < ncorner; ++cI) {
-            double x[MAXD], da = 0.0;
-            for (int d = 0; d < nd; ++d) x[d] = (cI >> d) & 1 ? S.bbmax[d] : S.bbmin[d];
-            for (int d = 0; d < nd; ++d) da += (x[d] - gh[k].points[b][d]) * gh[k].normals[b][d];
-            for (int d = 0; d < nd; ++d) {
-                double r = x[d] - 2.0 * da * gh[k].normals[b][d];
-                lo[d] = fmin(lo[d], fmin(r, x[d]));
-                hi[d] = fmax(hi[d], fmax(r, x[d]));
-            }
-        }
-    double pad = 2.0 * S.sort_cutoff;
-    for (int d = 0; d < nd; ++d) {
-        gi[k].bbmin[d] = lo[d] - pad;
-        gi[k].bbmax[d] = hi[d] + pad;
-    }
-    gi[k].n = S.n;  // upper bound on the count, used only for planning
 }
 
 // Stable counting sort of `S` (or of a ghost set when G != nullptr) over
@@ -1279,83 +1267,90 @@ AParts a_parts(gc_ctx* ctx, const DInter& D) {
     return AParts{A.F(F_X), A.N, A.inst_of, nullptr};
 }
 
+// system_b's particles of an interaction
+struct BParts {
+    const double* x;
+    int64_t N;
+    const int32_t* inst_of;
+    const int64_t* count;
+};
+BParts b_parts(gc_ctx* ctx, const DInter& D) {
+    if (D.btype == BT_GHOST) {
+        DGhost& G = ctx->ghosts[D.bghost];
+        return BParts{G.x[G.cur], G.CAP, G.ginst[G.cur], G.d_count};
+    }
+    DSlot& B = ctx->slots[D.bslot];
+    return BParts{B.F(F_X), B.N, B.inst_of, nullptr};
+}
+
+// system_a's CSR on the interaction's grid.
+int count_csa(gc_ctx* ctx, DInter& D, int64_t cells) {
+    const AParts ap = a_parts(ctx, D);
+    TRY(ensure_cells(ctx, cells));
+    launch_grid_count(ap.x, ap.N, ctx->slots[D.a].nd, ap.inst_of, ap.count, D.d_gi, ctx->hist, cells, ctx->d_err,
+                      ctx->d_incons, ctx->stream);
+    scan_exclusive_clear(ctx->hist, D.cs_a, cells, ctx->scan_tmp, ctx->stream);
+    return GC_OK;
+}
+
+void grid_built(gc_ctx* ctx, DInter& D, int64_t cells) {
+    D.grid_valid = true;
+    D.cells = cells;
+    D.grid_ver = ++ctx->grid_version;
+    D.csa_ver = D.two_sided ? D.grid_ver : -1;
+}
+
 // allow_keep: system_b's positions have not changed since its CSR was last
 // counted, so an unchanged geometry keeps the CSR (decided on the device by
 // the step's plan, keep[1]).
 int build_grid(gc_ctx* ctx, DInter& D, int64_t cells, bool allow_keep = false) {
     TRY(ensure_inter_cells(ctx, D, cells));
-    DSlot& A = ctx->slots[D.a];
     const int* skip = nullptr;
     if (D.d_keep) {
         if (allow_keep) skip = D.d_keep + 1;
         else CU(cudaMemsetAsync(D.d_keep, 0, sizeof(int), ctx->stream));  // counted on a geometry not recorded
     }
-    const double* bx;
-    const int32_t* binst;
-    const int64_t* bcount = nullptr;
-    int64_t bN;
-    if (D.btype == BT_GHOST) {
-        DGhost& G = ctx->ghosts[D.bghost];
-        bx = G.x[G.cur];
-        binst = G.ginst[G.cur];
-        bcount = G.d_count;
-        bN = G.CAP;
-    } else {
-        DSlot& B = ctx->slots[D.bslot];
-        bx = B.F(F_X);
-        binst = B.inst_of;
-        bN = B.N;
-    }
-    launch_grid_count(bx, bN, A.nd, binst, bcount, D.d_gi, ctx->hist, cells, ctx->d_err, ctx->d_incons, ctx->stream,
-                      skip);
+    const BParts b = b_parts(ctx, D);
+    launch_grid_count(b.x, b.N, ctx->slots[D.a].nd, b.inst_of, b.count, D.d_gi, ctx->hist, cells, ctx->d_err,
+                      ctx->d_incons, ctx->stream, skip);
     scan_exclusive_clear(ctx->hist, D.cs, cells, ctx->scan_tmp, ctx->stream, skip);
-    if (D.two_sided) {
-        const AParts ap = a_parts(ctx, D);
-        launch_grid_count(ap.x, ap.N, A.nd, ap.inst_of, ap.count, D.d_gi, ctx->hist, cells, ctx->d_err,
-                          ctx->d_incons, ctx->stream);
-        scan_exclusive_clear(ctx->hist, D.cs_a, cells, ctx->scan_tmp, ctx->stream);
-    }
-    D.grid_valid = true;
-    D.cells = cells;
-    D.grid_ver = ++ctx->grid_version;
-    D.csa_ver = D.two_sided ? D.grid_ver : -1;
+    if (D.two_sided) TRY(count_csa(ctx, D, cells));
+    grid_built(ctx, D, cells);
     return check_launch(ctx, "grid");
 }
 
-// The grids of interactions against a system_b that does not move, built
-// together: one count and one scan launch for all of them, each returning
-// at once on the device while its grid's geometry is unchanged (keep[1]).
-int build_still_grids(gc_ctx* ctx, const std::vector<DInter*>& L, const std::vector<int64_t>& need) {
-    for (size_t i0 = 0; i0 < L.size(); i0 += STILL_MAX) {
-        StillGridArgs a{};
-        a.n = (int)std::min<size_t>(STILL_MAX, L.size() - i0);
+// The grids of several interactions: one count and two scan launches for all
+// of them.  An interaction against a system_b that does not move returns at
+// once on the device while its grid's geometry is unchanged (keep[1]).
+int build_grids(gc_ctx* ctx, const std::vector<DInter*>& L, const std::vector<int64_t>& need) {
+    for (size_t i0 = 0; i0 < L.size(); i0 += GRIDS_MAX) {
+        GridBuildArgs a{};
+        a.n = (int)std::min<size_t>(GRIDS_MAX, L.size() - i0);
         a.err = ctx->d_err;
         a.incons = ctx->d_incons;
         for (int i = 0; i < a.n; ++i) {
             DInter& D = *L[i0 + i];
             const int64_t cells = need[D.need_slot];
             TRY(ensure_inter_cells(ctx, D, cells));  // sizes the histogram with the CSR
-            DSlot& B = ctx->slots[D.bslot];
             a.nd = ctx->slots[D.a].nd;
-            a.g[i] = StillGrid{B.F(F_X), B.inst_of, B.N, D.d_gi, D.d_keep, D.hist, D.cs, cells};
-            D.grid_valid = true;
-            D.cells = cells;
-            D.grid_ver = ++ctx->grid_version;
-            D.csa_ver = -1;
+            const BParts b = b_parts(ctx, D);
+            a.g[i] = GridBuild{b.x, b.inst_of, b.N, b.count, D.d_gi, D.d_keep, D.hist, D.hist + D.cap_cells, D.cs,
+                               cells};
         }
-        launch_still_grids(a, ctx->stream);
+        launch_grids(a, ctx->stream);
+        for (int i = 0; i < a.n; ++i) {
+            DInter& D = *L[i0 + i];
+            if (D.two_sided) TRY(count_csa(ctx, D, need[D.need_slot]));
+            grid_built(ctx, D, need[D.need_slot]);
+        }
     }
-    return check_launch(ctx, "still grids");
+    return check_launch(ctx, "grids");
 }
 
 // CSR of system_a's particles on a coupled interaction's grid.
 int ensure_csa(gc_ctx* ctx, DInter& D) {
     if (D.btype == BT_SELF || D.csa_ver == D.grid_ver) return GC_OK;
-    const AParts ap = a_parts(ctx, D);
-    TRY(ensure_cells(ctx, D.cells));
-    launch_grid_count(ap.x, ap.N, ctx->slots[D.a].nd, ap.inst_of, ap.count, D.d_gi, ctx->hist, D.cells, ctx->d_err,
-                      ctx->d_incons, ctx->stream);
-    scan_exclusive_clear(ctx->hist, D.cs_a, D.cells, ctx->scan_tmp, ctx->stream);
+    TRY(count_csa(ctx, D, D.cells));
     D.csa_ver = D.grid_ver;
     return check_launch(ctx, "grid (system_a)");
 }
@@ -1365,21 +1360,8 @@ int ensure_csa(gc_ctx* ctx, DInter& D) {
 template <class St>
 int build_groups(gc_ctx* ctx, St& S, DInter& D, int64_t key, const int32_t* cs) {
     if (S.groups_key == key && S.groups_ver == D.grid_ver) return GC_OK;
-    const int64_t ncols_cap = D.cells;
-    if (ncols_cap + 1 > S.cap_gcols) {
-        CU(cudaStreamSynchronize(ctx->stream));
-        dfree(ctx, S.gcnt, S.cap_gcols);
-        dfree(ctx, S.goff, S.cap_gcols);
-        int64_t cap = ncols_cap + 1 + ncols_cap / 4;
-        TRY(dalloc(ctx, &S.gcnt, (size_t)cap));
-        TRY(dalloc(ctx, &S.goff, (size_t)cap));
-        S.cap_gcols = cap;
-    }
-    TRY(ensure_cells(ctx, ncols_cap));  // scan scratch
-    const int nd = ctx->slots[D.a].nd;
-    launch_groups_count(D.d_gi, ninst(ctx), nd, cs, ncols_cap, D.cells, S.gcnt, ctx->stream);
-    scan_exclusive(S.gcnt, S.goff, ncols_cap, ctx->scan_tmp, ctx->stream);
-    launch_groups_fill(D.d_gi, ninst(ctx), nd, cs, S.goff, ncols_cap, D.cells, S.groups, S.d_ngroups, ctx->stream);
+    launch_groups(D.d_gi, ninst(ctx), ctx->slots[D.a].nd, cs, D.cells, D.cells, S.groups, S.d_ngroups,
+                  ctx->d_gscratch, ctx->stream);
     S.groups_key = key;
     S.groups_ver = D.grid_ver;
     return check_launch(ctx, "groups");
@@ -1402,16 +1384,6 @@ int ensure_groups(gc_ctx* ctx, int slot, int id, bool b_side) {
     return build_groups(ctx, S, D, key, cs);
 }
 
-// Capacity mode: record the largest plans, and flag every plan that does
-// not fit its buffers (the window is then rolled back and re-run exactly).
-__global__ void k_need_max(const int64_t* need, int64_t* need_max, const int64_t* cap, int n, int* err) {
-    pdl_enter();
-    for (int i = threadIdx.x; i < n; i += blockDim.x) {
-        if (need[i] > need_max[i]) need_max[i] = need[i];
-        if (need[i] > cap[i]) atomicOr(err, ERR_CAPACITY);
-    }
-}
-
 // Cell bound for sorts and for interaction D's grid in capacity mode: the
 // shared histogram and the interaction's CSR both have to hold it.
 int64_t cap_sort_cells(gc_ctx* ctx) { return ctx->cap_cells - 1; }
@@ -1423,27 +1395,23 @@ int64_t cap_grid_cells(gc_ctx* ctx, const DInter& D) { return std::min(D.cap_cel
 // (no host read), and the kernels flag any plan that does not fit.
 int prepare(gc_ctx* ctx, const std::vector<char>& sort_mask) {
     const int ni = ninst(ctx);
-    CU(cudaMemsetAsync(ctx->d_need, 0, sizeof(int64_t) * ctx->nneed, ctx->stream));
     // bounding boxes of every real system (positions are current); a system
     // that does not move keeps the box computed after its last upload
     for (auto& S : ctx->slots)
         if (S.xmoves() || !S.sorted_once) TRY(bbox_slot(ctx, S));
-    for (size_t s = 0; s < ctx->slots.size(); ++s)
-        if (sort_mask[s])
-            launch_sort_plan(ctx->slots[s].d_inst, ni, ctx->slots[s].nd, ctx->d_need + s, ctx->d_err, ctx->stream);
-    for (auto& G : ctx->ghosts) {
-        k_ghost_bound<<<(ni + 127) / 128, 128, 0, ctx->stream>>>(G.d_gh, ctx->slots[G.src].d_inst, G.d_inst, ni, G.nd,
-                                                                 G.nplanes);
-        g_launches.fetch_add(1, std::memory_order_relaxed);
-        launch_sort_plan(G.d_inst, ni, G.nd, ctx->d_need + G.need_slot, ctx->d_err, ctx->stream);
+    for (int i0 = 0; i0 < ctx->nneed; i0 += PLAN_MAX) {
+        const int n = std::min(PLAN_MAX, ctx->nneed - i0);
+        PlanMask mask{};
+        for (int i = 0; i < n; ++i) {
+            const size_t s = (size_t)(i0 + i);  // ghosts follow the slots
+            if (s >= ctx->slots.size() || sort_mask[s]) mask.w[i >> 6] |= 1ull << (i & 63);
+        }
+        launch_plan_all(ctx->d_plans + i0, n, ni, mask, ctx->d_need + i0, ctx->capmode ? ctx->d_need_max + i0 : nullptr,
+                        ctx->d_need_cap + i0, ctx->d_err, ctx->stream);
     }
-    launch_grid_plan_all(ctx->d_plan_args, ctx->nplan, ctx->stream);
     TRY(check_launch(ctx, "plan"));
     std::vector<int64_t> need(ctx->nneed);
     if (ctx->capmode) {
-        k_need_max<<<1, 128, 0, ctx->stream>>>(ctx->d_need, ctx->d_need_max, ctx->d_need_cap, ctx->nneed,
-                                                ctx->d_err);
-        g_launches.fetch_add(1, std::memory_order_relaxed);
         for (size_t s = 0; s < ctx->slots.size(); ++s) need[s] = cap_sort_cells(ctx);
         for (auto& G : ctx->ghosts) need[G.need_slot] = cap_sort_cells(ctx);
         for (auto& D : ctx->inters) need[D.need_slot] = D.probe ? 0 : cap_grid_cells(ctx, D);
@@ -1465,18 +1433,19 @@ int prepare(gc_ctx* ctx, const std::vector<char>& sort_mask) {
     }
     // grids (ghost-b plans are recomputed from the exact ghost boxes; the
     // cell count cannot exceed the planned bound)
-    std::vector<DInter*> still;
+    std::vector<DInter*> batch;
     for (auto& D : ctx->inters) {
         if (D.probe) continue;
         if (D.btype == BT_GHOST || D.ag >= 0) launch_grid_plan(grid_plan_args(ctx, D), ctx->stream);
         const bool b_still = D.d_keep && !sort_mask[D.bslot] && !ctx->slots[D.bslot].xmoves();
-        if (b_still && ctx->slots[D.bslot].N > 0 && need[D.need_slot] <= STILL_MAX_CELLS) {
-            still.push_back(&D);
+        const int64_t bN = D.btype == BT_GHOST ? ctx->ghosts[D.bghost].CAP : ctx->slots[D.bslot].N;
+        if (bN > 0 && need[D.need_slot] <= GRIDS_MAX_CELLS && (b_still || !D.d_keep)) {
+            batch.push_back(&D);
             continue;
         }
         TRY(build_grid(ctx, D, need[D.need_slot], b_still));
     }
-    return build_still_grids(ctx, still, need);
+    return build_grids(ctx, batch, need);
 }
 
 StepArgs step_args(DSlot& S) {
@@ -2347,19 +2316,6 @@ bool tuning(gc_ctx* ctx) {
     return false;
 }
 
-template <class St>
-int grow_gcols(gc_ctx* ctx, St& S, int64_t ncols) {
-    if (ncols + 1 <= S.cap_gcols) return GC_OK;
-    CU(cudaStreamSynchronize(ctx->stream));
-    dfree(ctx, S.gcnt, S.cap_gcols);
-    dfree(ctx, S.goff, S.cap_gcols);
-    int64_t cap = ncols + 1 + ncols / 4;
-    TRY(dalloc(ctx, &S.gcnt, (size_t)cap));
-    TRY(dalloc(ctx, &S.goff, (size_t)cap));
-    S.cap_gcols = cap;
-    return GC_OK;
-}
-
 // Capacities for capacity-mode steps: every planned cell count seen so far,
 // times the margin.  Growth happens here, at a verified point, never inside
 // a captured step.
@@ -2388,14 +2344,6 @@ int size_capacities(gc_ctx* ctx) {
         dfree(ctx, ctx->scan_tmp, ctx->cap_scan);
         TRY(dalloc(ctx, &ctx->scan_tmp, (size_t)st));
         ctx->cap_scan = st;
-    }
-    // warp-group column tables of every system a grid groups
-    for (auto& D : ctx->inters) {
-        if (D.probe) continue;
-        const int64_t cells = cap_grid_cells(ctx, D);
-        TRY(grow_gcols(ctx, ctx->slots[D.a], cells));
-        if (D.two_sided && D.bslot >= 0) TRY(grow_gcols(ctx, ctx->slots[D.bslot], cells));
-        if (D.vadj && D.btype == BT_GHOST) TRY(grow_gcols(ctx, ctx->ghosts[D.bghost], cells));
     }
     // the bound each plan entry is checked against inside the steps
     std::vector<int64_t> cap(n);
@@ -2732,8 +2680,6 @@ int gc_ctx_destroy(gc_ctx* ctx) {
         dev_free(ctx, S.inst_of);
         dev_free(ctx, S.groups);
         dev_free(ctx, S.d_ngroups);
-        dev_free(ctx, S.gcnt);
-        dev_free(ctx, S.goff);
         dev_free(ctx, S.d_inst);
         dev_free(ctx, S.d_mass);
         dev_free(ctx, S.d_c);
@@ -2764,8 +2710,6 @@ int gc_ctx_destroy(gc_ctx* ctx) {
         dev_free(ctx, G.fpk);
         dev_free(ctx, G.groups);
         dev_free(ctx, G.d_ngroups);
-        dev_free(ctx, G.gcnt);
-        dev_free(ctx, G.goff);
         dev_free(ctx, G.gadj);
     }
     for (auto& V : ctx->virts) {
@@ -2802,7 +2746,8 @@ int gc_ctx_destroy(gc_ctx* ctx) {
     if (ctx->h_need) cudaFreeHost(ctx->h_need);
     dev_free(ctx, ctx->d_need_max);
     dev_free(ctx, ctx->d_need_cap);
-    dev_free(ctx, ctx->d_plan_args);
+    dev_free(ctx, ctx->d_plans);
+    dev_free(ctx, ctx->d_gscratch);
     if (ctx->h_need_max) cudaFreeHost(ctx->h_need_max);
     drop_graphs(ctx);
     for (auto& sn : ctx->snaps) {

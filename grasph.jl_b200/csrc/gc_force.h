@@ -85,10 +85,10 @@ __host__ __device__ inline int group_count(int2 g) { return g.y & 63; }
 __host__ __device__ inline int group_inst(int2 g) { return g.y >> 6; }
 
 int launch_force_f64(const ForceArgs& A, bool count_only, cudaStream_t s);
-void launch_groups_count(const GridInst* gi, int ninst, int nd, const int32_t* cs, int64_t ncols_cap,
-                         int64_t cells_cap, int32_t* cnt, cudaStream_t s);
-void launch_groups_fill(const GridInst* gi, int ninst, int nd, const int32_t* cs, const int32_t* off,
-                        int64_t ncols_cap, int64_t cells_cap, int2* groups, int64_t* ngroups, cudaStream_t s);
+// Warp groups of the columns of a grid into groups[0, *ngroups).  scratch: two
+// words, zero between launches.
+void launch_groups(const GridInst* gi, int ninst, int nd, const int32_t* cs, int64_t ncols_cap, int64_t cells_cap,
+                   int2* groups, int64_t* ngroups, unsigned long long* scratch, cudaStream_t s);
 // Mode of a functor's records.
 __host__ __device__ constexpr int aux_mode(int pfn) {
     return pfn == GC_PFN_FLUID || pfn == PFN_FLUID2 ? AUX_P_OVER_RHO2

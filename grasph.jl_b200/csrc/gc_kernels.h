@@ -88,38 +88,61 @@ struct GridPlanArgs {
     int* keep;
 };
 void launch_grid_plan(const GridPlanArgs& a, cudaStream_t s);
-// The plans of n interactions (device array of arguments), one block each.
-void launch_grid_plan_all(const GridPlanArgs* d_args, int n, cudaStream_t s);
+// One entry of a step's plans (launch_plan_all): what entry i of `need` asks
+// for, and the ghost sets to bound first.
+struct GhostBound {
+    const GhostInst* gh;
+    const SysInst* src;  // the source's boxes
+    SysInst* inst;       // the ghosts' (bounds written)
+    int nd, nplanes;
+};
+enum { PLAN_NONE = 0, PLAN_SORT = 1, PLAN_GRID = 2 };
+struct PlanItem {
+    int kind;
+    SysInst* inst;  // PLAN_SORT
+    int nd;
+    GridPlanArgs grid;  // PLAN_GRID
+    int nbound;
+    GhostBound bound[2];
+};
+constexpr int PLAN_MAX = 256;  // entries per launch
+struct PlanMask {
+    uint64_t w[PLAN_MAX / 64];  // which sorts to plan
+};
+// need_max, need_cap: capacity mode (nullptr otherwise).
+void launch_plan_all(const PlanItem* items, int n, int ninst, const PlanMask& mask, int64_t* need, int64_t* need_max,
+                     const int64_t* need_cap, int* err, cudaStream_t s);
 // cell histogram of the particles of one slot on an interaction's grid
 // (skip: optional device flag; when set, the launch returns at once).
 void launch_grid_count(const double* x, int64_t N, int nd, const int32_t* inst_of, const int64_t* count,
                        const GridInst* gi, int32_t* hist, int64_t cells_cap, int* err,
                        unsigned long long* incons, cudaStream_t s, const int* skip = nullptr);
-// The grids of the interactions whose system_b does not move, counted and
-// scanned in one launch each: entry y of the table is interaction y's CSR,
-// counted into its own histogram (zero between uses; the scan clears it)
-// and skipped on the device while keep[1] is set.  cells <= STILL_MAX_CELLS.
-constexpr int STILL_MAX = 16;
-constexpr int64_t STILL_MAX_CELLS = 2048LL * 2048LL;
-struct StillGrid {
+// A step's grids, counted and scanned in one launch each: entry y of the
+// table is an interaction's CSR, counted into its own histogram (zero between
+// uses; the scan clears it) and skipped on the device while keep[1] is set.
+constexpr int GRIDS_MAX = 16;
+constexpr int64_t GRIDS_MAX_CELLS = 2048LL * 2048LL;
+struct GridBuild {
     const double* x;
     const int32_t* inst_of;
-    int64_t N;      // system_b's particles
+    int64_t N;             // system_b's particles (capacity of a ghost set)
+    const int64_t* count;  // ghosts: their count, else nullptr
     const GridInst* gi;
-    const int* keep;
-    int32_t* hist;  // cells entries, then the scan's tile sums
-    int32_t* cs;    // CSR, cells + 1 entries
+    const int* keep;       // a system_b that does not move, else nullptr
+    int32_t* hist;         // cells entries
+    int32_t* sums;         // the scan's tile sums (grid_scan_tiles(cells) entries)
+    int32_t* cs;           // CSR, cells + 1 entries
     int64_t cells;
 };
-struct StillGridArgs {
-    StillGrid g[STILL_MAX];
+struct GridBuildArgs {
+    GridBuild g[GRIDS_MAX];
     int n, nd;
     int* err;
     unsigned long long* incons;
+    int count0[GRIDS_MAX + 1], scan0[GRIDS_MAX + 1];  // first blocks of the entries (launch_grids)
 };
-// Tile sums after the histogram's cells: entries of hist beyond cells.
-int64_t still_hist_elems(int64_t cells);
-void launch_still_grids(const StillGridArgs& a, cudaStream_t s);
+int64_t grid_scan_tiles(int64_t cells);
+void launch_grids(GridBuildArgs& a, cudaStream_t s);
 
 // ---------------------------------------------------------------- ghosts
 struct GhostGenArgs {

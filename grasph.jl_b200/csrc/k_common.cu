@@ -421,8 +421,39 @@ void launch_bbox(const double* x, int64_t N, int nd, const int32_t* inst_of, con
 }
 
 // ================================================================== sort
-__global__ void k_sort_plan(SysInst* inst, int ninst, int nd, int64_t* need, int* err) {
-    pdl_enter();
+// set(k, exclusive prefix sum of get over [0, n)) by the whole block, which
+// returns the total.
+template <class Get, class Set>
+__device__ int64_t block_bases(int n, Get get, Set set) {
+    __shared__ int64_t wsum[32];
+    __shared__ int64_t carry;
+    const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5, nw = blockDim.x >> 5;
+    if (threadIdx.x == 0) carry = 0;
+    for (int k0 = 0; k0 < n; k0 += blockDim.x) {
+        const int k = k0 + threadIdx.x;
+        const int64_t v = k < n ? get(k) : 0;
+        int64_t x = v;
+#pragma unroll
+        for (int o = 1; o < 32; o <<= 1) {
+            const int64_t y = __shfl_up_sync(0xffffffffu, x, o);
+            if (lane >= o) x += y;
+        }
+        if (lane == 31) wsum[wid] = x;
+        __syncthreads();
+        int64_t base = carry;
+        for (int w = 0; w < wid; ++w) base += wsum[w];
+        if (k < n) set(k, base + x - v);
+        __syncthreads();
+        if (threadIdx.x == 0)
+            for (int w = 0; w < nw; ++w) carry += wsum[w];
+        __syncthreads();
+    }
+    __syncthreads();
+    return carry;
+}
+
+// Per-instance key lattice from the bbox; *need the total cells.
+__device__ void sort_plan_block(SysInst* inst, int ninst, int nd, int64_t* need, int* err) {
     for (int k = threadIdx.x; k < ninst; k += blockDim.x) {
         SysInst& S = inst[k];
         int64_t cells = S.n > 0 ? 1 : 0;
@@ -444,18 +475,21 @@ __global__ void k_sort_plan(SysInst* inst, int ninst, int nd, int64_t* need, int
         S.sort_ncells = cells;
     }
     __syncthreads();
-    if (threadIdx.x == 0) {
-        int64_t base = 0;
-        for (int k = 0; k < ninst; ++k) {
-            inst[k].sort_cellbase = base;
-            base += inst[k].sort_ncells;
-        }
-        *need = base;
-    }
+    const int64_t total = block_bases(
+        ninst, [&](int k) { return inst[k].sort_ncells; }, [&](int k, int64_t b) { inst[k].sort_cellbase = b; });
+    if (threadIdx.x == 0) *need = total;
+}
+
+// A block of the plan kernels: its threads cover the instances.
+static int plan_threads(int ninst) { return std::min(1024, (ninst + 31) / 32 * 32); }
+
+__global__ void k_sort_plan(SysInst* inst, int ninst, int nd, int64_t* need, int* err) {
+    pdl_enter();
+    sort_plan_block(inst, ninst, nd, need, err);
 }
 
 void launch_sort_plan(SysInst* inst, int ninst, int nd, int64_t* need, int* err, cudaStream_t s) {
-    k_sort_plan<<<1, 1024, 0, s>>>(inst, ninst, nd, need, err);
+    k_sort_plan<<<1, plan_threads(ninst), 0, s>>>(inst, ninst, nd, need, err);
     COUNTED(1);
 }
 
@@ -787,18 +821,6 @@ void launch_gather_i32(const int32_t* src, int32_t* dst, int64_t N, const int32_
 // ================================================================== grid
 // src/Interaction.jl:131-193: origin snapped to a multiple of the cell
 // size below min−2h, ngridx = floor((max+2h − origin)/h2) + 1.
-__device__ void grid_plan_block(const GridPlanArgs& a);
-__global__ void k_grid_plan(GridPlanArgs a) {
-    pdl_enter(); grid_plan_block(a); }
-__global__ void k_grid_plan_all(const GridPlanArgs* __restrict__ args) {
-    pdl_enter(); grid_plan_block(args[blockIdx.x]); }
-
-void launch_grid_plan_all(const GridPlanArgs* d_args, int n, cudaStream_t s) {
-    if (n <= 0) return;
-    k_grid_plan_all<<<n, 1024, 0, s>>>(d_args);
-    COUNTED(1);
-}
-
 __device__ void grid_plan_block(const GridPlanArgs& a) {
     for (int k = threadIdx.x; k < a.ninst; k += blockDim.x) {
         GridInst& G = a.gi[k];
@@ -846,16 +868,11 @@ __device__ void grid_plan_block(const GridPlanArgs& a) {
         G.ncols = cells / G.ng[a.nd - 1];
     }
     __syncthreads();
-    if (threadIdx.x == 0) {
-        int64_t base = 0, cb = 0;
-        for (int k = 0; k < a.ninst; ++k) {
-            a.gi[k].cellbase = base;
-            a.gi[k].colbase = cb;
-            base += a.gi[k].ncells;
-            cb += a.gi[k].ncols;
-        }
-        *a.need = base;
-    }
+    block_bases(
+        a.ninst, [&](int k) { return a.gi[k].ncols; }, [&](int k, int64_t b) { a.gi[k].colbase = b; });
+    const int64_t total = block_bases(
+        a.ninst, [&](int k) { return a.gi[k].ncells; }, [&](int k, int64_t b) { a.gi[k].cellbase = b; });
+    if (threadIdx.x == 0) *a.need = total;
     if (a.gi_b) {
         // the system_b-side copy keeps its own neighbour mass and sound speed
         __syncthreads();
@@ -894,8 +911,75 @@ __device__ void grid_plan_block(const GridPlanArgs& a) {
     }
 }
 
+__global__ void k_grid_plan(GridPlanArgs a) {
+    pdl_enter();
+    grid_plan_block(a);
+}
+
 void launch_grid_plan(const GridPlanArgs& a, cudaStream_t s) {
-    k_grid_plan<<<1, 1024, 0, s>>>(a);
+    k_grid_plan<<<1, plan_threads(a.ninst), 0, s>>>(a);
+    COUNTED(1);
+}
+
+// Conservative ghost extent before generation: the reflection of the source
+// bounding box's corners across every plane, padded by one cell.
+__device__ void ghost_bound_block(const GhostBound& g, int ninst) {
+    for (int k = threadIdx.x; k < ninst; k += blockDim.x) {
+        const SysInst& S = g.src[k];
+        double lo[MAXD], hi[MAXD];
+        for (int d = 0; d < g.nd; ++d) {
+            lo[d] = 1e300;
+            hi[d] = -1e300;
+        }
+        const int ncorner = 1 << g.nd;
+        for (int b = 0; b < g.nplanes; ++b)
+            for (int cI = 0; cI < ncorner; ++cI) {
+                double x[MAXD], da = 0.0;
+                for (int d = 0; d < g.nd; ++d) x[d] = (cI >> d) & 1 ? S.bbmax[d] : S.bbmin[d];
+                for (int d = 0; d < g.nd; ++d) da += (x[d] - g.gh[k].points[b][d]) * g.gh[k].normals[b][d];
+                for (int d = 0; d < g.nd; ++d) {
+                    const double r = x[d] - 2.0 * da * g.gh[k].normals[b][d];
+                    lo[d] = fmin(lo[d], fmin(r, x[d]));
+                    hi[d] = fmax(hi[d], fmax(r, x[d]));
+                }
+            }
+        const double pad = 2.0 * S.sort_cutoff;
+        for (int d = 0; d < g.nd; ++d) {
+            g.inst[k].bbmin[d] = lo[d] - pad;
+            g.inst[k].bbmax[d] = hi[d] + pad;
+        }
+        g.inst[k].n = S.n;  // upper bound on the count, used only for planning
+    }
+    __syncthreads();
+}
+
+// Every plan of a step in one launch, a block per entry of `need`: a sort, a
+// ghost set's bound and sort, or an interaction's grid (which bounds the
+// ghosts that it reads itself: every block writes the same values), then the
+// largest plan so far and the check against the capacity.  One launch in
+// place of a clear, a launch per sorted system and ghost set, the grids' and
+// the check's: each took about 2 us of the step's chain.
+__global__ void k_plan_all(const PlanItem* __restrict__ items, int ninst, PlanMask mask, int64_t* need,
+                           int64_t* need_max, const int64_t* need_cap, int* err) {
+    pdl_enter();
+    const int i = blockIdx.x;
+    const PlanItem& it = items[i];
+    if (threadIdx.x == 0) need[i] = 0;
+    __syncthreads();
+    for (int q = 0; q < it.nbound; ++q) ghost_bound_block(it.bound[q], ninst);
+    if (it.kind == PLAN_SORT && (mask.w[i >> 6] >> (i & 63) & 1)) sort_plan_block(it.inst, ninst, it.nd, need + i, err);
+    if (it.kind == PLAN_GRID) grid_plan_block(it.grid);
+    if (need_max && threadIdx.x == 0) {
+        const int64_t n = need[i];
+        if (n > need_max[i]) need_max[i] = n;
+        if (n > need_cap[i]) atomicOr(err, ERR_CAPACITY);
+    }
+}
+
+void launch_plan_all(const PlanItem* items, int n, int ninst, const PlanMask& mask, int64_t* need, int64_t* need_max,
+                     const int64_t* need_cap, int* err, cudaStream_t s) {
+    if (n <= 0) return;
+    k_plan_all<<<n, plan_threads(ninst), 0, s>>>(items, ninst, mask, need, need_max, need_cap, err);
     COUNTED(1);
 }
 
@@ -976,31 +1060,42 @@ void launch_grid_count(const double* x, int64_t N, int nd, const int32_t* inst_o
     COUNTED(1);
 }
 
-// ------------------------------------------------ still grids, batched
-// Every interaction whose system_b does not move recounts its CSR only when
-// its grid's geometry changed (keep[1], set by the plan).  Their counts and
-// scans run as one launch each over a table of interactions (blockIdx.y),
-// with a few blocks per interaction striding over the work: on the usual
-// step every block returns at once, and separate launches of one block per
-// tile would cost more in launch latency than the work they skip.
-int64_t still_hist_elems(int64_t cells) { return cells + (cells + SCAN_TILE - 1) / SCAN_TILE + 1; }
+// ------------------------------------------------------ grids, batched
+// The step's grids are counted and scanned together, three launches for all
+// of them: entry y of the table is an interaction's CSR, counted into its
+// own histogram, and its blocks follow those of the entry before it.  An
+// interaction whose system_b does not move recounts its CSR only when its
+// grid's geometry changed (keep[1], set by the plan): its few blocks return
+// at once on the usual step.
+int64_t grid_scan_tiles(int64_t cells) { return (cells + SCAN_TILE - 1) / SCAN_TILE; }
 
-__global__ void k_still_count(const __grid_constant__ StillGridArgs a) {
-    pdl_enter();
-    const StillGrid& g = a.g[blockIdx.y];
-    if (g.keep[1]) return;
-    grid_count_blocks(g.x, g.N, a.nd, g.inst_of, nullptr, g.gi, g.hist, g.cells, a.err, a.incons, blockIdx.x,
-                      gridDim.x);
+// The entry of a block, and the block's number and the number of blocks in it.
+__device__ __forceinline__ const GridBuild& grid_of_block(const GridBuildArgs& a, const int* first, int64_t& bid,
+                                                          int64_t& nblocks) {
+    int y = 0;
+    while (y + 1 < a.n && (int)blockIdx.x >= first[y + 1]) ++y;
+    bid = blockIdx.x - first[y];
+    nblocks = first[y + 1] - first[y];
+    return a.g[y];
 }
 
-// Tile sums of each histogram, after its cells.
-__global__ void k_still_scan_reduce(const __grid_constant__ StillGridArgs a) {
+__global__ void k_grids_count(const __grid_constant__ GridBuildArgs a) {
     pdl_enter();
-    const StillGrid& g = a.g[blockIdx.y];
-    if (g.keep[1]) return;
+    int64_t bid, nblocks;
+    const GridBuild& g = grid_of_block(a, a.count0, bid, nblocks);
+    if (g.keep && g.keep[1]) return;
+    grid_count_blocks(g.x, g.N, a.nd, g.inst_of, g.count, g.gi, g.hist, g.cells, a.err, a.incons, bid, nblocks);
+}
+
+// Tile sums of each histogram.
+__global__ void k_grids_scan_reduce(const __grid_constant__ GridBuildArgs a) {
+    pdl_enter();
+    int64_t bid, nblocks;
+    const GridBuild& g = grid_of_block(a, a.scan0, bid, nblocks);
+    if (g.keep && g.keep[1]) return;
     const int64_t nb = (g.cells + SCAN_TILE - 1) / SCAN_TILE;
-    int32_t* bsum = g.hist + g.cells;
-    for (int64_t b = blockIdx.x; b < nb; b += gridDim.x) {
+    int32_t* bsum = g.sums;
+    for (int64_t b = bid; b < nb; b += nblocks) {
         const int64_t t0 = b * SCAN_TILE + (int64_t)threadIdx.x * SCAN_I;
         int32_t s = 0;
 #pragma unroll
@@ -1014,14 +1109,15 @@ __global__ void k_still_scan_reduce(const __grid_constant__ StillGridArgs a) {
 
 // Exclusive scan of each histogram into its CSR (cells + 1 entries), the
 // histogram cleared as it is read; each tile adds up the sums before it.
-__global__ void k_still_scan_apply(const __grid_constant__ StillGridArgs a) {
+__global__ void k_grids_scan_apply(const __grid_constant__ GridBuildArgs a) {
     pdl_enter();
-    const StillGrid& g = a.g[blockIdx.y];
-    if (g.keep[1]) return;
+    int64_t bid, nblocks;
+    const GridBuild& g = grid_of_block(a, a.scan0, bid, nblocks);
+    if (g.keep && g.keep[1]) return;
     const int64_t n = g.cells;
     const int64_t nb = (n + SCAN_TILE - 1) / SCAN_TILE;
-    const int32_t* bsum = g.hist + n;
-    for (int64_t b = blockIdx.x; b < nb; b += gridDim.x) {
+    const int32_t* bsum = g.sums;
+    for (int64_t b = bid; b < nb; b += nblocks) {
         int32_t off;
         {
             int32_t s = 0;
@@ -1050,18 +1146,22 @@ __global__ void k_still_scan_apply(const __grid_constant__ StillGridArgs a) {
     }
 }
 
-void launch_still_grids(const StillGridArgs& a, cudaStream_t s) {
+void launch_grids(GridBuildArgs& a, cudaStream_t s) {
     if (a.n <= 0) return;
-    int64_t maxN = 1, maxnb = 1;
+    a.count0[0] = a.scan0[0] = 0;
     for (int i = 0; i < a.n; ++i) {
-        maxN = std::max(maxN, a.g[i].N);
-        maxnb = std::max(maxnb, (a.g[i].cells + SCAN_TILE - 1) / SCAN_TILE);
+        // a still entry strides over its work with a few blocks: on the usual
+        // step they only start and return
+        const GridBuild& g = a.g[i];
+        const int64_t bc = std::min<int64_t>(nblk(g.N), g.keep ? 2 * 148 : 1 << 20);
+        const int64_t bs = std::min<int64_t>(std::max<int64_t>((g.cells + SCAN_TILE - 1) / SCAN_TILE, 1),
+                                             g.keep ? 148 : 1 << 20);
+        a.count0[i + 1] = a.count0[i] + (int)bc;
+        a.scan0[i + 1] = a.scan0[i] + (int)bs;
     }
-    const unsigned bc = (unsigned)std::min<int64_t>(nblk(maxN), 2 * 148);
-    const unsigned bs = (unsigned)std::min<int64_t>(maxnb, 148);
-    k_still_count<<<dim3(bc, a.n), TPB, 0, s>>>(a);
-    k_still_scan_reduce<<<dim3(bs, a.n), SCAN_T, 0, s>>>(a);
-    k_still_scan_apply<<<dim3(bs, a.n), SCAN_T, 0, s>>>(a);
+    k_grids_count<<<a.count0[a.n], TPB, 0, s>>>(a);
+    k_grids_scan_reduce<<<a.scan0[a.n], SCAN_T, 0, s>>>(a);
+    k_grids_scan_apply<<<a.scan0[a.n], SCAN_T, 0, s>>>(a);
     COUNTED(3);
 }
 

@@ -35,63 +35,69 @@ __device__ __forceinline__ int find_inst(const GridInst* gi, int ninst, int64_t 
 
 // `cells_cap`: cells of `cs` that are valid (cs holds cells_cap + 1
 // entries); an instance whose grid reaches beyond them contributes nothing
-// (the grid build has flagged the overflow).
-__global__ void k_groups_count(const GridInst* __restrict__ gi, int ninst, int nd, const int32_t* __restrict__ cs,
-                               int64_t ncols_cap, int64_t cells_cap, int32_t* __restrict__ cnt) {
+// (the grid build has flagged the overflow).  A warp takes 32 columns, adds up
+// their groups, and reserves them with one add on scratch[0]; the groups'
+// order does not matter (each is swept by itself), so no scan over the
+// columns is needed: one launch in place of four.  The last block
+// (scratch[1] counts them) writes the total and clears the scratch.
+__global__ void k_groups(const GridInst* __restrict__ gi, int ninst, int nd, const int32_t* __restrict__ cs,
+                         int64_t ncols_cap, int64_t cells_cap, int2* __restrict__ groups, int64_t* ngroups,
+                         unsigned long long* scratch) {
     pdl_enter();
-    const int64_t T = gi[ninst - 1].colbase + gi[ninst - 1].ncols;
-    for (int64_t c = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; c < ncols_cap;
-         c += (int64_t)gridDim.x * blockDim.x) {
-        if (c >= T) {
-            cnt[c] = 0;
-            continue;
+    const unsigned FULL = 0xffffffffu;
+    const int lane = threadIdx.x & 31;
+    const int64_t all = gi[ninst - 1].colbase + gi[ninst - 1].ncols;
+    const int64_t T = all < ncols_cap ? all : ncols_cap;
+    const int64_t nwarps = ((int64_t)gridDim.x * blockDim.x) >> 5;
+    for (int64_t c0 = (((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5) * 32; c0 < T; c0 += nwarps * 32) {
+        const int64_t c = c0 + lane;
+        int k = 0;
+        int32_t s0 = 0, n = 0;
+        if (c < T) {
+            k = find_inst(gi, ninst, c);
+            const GridInst& G = gi[k];
+            if (G.cellbase + G.ncells <= cells_cap) {
+                const int64_t ngl = G.ng[nd - 1];
+                const int64_t b = G.cellbase + (c - G.colbase) * ngl;
+                s0 = cs[b];
+                n = cs[b + ngl] - s0;
+            }
         }
-        const GridInst& G = gi[find_inst(gi, ninst, c)];
-        const int64_t ngl = G.ng[nd - 1];
-        const int64_t local = c - G.colbase;
-        const int64_t b = G.cellbase + local * ngl;
-        if (G.cellbase + G.ncells > cells_cap) {
-            cnt[c] = 0;
-            continue;
+        const int32_t m = (n + 31) / 32;
+        int32_t at = m;
+#pragma unroll
+        for (int o = 1; o < 32; o <<= 1) {
+            const int32_t y = __shfl_up_sync(FULL, at, o);
+            if (lane >= o) at += y;
         }
-        const int32_t n = cs[b + ngl] - cs[b];
-        cnt[c] = (n + 31) / 32;
+        const int32_t total = __shfl_sync(FULL, at, 31);
+        unsigned long long base = 0;
+        if (lane == 0 && total > 0) base = atomicAdd(&scratch[0], (unsigned long long)total);
+        const int64_t first = (int64_t)__shfl_sync(FULL, base, 0) + at - m;
+        for (unsigned left = __ballot_sync(FULL, m > 0); left; left &= left - 1) {
+            const int l = __ffs(left) - 1;
+            const int64_t o = __shfl_sync(FULL, first, l);
+            const int32_t sl = __shfl_sync(FULL, s0, l), nl = __shfl_sync(FULL, n, l), ml = __shfl_sync(FULL, m, l);
+            const int kl = __shfl_sync(FULL, k, l);
+            for (int32_t q = lane; q < ml; q += 32)
+                groups[o + q] = group_of(sl + 32 * q, nl - 32 * q < 32 ? nl - 32 * q : 32, kl);
+        }
+    }
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        __threadfence();
+        if (atomicAdd(&scratch[1], 1ull) == gridDim.x - 1) {
+            *ngroups = (int64_t)atomicExch(&scratch[0], 0ull);
+            scratch[1] = 0ull;
+        }
     }
 }
 
-__global__ void k_groups_fill(const GridInst* __restrict__ gi, int ninst, int nd, const int32_t* __restrict__ cs,
-                              const int32_t* __restrict__ off, int64_t ncols_cap, int64_t cells_cap,
-                              int2* __restrict__ groups, int64_t* ngroups) {
-    pdl_enter();
-    const int64_t T = gi[ninst - 1].colbase + gi[ninst - 1].ncols;
-    for (int64_t c = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; c < T && c < ncols_cap;
-         c += (int64_t)gridDim.x * blockDim.x) {
-        const int k = find_inst(gi, ninst, c);
-        const GridInst& G = gi[k];
-        if (G.cellbase + G.ncells > cells_cap) continue;
-        const int64_t ngl = G.ng[nd - 1];
-        const int64_t local = c - G.colbase;
-        const int64_t b = G.cellbase + local * ngl;
-        const int32_t s0 = cs[b], n = cs[b + ngl] - s0;
-        int32_t o = off[c];
-        for (int32_t q = 0; q < n; q += 32) groups[o++] = group_of(s0 + q, n - q < 32 ? n - q : 32, k);
-    }
-    if (blockIdx.x == 0 && threadIdx.x == 0) *ngroups = off[ncols_cap];
-}
-
-void launch_groups_count(const GridInst* gi, int ninst, int nd, const int32_t* cs, int64_t ncols_cap,
-                         int64_t cells_cap, int32_t* cnt, cudaStream_t s) {
+void launch_groups(const GridInst* gi, int ninst, int nd, const int32_t* cs, int64_t ncols_cap, int64_t cells_cap,
+                   int2* groups, int64_t* ngroups, unsigned long long* scratch, cudaStream_t s) {
     int64_t b = (ncols_cap + 255) / 256;
-    if (b < 1) b = 1;
-    k_groups_count<<<(int)b, 256, 0, s>>>(gi, ninst, nd, cs, ncols_cap, cells_cap, cnt);
-    g_launches.fetch_add(1, std::memory_order_relaxed);
-}
-
-void launch_groups_fill(const GridInst* gi, int ninst, int nd, const int32_t* cs, const int32_t* off,
-                        int64_t ncols_cap, int64_t cells_cap, int2* groups, int64_t* ngroups, cudaStream_t s) {
-    int64_t b = (ncols_cap + 255) / 256;
-    if (b < 1) b = 1;
-    k_groups_fill<<<(int)b, 256, 0, s>>>(gi, ninst, nd, cs, off, ncols_cap, cells_cap, groups, ngroups);
+    b = b < 1 ? 1 : b > 2 * 148 ? 2 * 148 : b;
+    k_groups<<<(int)b, 256, 0, s>>>(gi, ninst, nd, cs, ncols_cap, cells_cap, groups, ngroups, scratch);
     g_launches.fetch_add(1, std::memory_order_relaxed);
 }
 
