@@ -3447,7 +3447,8 @@ int gc_upload_field(gc_ctx* ctx, int inst, int handle, int field, const void* ho
     return gc_upload_fields(ctx, 1, &f);
 }
 
-int gc_download_fields(gc_ctx* ctx, int nio, const gc_field_io* io) {
+// f32: the fields to round to FP32 on the device (nullptr: none).
+static int download_fields(gc_ctx* ctx, int nio, const gc_field_io* io, const unsigned char* f32) {
     if (!ctx || nio < 0 || (nio && !io)) return GC_ERR_ARG;
     std::vector<HandleRef> ref(nio);
     std::vector<int> comps(nio);
@@ -3456,6 +3457,9 @@ int gc_download_fields(gc_ctx* ctx, int nio, const gc_field_io* io) {
         const gc_field_io& f = io[q];
         if (!f.host) return seterr(ctx, GC_ERR_ARG, "null host buffer");
         TRY(resolve(ctx, f.inst, f.handle, &ref[q]));
+        const bool narrow = f32 && f32[q];
+        if (narrow && (ref[q].ghost || ref[q].virt || f.field == GC_FIELD_ID))
+            return seterr(ctx, GC_ERR_ARG, "only a particle system's real fields are downloaded in FP32");
         if (ref[q].ghost) continue;
         const HSys& hs = ctx->inst[f.inst].sys[ref[q].sys];
         if (ref[q].virt && (f.field == GC_FIELD_W_SUM || !ref[q].slot)) {
@@ -3468,7 +3472,7 @@ int gc_download_fields(gc_ctx* ctx, int nio, const gc_field_io* io) {
         }
         comps[q] = sys_comps(hs, f.field);
         if (comps[q] < 0) return seterr(ctx, GC_ERR_ARG, "field %d not present on this system", f.field);
-        if (f.bytes != (size_t)(hs.n * comps[q] * 8))
+        if (f.bytes != (size_t)(hs.n * comps[q] * (narrow ? 4 : 8)))
             return seterr(ctx, GC_ERR_ARG, "byte count mismatch (%zu)", f.bytes);
         total += hs.n * comps[q];
     }
@@ -3491,6 +3495,8 @@ int gc_download_fields(gc_ctx* ctx, int nio, const gc_field_io* io) {
         }
         if (n == 0) continue;
         if (f.field == GC_FIELD_ID) launch_i32_to_i64(S.id[S.cur] + base, (int64_t*)st, n, ctx->stream);
+        else if (f32 && f32[q])
+            launch_planar_to_aos(S.F(field_slot(f.field)), (float*)st, n, comps[q], S.N, base, ctx->stream);
         else launch_planar_to_aos(S.F(field_slot(f.field)), st, n, comps[q], S.N, base, ctx->stream);
         CU(cudaMemcpyAsync(f.host, st, f.bytes, cudaMemcpyDeviceToHost, ctx->stream));
     }
@@ -3499,6 +3505,12 @@ int gc_download_fields(gc_ctx* ctx, int nio, const gc_field_io* io) {
     for (int q = 0; q < nio; ++q)
         if (ref[q].ghost) TRY(ghost_field_io(ctx, io[q].inst, *ref[q].ghost, io[q].field, io[q].host, io[q].bytes));
     return GC_OK;
+}
+
+int gc_download_fields(gc_ctx* ctx, int nio, const gc_field_io* io) { return download_fields(ctx, nio, io, nullptr); }
+
+int gc_download_fields_as(gc_ctx* ctx, int nio, const gc_field_io* io, const unsigned char* f32) {
+    return download_fields(ctx, nio, io, f32);
 }
 
 int gc_download_field(gc_ctx* ctx, int inst, int handle, int field, void* host, size_t bytes) {

@@ -174,6 +174,9 @@ void launch_aos_to_planar(const double* src, double* dst, int64_t n, int comps, 
                           cudaStream_t s);
 void launch_planar_to_aos(const double* src, double* dst, int64_t n, int comps, int64_t N, int64_t base,
                           cudaStream_t s);
+// (rounded to FP32)
+void launch_planar_to_aos(const double* src, float* dst, int64_t n, int comps, int64_t N, int64_t base,
+                          cudaStream_t s);
 void launch_i64_to_i32(const int64_t* src, int32_t* dst, int64_t n, cudaStream_t s);
 void launch_i32_to_i64(const int32_t* src, int64_t* dst, int64_t n, cudaStream_t s);
 

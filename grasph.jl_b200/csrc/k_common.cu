@@ -1354,14 +1354,15 @@ __global__ void k_aos_to_planar(const double* __restrict__ src, double* __restri
         dst[c * N + base + i] = src[t];
     }
 }
-__global__ void k_planar_to_aos(const double* __restrict__ src, double* __restrict__ dst, int64_t n, int comps,
-                                int64_t N, int64_t base) {
+template <class T>
+__global__ void k_planar_to_aos(const double* __restrict__ src, T* __restrict__ dst, int64_t n, int comps, int64_t N,
+                                int64_t base) {
     pdl_enter();
     for (int64_t t = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; t < n * comps;
          t += (int64_t)gridDim.x * blockDim.x) {
         int64_t i = t / comps;
         int c = (int)(t - i * comps);
-        dst[t] = src[c * N + base + i];
+        dst[t] = (T)src[c * N + base + i];
     }
 }
 __global__ void k_i64_to_i32(const int64_t* __restrict__ src, int32_t* __restrict__ dst, int64_t n) {
@@ -1383,13 +1384,19 @@ void launch_aos_to_planar(const double* src, double* dst, int64_t n, int comps, 
     k_aos_to_planar<<<b, TPB, 0, s>>>(src, dst, n, comps, N, base);
     COUNTED(1);
 }
+template <class T>
+static void planar_to_aos(const double* src, T* dst, int64_t n, int comps, int64_t N, int64_t base, cudaStream_t s) {
+    if (n <= 0) return;
+    k_planar_to_aos<<<std::min(nblk(n * comps), 148 * 32), TPB, 0, s>>>(src, dst, n, comps, N, base);
+    COUNTED(1);
+}
 void launch_planar_to_aos(const double* src, double* dst, int64_t n, int comps, int64_t N, int64_t base,
                           cudaStream_t s) {
-    if (n <= 0) return;
-    int b = nblk(n * comps);
-    if (b > 148 * 32) b = 148 * 32;
-    k_planar_to_aos<<<b, TPB, 0, s>>>(src, dst, n, comps, N, base);
-    COUNTED(1);
+    planar_to_aos(src, dst, n, comps, N, base, s);
+}
+void launch_planar_to_aos(const double* src, float* dst, int64_t n, int comps, int64_t N, int64_t base,
+                          cudaStream_t s) {
+    planar_to_aos(src, dst, n, comps, N, base, s);
 }
 void launch_i64_to_i32(const int64_t* src, int32_t* dst, int64_t n, cudaStream_t s) {
     if (n <= 0) return;

@@ -113,6 +113,7 @@ def load_library(path: os.PathLike | None = None):
         "gc_set_sweep_config": (ct.c_int, [ct.c_void_p, ct.c_int]),
         "gc_upload_fields": (ct.c_int, [ct.c_void_p, ct.c_int, ct.c_void_p]),
         "gc_download_fields": (ct.c_int, [ct.c_void_p, ct.c_int, ct.c_void_p]),
+        "gc_download_fields_as": (ct.c_int, [ct.c_void_p, ct.c_int, ct.c_void_p, ct.c_void_p]),
         "gc_stage_field": (ct.c_int, [ct.c_void_p, ct.c_int, ct.c_int, ct.c_int, ct.c_void_p, ct.c_size_t]),
         "gc_serve_create": (ct.c_int, [ct.c_int, ct.c_size_t, ct.c_int, ct.c_int, ct.POINTER(ct.c_void_p)]),
         "gc_serve_destroy": (ct.c_int, [ct.c_void_p]),
@@ -270,12 +271,14 @@ class CudaBackend:
         self._chk(self.lib.gc_upload_fields(self.ctx, len(items), arr), "gc_upload_fields")
 
     def download_many(self, items):
-        """items: (inst, handle, field, out_array) tuples, filled in place."""
+        """items: (inst, handle, field, out_array) tuples, filled in place (a
+        Float32 array with the field rounded to Float32 on the device)."""
         arr = (FieldIO * max(len(items), 1))()
+        f32 = bytes(a.dtype == np.float32 for *_, a in items)
         for q, (inst, h, f, a) in enumerate(items):
             assert a.flags["C_CONTIGUOUS"]
             arr[q] = FieldIO(inst, h, f, 0, a.ctypes.data, a.nbytes)
-        self._chk(self.lib.gc_download_fields(self.ctx, len(items), arr), "gc_download_fields")
+        self._chk(self.lib.gc_download_fields_as(self.ctx, len(items), arr, f32), "gc_download_fields")
 
     def download_into(self, inst, handle, field, out):
         self._chk(self.lib.gc_download_field(self.ctx, inst, handle, field, out.ctypes.data, out.nbytes),
@@ -492,33 +495,63 @@ def upload_instance(backend, m: InstanceMap, systems=None):
             backend.upload(inst, h, fid, a)
 
 
-def download_instance(backend, m: InstanceMap, with_ghosts=True, systems=None):
-    items, narrow = [], []
-    for ps in m.systems:
-        if systems is not None and not any(ps is q for q in systems):
-            continue
-        for name, fid in ps.particle_fields():
-            a = getattr(ps, name)
-            if a.dtype == np.float32:
-                # downloaded in Float64, rounded to the system's Float32
-                w = np.empty(a.shape)
-                narrow.append((a, w))
-                a = w
-            items.append((m.inst, m.h(ps), fid, a))
-    if hasattr(backend, "download_many"):
+def _download_systems(backend, maps, systems=None):
+    """Every field of every system (or of `systems` only) of the instances."""
+    if not hasattr(backend, "download_many"):
+        for m in maps:
+            for ps in m.systems:
+                if systems is not None and not any(ps is q for q in systems):
+                    continue
+                for name, fid in ps.particle_fields():
+                    a = getattr(ps, name)
+                    if a.dtype == np.float32:
+                        # downloaded in Float64, rounded to the system's Float32
+                        a[...] = backend.download_into(m.inst, m.h(ps), fid, np.empty(a.shape))
+                    else:
+                        backend.download_into(m.inst, m.h(ps), fid, a)
+        return
+    # as many instances a call as DOWNLOAD_BYTES of fields hold: one device
+    # synchronisation for all of them, and a bounded staging buffer
+    wanted = None if systems is None else {id(ps) for ps in systems}
+    items, held, apart = [], 0, []
+    for m in maps:
+        for ps in m.systems:
+            if wanted is not None and id(ps) not in wanted:
+                continue
+            fields = [(m.inst, m.h(ps), fid, getattr(ps, name)) for name, fid in ps.particle_fields()]
+            for q, (inst, h, fid, a) in enumerate(fields):
+                if a.dtype == np.float32 and not a.flags["C_CONTIGUOUS"]:
+                    apart.append((a, np.empty(a.shape, np.float32)))
+                    fields[q] = (inst, h, fid, apart[-1][1])
+            size = sum(a.size for *_, a in fields) * 8
+            if items and held + size > DOWNLOAD_BYTES:
+                backend.download_many(items)
+                items, held = [], 0
+            items += fields
+            held += size
+    if items:
         backend.download_many(items)
-    else:
-        for inst, h, fid, a in items:
-            backend.download_into(inst, h, fid, a)
-    for a, w in narrow:
+    for a, w in apart:
         a[...] = w
+
+
+DOWNLOAD_BYTES = 256 << 20
+
+
+def download_instance(backend, m: InstanceMap, with_ghosts=True, systems=None):
+    _download_systems(backend, [m], systems)
     if with_ghosts:
-        for ge in m.ghosts:
-            download_ghost(backend, m, ge)
-        for vps in m.virtuals:
-            backend.download_into(m.inst, m.h(vps), C.GC_FIELD_W_SUM, vps.w_sum)
-        for pr in m.probes:
-            download_probe(backend, m, pr)
+        _download_derived(backend, m)
+
+
+def _download_derived(backend, m: InstanceMap):
+    """The ghosts, the virtual systems' w_sum and the probes of an instance."""
+    for ge in m.ghosts:
+        download_ghost(backend, m, ge)
+    for vps in m.virtuals:
+        backend.download_into(m.inst, m.h(vps), C.GC_FIELD_W_SUM, vps.w_sum)
+    for pr in m.probes:
+        download_probe(backend, m, pr)
 
 
 def download_probe(backend, m: InstanceMap, pr):
@@ -597,8 +630,10 @@ class Session:
 
     def pull(self, with_ghosts=True, systems=None):
         """Download every field of every system (or of `systems` only)."""
-        for m in self.maps:
-            download_instance(self.backend, m, with_ghosts, systems)
+        _download_systems(self.backend, self.maps, systems)
+        if with_ghosts:
+            for m in self.maps:
+                _download_derived(self.backend, m)
 
     def step(self, nsteps, cfl):
         self.backend.step(nsteps, cfl)

@@ -296,6 +296,10 @@ typedef struct gc_field_io {
 } gc_field_io;
 int gc_upload_fields(gc_ctx* ctx, int n, const gc_field_io* io);
 int gc_download_fields(gc_ctx* ctx, int n, const gc_field_io* io);
+/* The same with fields rounded to Float32 on the device: where f32[q] is not
+ * zero, io[q].host is a float array and io[q].bytes its size (the real
+ * fields of particle systems only).                                       */
+int gc_download_fields_as(gc_ctx* ctx, int nio, const gc_field_io* io, const unsigned char* f32);
 /* Current particle count of a handle (ghost counts change every step).    */
 int gc_get_count(gc_ctx* ctx, int inst, int handle, int64_t* n_out);
 
