@@ -119,6 +119,7 @@ struct DSlot {
     int64_t xpk_epoch = -1;    // pack_epoch the position records were made in
     bool xpk_static = false;   // position records of a system that does not move are current
     bool xpk_fp32 = false;     // their precision
+    bool box_fresh = false;    // the boxes are those of the current positions (kept by the full step)
     bool written = false;      // some functor writes this system
     bool moving = true;        // sorted and integrated every step
     bool vsrc = false;         // source of a virtual system: never integrated
@@ -130,6 +131,7 @@ struct DSlot {
     // updaters: [stage][chain] -> per-instance UpdInst device array
     std::vector<std::vector<UpdInst*>> d_upd;
     std::vector<std::vector<int>> upd_kind;
+    std::vector<std::vector<uint32_t>> upd_zeroed;  // the fields every instance's ZERO_FIELDS zeroes
     bool upd_set = false;
     int nupd = 0;
     // the fused half step of this pack_epoch already ran the stage-1
@@ -733,6 +735,7 @@ int finalize(gc_ctx* ctx) {
         D.nupd = (int)h0.upd.size();
         D.d_upd.resize(h0.upd.size());
         D.upd_kind.resize(h0.upd.size());
+        D.upd_zeroed.resize(h0.upd.size());
         for (size_t t = 0; t < h0.upd.size(); ++t) {
             for (size_t q = 0; q < h0.upd[t].size(); ++q) {
                 std::vector<UpdInst> per(ninst);
@@ -742,6 +745,9 @@ int finalize(gc_ctx* ctx) {
                 CU(cudaMemcpyAsync(d, per.data(), ninst * sizeof(UpdInst), cudaMemcpyHostToDevice, ctx->stream));
                 D.d_upd[t].push_back(d);
                 D.upd_kind[t].push_back(h0.upd[t][q].kind);
+                uint32_t z = ~0u;
+                for (const UpdInst& u : per) z &= u.zmask;
+                D.upd_zeroed[t].push_back(z);
             }
         }
         // Host-side copies must outlive the async copies above.
@@ -1131,7 +1137,9 @@ int bbox_slot(gc_ctx* ctx, DSlot& S) {
 // Stable counting sort of `S` (or of a ghost set when G != nullptr) over
 // `cells` packed key cells (an upper bound on the planned total, which the
 // device holds at `total`).
-int sort_particles_slot(gc_ctx* ctx, DSlot* S, DGhost* G, int64_t cells, const int64_t* total) {
+// half: the gather is the fused half step's (gather_halfstep).
+int gather_halfstep(gc_ctx* ctx, DSlot& S);
+int sort_particles_slot(gc_ctx* ctx, DSlot* S, DGhost* G, int64_t cells, const int64_t* total, bool half = false) {
     const int ni = ninst(ctx);
     // The histogram and fill counters are zero on entry and left zero: the
     // scan clears what the keys counted, the fix-up what the scatter filled.
@@ -1144,6 +1152,11 @@ int sort_particles_slot(gc_ctx* ctx, DSlot* S, DGhost* G, int64_t cells, const i
         launch_sort_scatter(ctx->key, S->N, nullptr, ctx->start, ctx->fill, ctx->perm, ctx->stream, ctx->d_unsorted);
         launch_sort_fixup_clear(ctx->start, cells, total, ctx->perm, ctx->fill, ctx->stream, ctx->d_unsorted,
                                 ctx->d_sorts_in_order);
+        if (half) {
+            TRY(gather_halfstep(ctx, *S));
+            S->xpk_static = false;
+            return check_launch(ctx, "sort");
+        }
         for (int f = 0; f < NF; ++f)
             if (S->ncomp[f]) {
                 ga.src[ga.nf] = S->F(f);
@@ -1393,12 +1406,13 @@ int64_t cap_grid_cells(gc_ctx* ctx, const DInter& D) { return std::min(D.cap_cel
 // system slots are sorted.  Exact mode reads the planned cell counts back
 // to size every buffer; capacity mode sizes from the buffers' capacities
 // (no host read), and the kernels flag any plan that does not fit.
-int prepare(gc_ctx* ctx, const std::vector<char>& sort_mask) {
+// half: the moving systems' half steps are part of their sorts.
+int prepare(gc_ctx* ctx, const std::vector<char>& sort_mask, bool half) {
     const int ni = ninst(ctx);
     // bounding boxes of every real system (positions are current); a system
     // that does not move keeps the box computed after its last upload
     for (auto& S : ctx->slots)
-        if (S.xmoves() || !S.sorted_once) TRY(bbox_slot(ctx, S));
+        if ((S.xmoves() || !S.sorted_once) && !S.box_fresh) TRY(bbox_slot(ctx, S));
     for (int i0 = 0; i0 < ctx->nneed; i0 += PLAN_MAX) {
         const int n = std::min(PLAN_MAX, ctx->nneed - i0);
         PlanMask mask{};
@@ -1424,7 +1438,9 @@ int prepare(gc_ctx* ctx, const std::vector<char>& sort_mask) {
     }
     // sorts
     for (size_t s = 0; s < ctx->slots.size(); ++s)
-        if (sort_mask[s]) TRY(sort_particles_slot(ctx, &ctx->slots[s], nullptr, need[s], ctx->d_need + s));
+        if (sort_mask[s])
+            TRY(sort_particles_slot(ctx, &ctx->slots[s], nullptr, need[s], ctx->d_need + s,
+                                    half && ctx->slots[s].moving));
     // ghosts: generate, bound-checked plan, sort
     for (auto& G : ctx->ghosts) {
         TRY(generate_ghosts(ctx, G));
@@ -2127,19 +2143,41 @@ int xsph_pass(gc_ctx* ctx) {
     return check_launch(ctx, "XSPH correction");
 }
 
-// The LeapFrog half step of slot `a` fused with the stage-1 work that
-// follows it for the same particles: its stage-1 updater when that is one
-// light elementwise kind (moved here from _sweep_all_stages!, :401-419;
-// nothing between the two reads or writes what it touches) and the records
-// of the first sweep after it
-// (sweep_group then finds them packed).
-int halfstep_stage1(gc_ctx* ctx, int a) {
-    DSlot& S = ctx->slots[a];
-    UpdArgs u{};
-    u.kind = -1;
+// The LeapFrog half step of a slot fused with the gather of its sort before
+// it and the stage-1 work that follows it for the same particles: its stage-1
+// updater when that is one light elementwise kind (moved here from
+// _sweep_all_stages!, :401-419; nothing between the two reads or writes what
+// it touches) and the records of the first sweep after it (sweep_group then
+// finds them packed).  Between the sort and the half step the ghosts and the
+// grids are built, from positions alone.
+int gather_halfstep(gc_ctx* ctx, DSlot& S) {
+    const int a = (int)(&S - ctx->slots.data());
+    const StepSrc src{S.F(F_X), S.F(F_V), S.F(F_RHO), S.F(F_DVDT), S.F(F_DRHODT), S.id[S.cur], S.id[S.cur ^ 1]};
+    GatherArgs rest{};
+    rest.clear = ctx->d_unsorted;
     // a stage-1 chain of at most one light updater moves into the half step
     const bool has1 = !S.vsrc && S.upd_set && S.nupd == ctx->nstages && ctx->nstages >= 1 && !S.d_upd.empty();
     const bool upd = has1 && S.d_upd[0].size() == 1 && halfstep_fuses(S.upd_kind[0][0]);
+    // the fields that the updater overwrites need not be carried over
+    uint32_t drops = 0;
+    if (upd && (S.upd_kind[0][0] == GC_UPD_TAIT_EOS || S.upd_kind[0][0] == GC_UPD_LINEAR_EOS)) drops |= 1u << F_P;
+    if (upd && S.upd_kind[0][0] == GC_UPD_ZERO_FIELDS) {
+        const uint32_t z = S.upd_zeroed[0][0];
+        if (z >> GC_FIELD_STRAIN_RATE & 1u) drops |= 1u << F_SR;
+        if (z >> GC_FIELD_VORTICITY & 1u) drops |= 1u << F_VORT;
+        if (z >> GC_FIELD_P & 1u) drops |= 1u << F_P;
+        if (z >> GC_FIELD_STRESS & 1u) drops |= 1u << F_STRESS;
+    }
+    for (int f = 0; f < NF; ++f) {
+        if (!S.ncomp[f] || f == F_X || f == F_V || f == F_RHO || f == F_DVDT || f == F_DRHODT) continue;
+        if (drops >> f & 1u) continue;
+        rest.src[rest.nf] = S.F(f);
+        rest.dst[rest.nf] = S.A(f);
+        rest.ncomp[rest.nf++] = S.ncomp[f];
+    }
+    S.cur ^= 1;
+    UpdArgs u{};
+    u.kind = -1;
     if (upd) u = upd_args(S, 1, 0, NAN);
     PackArgs pk{};
     if (upd || !has1 || S.d_upd[0].empty()) {  // the pack follows the stage-1 updaters
@@ -2159,8 +2197,24 @@ int halfstep_stage1(gc_ctx* ctx, int a) {
             }
         }
     }
-    launch_halfstep_fused(step_args(S), u, pk, ctx->stream);
+    launch_gather_halfstep(step_args(S), src, rest, ctx->perm, u, pk, ctx->stream);
     if (upd) S.upd_fused_epoch = ctx->pack_epoch;
+    return GC_OK;
+}
+
+// Whether a LeapFrog step leaves the slot's boxes with its full step (XSPH
+// and prescribed velocities move positions after it).
+bool box_kept(gc_ctx* ctx, const DSlot& S) {
+    return ctx->inst[0].integ != GC_INTEGRATOR_RK4 && S.moving && !S.vmoves && !ctx->xsph;
+}
+
+// The boxes that captured steps take as given.
+int ensure_boxes(gc_ctx* ctx) {
+    for (auto& S : ctx->slots)
+        if (box_kept(ctx, S) && !S.box_fresh) {
+            TRY(bbox_slot(ctx, S));
+            S.box_fresh = true;
+        }
     return GC_OK;
 }
 
@@ -2172,17 +2226,17 @@ int one_step(gc_ctx* ctx) {
         DSlot& S = ctx->slots[s];
         mask[s] = !S.probe && (S.xmoves() || !S.sorted_once);  // probes: sorted at measurement
     }
-    TRY(prepare(ctx, mask));
+    TRY(prepare(ctx, mask, true));
     for (size_t s = 0; s < ctx->slots.size(); ++s)
         if (mask[s]) ctx->slots[s].sorted_once = true;
     ctx->resorts += 1;
-    for (size_t a = 0; a < ctx->slots.size(); ++a)
-        if (ctx->slots[a].moving) TRY(halfstep_stage1(ctx, (int)a));
-    TRY(check_launch(ctx, "half step"));
     for (auto& G : ctx->ghosts) TRY(ghost_kinematics(ctx, G));
     TRY(sweep_all_stages(ctx));
     for (auto& S : ctx->slots)
-        if (S.moving) launch_fullstep(step_args(S), ctx->stream);
+        if (S.moving) {
+            S.box_fresh = box_kept(ctx, S);
+            launch_fullstep(step_args(S), S.box_fresh ? ctx->bbox_scratch : nullptr, S.d_inst, ninst(ctx), ctx->stream);
+        }
     TRY(check_launch(ctx, "full step"));
     if (ctx->xsph) TRY(xsph_pass(ctx));
     TRY(advance_virtuals(ctx));
@@ -2203,7 +2257,8 @@ int one_step_rk4(gc_ctx* ctx) {
             TRY(dalloc(ctx, &S.accrho, (size_t)S.N));
         }
     }
-    TRY(prepare(ctx, mask));
+    TRY(prepare(ctx, mask, false));
+    for (auto& S : ctx->slots) S.box_fresh = false;
     for (size_t s = 0; s < ctx->slots.size(); ++s)
         if (mask[s]) ctx->slots[s].sorted_once = true;
     ctx->resorts += 1;
@@ -2577,6 +2632,7 @@ int run_steps(gc_ctx* ctx, int nsteps) {
             ctx->graphs_epoch = ctx->alloc_epoch;
             ctx->graphs_key = graph_key(ctx);
         }
+        TRY(ensure_boxes(ctx));
         int ran = 0;
         int cap_err = GC_OK;
         ctx->capmode = true;
@@ -2604,6 +2660,7 @@ int run_steps(gc_ctx* ctx, int nsteps) {
             // steps exactly (which size every buffer from the plan)
             if (!snap) set_parity(ctx, par0);
             else TRY(restore(ctx, par0));
+            for (auto& S : ctx->slots) S.box_fresh = false;
             ctx->steps_done -= ran;
             ctx->resorts -= ran;
             ctx->graph_steps -= ran;
@@ -3426,6 +3483,7 @@ int gc_upload_fields(gc_ctx* ctx, int nio, const gc_field_io* io) {
             // a system that is not sorted every step is sorted again
             if (!S.moving) structural = true;
             S.sorted_once = false;
+            S.box_fresh = false;
             S.xpk_static = false;
             S.xpk_epoch = -1;
         }

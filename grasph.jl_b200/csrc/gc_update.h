@@ -5,6 +5,7 @@
 #include <cuda_runtime.h>
 
 #include "gc_internal.h"
+#include "gc_kernels.h"
 
 namespace gc {
 
@@ -42,18 +43,28 @@ struct PackArgs {
     float4 *pos, *rec;
 };
 
-void launch_halfstep(const StepArgs& a, cudaStream_t s);
-// The half step fused with what follows it for the same particles before
-// the first sweeps (src/TimeIntegration.jl:158, then _sweep_all_stages!'s
-// stage-1 state updater :401-419): per particle the half step, the updater
-// u (u.kind < 0: none; an elementwise kind), then (pk.pos or pk.rec set) the
-// records of the stage's first sweep.  One pass over the state instead
-// of three.
-void launch_halfstep_fused(const StepArgs& a, const UpdArgs& u, const PackArgs& pk, cudaStream_t s);
-// Whether launch_halfstep_fused takes updater kind `kind` (the light,
+// The half step on a sort's permutation, fused with what follows it for the
+// same particles before the first sweeps (src/TimeIntegration.jl:158, then
+// _sweep_all_stages!'s stage-1 state updater :401-419): per particle the
+// gather (every field read at perm[g] of its old buffer and written at g of
+// the new one: the half step's from `src`, the others as launch_gather_fields
+// would), the half step, the updater u (u.kind < 0: none; an elementwise
+// kind), then (pk.pos or pk.rec set) the records of the stage's first sweep.
+// One pass over the state instead of four.
+struct StepSrc {
+    const double *x, *v, *rho, *dvdt, *drhodt;
+    const int32_t* id;
+    int32_t* id_to;
+};
+void launch_gather_halfstep(const StepArgs& a, const StepSrc& src, const GatherArgs& rest, const int32_t* perm,
+                            const UpdArgs& u, const PackArgs& pk, cudaStream_t s);
+// Whether launch_gather_halfstep takes updater kind `kind` (the light,
 // elementwise ones; the stress updaters keep their own launch).
 bool halfstep_fuses(int kind);
-void launch_fullstep(const StepArgs& a, cudaStream_t s);
+// box_scratch (launch_bbox_fused's): the moved positions' boxes too, into
+// box_inst; a non-finite position is left to the next plan to report.
+void launch_fullstep(const StepArgs& a, unsigned long long* box_scratch, SysInst* box_inst, int ninst,
+                     cudaStream_t s);
 // RK4 (src/TimeIntegration.jl:712-838): q0 snapshot, zero accumulators and
 // dqdt reset; stage advance q = q0 + f·dt·dqdt (f = 0.5 or 1) and dqdt reset;
 // damping and acc += w·dqdt after a stage's sweeps; q = q0 + dt·acc, zero

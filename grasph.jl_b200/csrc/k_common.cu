@@ -8,6 +8,7 @@
 #include <atomic>
 #include <cstdio>
 
+#include "gc_box.cuh"
 #include "gc_device.cuh"
 #include "gc_kernels.h"
 
@@ -294,18 +295,8 @@ __global__ void k_bbox_fused(const double* __restrict__ x, int64_t N, int nd, co
                              const int64_t* count, unsigned long long* scratch, SysInst* inst, int ninst, int* err,
                              int64_t tiles_per_block) {
     pdl_enter();
-    // each block reduces a contiguous run of 256-particle tiles: every thread
-    // keeps the running min/max of its particles while they belong to one
-    // instance (flushing with atomics when the instance changes), and the
-    // block reduces them once at the end, so one block makes 2·nd atomics,
-    // not 2·nd per tile (ordered keys: min/max is exact in any order)
     const int64_t n = count ? *count : N;
-    int krun = -1;
-    unsigned long long amn[MAXD], amx[MAXD];
-    for (int d = 0; d < MAXD; ++d) {
-        amn[d] = ~0ull;
-        amx[d] = 0ull;
-    }
+    BoxRun run;
     bool bad = false;
     for (int64_t tile = (int64_t)blockIdx.x * tiles_per_block;
          tile < (int64_t)(blockIdx.x + 1) * tiles_per_block && tile * blockDim.x < n; ++tile) {
@@ -313,101 +304,20 @@ __global__ void k_bbox_fused(const double* __restrict__ x, int64_t N, int nd, co
         if (g >= n) continue;
         double xv[MAXD];
         load_pos(x, N, g, nd, xv);
-        const int k = inst_of[g];
-        if (k != krun) {
-            if (krun >= 0)
-                #pragma unroll
-                for (int d = 0; d < MAXD; ++d) {
-                    if (d >= nd) break;
-                    atomicMin(&scratch[(krun * 2 + 0) * MAXD + d], amn[d]);
-                    atomicMax(&scratch[(krun * 2 + 1) * MAXD + d], amx[d]);
-                }
-            krun = k;
-            for (int d = 0; d < MAXD; ++d) {
-                amn[d] = ~0ull;
-                amx[d] = 0ull;
-            }
-        }
-        #pragma unroll
-        for (int d = 0; d < MAXD; ++d) {
-            if (d >= nd) break;
-            const double v = xv[d];
-            if (!isfinite(v)) bad = true;
-            const unsigned long long key = ord_key(v);
-            amn[d] = key < amn[d] ? key : amn[d];
-            amx[d] = key > amx[d] ? key : amx[d];
-        }
+#pragma unroll
+        for (int d = 0; d < MAXD; ++d)
+            if (d < nd && !isfinite(xv[d])) bad = true;
+        run.add(scratch, inst_of[g], xv, nd);
     }
     if (bad) atomicOr(err, ERR_NONFINITE);
-    // thread 0 holds the block's first particle, so its instance is the
-    // block's whenever the block has any
-    __shared__ int k0;
-    if (threadIdx.x == 0) k0 = krun;
-    __syncthreads();
-    const int uniform = __syncthreads_and(krun < 0 || krun == k0);
-    if (uniform && k0 >= 0) {
-        __shared__ unsigned long long smn[TPB / 32][MAXD], smx[TPB / 32][MAXD];
-        const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
-        #pragma unroll
-        for (int d = 0; d < MAXD; ++d) {
-            if (d >= nd) break;
-            unsigned long long a = amn[d], b = amx[d];
-            for (int o = 16; o > 0; o >>= 1) {
-                unsigned long long a2 = __shfl_down_sync(0xffffffffu, a, o);
-                unsigned long long b2 = __shfl_down_sync(0xffffffffu, b, o);
-                a = a2 < a ? a2 : a;
-                b = b2 > b ? b2 : b;
-            }
-            if (lane == 0) {
-                smn[wid][d] = a;
-                smx[wid][d] = b;
-            }
-        }
-        __syncthreads();
-        if (threadIdx.x < nd) {
-            const int d = threadIdx.x;
-            unsigned long long a = ~0ull, b = 0ull;
-            for (int w = 0; w < (int)(blockDim.x / 32); ++w) {
-                a = smn[w][d] < a ? smn[w][d] : a;
-                b = smx[w][d] > b ? smx[w][d] : b;
-            }
-            atomicMin(&scratch[(k0 * 2 + 0) * MAXD + d], a);
-            atomicMax(&scratch[(k0 * 2 + 1) * MAXD + d], b);
-        }
-    } else if (krun >= 0) {
-        #pragma unroll
-        for (int d = 0; d < MAXD; ++d) {
-            if (d >= nd) break;
-            atomicMin(&scratch[(krun * 2 + 0) * MAXD + d], amn[d]);
-            atomicMax(&scratch[(krun * 2 + 1) * MAXD + d], amx[d]);
-        }
-    }
-    unsigned long long* counter = scratch + (size_t)ninst * 2 * MAXD;
-    __shared__ bool last;
-    __threadfence();
-    __syncthreads();
-    if (threadIdx.x == 0) last = atomicAdd(counter, 1ull) == gridDim.x - 1;
-    __syncthreads();
-    if (!last) return;
-    __threadfence();
-    for (int k = threadIdx.x; k < ninst; k += blockDim.x) {
-        #pragma unroll
-        for (int d = 0; d < MAXD; ++d) {
-            if (d >= nd) break;
-            unsigned long long a = atomicExch(&scratch[(k * 2 + 0) * MAXD + d], ~0ull);
-            unsigned long long b = atomicExch(&scratch[(k * 2 + 1) * MAXD + d], 0ull);
-            inst[k].bbmin[d] = a == ~0ull ? 0.0 : ord_val(a);
-            inst[k].bbmax[d] = b == 0ull ? 0.0 : ord_val(b);
-        }
-    }
-    if (threadIdx.x == 0) atomicExch(counter, 0ull);
+    run.finish(scratch, inst, ninst, nd);
 }
 
 void launch_bbox_fused(const double* x, int64_t N, int nd, const int32_t* inst_of, const int64_t* count,
                        SysInst* inst, unsigned long long* scratch, int ninst, int* err, cudaStream_t s) {
-    const int64_t tiles = std::max<int64_t>((N + TPB - 1) / TPB, 1);
-    const int64_t per = std::max<int64_t>((tiles + 1183) / 1184, 1);  // about 8 blocks per SM
-    const int blocks = (int)((tiles + per - 1) / per);
+    constexpr int wave = 148 * 8;
+    const int64_t per = box_tiles_per_block(N, TPB, wave);
+    const int blocks = box_blocks(N, TPB, wave);
     k_bbox_fused<<<blocks, TPB, 0, s>>>(x, N, nd, inst_of, count, scratch, inst, ninst, err, per);
     COUNTED(1);
 }

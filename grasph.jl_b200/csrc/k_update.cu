@@ -4,6 +4,7 @@
 // (src/Utils.jl:19-29) is a fused multiply-add; on SVector fields the
 // FastMath operators fall back to plain `*` and `+`, two roundings.
 // Compiled with -fmad=false; fused operations are explicit fma().
+#include "gc_box.cuh"
 #include "gc_device.cuh"
 #include "gc_kernels.h"
 #include "gc_update.h"
@@ -18,19 +19,20 @@ static inline int ublk(int64_t n) {
     return (int)(b < 1 ? 1 : b);
 }
 
-// src/TimeIntegration.jl:158 (_halfstep_ps!) with the q0 snapshot of :220.
-// Every load comes before the first store: the fields are separate arrays,
-// but the compiler cannot know that, and would otherwise wait out a memory
-// round trip per component.
-__device__ __forceinline__ void halfstep_one(const StepArgs& a, int64_t g) {
+// src/TimeIntegration.jl:158 (_halfstep_ps!) with the q0 snapshot of :220, on
+// particle o of `src` into particle g.  Every load comes before the first
+// store: the fields are separate arrays, but the compiler cannot know that,
+// and would otherwise wait out a memory round trip per component.
+__device__ __forceinline__ void halfstep_from(const StepArgs& a, const double* sv, const double* srho,
+                                              const double* sdv, const double* sdrho, int64_t o, int64_t g) {
     double v[MAXD], dv[MAXD];
 #pragma unroll
     for (int d = 0; d < MAXD; ++d)
         if (d < a.nd) {
-            v[d] = a.v[d * a.N + g];
-            dv[d] = a.dvdt[d * a.N + g];
+            v[d] = sv[d * a.N + o];
+            dv[d] = sdv[d * a.N + o];
         }
-    const double r = a.rho[g], dr = a.drhodt[g];
+    const double r = srho[o], dr = sdrho[o];
     const SysInst& S = a.inst[a.inst_of[g]];
     const double h = S.half_dt;
 #pragma unroll
@@ -45,21 +47,45 @@ __device__ __forceinline__ void halfstep_one(const StepArgs& a, int64_t g) {
     a.drhodt[g] = S.srcrho;
 }
 
-__global__ void k_halfstep(StepArgs a) {
-    pdl_enter();
-    for (int64_t g = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; g < a.N; g += (int64_t)gridDim.x * blockDim.x)
-        halfstep_one(a, g);
-}
-
 template <int KIND>
 __device__ __forceinline__ void update_one(const UpdArgs& a, int64_t g);
 
-// KIND: the updater's GC_UPD_* kind, or -1 for none
+// The half step on a sort's permutation.  HBM-bound; separately the gather
+// reads and writes every carried field and the half step reads and writes
+// most of them again: 46 and 43 us for a million particles of water, 57 together
+// (292 MB; limits on registers and one-wave grids give the same within 3).
+// KIND: the updater's GC_UPD_* kind, or -1 for none.
 template <int KIND>
-__global__ void k_halfstep_fused(StepArgs a, UpdArgs u, PackArgs pk) {
+__global__ void k_gather_halfstep(StepArgs a, StepSrc src, const __grid_constant__ GatherArgs rest,
+                                  const int32_t* __restrict__ perm, UpdArgs u, PackArgs pk) {
     pdl_enter();
+    if (rest.clear && blockIdx.x == 0 && threadIdx.x == 0) *rest.clear = 0;
     for (int64_t g = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; g < a.N; g += (int64_t)gridDim.x * blockDim.x) {
-        halfstep_one(a, g);
+        int64_t o = perm[g];
+        // a permutation left incomplete by a flagged key overflow may hold
+        // stale entries: keep every read inside the array
+        if ((uint64_t)o >= (uint64_t)a.N) o = g;
+        double x[MAXD];
+#pragma unroll
+        for (int d = 0; d < MAXD; ++d)
+            if (d < a.nd) x[d] = __ldg(src.x + d * a.N + o);
+        const int32_t id = __ldg(src.id + o);
+        halfstep_from(a, src.v, src.rho, src.dvdt, src.drhodt, o, g);
+#pragma unroll
+        for (int d = 0; d < MAXD; ++d)
+            if (d < a.nd) a.x[d * a.N + g] = x[d];
+        src.id_to[g] = id;
+        for (int f = 0; f < rest.nf; ++f) {
+            const double* __restrict__ from = rest.src[f];
+            double* __restrict__ to = rest.dst[f];
+            double w[MAXS];
+#pragma unroll
+            for (int c = 0; c < MAXS; ++c)
+                if (c < rest.ncomp[f]) w[c] = __ldg(from + c * a.N + o);
+#pragma unroll
+            for (int c = 0; c < MAXS; ++c)
+                if (c < rest.ncomp[f]) to[c * a.N + g] = w[c];
+        }
         if (KIND >= 0) update_one<KIND>(u, g);
         if (pk.pos || pk.rec) pack_one(pk, g);
     }
@@ -67,10 +93,23 @@ __global__ void k_halfstep_fused(StepArgs a, UpdArgs u, PackArgs pk) {
 
 // src/TimeIntegration.jl:673-682: damping, full step, zero XSPH pass, x += dt·v
 // (every load before the first store, as in halfstep_one).
-__global__ void k_fullstep(StepArgs a) {
+// BOX: the moved positions' bounding boxes too (gc_box.cuh), which the next
+// step's plan would otherwise read all positions for (16 us of a million
+// particles' step, and a launch).
+// One wave of blocks, four per SM, each with its run of tiles: 34 us for a
+// million particles, against 46 with 1184 blocks (a nearly empty second
+// wave; 31 us without the boxes).
+constexpr int FULL_PER_SM = 4;
+template <bool BOX>
+__global__ void __launch_bounds__(UTPB, FULL_PER_SM) k_fullstep(StepArgs a, unsigned long long* scratch, SysInst* box, int ninst, int64_t tiles_per_block) {
     pdl_enter();
-    for (int64_t g = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; g < a.N; g += (int64_t)gridDim.x * blockDim.x) {
-        const SysInst& S = a.inst[a.inst_of[g]];
+    BoxRun run;
+    for (int64_t tile = (int64_t)blockIdx.x * tiles_per_block;
+         tile < (int64_t)(blockIdx.x + 1) * tiles_per_block && tile * blockDim.x < a.N; ++tile) {
+        const int64_t g = tile * blockDim.x + threadIdx.x;
+        if (g >= a.N) continue;
+        const int k = a.inst_of[g];
+        const SysInst& S = a.inst[k];
         const double dt = S.dt;
         const bool damp = S.gamma_dt != 0.0;
         double dvl[MAXD], q0[MAXD], vo[MAXD], xa[MAXD];  // xa: x, or v_adjustment with XSPH
@@ -100,11 +139,14 @@ __global__ void k_fullstep(StepArgs a) {
             } else {
                 v = (v + (-1.0 * 0.0)) + 1.0 * 0.0;
                 a.v[d * a.N + g] = v;
-                a.x[d * a.N + g] = xa[d] + dt * v;
+                xa[d] = xa[d] + dt * v;
+                a.x[d * a.N + g] = xa[d];
             }
         }
         a.rho[g] = fma(dt, dr, q0r);
+        if (BOX) run.add(scratch, k, xa, a.nd);
     }
+    if (BOX) run.finish(scratch, box, ninst, a.nd);
 }
 
 // :434 and :684-685: v += v_adjustment, then x += dt·v.
@@ -214,23 +256,27 @@ void launch_xsph_final(const StepArgs& a, cudaStream_t s) {
     g_launches.fetch_add(a.N > 0, std::memory_order_relaxed);
 }
 
-void launch_halfstep(const StepArgs& a, cudaStream_t s) {
-    if (a.N > 0) k_halfstep<<<ublk(a.N), UTPB, 0, s>>>(a);
-    g_launches.fetch_add(a.N > 0, std::memory_order_relaxed);
-}
-void launch_halfstep_fused(const StepArgs& a, const UpdArgs& u, const PackArgs& pk, cudaStream_t s) {
+void launch_gather_halfstep(const StepArgs& a, const StepSrc& src, const GatherArgs& rest, const int32_t* perm,
+                            const UpdArgs& u, const PackArgs& pk, cudaStream_t s) {
     if (a.N <= 0) return;
+    const int b = ublk(a.N);
     switch (u.kind) {
-        case GC_UPD_ZERO_FIELDS: k_halfstep_fused<GC_UPD_ZERO_FIELDS><<<ublk(a.N), UTPB, 0, s>>>(a, u, pk); break;
-        case GC_UPD_TAIT_EOS: k_halfstep_fused<GC_UPD_TAIT_EOS><<<ublk(a.N), UTPB, 0, s>>>(a, u, pk); break;
-        case GC_UPD_LINEAR_EOS: k_halfstep_fused<GC_UPD_LINEAR_EOS><<<ublk(a.N), UTPB, 0, s>>>(a, u, pk); break;
-        default: k_halfstep_fused<-1><<<ublk(a.N), UTPB, 0, s>>>(a, u, pk); break;
+        case GC_UPD_ZERO_FIELDS: k_gather_halfstep<GC_UPD_ZERO_FIELDS><<<b, UTPB, 0, s>>>(a, src, rest, perm, u, pk); break;
+        case GC_UPD_TAIT_EOS: k_gather_halfstep<GC_UPD_TAIT_EOS><<<b, UTPB, 0, s>>>(a, src, rest, perm, u, pk); break;
+        case GC_UPD_LINEAR_EOS: k_gather_halfstep<GC_UPD_LINEAR_EOS><<<b, UTPB, 0, s>>>(a, src, rest, perm, u, pk); break;
+        default: k_gather_halfstep<-1><<<b, UTPB, 0, s>>>(a, src, rest, perm, u, pk); break;
     }
     g_launches.fetch_add(1, std::memory_order_relaxed);
 }
-void launch_fullstep(const StepArgs& a, cudaStream_t s) {
-    if (a.N > 0) k_fullstep<<<ublk(a.N), UTPB, 0, s>>>(a);
-    g_launches.fetch_add(a.N > 0, std::memory_order_relaxed);
+void launch_fullstep(const StepArgs& a, unsigned long long* box_scratch, SysInst* box_inst, int ninst,
+                     cudaStream_t s) {
+    if (a.N <= 0) return;
+    constexpr int wave = 148 * FULL_PER_SM;
+    const int64_t per = box_tiles_per_block(a.N, UTPB, wave);
+    const int blocks = box_blocks(a.N, UTPB, wave);
+    if (box_scratch) k_fullstep<true><<<blocks, UTPB, 0, s>>>(a, box_scratch, box_inst, ninst, per);
+    else k_fullstep<false><<<blocks, UTPB, 0, s>>>(a, nullptr, nullptr, 0, per);
+    g_launches.fetch_add(1, std::memory_order_relaxed);
 }
 
 // ------------------------------------------------------------- updaters
