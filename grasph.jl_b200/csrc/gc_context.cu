@@ -142,7 +142,8 @@ struct DSlot {
     bool pack_done_fp32 = false;
     // warp groups of this system's particles (one grid's columns)
     int2* groups = nullptr;
-    int64_t* d_ngroups = nullptr;
+    int64_t* d_ngroups = nullptr;  // in d_need_max
+    int sm_blocks = 0;             // most blocks of a captured sweep on an SM, 0: as many as fit
     int64_t groups_key = -1, groups_ver = -1;
     double* F(int k) { return f[cur][k]; }
     double* A(int k) { return f[cur ^ 1][k]; }
@@ -704,7 +705,6 @@ int finalize(gc_ctx* ctx) {
         TRY(dalloc(ctx, &D.q0rho, (size_t)D.N));
         TRY(dalloc(ctx, &D.inst_of, (size_t)D.N));
         TRY(dalloc(ctx, &D.groups, (size_t)D.N + 1));
-        TRY(dalloc(ctx, &D.d_ngroups, 1));
         std::vector<int32_t> io(D.N);
         for (int k = 0; k < ninst; ++k)
             for (int64_t i = 0; i < D.h_inst[k].n; ++i) io[D.h_inst[k].base + i] = k;
@@ -1025,9 +1025,13 @@ int finalize(gc_ctx* ctx) {
     ctx->nneed = (int)(ctx->slots.size() + ctx->ghosts.size() + ctx->inters.size());
     TRY(dalloc(ctx, &ctx->d_need, (size_t)ctx->nneed));
     CU(cudaMallocHost(&ctx->h_need, sizeof(int64_t) * ctx->nneed));
-    TRY(dalloc(ctx, &ctx->d_need_max, (size_t)ctx->nneed));
+    // the slots' group counts follow the plans' maxima: one read takes both
+    const size_t nmax = (size_t)ctx->nneed + ctx->slots.size();
+    TRY(dalloc(ctx, &ctx->d_need_max, nmax));
+    CU(cudaMemsetAsync(ctx->d_need_max, 0, sizeof(int64_t) * nmax, ctx->stream));
+    for (size_t s = 0; s < ctx->slots.size(); ++s) ctx->slots[s].d_ngroups = ctx->d_need_max + ctx->nneed + s;
     TRY(dalloc(ctx, &ctx->d_need_cap, (size_t)ctx->nneed));
-    CU(cudaMallocHost(&ctx->h_need_max, sizeof(int64_t) * ctx->nneed));
+    CU(cudaMallocHost(&ctx->h_need_max, sizeof(int64_t) * nmax));
     ctx->need_max.assign(ctx->nneed, 0);
     for (size_t g = 0; g < ctx->ghosts.size(); ++g) ctx->ghosts[g].need_slot = (int64_t)(ctx->slots.size() + g);
     for (size_t i = 0; i < ctx->inters.size(); ++i)
@@ -1874,6 +1878,7 @@ int sweep_group(gc_ctx* ctx, int a, const std::vector<int>& ids, int stage, bool
     TRY(ensure_groups(ctx, a, ids[0], false));
     A.groups = S.groups;
     A.ngroups = S.d_ngroups;
+    A.sm_blocks = S.sm_blocks;
     for (int id : ids) {
         DInter& D = ctx->inters[id];
         if (!D.grid_valid) return seterr(ctx, GC_ERR_STATE, "sweep before create_grid");
@@ -2376,9 +2381,21 @@ bool tuning(gc_ctx* ctx) {
 // a captured step.
 int size_capacities(gc_ctx* ctx) {
     const int n = ctx->nneed;
-    CU(cudaMemcpyAsync(ctx->h_need_max, ctx->d_need_max, sizeof(int64_t) * n, cudaMemcpyDeviceToHost, ctx->stream));
+    CU(cudaMemcpyAsync(ctx->h_need_max, ctx->d_need_max, sizeof(int64_t) * (n + ctx->slots.size()),
+                       cudaMemcpyDeviceToHost, ctx->stream));
     CU(cudaStreamSynchronize(ctx->stream));
     for (int i = 0; i < n; ++i) ctx->need_max[i] = std::max(ctx->need_max[i], ctx->h_need_max[i]);
+    // Captured sweeps of few groups spread them over all SMs: the blocks an SM
+    // holds at most are those an even spread of the last step's groups needs,
+    // a quarter more, and one (launch_win).  It only ever rises.
+    for (size_t s = 0; s < ctx->slots.size(); ++s) {
+        const int64_t wave = (int64_t)ctx->num_sms * (WIN_TPB / 32), ng = ctx->h_need_max[n + s];
+        if (ng == 0) continue;
+        const int r = (int)std::min<int64_t>((ng * 5 / 4 + wave - 1) / wave + 1, WIN_SM_BLOCKS);
+        if (r <= ctx->slots[s].sm_blocks) continue;
+        ctx->slots[s].sm_blocks = r;
+        ctx->alloc_epoch++;  // capture the steps again
+    }
     const double m = ctx->cap_margin;
     auto want = [&](int64_t need) { return (int64_t)((double)need * m) + 1024; };
     auto low = [&](int64_t need) { return (int64_t)((double)need * (1.0 + (m - 1.0) / 2.0)) + 512; };
@@ -2736,7 +2753,6 @@ int gc_ctx_destroy(gc_ctx* ctx) {
         dev_free(ctx, S.accrho);
         dev_free(ctx, S.inst_of);
         dev_free(ctx, S.groups);
-        dev_free(ctx, S.d_ngroups);
         dev_free(ctx, S.d_inst);
         dev_free(ctx, S.d_mass);
         dev_free(ctx, S.d_c);

@@ -9,7 +9,7 @@
 namespace gc {
 
 constexpr int FORCE_TPB = 128;  // threads per block of the sweep
-constexpr int WIN_TPB = 64;     // threads per block of the FP32-compensated sweep
+constexpr int WIN_TPB = 64;     // threads per block of the window sweep
 constexpr int FORCE_BUF = 64;   // staged-neighbour column of the counting sweep (shared memory)
 
 // Launch configurations of the window sweep: resident blocks per SM and
@@ -21,6 +21,7 @@ struct WinCfg {
 constexpr int NUM_FORCE_CFG = GC_NUM_SWEEP_CONFIGS;
 constexpr WinCfg WIN_CFGS32[NUM_FORCE_CFG] = {{8, 192}, {7, 192}, {6, 224}, {10, 160}};
 constexpr WinCfg WIN_CFGS64[NUM_FORCE_CFG] = {{6, 192}, {5, 192}, {7, 160}, {8, 128}};
+constexpr int WIN_SM_BLOCKS = 10;  // no configuration holds more blocks on an SM
 constexpr int MAX_REFS = 8;     // interactions fused into one launch
 
 // system_b kinds as seen by a functor (src/PairwiseFunctors.jl dispatch)
@@ -68,6 +69,7 @@ struct ForceArgs {
     const int2* groups;        // warp groups of system_a particles (group_of)
     const int64_t* ngroups;    // device count of groups
     int num_sms;
+    int sm_blocks;             // most blocks of the window sweep on an SM, 0: as many as fit
     int cfg;                   // index into WIN_CFGS32 / WIN_CFGS64
     int imask, iwsum;          // InterpolateFieldFn: fields (1<<GC_FIELD_*), accumulate w_sum into avort
     int nref;

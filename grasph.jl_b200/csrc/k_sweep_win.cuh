@@ -401,20 +401,29 @@ __global__ void __launch_bounds__(WIN_TPB, MINB) k_sweep_win(ForceArgs A) {
     }
 }
 
+// Shared memory of a block of which an SM holds `blocks` (228 KB, of which 1 KB
+// a block is the system's; 1 KB to spare).
+constexpr size_t sm_share(int blocks) { return (size_t)(228 * 1024 / (blocks < 2 ? 2 : blocks) - 2048); }
+
 template <class Phys, int ND, int PFN, int C>
 static void launch_win(const ForceArgs& A, cudaStream_t s) {
     constexpr WinCfg cf = Phys::EXACT ? WIN_CFGS64[C] : WIN_CFGS32[C];
     int64_t blocks = (A.aN * 32 + WIN_TPB - 1) / WIN_TPB;
     if (blocks > (int64_t)A.num_sms * cf.minb * 4) blocks = (int64_t)A.num_sms * cf.minb * 4;
     if (blocks < 1) blocks = 1;
-    constexpr size_t smem = (size_t)(WIN_TPB / 32) * win_warp_bytes<ND, Phys::NQ, cf.chunk>();
+    constexpr size_t need = (size_t)(WIN_TPB / 32) * win_warp_bytes<ND, Phys::NQ, cf.chunk>();
     auto kern = k_sweep_win<Phys, ND, PFN, cf.minb, cf.chunk>;
-    if (smem > 48 * 1024) {
-        static bool opted = false;
-        if (!opted) {
-            cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-            opted = true;
-        }
+    // Few groups: a sweep launched while the kernel before it still runs
+    // (programmatic dependent launch) finds free the SMs that finished first
+    // and piles its blocks on those; with shared memory asked for beyond what
+    // it needs no SM takes more than its even share.  18135 particles of 3-D
+    // water, 8 blocks an SM at most: step 107 us; 5, 4 or 3: 93; 2: 96.
+    size_t smem = need;
+    if (A.sm_blocks && A.sm_blocks < cf.minb) smem = std::max(need, sm_share(A.sm_blocks));
+    if constexpr (cf.minb > 2) {
+        static const cudaError_t opted = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                                              (int)std::max(need, sm_share(2)));
+        (void)opted;
     }
     kern<<<(int)blocks, WIN_TPB, smem, s>>>(A);
     g_launches.fetch_add(1, std::memory_order_relaxed);
