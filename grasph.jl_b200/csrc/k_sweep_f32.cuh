@@ -10,9 +10,9 @@
 //     factor multiplies the sums, not the terms;
 //   * components go through packed FP32x2 arithmetic.
 // Three-dimensional dam break of a million jittered particles: 894 us a launch
-// with strips staged one at a time and FP64 differences, 704-716 us with this
-// kernel; 64 batched columns (1.07 M particles) 292 to 226 us; a
-// Lennard-Jones box of 18 k particles 72 to 46 us.  Sixteen warps per SM (128
+// with strips staged one at a time and FP64 differences, 700 us with this
+// kernel; 64 batched columns (1.07 M particles) 292 to 230 us; a
+// Lennard-Jones box of 18 k particles 72 to 45 us.  Sixteen warps per SM (128
 // registers, chunks of 192) beat eighteen to twenty-four at 80-96 registers,
 // whose spills cost more than the occupancy gives.
 //
@@ -328,7 +328,11 @@ struct PhysF32 {
                                                 float da, Rec& b, float2 d, float dz, float rr, bool in, Acc& acc) {
         const int bt = BTK >= 0 ? BTK : p.bt;
         if (bt == BT_DYNAMIC) mirror(G, o, da, d, dz, b);
-        const float ri = rsqrt_fast(rr);
+        float ri = rsqrt_fast(rr);
+        // One Newton step: the seed's error, the same for every pair at a
+        // distance, would be the largest of the term (dρ/dt of a resting 3-D
+        // lattice 2.1e-7 of scale, 0.7e-7 with it; 1.6% of the sweep).
+        ri = fmaf(0.5f * ri, fmaf(-(rr * ri), ri, 1.f), ri);
         const float g = kgrad(p, rr, ri);
         const float2 dv = sub2(o.v, b.v);
         const float dvz = ND == 3 ? o.vz - b.vz : 0.f;

@@ -8,8 +8,8 @@
 // what is left), with fused multiply-adds, dv·∇W as W'·(dv·dx), and the
 // kernel's constant factor on the sums.  Every quantity stays FP64; a term
 // differs from the reference's expression by a few units in the last place.
-// Sweep of a 224 k particle 3-D dam break 847 -> 242 us, 5,000 particles in 2-D
-// 61 -> 25 us, an 80 k column 79 -> 40 us a launch.  Blocks few enough that
+// Sweep of a 224 k particle 3-D dam break 847 -> 246 us, 5,000 particles in 2-D
+// 61 -> 22.5 us, an 80 k column 79 -> 42 us a launch.  Blocks few enough that
 // nothing spills (168 registers, twelve warps per SM) are the fastest.
 // The acceptance test keeps the reference's unfused r² < (2h)², so the
 // neighbour sets are bit-identical.
