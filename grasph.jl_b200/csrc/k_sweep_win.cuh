@@ -358,17 +358,30 @@ __global__ void __launch_bounds__(WIN_TPB, MINB) k_sweep_win(ForceArgs A) {
                         };
                         if (self && !Phys::diffuses(par)) pairs(std::integral_constant<int, BT_SELF>{});
                         else pairs(std::integral_constant<int, -1>{});
-                        // rare: candidates so near the cutoff that FP64 decides (counts them)
+                        // rare, but for particles at rest on a lattice with 2h a multiple of
+                        // its spacing: candidates so near the cutoff that FP64 decides (counts
+                        // them).  The masks are cut down to these first, so that the lanes wait
+                        // for their FP64 positions together: the resting 80 k column's sweep
+                        // 61 -> 40 us, the others unchanged.
                         if (!Phys::EXACT && nearest <= Phys::band(par)) {
                             for (int mi = 0; mi < nm; ++mi) {
                                 const int b = (bn >> (4 * mi) & 15u) * 32;
+                                unsigned near = 0;
                                 for (unsigned cur = masks[mi * 32]; cur;) {
-                                    const int t = b + __clz(cur);
-                                    cur ^= 0x80000000u >> (t - b);
-                                    if (Phys::in_band(par, o, [&](int q) { return slots[q * CH + t]; }) &&
-                                        exact_slot(wc, cc, t))
-                                        ++accepted;
+                                    const int t = __clz(cur);
+                                    cur ^= 0x80000000u >> t;
+                                    if (Phys::in_band(par, o, [&](int q) { return slots[q * CH + b + t]; }))
+                                        near |= 0x80000000u >> t;
                                 }
+                                masks[mi * 32] = near;
+                            }
+                            unsigned near = 0;
+                            for (int mi = -1;;) {
+                                while (!near && ++mi < nm) near = masks[mi * 32];
+                                if (!near) break;
+                                const int t = __clz(near);
+                                near ^= 0x80000000u >> t;
+                                if (exact_slot(wc, cc, (int)(bn >> (4 * mi) & 15u) * 32 + t)) ++accepted;
                             }
                         }
                         __syncwarp();  // every lane is done with the chunk before the next one lands
