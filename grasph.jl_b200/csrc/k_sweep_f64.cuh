@@ -91,7 +91,11 @@ struct PhysF64 {
 
     struct Par {
         double cut, sure;    // (2h)²; below `sure` the strip range cannot matter
-        double qs, kf;       // kernel argument's factor; the gradient's, with the term's mass
+        double qs;           // kernel argument's factor
+        // the gradient's, with the term's mass, by which the sums are multiplied
+        // at the end; a Lennard-Jones wall's terms take it one by one (kq, with
+        // kf = 1), as its mass, which may be 0, is not the force's
+        double kq, kf;
         double eps, am, beta;  // 0.01·h², α·c̄·h, β·h² of the artificial viscosity
         double dd;             // 2·δ·c̄·h of the density diffusion (0: none)
         double c;              // system_a's sound speed
@@ -117,6 +121,8 @@ struct PhysF64 {
             p.beta = P.beta * P.h * P.h;
             if (P.has_delta) p.dd = 2.0 * P.delta * (two ? cm : ca) * P.h;
         }
+        p.kq = p.kf;
+        if ((FLUID || CAUCHY) && r.btype == BT_STATIC) p.kf = 1.0;
         return p;
     }
     static __device__ __forceinline__ bool diffuses(const Par& p) { return p.dd != 0.0; }
@@ -243,9 +249,8 @@ struct PhysF64 {
             const double mu = (vr < 0.0 ? vr : 0.0) * rcp_newton(rr + p.eps);
             const double pj = fma(p.beta, mu, -p.am) * mu * (2.0 * o.irho);  // π·ρ_j
             if (bt == BT_STATIC) {
-                // Lennard-Jones wall, src/PairwiseFunctors.jl:210-219 (kf carries system_b's mass)
-                const double lj = lennard_jones<ND>(d, rr, G.ljcut, p.c) / p.kf;
-                const double s = lj - g * pj * b.irho;
+                // Lennard-Jones wall, src/PairwiseFunctors.jl:210-219 (kq with system_b's mass)
+                const double s = lennard_jones<ND>(d, rr, G.ljcut, p.c) - p.kq * g * pj * b.irho;
 #pragma unroll
                 for (int q = 0; q < ND; ++q) acc.s[q] = fma(s, d[q], acc.s[q]);
                 return;

@@ -694,3 +694,26 @@ def test_static_boundary_lennard_jones_pair(be, nd, sep):
     if sep < 1.0:
         # the repulsion points away from the wall and dominates
         assert f.dvdt[0, -1] > 0.0
+
+
+@pytest.mark.parametrize("be", BACKENDS)
+@pytest.mark.parametrize("nd", [2, 3])
+def test_static_boundary_without_mass(be, nd):
+    """A wall's mass scales its viscosity alone: without one the repulsion stays."""
+    h, c, dx_sp = 0.6, 30.0, 0.5
+    f = G.FluidParticleSystem("f", 1, nd, 125.0, c)
+    w = G.BasicParticleSystem("w", 1, nd, 0.0, c)
+    f.x[0] = [0.1] * (nd - 1) + [0.4]
+    w.x[0] = [0.0] * nd
+    f.v[0, -1] = -0.3
+    f.rho[:] = 1003.0
+    w.rho[:] = 998.0
+    si = G.SystemInteraction(G.CubicSplineKernel(h, ndims=nd), G.FluidPfn(0.1, 0.2, h), f,
+                             G.StaticBoundarySystem(w, dx_sp))
+    lf, s = session(be, [f, w], [si])
+    s.create_grid(si)
+    s.sweep(si, 1)
+    s.pull()
+    want = _lj_expected(f.x[0], w.x[0], f.v[0], w.v[0], 1003.0, 998.0, 0.0, c, h, 0.1, 0.2, dx_sp)
+    assert want[-1] > 0.0
+    assert np.allclose(f.dvdt[0], want, rtol=1e-13, atol=0.0), (f.dvdt[0], want)
