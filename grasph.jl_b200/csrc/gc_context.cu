@@ -173,6 +173,7 @@ struct DGhost {
     int64_t cap_fpk = 0;
     int64_t xpk_epoch = -1;
     bool xpk_static = false;  // never set: ghosts are regenerated every step
+    int64_t pack_done_epoch = -1;  // never set: packed for every sweep
     std::vector<std::vector<std::pair<int, int>>> copiers;
     bool ex_p = false, ex_stress = false;
     int64_t need_slot = -1;  // index into need[] for its sort cells
@@ -1600,8 +1601,9 @@ int ensure_fpk(gc_ctx* ctx, T& X, int64_t N, int nd, int mode, bool fp32) {
         dfree(ctx, X.fpk, X.cap_fpk);
         TRY(dalloc(ctx, &X.fpk, (size_t)need));
         X.cap_fpk = need;
-        X.xpk_epoch = -1;  // the new buffer holds no positions yet
+        X.xpk_epoch = -1;  // the new buffer holds no positions and no records yet
         X.xpk_static = false;
+        X.pack_done_epoch = -1;
     }
     return GC_OK;
 }

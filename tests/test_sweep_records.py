@@ -1,0 +1,78 @@
+"""A sweep reads the records of the state, functor and precision that it is
+for: when a system's buffer grows under another system's sweep.
+
+Compared, bit by bit, with an order of the same interactions in which every
+sweep finds its records where the half step or its own pack has just put
+them."""
+import numpy as np
+import pytest
+
+import grasph_b200 as G
+from gc_helpers import make_backend
+
+pytestmark = pytest.mark.gpu
+
+H, DX, C0 = 0.03, 0.02, 40.0
+PRECISIONS = [G.PRECISION_FP64, G.PRECISION_FP32_COMPENSATED]
+
+
+def _block(ps, n, origin, seed):
+    rng = np.random.default_rng(seed)
+    i, j = np.meshgrid(np.arange(n[0]), np.arange(n[1]), indexing="ij")
+    ps.x[:] = np.stack([i.ravel(), j.ravel()], axis=1) * DX + np.asarray(origin) + rng.uniform(-2e-3, 2e-3, ps.x.shape)
+    ps.v[:] = rng.uniform(-1.0, 1.0, ps.x.shape)
+    ps.rho[:] = rng.uniform(990.0, 1010.0, ps.n)
+    if hasattr(ps, "stress"):
+        ps.stress[:] = rng.uniform(-300.0, 100.0, ps.stress.shape)
+    if hasattr(ps, "p"):
+        ps.p[:] = rng.uniform(-50.0, 500.0, ps.n)
+    return ps
+
+
+def _soil(n, origin, seed):
+    return _block(G.ElastoPlasticParticleSystem(f"s{seed}", n[0] * n[1], 2, 4, 0.4, C0), n, origin, seed)
+
+
+def _water(n, origin, seed):
+    return _block(G.FluidParticleSystem(f"w{seed}", n[0] * n[1], 2, 0.4, C0), n, origin, seed)
+
+
+def _wall(ps, y):
+    return G.DynamicBoundarySystem(ps, [0.0, 1.0], [0.0, y], 1.5)
+
+
+def _session(lf, precision):
+    s = G.Session([lf], backend=make_backend("cuda"), precision=precision)
+    s.push()
+    return s
+
+
+def _equal(got, want):
+    assert np.abs(got.systems[0].dvdt).max() > 0.0
+    want = {ps.name: ps for ps in want.systems}
+    for ps in got.systems:
+        for f, _ in ps.particle_fields():
+            a, b = getattr(ps, f), getattr(want[ps.name], f)
+            assert np.isfinite(a).all() and np.array_equal(a, b), f"{ps.name} {f}"
+
+
+def _growing(turned):
+    """Soil on a moving fluid as its wall: the soil's larger records grow the
+    fluid's buffer after the fluid's half step has filled it (turned: after
+    the fluid's own sweep)."""
+    s, w = _soil((12, 8), (0.0, 0.0), 1), _water((12, 6), (0.0, -0.12), 2)
+    k = G.CubicSplineKernel(H, ndims=2)
+    return G.LeapFrogTimeIntegrator([w, s] if turned else [s, w], [
+        G.SystemInteraction(k, G.CauchyFluidPfn(0.1, 0.1, H), s, _wall(w, -0.01)),
+        G.SystemInteraction(k, G.FluidPfn(0.1, 0.1, H), w)])
+
+
+@pytest.mark.parametrize("precision", PRECISIONS)
+@pytest.mark.parametrize("build", [_growing])
+def test_one_step(build, precision):
+    got, want = build(False), build(True)
+    for lf in (got, want):
+        s = _session(lf, precision)
+        s.step(1, 0.01)
+        s.pull()
+    _equal(got, want)
