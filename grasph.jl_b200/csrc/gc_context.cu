@@ -1815,10 +1815,12 @@ int sweep_group(gc_ctx* ctx, int a, const std::vector<int>& ids, int stage, bool
         // the fused half step of this step may have packed these records
         const bool done = S.pack_done_epoch == ctx->pack_epoch && S.pack_done_stage == stage &&
                           S.pack_done_mode == mode && S.pack_done_ns == pk_ns && S.pack_done_fp32 == fp32;
-        if (!done)
+        if (!done) {
             launch_pack(fp32, mode, S.N, nullptr, S.nd, pk_ns, S.F(F_X), S.F(F_V), S.F(F_RHO), S.F(F_P),
                         S.F(F_STRESS), S.inst_of, S.d_mass, hpos_of(S.fpk), nullptr, rec_of(S.fpk, S.N, S.nd),
                         ctx->stream);
+            S.pack_done_epoch = -1;  // no longer the half step's: a later functor of its mode packs again
+        }
     }
     ForceArgs A{};
     A.nd = S.nd;

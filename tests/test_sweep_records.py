@@ -1,9 +1,10 @@
 """A sweep reads the records of the state, functor and precision that it is
-for: when a system's buffer grows under another system's sweep.
+for: when a system's buffer grows under another system's sweep, and when two
+functors of one stage take turns.
 
-Compared, bit by bit, with an order of the same interactions in which every
-sweep finds its records where the half step or its own pack has just put
-them."""
+Each is compared, bit by bit, with an order of the same interactions in which
+every sweep finds its records where the half step or its own pack has just
+put them."""
 import numpy as np
 import pytest
 
@@ -67,8 +68,21 @@ def _growing(turned):
         G.SystemInteraction(k, G.FluidPfn(0.1, 0.1, H), w)])
 
 
+def _turns(turned):
+    """One stage with strain rate, Cauchy and strain rate functors (turned:
+    the Cauchy one first)."""
+    s, a, b = _soil((12, 8), (0.0, 0.0), 1), _water((12, 2), (0.0, -0.04), 2), _water((12, 2), (0.0, 0.16), 3)
+    k = G.CubicSplineKernel(H, ndims=2)
+    inters = [G.SystemInteraction(k, G.StrainRatePfn(), s),
+              G.SystemInteraction(k, G.CauchyFluidPfn(0.1, 0.1, H), s, _wall(a, -0.01)),
+              G.SystemInteraction(k, G.StrainRateVorticityPfn(), s, _wall(b, 0.15))]
+    if turned:
+        inters = [inters[1], inters[0], inters[2]]
+    return G.LeapFrogTimeIntegrator([s, a, b], inters)
+
+
 @pytest.mark.parametrize("precision", PRECISIONS)
-@pytest.mark.parametrize("build", [_growing])
+@pytest.mark.parametrize("build", [_growing, _turns])
 def test_one_step(build, precision):
     got, want = build(False), build(True)
     for lf in (got, want):
