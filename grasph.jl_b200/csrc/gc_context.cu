@@ -334,7 +334,7 @@ struct gc_ctx {
     unsigned long long* d_gscratch = nullptr;  // launch_groups' scratch
     std::vector<Snapshot> snaps;    // per slot (moving slots only)
     int64_t graph_steps = 0, rollbacks = 0;
-    int64_t pack_epoch = 0;  // bumps at the start of every issued step (never rolled back)
+    int64_t pack_epoch = 0;  // bumps at the start of every issued step and single sweep (never rolled back)
     double params_cfl = NAN;  // CFL number the per-instance parameters were pushed for
     bool params_dirty = true;
 };
@@ -3824,6 +3824,7 @@ int gc_sweep(gc_ctx* ctx, int inst, int inter, int stage) {
     DInter& D = ctx->inters[inter];
     if (stage < 1 || stage > D.nstages || D.pk[stage - 1] == GC_PFN_NONE) return GC_OK;
     CU(cudaMemsetAsync(ctx->d_err, 0, sizeof(int), ctx->stream));
+    ctx->pack_epoch++;  // the state is not the last step's: nothing packed in it counts
     TRY(sweep_group(ctx, D.a, std::vector<int>{inter}, stage, false));
     return finish_status(ctx);
 }

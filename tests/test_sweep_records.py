@@ -1,10 +1,10 @@
 """A sweep reads the records of the state, functor and precision that it is
-for: when a system's buffer grows under another system's sweep, and when two
-functors of one stage take turns.
+for: when a system's buffer grows under another system's sweep, when two
+functors of one stage take turns, and when a single sweep follows a step.
 
-Each is compared, bit by bit, with an order of the same interactions in which
-every sweep finds its records where the half step or its own pack has just
-put them."""
+Each is compared, bit by bit, with an order of the same interactions (or a
+fresh session) in which every sweep finds its records where the half step or
+its own pack has just put them."""
 import numpy as np
 import pytest
 
@@ -89,4 +89,40 @@ def test_one_step(build, precision):
         s = _session(lf, precision)
         s.step(1, 0.01)
         s.pull()
+    _equal(got, want)
+
+
+@pytest.mark.parametrize("precision", PRECISIONS)
+@pytest.mark.parametrize("wall", [False, True])
+def test_single_sweep_after_a_step(precision, wall):
+    """The state pushed between the step and the sweep is the one swept."""
+    def build(seed):
+        w = _water((12, 9), (0.0, 0.0), seed)
+        k = G.CubicSplineKernel(H, ndims=2)
+        systems, inters = [w], [G.SystemInteraction(k, G.FluidPfn(0.1, 0.1, H), w)]
+        if wall:  # a moving system that lends its positions
+            systems.append(_water((12, 3), (0.0, -0.06), seed + 1))
+            inters.append(G.SystemInteraction(k, G.FluidPfn(0.1, 0.1, H), w, _wall(systems[1], -0.01)))
+        for i, ps in enumerate(systems):
+            ps.name = f"w{i}"
+        return G.LeapFrogTimeIntegrator(systems, inters)
+
+    def sweep(lf, s):
+        for ps in lf.systems:
+            s.sort_particles(ps, 2.0 * H)
+        for si in lf.interactions:
+            s.create_grid(si)
+            s.sweep(si, 1)
+        s.pull()
+
+    want = build(7)
+    sweep(want, _session(want, precision))
+    got, new = build(1), build(7)
+    s = _session(got, precision)
+    s.step(1, 0.01)
+    for ps, to in zip(got.systems, new.systems):
+        for f, _ in ps.particle_fields():
+            getattr(ps, f)[:] = getattr(to, f)
+    s.push()
+    sweep(got, s)
     _equal(got, want)
