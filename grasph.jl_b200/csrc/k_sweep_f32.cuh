@@ -3,9 +3,11 @@
 // What bounds it is instruction issue (65% of the slots, the FMA pipe half
 // busy, shared memory half busy), so the pair term is written for few
 // instructions:
-//   * positions are FP32 pairs whose difference is the FP64 one rounded to
-//     FP32 (a few adds per pair instead of eight FP64 operations and four
-//     conversions), and a record is two or three 16-byte quads;
+//   * positions are FP32 pairs whose difference is the FP64 one to within two
+//     roundings to FP32 (one where the pairs' high parts subtract exactly, as
+//     they do but next to the origin), by a few adds per pair instead of eight
+//     FP64 operations and four conversions; a record is two or three 16-byte
+//     quads;
 //   * dv·∇W is W'·(dv·dx), so ∇W itself is never formed; the kernel's constant
 //     factor multiplies the sums, not the terms;
 //   * components go through packed FP32x2 arithmetic.
@@ -139,8 +141,9 @@ struct PhysF32 {
         Par p;
         p.bt = r.btype;
         p.cut = (float)G.cutoff_sq;
-        // FP32 r² is off by less than 1e-6 of the cutoff's, plus what the
-        // FP32 pairs lose of coordinates |x| (2^-48·|x| each)
+        // FP32 r² is off by less than 1e-6 of the cutoff's (ten roundings of
+        // terms below 1.3 of it: 8e-7), plus what the FP32 pairs lose of
+        // coordinates |x| (2^-47·|x| each, so less than 3e-14·|x|/2h of r²)
         p.band = p.cut * (2e-6f + (float)strip_doubt<ND>(G) + 1e-13f * xmax * (float)G.inv_cell);
         p.qs = G.f_qs;
         p.kf = G.kq;
@@ -254,9 +257,11 @@ struct PhysF32 {
         d = __fadd2_rn(h, l);
         const float hz = ND == 3 ? o.hz - b.hz : 0.f, lz = ND == 3 ? o.lz - b.lz : 0.f;
         dz = hz + lz;
-        // h² + 2hl, not d²: d's rounding stays out of r²
-        float s = dot(h, hz, l, lz);
-        s += s;
+        // h² + (2h + l)·l, not d²: d's rounding stays out of r².  l counts in
+        // full: it reaches an ulp of the coordinate, 3% of 2h at 2^18 cells from
+        // the origin.  (2h + l does not wait for d = h + l: 712 us on the million
+        // particles, 729 as d + h, 711 with 2h·l alone.)
+        float s = dot(__ffma2_rn(h, bc2(2.f), l), fmaf(2.f, hz, lz), l, lz);
         s = fmaf(h.x, h.x, s);
         s = fmaf(h.y, h.y, s);
         if (ND == 3) s = fmaf(hz, hz, s);

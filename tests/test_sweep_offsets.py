@@ -1,0 +1,91 @@
+"""The window sweep away from the origin: its neighbour counts and rates are
+those of the same arithmetic next to it, up to where FP64 differences take
+over (2^20 cells), and beyond.
+
+Tolerance: that of the window sweep's rates (test_sweep_window.py)."""
+import numpy as np
+import pytest
+
+import grasph_b200 as G
+import parity
+from gc_helpers import make_backend
+
+pytestmark = pytest.mark.gpu
+
+DX = 0.02
+
+
+def _build(nd, functor, cells, wall):
+    h, c = 1.3 * DX, 40.0
+    n = (16, 30) if nd == 2 else (7, 8, 10)
+    rng = np.random.default_rng(3)
+    x = np.stack([a.ravel() for a in np.meshgrid(*[(np.arange(m) + 0.5) * DX for m in n], indexing="ij")], axis=1)
+    x += rng.uniform(-0.1, 0.1, x.shape) * DX
+    # every coordinate as far out, on either side of the origin
+    off = 2.0 * h * cells * np.array([1.0, -1.0, 1.0])[:nd]
+    k = G.CubicSplineKernel(h, ndims=nd)
+    if functor == "fluid":
+        ps = G.FluidParticleSystem("f", len(x), nd, 1000.0 * DX ** nd, c)
+        ps.p[:] = rng.uniform(-50.0, 500.0, ps.n)
+        pfn = G.FluidPfn(0.05, 0.1, h, delta=0.1)
+    else:
+        ps = G.ElastoPlasticParticleSystem("s", len(x), nd, 4 if nd == 2 else 6, 1000.0 * DX ** nd, c)
+        ps.stress[:] = rng.uniform(-300.0, 100.0, ps.stress.shape)
+        pfn = (G.StrainRateVorticityPfn(), G.CauchyFluidPfn(0.05, 0.1, h, delta=0.1))
+    ps.v[:] = rng.uniform(-1.0, 1.0, x.shape)
+    ps.rho[:] = rng.uniform(990.0, 1010.0, ps.n)
+    ps.x[:] = x + off
+    systems, inters = [ps], [G.SystemInteraction(k, pfn, ps)]
+    if wall:
+        w = x[x[:, -1] < 3 * DX] * np.array([1.0] * (nd - 1) + [-1.0])
+        b = G.BasicParticleSystem("w", len(w), nd, 1000.0 * DX ** nd, c)
+        b.x[:] = w + off
+        b.rho[:] = 1000.0
+        systems.append(b)
+        inters.append(G.SystemInteraction(k, pfn, ps,
+                                          G.DynamicBoundarySystem(b, [0.0] * (nd - 1) + [1.0], off, 1.5)))
+    return G.LeapFrogTimeIntegrator(systems, inters)
+
+
+def _pairs(nd, functor, cells, wall):
+    """Accepted pairs, from the counting sweep."""
+    lf = _build(nd, functor, cells, wall)
+    s = G.Session([lf], backend=make_backend("cuda"))
+    s.push()
+    for ps in lf.systems:
+        s.sort_particles(ps, 2.0 * lf.interactions[0].kernel.h)
+    counts = []
+    for si in lf.interactions:
+        s.create_grid(si)
+        counts.append(s.neighbor_counts(si))
+    return counts[0].sum() // 2 + sum(int(c.sum()) for c in counts[1:]), max(c.max() for c in counts)
+
+
+@pytest.mark.parametrize("cells", [0, 5e3, 1e4, 1e5, 9e5, 1.5e6])
+@pytest.mark.parametrize("nd,functor,wall", [(2, "fluid", True), (2, "stress", False), (3, "fluid", False),
+                                             (3, "stress", True)])
+def test_offset(nd, functor, wall, cells):
+    runs = {}
+    for name in ("oracle", "fp64", "fp32c"):
+        lf = _build(nd, functor, cells, wall)
+        prec = G.PRECISION_FP32_COMPENSATED if name == "fp32c" else G.PRECISION_FP64
+        be = make_backend("oracle", track=parity.INPUTS) if name == "oracle" else make_backend("cuda")
+        s = G.Session([lf], backend=be, precision=prec)
+        s.push()
+        s.step(1, 0.01)
+        s.pull()
+        runs[name] = (lf, s)
+    ref, so = runs["oracle"]
+    ps = ref.systems[0]
+    scales = parity.particle_scales(ps, parity.oracle_magnitudes(so, ref)[id(ps)])
+    pairs, most = _pairs(nd, functor, cells, wall)
+    for name in ("fp64", "fp32c"):
+        got = runs[name][0].systems[0]
+        assert runs[name][1].stats()["pairs_last_step"] == pairs
+        assert np.array_equal(ps.id, got.id)
+        tol = 25 * 2.0 ** -24 if name == "fp32c" else 2.0 * (40 + most) * 2.0 ** -53
+        for f in ("dvdt", "drhodt") + (("strain_rate", "vorticity") if functor == "stress" else ()):
+            a, b = (np.asarray(getattr(q, f), float).reshape(ps.n, -1) for q in (got, ps))
+            scale = np.max(np.asarray(scales[f]).reshape(ps.n, -1), axis=1, keepdims=True)
+            worst = np.max(np.abs(a - b) / np.maximum(scale, 1e-300))
+            assert np.all(np.abs(a - b) <= tol * scale), f"{name} {f}: {worst:.2e} against {tol:.2e}"
