@@ -185,10 +185,14 @@ struct PhysF32 {
     // Running compensated sums of one lane, component pairs together: (x, y)
     // and (z, dρ/dt); or (xx, yy), (xy, yx), (zz, xz), (zx, yz), (zy, -).
     static constexpr int NP = FLUID || CAUCHY || ND == 2 ? 2 : 5;
+    // Beside a strain rate with a zz component, Σ f·0.
+    static constexpr bool ZZ = !FLUID && !CAUCHY && ND == 2 && NS == 4;
     struct Acc {
         float2 s[NP], c[NP];  // Kahan: the sum, and minus its rounding error
+        float zz;
     };
     static __device__ __forceinline__ void zero(Acc& a) {
+        a.zz = 0.f;
 #pragma unroll
         for (int q = 0; q < NP; ++q) a.s[q] = a.c[q] = make_float2(0.f, 0.f);
     }
@@ -221,6 +225,7 @@ struct PhysF32 {
             put(A.asr, 1, sum(1));
             if (ND == 3) put(A.asr, 2, sum(4));
             put(A.asr, ND == 3 ? 3 : NS == 4 ? 3 : 2, 0.5 * (sum(2) + sum(3)));
+            if (ZZ && acc.zz != 0.f) put(A.asr, 2, (double)acc.zz);
             if (ND == 3) {
                 put(A.asr, 4, 0.5 * (sum(5) + sum(6)));
                 put(A.asr, 5, 0.5 * (sum(7) + sum(8)));
@@ -344,6 +349,7 @@ struct PhysF32 {
         if constexpr (!FLUID && !CAUCHY) {
             // strain rate and vorticity: f·(v_j − v_i)⊗∇W, f = m_j/ρ_j
             const float f = in ? -g * b.aux : 0.f;
+            if (ZZ) acc.zz = fmaf(f, 0.f, acc.zz);  // NaN beside a neighbour of no finite volume
             const float2 u = make_float2(in ? dv.x : 0.f, in ? dv.y : 0.f);
             const float2 w = __fmul2_rn(bc2(f), d);
             add(acc, 0, u, w);

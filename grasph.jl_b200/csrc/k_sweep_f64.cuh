@@ -152,10 +152,14 @@ struct PhysF64 {
 
     // Sums: dv/dt then dρ/dt; or the products f·dv_a·∂W_b (row a, column b)
     static constexpr int NSUM = FLUID || CAUCHY ? ND + 1 : ND * ND;
+    // ... and, beside a strain rate with a zz component, Σ f·0
+    static constexpr bool ZZ = !FLUID && !CAUCHY && ND == 2 && NS == 4;
     struct Acc {
         double s[NSUM];
+        double zz;
     };
     static __device__ __forceinline__ void zero(Acc& a) {
+        a.zz = 0.0;
 #pragma unroll
         for (int q = 0; q < NSUM; ++q) a.s[q] = 0.0;
     }
@@ -172,6 +176,7 @@ struct PhysF64 {
 #pragma unroll
             for (int d = 0; d < ND; ++d) put(A.asr, d, m(d, d));
             put(A.asr, ND == 3 ? 3 : NS == 4 ? 3 : 2, 0.5 * (m(0, 1) + m(1, 0)));
+            if (ZZ && acc.zz != 0.0) put(A.asr, 2, acc.zz);
             if (ND == 3) {
                 put(A.asr, 4, 0.5 * (m(0, 2) + m(2, 0)));
                 put(A.asr, 5, 0.5 * (m(1, 2) + m(2, 1)));
@@ -237,6 +242,7 @@ struct PhysF64 {
         if constexpr (!FLUID && !CAUCHY) {
             // strain rate and vorticity: f·(v_j − v_i)⊗∇W, f = m_j/ρ_j
             const double f = -g * b.aux;
+            if (ZZ) acc.zz = fma(f, 0.0, acc.zz);  // NaN beside a neighbour of no finite volume
 #pragma unroll
             for (int c = 0; c < ND; ++c) {
                 const double w = f * d[c];
@@ -246,7 +252,8 @@ struct PhysF64 {
         } else {
             // dv·∇W = g·(dv·dx); artificial viscosity src/PairwisePhysics.jl:29-34
             const double vr = dot(d, dv);
-            const double mu = (vr < 0.0 ? vr : 0.0) * rcp_newton(rr + p.eps);
+            // (a comparison that leaves NaN as it is, like Julia's min)
+            const double mu = (vr > 0.0 ? 0.0 : vr) * rcp_newton(rr + p.eps);
             const double pj = fma(p.beta, mu, -p.am) * mu * (2.0 * o.irho);  // π·ρ_j
             if (bt == BT_STATIC) {
                 // Lennard-Jones wall, src/PairwiseFunctors.jl:210-219 (kq with system_b's mass)
@@ -255,7 +262,8 @@ struct PhysF64 {
                 for (int q = 0; q < ND; ++q) acc.s[q] = fma(s, d[q], acc.s[q]);
                 return;
             }
-            double q = vr;
+            // the diffusion's ψ/ρ_j with ψ = 0: NaN when ρ_j is 0 or NaN, else vr
+            double q = fma(0.0, b.irho, vr);
             // density diffusion (the plain fluid and the specialised self form are without it)
             if (PFN != GC_PFN_FLUID && BTK != BT_SELF && p.dd != 0.0) q = fma(p.dd * (o.rho - b.rho), b.irho, q);
             double* dr = &acc.s[NSUM > ND ? ND : 0];

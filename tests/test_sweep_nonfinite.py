@@ -1,0 +1,68 @@
+"""Not-a-number inputs of the window sweep: what is not finite in the oracle's
+rates is not finite here, and everything else agrees with them, on the scale
+of the field's largest rate."""
+import numpy as np
+import pytest
+
+import grasph_b200 as G
+from gc_helpers import make_backend
+
+pytestmark = pytest.mark.gpu
+
+DX = 0.02
+H = 1.3 * DX
+
+
+def _build(nd, functor, kernel, spoil, at=0.0):
+    n = (9, 8) if nd == 2 else (6, 5, 4)
+    rng = np.random.default_rng(2)
+    x = np.stack([a.ravel() for a in np.meshgrid(*[(np.arange(m) + 0.5) * DX for m in n], indexing="ij")], axis=1)
+    x += rng.uniform(-0.1, 0.1, x.shape) * DX
+    k = {"spline": G.CubicSplineKernel, "wendland": G.WenlandC2Kernel}[kernel](H, ndims=nd)
+    if functor == "fluid":
+        ps = G.FluidParticleSystem("f", len(x), nd, 1000.0 * DX ** nd, 40.0)
+        ps.p[:] = rng.uniform(-50.0, 500.0, ps.n)
+        pfn = G.FluidPfn(0.05, 0.1, H)
+    else:
+        ps = G.ElastoPlasticParticleSystem("s", len(x), nd, 4 if nd == 2 else 6, 1000.0 * DX ** nd, 40.0)
+        ps.stress[:] = rng.uniform(-300.0, 100.0, ps.stress.shape)
+        pfn = (G.StrainRateVorticityPfn(), G.CauchyFluidPfn(0.05, 0.1, H))
+    ps.x[:] = x
+    ps.v[:] = rng.uniform(-1.0, 1.0, x.shape)
+    ps.rho[:] = rng.uniform(990.0, 1010.0, ps.n)
+    spoil(ps)
+    return G.LeapFrogTimeIntegrator([ps], [G.SystemInteraction(k, pfn, ps)])
+
+
+def _check(build, precision, tol, fields):
+    """One sweep of every stage (a step would integrate what is not finite)."""
+    runs = {}
+    for name in ("oracle", "cuda"):
+        lf = build()
+        s = G.Session([lf], backend=make_backend(name), precision=precision if name == "cuda" else G.PRECISION_FP64)
+        s.push()
+        ps, si = lf.systems[0], lf.interactions[0]
+        s.sort_particles(ps, 2.0 * H)
+        s.create_grid(si)
+        for stage in range(1, len(si.pfns) + 1):
+            s.sweep(si, stage)
+        s.pull()
+        runs[name] = ps
+    for f in fields:
+        a, b = (np.asarray(getattr(runs[q], f), float) for q in ("cuda", "oracle"))
+        assert np.array_equal(np.isfinite(a), np.isfinite(b)), f
+        ok = np.isfinite(b)
+        assert np.all(np.abs(a[ok] - b[ok]) <= tol * np.abs(b[ok]).max()), f
+    return runs["oracle"]
+
+
+FIELDS = {"fluid": ("dvdt", "drhodt"), "stress": ("dvdt", "drhodt", "strain_rate", "vorticity")}
+
+
+@pytest.mark.parametrize("field,value", [("v", np.nan), ("rho", np.nan), ("rho", 0.0)])
+@pytest.mark.parametrize("nd,functor", [(2, "fluid"), (3, "fluid"), (2, "stress"), (3, "stress")])
+def test_fp64_neighbour_not_a_number(nd, functor, field, value):
+    def spoil(ps):
+        getattr(ps, field)[ps.n // 2] = value
+    ps = _check(lambda: _build(nd, functor, "spline", spoil), G.PRECISION_FP64, 1e-12, FIELDS[functor])
+    assert np.isnan(ps.dvdt).any(axis=1).sum() > 4 and np.isnan(ps.drhodt).sum() > 4
