@@ -37,6 +37,11 @@ __device__ __forceinline__ float rcp_fast(float x) {
     asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
     return y;
 }
+__device__ __forceinline__ float min3(float a, float b, float c) {
+    float y;
+    asm("min.f32 %0, %1, %2, %3;" : "=f"(y) : "f"(a), "f"(b), "f"(c));
+    return y;
+}
 __device__ __forceinline__ float2 bc2(float x) { return make_float2(x, x); }
 // a - b, exactly rounded (b·(−1) is exact)
 __device__ __forceinline__ float2 sub2(float2 a, float2 b) { return __ffma2_rn(b, bc2(-1.0f), a); }
@@ -171,12 +176,12 @@ struct PhysF32 {
             const float a = fmaf(r, -p.qs, 1.f), b = __saturatef(fmaf(r, -2.f * p.qs, 1.f));
             return ri * fmaf(a, a, -(b * b));
         } else {
-            const float a = fmaxf(fmaf(r, -p.qs, 2.f), 0.f);
+            const float a = fmaf(r, -p.qs, 2.f);  // (only pairs with r < 2h are added)
             return a * a * a;
         }
     }
-    static __device__ __forceinline__ float dot(float2 a, float az, float2 b, float bz) {
-        float s = a.x * b.x;
+    static __device__ __forceinline__ float dot(float2 a, float az, float2 b, float bz, float s0 = 0.f) {
+        float s = fmaf(a.x, b.x, s0);
         s = fmaf(a.y, b.y, s);
         if (ND == 3) s = fmaf(az, bz, s);
         return s;
@@ -266,7 +271,9 @@ struct PhysF32 {
         // full: it reaches an ulp of the coordinate, 3% of 2h at 2^18 cells from
         // the origin.  (2h + l does not wait for d = h + l: 712 us on the million
         // particles, 729 as d + h, 711 with 2h·l alone.)
-        float s = dot(__ffma2_rn(h, bc2(2.f), l), fmaf(2.f, hz, lz), l, lz);
+        // FLT_MIN keeps r² of particles nearly at one place out of the subnormals
+        // (whose 1/r the seed cannot give) and is lost in any other.
+        float s = dot(__ffma2_rn(h, bc2(2.f), l), fmaf(2.f, hz, lz), l, lz, FLT_MIN);
         s = fmaf(h.x, h.x, s);
         s = fmaf(h.y, h.y, s);
         if (ND == 3) s = fmaf(hz, hz, s);
@@ -281,21 +288,31 @@ struct PhysF32 {
 
     static __device__ __forceinline__ bool diffuses(const Par& p) { return p.dd != 0.f; }
     static __device__ __forceinline__ float band(const Par& p) { return p.band; }
+    static __device__ __forceinline__ bool lj_wall(int bt) { return (FLUID || CAUCHY) && bt == BT_STATIC; }
+    // The sums of a lane with a neighbour at no distance: NaN (a Lennard-Jones
+    // wall's terms are so by themselves).
+    static __device__ __forceinline__ void spoil(const Par& p, Acc& a) {
+        if (lj_wall(p.bt)) return;
+#pragma unroll
+        for (int q = 0; q < NP; ++q) a.s[q] = bc2(CUDART_NAN_F);
+    }
     // whether pair() left this candidate to the FP64 test
     template <class Q>
-    static __device__ __forceinline__ bool in_band(const Par& p, const Rec& o, const Q& quad) {
+    static __device__ __forceinline__ bool in_band(const Par& p, const Rec& o, const Q& quad, Acc& a) {
         Rec b;
         float2 d;
         float dz;
         pos_read(quad, b);
-        return fabsf(delta(o, b, d, dz) - p.cut) <= p.band;
+        const float rr = delta(o, b, d, dz);
+        if (rr <= FLT_MIN) spoil(p, a);
+        return fabsf(rr - p.cut) <= p.band;
     }
 
     // One candidate: r² from the FP32 pairs, then the functor's term when it
     // lies below the band around the cutoff (returns 1); `nearest` keeps how
-    // near to the cutoff an r² came.  The pairs inside the band are left to
-    // the caller to count: the kernel's gradient there is below 1e-11 of its
-    // peak, so their terms vanish in FP32.  Only a Lennard-Jones wall, whose
+    // near to the cutoff, or to 0, an r² came (one three-input minimum).  The
+    // pairs inside the band are left to the caller to count: the kernel's
+    // gradient there is below 1e-11 of its peak, so their terms vanish in FP32.  Only a Lennard-Jones wall, whose
     // force need not, has exact() decide them here.  o: own record; da: own
     // distance to a dynamic boundary's plane.  BTK: the system_b kind when
     // known at compile time (BT_SELF then has no density diffusion).
@@ -311,13 +328,13 @@ struct PhysF32 {
         float dz;
         float rr = delta(o, b, d, dz);
         // a Lennard-Jones force goes with r^-14: its r² from FP64
-        if (bt == BT_STATIC) rr = delta64(o, b);
+        if (lj_wall(bt)) rr = delta64(o, b);
         const float off = rr - p.cut;
         bool in = off < -p.band;
-        if (bt == BT_STATIC) {
+        if (lj_wall(bt)) {
             if (fabsf(off) <= p.band) in = exact();
         } else {
-            nearest = fminf(nearest, fabsf(off));
+            nearest = min3(nearest, fabsf(off), rr);
         }
         term<BTK>(p, G, P, o, da, b, d, dz, rr, in, acc);
         return in ? 1 : 0;
@@ -326,8 +343,10 @@ struct PhysF32 {
     // The term of an accepted pair from its FP64 differences.
     static __device__ __forceinline__ void walked(const Par& p, const GridInst& G, const PfnInst& P, const Rec& o,
                                                   float da, Rec& b, const double* y, double r2, Acc& acc) {
-        term<-1>(p, G, P, o, da, b, make_float2((float)y[0], (float)y[1]), ND == 3 ? (float)y[ND - 1] : 0.f, (float)r2,
-                 true, acc);
+        const float rr = lj_wall(p.bt) ? (float)r2 : fmaxf((float)r2, FLT_MIN);
+        term<-1>(p, G, P, o, da, b, make_float2((float)y[0], (float)y[1]), ND == 3 ? (float)y[ND - 1] : 0.f, rr, true,
+                 acc);
+        if (r2 == 0.0) spoil(p, acc);
     }
 
     // The functor's term of a pair at distance (d, dz), r² = rr, onto the
@@ -365,7 +384,7 @@ struct PhysF32 {
             const float vr = dot(d, dz, dv, dvz);
             const float mu = fminf(vr, 0.f) * rcp_fast(rr + p.eps);
             const float pj = fmaf(p.beta, mu, -p.am) * mu * (2.f * o.irho);  // π·ρ_j
-            if (bt == BT_STATIC) {
+            if (lj_wall(bt)) {
                 // Lennard-Jones wall, src/PairwiseFunctors.jl:210-219 (kq with system_b's mass)
                 const float x = G.f_ljcut * ri, x2 = x * x, x6 = x2 * x2 * x2;
                 const float lj = x > 1.f ? p.ljc * __fdividef(x6 * x6 - x6, rr) : 0.f;

@@ -18,7 +18,8 @@
 
 namespace gc {
 
-// 1/x and 1/sqrt(x) of a positive normal x, by Newton-Raphson.
+// 1/x and 1/sqrt(x) of a positive normal x, by Newton-Raphson.  (1/sqrt of a
+// smaller x, whose seed is infinite, is some number above 2^511.)
 __device__ __forceinline__ double rcp_newton(double x) {
     double y;
     asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(x));
@@ -28,6 +29,7 @@ __device__ __forceinline__ double rcp_newton(double x) {
 __device__ __forceinline__ double rsqrt_newton(double x) {
     double y;
     asm("rsqrt.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(x));
+    y = __hiloint2double(min(__double2hiint(y), 0x5fe00000), __double2loint(y));
     const double h = -0.5 * x;
     y = fma(y, fma(h * y, y, 0.5), y);
     return fma(y, fma(h * y, y, 0.5), y);
@@ -126,9 +128,8 @@ struct PhysF64 {
         return p;
     }
     static __device__ __forceinline__ bool diffuses(const Par& p) { return p.dd != 0.0; }
-    static __device__ __forceinline__ float band(const Par&) { return 0.f; }
-    template <class Q>
-    static __device__ __forceinline__ bool in_band(const Par&, const Rec&, const Q&) { return false; }
+    // (pair()'s `nearest` is r²'s high word, as a float: subnormal or 0 up to this)
+    static __device__ __forceinline__ float band(const Par&) { return __int_as_float(0x000fffff); }
 
     // ∇W = (the kernel's factor)·kgrad·dx for a pair at r² (ri = 1/r)
     static __device__ __forceinline__ double kgrad(const Par& p, double rr, double ri) {
@@ -162,6 +163,23 @@ struct PhysF64 {
         a.zz = 0.0;
 #pragma unroll
         for (int q = 0; q < NSUM; ++q) a.s[q] = 0.0;
+    }
+    // The sums of a lane with a neighbour at no distance: NaN (a Lennard-Jones
+    // wall's terms are so by themselves).
+    static __device__ __forceinline__ void spoil(const Par& p, Acc& a) {
+        if ((FLUID || CAUCHY) && p.bt == BT_STATIC) return;
+#pragma unroll
+        for (int q = 0; q < NSUM; ++q) a.s[q] = CUDART_NAN;
+    }
+    template <class Q>
+    static __device__ __forceinline__ bool in_band(const Par& p, const Rec& o, const Q& quad, Acc& a) {
+        Rec b;
+        pos_read(quad, b);
+        double d[ND];
+#pragma unroll
+        for (int q = 0; q < ND; ++q) d[q] = o.x[q] - b.x[q];
+        if (dot_exact<ND>(d, d) == 0.0) spoil(p, a);
+        return false;
     }
     static __device__ __forceinline__ void store(const ForceArgs& A, int64_t gi, const Acc& acc, double f) {
         const int64_t N = A.aN;
@@ -197,7 +215,8 @@ struct PhysF64 {
     // cells away otherwise.
     template <int BTK, class Q, class Exact>
     static __device__ __forceinline__ int pair(const Par& p, const GridInst& G, const PfnInst& P, const Rec& o,
-                                               double da, const Q& quad, const Exact& exact, float&, Acc& acc) {
+                                               double da, const Q& quad, const Exact& exact, float& nearest,
+                                               Acc& acc) {
         const int bt = BTK >= 0 ? BTK : p.bt;
         Rec b;
         if (bt == BT_DYNAMIC) pos_read(quad, b);
@@ -206,6 +225,7 @@ struct PhysF64 {
 #pragma unroll
         for (int q = 0; q < ND; ++q) d[q] = o.x[q] - b.x[q];
         const double rr = dot_exact<ND>(d, d);
+        nearest = fminf(nearest, __int_as_float(__double2hiint(rr)));
         bool in = rr < p.cut;
         if (in && rr > p.sure) in = exact();
         if (in) term<BTK>(p, G, P, o, da, b, d, rr, acc);
@@ -214,6 +234,7 @@ struct PhysF64 {
     static __device__ __forceinline__ void walked(const Par& p, const GridInst& G, const PfnInst& P, const Rec& o,
                                                   double da, Rec& b, const double* y, double r2, Acc& acc) {
         term<-1>(p, G, P, o, da, b, y, r2, acc);
+        if (r2 == 0.0) spoil(p, acc);
     }
 
     template <int BTK>

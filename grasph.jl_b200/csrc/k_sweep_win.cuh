@@ -16,6 +16,7 @@
 // next group's state is prefetched.
 #pragma once
 #include <cfloat>
+#include <math_constants.h>
 
 #include "k_force_impl.cuh"
 
@@ -362,26 +363,29 @@ __global__ void __launch_bounds__(WIN_TPB, MINB) k_sweep_win(ForceArgs A) {
                         // its spacing: candidates so near the cutoff that FP64 decides (counts
                         // them).  The masks are cut down to these first, so that the lanes wait
                         // for their FP64 positions together: the resting 80 k column's sweep
-                        // 61 -> 40 us, the others unchanged.
-                        if (!Phys::EXACT && nearest <= Phys::band(par)) {
+                        // 61 -> 40 us, the others unchanged.  And pairs at no distance, for
+                        // which the reference's kernel gradient is 0/0.
+                        if (nearest <= Phys::band(par)) {
                             for (int mi = 0; mi < nm; ++mi) {
                                 const int b = (bn >> (4 * mi) & 15u) * 32;
                                 unsigned near = 0;
                                 for (unsigned cur = masks[mi * 32]; cur;) {
                                     const int t = __clz(cur);
                                     cur ^= 0x80000000u >> t;
-                                    if (Phys::in_band(par, o, [&](int q) { return slots[q * CH + b + t]; }))
+                                    if (Phys::in_band(par, o, [&](int q) { return slots[q * CH + b + t]; }, acc))
                                         near |= 0x80000000u >> t;
                                 }
                                 masks[mi * 32] = near;
                             }
-                            unsigned near = 0;
-                            for (int mi = -1;;) {
-                                while (!near && ++mi < nm) near = masks[mi * 32];
-                                if (!near) break;
-                                const int t = __clz(near);
-                                near ^= 0x80000000u >> t;
-                                if (exact_slot(wc, cc, (int)(bn >> (4 * mi) & 15u) * 32 + t)) ++accepted;
+                            if (!Phys::EXACT) {
+                                unsigned near = 0;
+                                for (int mi = -1;;) {
+                                    while (!near && ++mi < nm) near = masks[mi * 32];
+                                    if (!near) break;
+                                    const int t = __clz(near);
+                                    near ^= 0x80000000u >> t;
+                                    if (exact_slot(wc, cc, (int)(bn >> (4 * mi) & 15u) * 32 + t)) ++accepted;
+                                }
                             }
                         }
                         __syncwarp();  // every lane is done with the chunk before the next one lands

@@ -1,6 +1,6 @@
-"""Not-a-number inputs of the window sweep: what is not finite in the oracle's
-rates is not finite here, and everything else agrees with them, on the scale
-of the field's largest rate."""
+"""Not-a-number and coincident inputs of the window sweep: what is not finite
+in the oracle's rates is not finite here, and everything else agrees with
+them, on the scale of the field's largest rate."""
 import numpy as np
 import pytest
 
@@ -13,7 +13,7 @@ DX = 0.02
 H = 1.3 * DX
 
 
-def _build(nd, functor, kernel, spoil, at=0.0):
+def _build(nd, functor, kernel, spoil, wall=None):
     n = (9, 8) if nd == 2 else (6, 5, 4)
     rng = np.random.default_rng(2)
     x = np.stack([a.ravel() for a in np.meshgrid(*[(np.arange(m) + 0.5) * DX for m in n], indexing="ij")], axis=1)
@@ -31,7 +31,16 @@ def _build(nd, functor, kernel, spoil, at=0.0):
     ps.v[:] = rng.uniform(-1.0, 1.0, x.shape)
     ps.rho[:] = rng.uniform(990.0, 1010.0, ps.n)
     spoil(ps)
-    return G.LeapFrogTimeIntegrator([ps], [G.SystemInteraction(k, pfn, ps)])
+    systems, b = [ps], None
+    if wall:
+        # a wall with one particle where one of the system's is
+        w = G.BasicParticleSystem("w", 1, nd, 1000.0 * DX ** nd, 40.0)
+        w.x[:] = ps.x[7]
+        w.rho[:] = 1000.0
+        systems.append(w)
+        b = (G.StaticBoundarySystem(w, DX) if wall == "static" else
+             G.DynamicBoundarySystem(w, [0.0] * (nd - 1) + [1.0], w.x[0] - DX, 1.5))
+    return G.LeapFrogTimeIntegrator(systems, [G.SystemInteraction(k, pfn, ps, b)])
 
 
 def _check(build, precision, tol, fields):
@@ -42,7 +51,8 @@ def _check(build, precision, tol, fields):
         s = G.Session([lf], backend=make_backend(name), precision=precision if name == "cuda" else G.PRECISION_FP64)
         s.push()
         ps, si = lf.systems[0], lf.interactions[0]
-        s.sort_particles(ps, 2.0 * H)
+        for q in lf.systems:
+            s.sort_particles(q, 2.0 * H)
         s.create_grid(si)
         for stage in range(1, len(si.pfns) + 1):
             s.sweep(si, stage)
@@ -66,3 +76,50 @@ def test_fp64_neighbour_not_a_number(nd, functor, field, value):
         getattr(ps, field)[ps.n // 2] = value
     ps = _check(lambda: _build(nd, functor, "spline", spoil), G.PRECISION_FP64, 1e-12, FIELDS[functor])
     assert np.isnan(ps.dvdt).any(axis=1).sum() > 4 and np.isnan(ps.drhodt).sum() > 4
+
+
+@pytest.mark.parametrize("precision", [G.PRECISION_FP64, G.PRECISION_FP32_COMPENSATED])
+@pytest.mark.parametrize("kernel", ["spline", "wendland"])
+@pytest.mark.parametrize("nd,functor", [(2, "fluid"), (3, "stress")])
+def test_coincident(nd, functor, kernel, precision):
+    def spoil(ps):
+        ps.x[7] = ps.x[8]
+    fields = FIELDS[functor]
+    ps = _check(lambda: _build(nd, functor, kernel, spoil), precision,
+                1e-12 if precision == G.PRECISION_FP64 else 1e-5, fields)
+    assert np.isnan(ps.drhodt).sum() == 2
+
+
+# The pair's r² is 2e-42 (a subnormal float) and 2e-312 (a subnormal double):
+# its terms vanish with the distance.
+@pytest.mark.parametrize("precision,sep", [(G.PRECISION_FP32_COMPENSATED, 1e-21), (G.PRECISION_FP64, 1e-156)])
+@pytest.mark.parametrize("kernel", ["spline", "wendland"])
+@pytest.mark.parametrize("nd,functor", [(2, "fluid"), (3, "stress")])
+def test_nearly_coincident(nd, functor, kernel, precision, sep):
+    def spoil(ps):
+        ps.x[:] -= ps.x[8]
+        ps.x[7] = 0.0
+        ps.x[7, :2] = sep
+    ps = _check(lambda: _build(nd, functor, kernel, spoil), precision,
+                1e-12 if precision == G.PRECISION_FP64 else 1e-5, FIELDS[functor])
+    assert np.isfinite(ps.dvdt).all() and np.isfinite(ps.drhodt).all()
+
+
+@pytest.mark.parametrize("precision", [G.PRECISION_FP64, G.PRECISION_FP32_COMPENSATED])
+@pytest.mark.parametrize("wall", ["static", "dynamic"])
+@pytest.mark.parametrize("functor", ["fluid", "stress"])
+def test_coincident_with_a_wall(functor, wall, precision):
+    ps = _check(lambda: _build(2, functor, "spline", lambda ps: None, wall), precision,
+                1e-12 if precision == G.PRECISION_FP64 else 1e-5, ("dvdt", "drhodt", *FIELDS[functor][2:]))
+    assert np.isnan(ps.dvdt).any(axis=1).sum() == 1
+
+
+@pytest.mark.parametrize("precision", [G.PRECISION_FP64, G.PRECISION_FP32_COMPENSATED])
+def test_coincident_far_out(precision):
+    """(where FP32-compensated takes FP64 differences)"""
+    def spoil(ps):
+        ps.x[:] += 2.0 * H * 3.0 * 2 ** 20
+        ps.x[7] = ps.x[8]
+    ps = _check(lambda: _build(2, "stress", "wendland", spoil), precision,
+                1e-12 if precision == G.PRECISION_FP64 else 1e-5, FIELDS["stress"])
+    assert np.isnan(ps.drhodt).sum() == 2
