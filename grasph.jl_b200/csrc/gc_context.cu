@@ -22,6 +22,7 @@
 #include <cstring>
 #include <map>
 #include <string>
+#include <unordered_map>
 #include <vector>
 
 #include "gc_force.h"
@@ -227,7 +228,6 @@ struct DInter {
     int* d_keep = nullptr;          // [0] cs is current for d_gi_prev, [1] this step's grid equals it
     GridInst* d_gi_prev = nullptr;  // geometry cs was last counted on, per instance
     int32_t* hist = nullptr;        // its own histogram (batched grids): zero between uses
-    int64_t cap_hist = 0;
 };
 
 // One captured step: valid for the buffer parities `pre` (cur of every slot,
@@ -255,6 +255,7 @@ struct Snapshot {
 struct gc_ctx {
     int device = 0;
     size_t budget = 0, allocated = 0;
+    std::unordered_map<void*, size_t> blocks;  // dalloc's, with their bytes
     cudaStream_t stream = nullptr;
     // device memory: cudaMalloc/cudaFree, or (contexts a server builds) a
     // stream-ordered pool that keeps freed memory for the next context, so
@@ -394,6 +395,7 @@ int dalloc(gc_ctx* ctx, T** p, size_t count) {
     if (e != cudaSuccess) return seterr(ctx, GC_ERR_OOM, "cudaMalloc(%zu): %s", bytes, cudaGetErrorString(e));
     CU(cudaMemsetAsync(q, 0, bytes, ctx->stream));
     ctx->allocated += bytes;
+    ctx->blocks[q] = bytes;
     *p = (T*)q;
     return GC_OK;
 }
@@ -406,12 +408,15 @@ void dev_free(gc_ctx* ctx, void* p) {
 }
 
 template <class T>
-void dfree(gc_ctx* ctx, T*& p, size_t count) {
+void dfree(gc_ctx* ctx, T*& p) {
     if (p) {
         ctx->alloc_epoch++;
         dev_free(ctx, p);
-        size_t bytes = count * sizeof(T);
-        ctx->allocated -= std::min(ctx->allocated, bytes ? bytes : 16);
+        auto held = ctx->blocks.find(p);
+        if (held != ctx->blocks.end()) {
+            ctx->allocated -= held->second;
+            ctx->blocks.erase(held);
+        }
         p = nullptr;
     }
 }
@@ -1079,45 +1084,52 @@ int finalize(gc_ctx* ctx) {
 }
 
 // ------------------------------------------------------------- capacity
-int ensure_cells(gc_ctx* ctx, int64_t cells) {
-    if (cells + 1 > ctx->cap_cells) {
-        int64_t cap = std::max<int64_t>(cells + 1 + cells / 4, 1024);
-        CU(cudaStreamSynchronize(ctx->stream));  // in-flight kernels may use the old buffers
-        dfree(ctx, ctx->hist, ctx->cap_cells);
-        dfree(ctx, ctx->start, ctx->cap_cells);
-        dfree(ctx, ctx->fill, ctx->cap_cells);
-        TRY(dalloc(ctx, &ctx->hist, (size_t)cap));
-        TRY(dalloc(ctx, &ctx->start, (size_t)cap));
-        TRY(dalloc(ctx, &ctx->fill, (size_t)cap));
-        ctx->cap_cells = cap;
-    }
-    int64_t st = scan_tmp_elems(ctx->cap_cells) + 16;
+// Scratch of a scan of n elements.
+int ensure_scan(gc_ctx* ctx, int64_t n) {
+    const int64_t st = scan_tmp_elems(n) + 16;
     if (st > ctx->cap_scan) {
         CU(cudaStreamSynchronize(ctx->stream));
-        dfree(ctx, ctx->scan_tmp, ctx->cap_scan);
+        ctx->cap_scan = 0;  // until the new one is there
+        dfree(ctx, ctx->scan_tmp);
         TRY(dalloc(ctx, &ctx->scan_tmp, (size_t)st));
         ctx->cap_scan = st;
     }
     return GC_OK;
 }
 
+int ensure_cells(gc_ctx* ctx, int64_t cells) {
+    if (cells + 1 > ctx->cap_cells) {
+        int64_t cap = std::max<int64_t>(cells + 1 + cells / 4, 1024);
+        CU(cudaStreamSynchronize(ctx->stream));  // in-flight kernels may use the old buffers
+        ctx->cap_cells = 0;  // until the new ones are there: an allocation may fail
+        dfree(ctx, ctx->hist);
+        dfree(ctx, ctx->start);
+        dfree(ctx, ctx->fill);
+        TRY(dalloc(ctx, &ctx->hist, (size_t)cap));
+        TRY(dalloc(ctx, &ctx->start, (size_t)cap));
+        TRY(dalloc(ctx, &ctx->fill, (size_t)cap));
+        ctx->cap_cells = cap;
+    }
+    return ensure_scan(ctx, ctx->cap_cells);
+}
+
 int ensure_inter_cells(gc_ctx* ctx, DInter& D, int64_t cells) {
     if (cells + 1 > D.cap_cells) {
         int64_t cap = std::max<int64_t>(cells + 1 + cells / 4, 1024);
         CU(cudaStreamSynchronize(ctx->stream));
-        dfree(ctx, D.cs, D.cap_cells);
-        dfree(ctx, D.cs_a, D.cap_cells);
+        D.cap_cells = 0;  // until the new ones are there
+        D.grid_valid = false;
+        dfree(ctx, D.cs);
+        dfree(ctx, D.cs_a);
         TRY(dalloc(ctx, &D.cs, (size_t)cap));
         if (D.btype != BT_SELF) TRY(dalloc(ctx, &D.cs_a, (size_t)cap));
-        D.cap_cells = cap;
         if (!D.probe) {
             // its own histogram for the batched grids (zero between uses), then
             // its scan's tile sums
-            dfree(ctx, D.hist, D.cap_hist);
-            D.cap_hist = cap + grid_scan_tiles(cap);
-            TRY(dalloc(ctx, &D.hist, (size_t)D.cap_hist));
-            CU(cudaMemsetAsync(D.hist, 0, sizeof(int32_t) * D.cap_hist, ctx->stream));
+            dfree(ctx, D.hist);
+            TRY(dalloc(ctx, &D.hist, (size_t)(cap + grid_scan_tiles(cap))));
         }
+        D.cap_cells = cap;
         // new buffer: nothing counted (the step's plan may already have set keep[1])
         if (D.d_keep) CU(cudaMemsetAsync(D.d_keep, 0, 2 * sizeof(int), ctx->stream));
     }
@@ -1248,15 +1260,8 @@ int generate_ghosts(gc_ctx* ctx, DGhost& G) {
     a.count = G.d_count;
     a.ginst_params = G.d_inst;
     launch_ghost_flags(a, ctx->stream);
-    int64_t n = G.CAP;
-    int64_t st = scan_tmp_elems(n) + 16;
-    if (st > ctx->cap_scan) {
-        CU(cudaStreamSynchronize(ctx->stream));
-        dfree(ctx, ctx->scan_tmp, ctx->cap_scan);
-        TRY(dalloc(ctx, &ctx->scan_tmp, (size_t)st));
-        ctx->cap_scan = st;
-    }
-    scan_exclusive(G.flags, G.pos, n, ctx->scan_tmp, ctx->stream);
+    TRY(ensure_scan(ctx, G.CAP));
+    scan_exclusive(G.flags, G.pos, G.CAP, ctx->scan_tmp, ctx->stream);
     launch_ghost_fill(a, ctx->stream);
     return check_launch(ctx, "ghost generation");
 }
@@ -1598,12 +1603,13 @@ int ensure_fpk(gc_ctx* ctx, T& X, int64_t N, int nd, int mode, bool fp32) {
     int64_t need = 4 * ((N * nd + 3) / 4 + N * (pos_quads(nd, fp32) + rec_quads(nd, mode, fp32)));
     if (need > X.cap_fpk) {
         CU(cudaStreamSynchronize(ctx->stream));
-        dfree(ctx, X.fpk, X.cap_fpk);
-        TRY(dalloc(ctx, &X.fpk, (size_t)need));
-        X.cap_fpk = need;
-        X.xpk_epoch = -1;  // the new buffer holds no positions and no records yet
+        X.cap_fpk = 0;     // until the new buffer is there,
+        X.xpk_epoch = -1;  // which holds no positions and no records yet
         X.xpk_static = false;
         X.pack_done_epoch = -1;
+        dfree(ctx, X.fpk);
+        TRY(dalloc(ctx, &X.fpk, (size_t)need));
+        X.cap_fpk = need;
     }
     return GC_OK;
 }
@@ -2414,13 +2420,7 @@ int size_capacities(gc_ctx* ctx) {
     // scan scratch for ghost flags and for every capacity-sized scan
     int64_t scan_n = ctx->cap_cells;
     for (auto& G : ctx->ghosts) scan_n = std::max(scan_n, G.CAP);
-    int64_t st = scan_tmp_elems(scan_n) + 16;
-    if (st > ctx->cap_scan) {
-        CU(cudaStreamSynchronize(ctx->stream));
-        dfree(ctx, ctx->scan_tmp, ctx->cap_scan);
-        TRY(dalloc(ctx, &ctx->scan_tmp, (size_t)st));
-        ctx->cap_scan = st;
-    }
+    TRY(ensure_scan(ctx, scan_n));
     // the bound each plan entry is checked against inside the steps
     std::vector<int64_t> cap(n);
     for (size_t s = 0; s < ctx->slots.size(); ++s) cap[s] = cap_sort_cells(ctx);
@@ -2439,8 +2439,9 @@ int snapshot(gc_ctx* ctx, std::vector<char>& par) {
         Snapshot& sn = ctx->snaps[s];
         if (!S.xmoves()) continue;
         if (sn.n != S.N) {
-            for (int f = 0; f < NF; ++f) dfree(ctx, sn.f[f], (size_t)S.ncomp[f] * sn.n);
-            dfree(ctx, sn.id, (size_t)sn.n);
+            sn.n = 0;  // until the new buffers are there
+            for (int f = 0; f < NF; ++f) dfree(ctx, sn.f[f]);
+            dfree(ctx, sn.id);
             for (int f = 0; f < NF; ++f)
                 if (S.ncomp[f]) TRY(dalloc(ctx, &sn.f[f], (size_t)S.ncomp[f] * S.N));
             TRY(dalloc(ctx, &sn.id, (size_t)S.N));
@@ -3349,7 +3350,8 @@ int gc_stage_field(gc_ctx* ctx, int inst, int handle, int field, const void* hos
 static int ensure_staging(gc_ctx* ctx, int64_t doubles) {
     if (doubles > ctx->cap_staging) {
         CU(cudaStreamSynchronize(ctx->stream));
-        dfree(ctx, ctx->staging, ctx->cap_staging);
+        ctx->cap_staging = 0;
+        dfree(ctx, ctx->staging);
         int64_t cap = std::max<int64_t>(doubles, 1 << 16);
         TRY(dalloc(ctx, &ctx->staging, (size_t)cap));
         ctx->cap_staging = cap;
@@ -3437,7 +3439,8 @@ __global__ void k_any_nonzero(const double* __restrict__ a, int64_t n, int* flag
 static int ensure_ioflags(gc_ctx* ctx, int n) {
     if (n > ctx->cap_ioflags) {
         CU(cudaStreamSynchronize(ctx->stream));
-        dfree(ctx, ctx->d_ioflags, (size_t)ctx->cap_ioflags);
+        ctx->cap_ioflags = 0;
+        dfree(ctx, ctx->d_ioflags);
         const int cap = std::max(n, 64);
         TRY(dalloc(ctx, &ctx->d_ioflags, (size_t)cap));
         ctx->cap_ioflags = cap;
@@ -3928,7 +3931,7 @@ int gc_measure_fp64_peak(gc_ctx* ctx, double* tflops_out) {
     CU(cudaEventElapsedTime(&ms, a, b));
     cudaEventDestroy(a);
     cudaEventDestroy(b);
-    dfree(ctx, out, 1);
+    dfree(ctx, out);
     double flops = 2.0 * 8.0 * (double)iters * threads * blocks;
     *tflops_out = flops / (ms * 1e-3) / 1e12;
     return GC_OK;
@@ -3954,7 +3957,7 @@ int gc_measure_fp32_peak(gc_ctx* ctx, double* tflops_out) {
     CU(cudaEventElapsedTime(&ms, a, b));
     cudaEventDestroy(a);
     cudaEventDestroy(b);
-    dfree(ctx, out, 1);
+    dfree(ctx, out);
     double flops = 2.0 * 8.0 * (double)iters * threads * blocks;
     *tflops_out = flops / (ms * 1e-3) / 1e12;
     return GC_OK;
@@ -4216,7 +4219,7 @@ int ctx_pack_fill(PackJob* J, gc_ctx* ctx, std::string* err) {
         if (dalloc(ctx, &d_seg, tab.size()) != GC_OK) return fail(GC_ERR_OOM);
         if (cudaMemcpyAsync(d_seg, tab.data(), sizeof(PackSeg) * tab.size(), cudaMemcpyHostToDevice, ctx->stream) !=
             cudaSuccess) {
-            dfree(ctx, d_seg, tab.size());
+            dfree(ctx, d_seg);
             return fail(seterr(ctx, GC_ERR_CUDA, "pack table upload"));
         }
         for (const Launch& L : launches) {
@@ -4228,7 +4231,7 @@ int ctx_pack_fill(PackJob* J, gc_ctx* ctx, std::string* err) {
         }
         // the host table lives until the copy has run
         cudaStreamSynchronize(ctx->stream);
-        dfree(ctx, d_seg, tab.size());
+        dfree(ctx, d_seg);
     }
     int st = check_launch(ctx, "pack");
     if (st) return fail(st);
