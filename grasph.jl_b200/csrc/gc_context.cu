@@ -1417,6 +1417,7 @@ int64_t cap_grid_cells(gc_ctx* ctx, const DInter& D) { return std::min(D.cap_cel
 // to size every buffer; capacity mode sizes from the buffers' capacities
 // (no host read), and the kernels flag any plan that does not fit.
 // half: the moving systems' half steps are part of their sorts.
+int size_step(gc_ctx* ctx, const std::vector<int64_t>& need);
 int prepare(gc_ctx* ctx, const std::vector<char>& sort_mask, bool half) {
     const int ni = ninst(ctx);
     // bounding boxes of every real system (positions are current); a system
@@ -1445,6 +1446,7 @@ int prepare(gc_ctx* ctx, const std::vector<char>& sort_mask, bool half) {
             need[i] = ctx->h_need[i];
             ctx->need_max[i] = std::max(ctx->need_max[i], need[i]);
         }
+        TRY(size_step(ctx, need));
     }
     // sorts
     for (size_t s = 0; s < ctx->slots.size(); ++s)
@@ -1807,6 +1809,34 @@ std::vector<std::vector<int>> stage_groups(gc_ctx* ctx, int a, int stage) {
             out.emplace_back(ids.begin() + off, ids.begin() + std::min(ids.size(), off + MAX_REFS));
     }
     return out;
+}
+
+// Every buffer of an exact step, before anything is sorted or moved: a step
+// that does not fit leaves the state as it was.
+int size_step(gc_ctx* ctx, const std::vector<int64_t>& need) {
+    TRY(ensure_cells(ctx, *std::max_element(need.begin(), need.end())));
+    for (auto& G : ctx->ghosts) TRY(ensure_scan(ctx, G.CAP));
+    for (auto& D : ctx->inters)
+        if (!D.probe) TRY(ensure_inter_cells(ctx, D, need[D.need_slot]));
+    for (int stage = 1; stage <= ctx->nstages; ++stage)
+        for (size_t a = 0; a < ctx->slots.size(); ++a)
+            for (auto& ids : stage_groups(ctx, (int)a, stage)) {
+                const PackPlan pl = pack_plan(ctx, (int)a, ids, stage, false);
+                if (!pl.records) continue;
+                DSlot& S = ctx->slots[a];
+                TRY(ensure_fpk(ctx, S, S.N, S.nd, pl.mode, pl.fp32));
+                for (int id : ids) {
+                    DInter& D = ctx->inters[id];
+                    if (D.btype == BT_GHOST) {
+                        DGhost& G = ctx->ghosts[D.bghost];
+                        TRY(ensure_fpk(ctx, G, G.CAP, G.nd, pl.mode, pl.fp32));
+                    } else if (D.btype != BT_SELF) {
+                        DSlot& B = ctx->slots[D.bslot];
+                        TRY(ensure_fpk(ctx, B, B.N, B.nd, pl.mode, pl.fp32));
+                    }
+                }
+            }
+    return GC_OK;
 }
 
 int sweep_group(gc_ctx* ctx, int a, const std::vector<int>& ids, int stage, bool count_only) {

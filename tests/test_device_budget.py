@@ -90,3 +90,21 @@ def test_a_step_that_does_not_fit_fails_again(kind):
             _fits(lambda: s.create_grid(si))  # noqa: B023
             assert not _step(s)
     assert met > 5
+
+
+@pytest.mark.parametrize("kind", ["water", "soil"])
+def test_a_step_that_does_not_fit_leaves_the_state(kind):
+    met = 0
+    for lf, s in _tight(kind):
+        met += 1
+        before = {}
+        for ps in lf.systems:
+            order = np.argsort(ps.id)
+            before[ps.name] = {f: np.array(getattr(ps, f))[order] for f, _ in ps.particle_fields()}
+        assert not _step(s)
+        s.pull()
+        for ps in lf.systems:
+            order = np.argsort(ps.id)
+            for f, _ in ps.particle_fields():
+                assert np.array_equal(getattr(ps, f)[order], before[ps.name][f]), f"{ps.name} {f}"
+    assert met > 5
