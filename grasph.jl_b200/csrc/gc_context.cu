@@ -2004,6 +2004,7 @@ int sweep_group(gc_ctx* ctx, int a, const std::vector<int>& ids, int stage, bool
     }
     if (tune_slot >= 0) CU(cudaEventRecord(ctx->tune_ev[tune_slot].first, ctx->stream));
     int st = launch_force_f64(A, count_only, ctx->stream);
+    if (st == GC_ERR_CUDA) return check_launch(ctx, "sweep");
     if (st) return seterr(ctx, st, "functor/system combination not implemented on the device");
     if (tune_slot >= 0) CU(cudaEventRecord(ctx->tune_ev[tune_slot].second, ctx->stream));
     if (e1)
@@ -2058,6 +2059,7 @@ int sweep_group(gc_ctx* ctx, int a, const std::vector<int>& ids, int stage, bool
         r.brec = records ? rec_of(S.fpk, S.N, S.nd) : nullptr;
         r.brq = rec_quads(S.nd, mode, fp32);
         st = launch_force_f64(R, false, ctx->stream);
+        if (st == GC_ERR_CUDA) return check_launch(ctx, "sweep (system_b side)");
         if (st) return seterr(ctx, st, "two-sided functor not implemented on the device");
         TRY(check_launch(ctx, "sweep (system_b side)"));
     }

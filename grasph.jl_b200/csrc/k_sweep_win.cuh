@@ -423,7 +423,7 @@ __global__ void __launch_bounds__(WIN_TPB, MINB) k_sweep_win(ForceArgs A) {
 constexpr size_t sm_share(int blocks) { return (size_t)(228 * 1024 / (blocks < 2 ? 2 : blocks) - 2048); }
 
 template <class Phys, int ND, int PFN, int C>
-static void launch_win(const ForceArgs& A, cudaStream_t s) {
+static int launch_win(const ForceArgs& A, cudaStream_t s) {
     constexpr WinCfg cf = Phys::EXACT ? WIN_CFGS64[C] : WIN_CFGS32[C];
     int64_t blocks = (A.aN * 32 + WIN_TPB - 1) / WIN_TPB;
     if (blocks > (int64_t)A.num_sms * cf.minb * 4) blocks = (int64_t)A.num_sms * cf.minb * 4;
@@ -437,25 +437,27 @@ static void launch_win(const ForceArgs& A, cudaStream_t s) {
     // water, 8 blocks an SM at most: step 107 us; 5, 4 or 3: 93; 2: 96.
     size_t smem = need;
     if (A.sm_blocks && A.sm_blocks < cf.minb) smem = std::max(need, sm_share(A.sm_blocks));
-    if constexpr (cf.minb > 2) {
-        static const cudaError_t opted = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                                              (int)std::max(need, sm_share(2)));
-        (void)opted;
-    }
+    // Beyond 48 KB a block asks for it.  The attribute belongs to the current
+    // device, and a process may have contexts on several: set at every such
+    // launch (captured steps launch once), always to the most of this kernel.
+    if (smem > 48 * 1024 &&
+        cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)std::max(need, sm_share(2))) !=
+            cudaSuccess)
+        return GC_ERR_CUDA;
     kern<<<(int)blocks, WIN_TPB, smem, s>>>(A);
     g_launches.fetch_add(1, std::memory_order_relaxed);
+    return 0;
 }
 
 template <template <int, int, int, int> class Phys, int ND, int NS, int PFN, int KK>
 static int launch_win_cfg(const ForceArgs& A, cudaStream_t s) {
     using P = Phys<ND, NS, PFN, KK>;
     switch (A.cfg) {
-        case 1: launch_win<P, ND, PFN, 1>(A, s); break;
-        case 2: launch_win<P, ND, PFN, 2>(A, s); break;
-        case 3: launch_win<P, ND, PFN, 3>(A, s); break;
-        default: launch_win<P, ND, PFN, 0>(A, s); break;
+        case 1: return launch_win<P, ND, PFN, 1>(A, s);
+        case 2: return launch_win<P, ND, PFN, 2>(A, s);
+        case 3: return launch_win<P, ND, PFN, 3>(A, s);
+        default: return launch_win<P, ND, PFN, 0>(A, s);
     }
-    return 0;
 }
 
 // The window sweep of A.pfn; GC_ERR_UNSUPPORTED for any other functor or
