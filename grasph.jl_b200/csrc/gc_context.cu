@@ -2588,6 +2588,10 @@ int capture_step(gc_ctx* ctx, StepGraph& g) {
         if (graph) cudaGraphDestroy(graph);
         cudaGetLastError();
         set_parity(ctx, g.pre);
+        for (auto& S : ctx->slots) {  // what it packed never ran
+            S.xpk_epoch = S.pack_done_epoch = -1;
+            S.xpk_static = false;
+        }
         if (st != GC_OK) return st;
         return seterr(ctx, GC_ERR_CUDA, "step capture: %s", cudaGetErrorString(e));
     }

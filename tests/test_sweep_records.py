@@ -126,3 +126,41 @@ def test_single_sweep_after_a_step(precision, wall):
     s.push()
     sweep(got, s)
     _equal(got, want)
+
+
+@pytest.mark.parametrize("first,then", [PRECISIONS, PRECISIONS[::-1]])
+def test_precision_changed_between_captured_steps(first, then):
+    """(the capture of the first step in the other precision is given up when
+    a record buffer has to grow, and what it had only recorded never ran)"""
+    def build():
+        rng = np.random.default_rng(8)
+        g = np.stack([a.ravel() for a in np.meshgrid(*[np.arange(m) for m in (6, 5, 6)], indexing="ij")], axis=1)
+        s = G.ElastoPlasticParticleSystem("s", len(g), 3, 6, 1000.0 * DX ** 3, C0)
+        s.x[:] = g * DX + rng.uniform(-2e-3, 2e-3, g.shape) + [0.0, 0.0, DX]
+        s.v[:] = rng.uniform(-1.0, 1.0, g.shape)
+        s.rho[:] = rng.uniform(990.0, 1010.0, s.n)
+        s.stress[:] = rng.uniform(-300.0, 100.0, s.stress.shape)
+        w = G.BasicParticleSystem("w", 60, 3, 1.0, C0)
+        w.x[:] = g[g[:, 2] < 2] * DX - [0.0, 0.0, DX + 1e-3]
+        w.rho[:] = 1000.0
+        pfns = (G.StrainRateVorticityPfn(), G.CauchyFluidPfn(0.1, 0.1, H))
+        k = G.CubicSplineKernel(H, ndims=3)
+        return G.LeapFrogTimeIntegrator([s, w], [
+            G.SystemInteraction(k, pfns, s),
+            G.SystemInteraction(k, pfns, s, G.DynamicBoundarySystem(w, [0.0, 0.0, 1.0], [0.0, 0.0, 0.0], 1.5))])
+
+    got, want = build(), build()
+    s = _session(got, first)
+    s.step(24, 1e-4)  # past the tuner, into captured steps
+    assert s.stats()["graph_steps"] > 0
+    s.pull()
+    for ps, to in zip(want.systems, got.systems):
+        for f, _ in ps.particle_fields():
+            getattr(ps, f)[:] = getattr(to, f)
+    s.backend.set_precision(then)
+    s.step(1, 1e-4)
+    s.pull()
+    t = _session(want, then)
+    t.step(1, 1e-4)
+    t.pull()
+    _equal(got, want)
