@@ -2026,6 +2026,7 @@ int sweep_group(gc_ctx* ctx, int a, const std::vector<int>& ids, int stage, bool
         ForceArgs R = A;
         R.groups = B.groups;
         R.ngroups = B.d_ngroups;
+        R.sm_blocks = B.sm_blocks;
         R.nd = B.nd;
         R.ns = B.ns;
         R.aN = B.N;
