@@ -464,6 +464,14 @@ double kernel_norm(int kind, int nd, double H) {
     return 21.0 / ((256.0 * pi) * (H * H * H));
 }
 
+// The factor of a kernel's gradient that all pairs share (GridInst.kq).
+long double gradient_factor(int kind, int nd, double H) {
+    const long double pi = 3.14159265358979323846264338327950288L, h = H, hd = nd == 3 ? h * h * h : nd == 2 ? h * h : h;
+    if (kind == GC_KERNEL_CUBIC_SPLINE)
+        return -3.0L * (nd == 3 ? 1.0L / pi : nd == 2 ? 10.0L / (7.0L * pi) : 2.0L / 3.0L) / (hd * h);
+    return -10.0L * (nd == 3 ? 21.0L / (256.0L * pi) : 7.0L / (64.0L * pi)) / (hd * h * h);
+}
+
 // Does stage `stage` (1-based; nstages + 1 is the velocity-adjust functor)
 // of an interaction also write system_b?  XSPHPfn's coupled form writes every
 // system_b kind: a wrapper's system, or a ghost's source at the ghost index.
@@ -916,7 +924,12 @@ int finalize(gc_ctx* ctx) {
             G.inv_cell = 1.0 / G.cell;
             const bool spline = h.kk == GC_KERNEL_CUBIC_SPLINE;
             G.f_qs = (float)(spline ? 0.5 / h.H : 1.0 / h.H);
-            G.kq = spline ? -3.0 * G.knorm / h.H : -10.0 * G.knorm / (h.H * h.H);
+            const long double kq = gradient_factor(h.kk, I.sys[h.a].nd, h.H);
+            G.kq = (double)kq;
+            G.kq_lo = (double)(kq - (long double)G.kq);
+            const long double qs = (spline ? 0.5L : 1.0L) / (long double)h.H;
+            G.qs = (double)qs;
+            G.qs_lo = (double)(qs - (long double)G.qs);
             if (h.b >= 0) {
                 const HHandle& hh = I.handles[h.b];
                 for (int d = 0; d < 3; ++d) {

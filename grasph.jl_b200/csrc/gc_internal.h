@@ -48,9 +48,10 @@ struct GridInst {
     double cutoff_sq;                  // (2h)^2
     double inv_cell;                   // 1/(2h), rounded
     double knorm;                      // kernel normalisation
-    // FP32-compensated sweep: the kernel's gradient and argument factors
-    // (cubic spline −3·knorm/h and 1/2h, Wendland C2 −10·knorm/h² and 1/h)
-    double kq;
+    // Window sweep: the kernel's gradient and argument factors (cubic spline
+    // −3·norm/h and 1/2h, Wendland C2 −10·norm/h² and 1/h), each the sum of two
+    // doubles, the second also in FP32
+    double kq, kq_lo, qs, qs_lo;
     float f_qs;
     double ming[MAXD];                 // grid origin (src/Interaction.jl:143)
     int64_t ng[MAXD];                  // cells per dimension (:179)

@@ -213,9 +213,11 @@ struct PhysF32 {
         const float s = j & 1 ? a.s[j >> 1].y : a.s[j >> 1].x, c = j & 1 ? a.c[j >> 1].y : a.c[j >> 1].x;
         return (double)s + (double)c;
     }
-    // The sums, times `f` in FP64, onto system_a's rates.
-    static __device__ __forceinline__ void store(const ForceArgs& A, int64_t gi, const Acc& acc, double f) {
+    // The sums, times kf in FP64, onto system_a's rates.
+    static __device__ __forceinline__ void store(const ForceArgs& A, const InterRef&, const GridInst&, int, const Par& p,
+                                                 int64_t gi, const Acc& acc) {
         const int64_t N = A.aN;
+        const double f = p.kf;
         // one lane alone adds to a word, in order, so fire-and-forget reductions
         // give the bits of a load, an add and a store without waiting for the load
         auto put = [&](double* to, int q, double x) { atomicAdd(to + q * N + gi, x); };

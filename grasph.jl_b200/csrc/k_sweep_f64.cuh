@@ -93,11 +93,8 @@ struct PhysF64 {
 
     struct Par {
         double cut, sure;    // (2h)²; below `sure` the strip range cannot matter
-        double qs;           // kernel argument's factor
-        // the gradient's, with the term's mass, by which the sums are multiplied
-        // at the end; a Lennard-Jones wall's terms take it one by one (kq, with
-        // kf = 1), as its mass, which may be 0, is not the force's
-        double kq, kf;
+        double qs, qs_lo;    // kernel argument's factor
+        double kq;           // the gradient's factor with system_b's mass (Lennard-Jones wall)
         double eps, am, beta;  // 0.01·h², α·c̄·h, β·h² of the artificial viscosity
         double dd;             // 2·δ·c̄·h of the density diffusion (0: none)
         double c;              // system_a's sound speed
@@ -109,22 +106,20 @@ struct PhysF64 {
         p.bt = r.btype;
         p.cut = G.cutoff_sq;
         p.sure = G.cutoff_sq * (1.0 - strip_doubt<ND>(G));
-        p.qs = KK == GC_KERNEL_CUBIC_SPLINE ? G.inv_cell : 2.0 * G.inv_cell;
-        p.kf = G.kq;
+        p.qs = G.qs;
+        p.qs_lo = G.qs_lo;
         p.eps = p.am = p.beta = p.dd = 0.0;
         if (FLUID || CAUCHY) {
             const double ca = A.a_c[k];
             p.c = ca;
             const bool two = PFN == PFN_FLUID2 && P.two;
             const double cm = (CAUCHY && r.btype == BT_GHOST) || two ? 0.5 * (ca + G.bc) : ca;
-            p.kf *= r.btype == BT_SELF || r.btype == BT_DYNAMIC ? A.a_mass[k] : G.bmass;
             p.eps = (P.h * P.h) * 0.01;
             p.am = P.alpha * cm * P.h;
             p.beta = P.beta * P.h * P.h;
             if (P.has_delta) p.dd = 2.0 * P.delta * (two ? cm : ca) * P.h;
         }
-        p.kq = p.kf;
-        if ((FLUID || CAUCHY) && r.btype == BT_STATIC) p.kf = 1.0;
+        p.kq = G.kq * G.bmass;
         return p;
     }
     static __device__ __forceinline__ bool diffuses(const Par& p) { return p.dd != 0.0; }
@@ -136,11 +131,15 @@ struct PhysF64 {
         const double r = rr * ri;
         if (KK == GC_KERNEL_CUBIC_SPLINE) {
             // −3·(¼(2−q)² − (1−q)²): with s = q/2, −3·((1−s)² − (1−2s)²)
-            const double s = r * p.qs, a = 1.0 - s, b = fma(-2.0, s, 1.0);
+            // (1/2h in two parts: rounded once, it would shift every pair's alike.
+            // With the sums' factor in two, FP64 errors of one sweep against long
+            // double 5-35% below what they were, and no larger than separately
+            // rounded square roots and divisions gave; 1.4% of the sweep.)
+            const double a0 = fma(-r, p.qs, 1.0), a = fma(-r, p.qs_lo, a0), b = fma(2.0, a0, -1.0);
             const double bb = b > 0.0 ? b * b : 0.0;
             return ri * fma(a, a, -bb);
         } else {
-            const double a = fma(-r, p.qs, 2.0);
+            const double a = fma(-r, p.qs_lo, fma(-r, p.qs, 2.0));
             return a * a * a;
         }
     }
@@ -181,10 +180,30 @@ struct PhysF64 {
         if (dot_exact<ND>(d, d) == 0.0) spoil(p, a);
         return false;
     }
-    static __device__ __forceinline__ void store(const ForceArgs& A, int64_t gi, const Acc& acc, double f) {
+    // The sums' factor, f + lo: the gradient's, with the terms' mass for dv/dt
+    // and dρ/dt.  A Lennard-Jones wall's terms carry it themselves (its mass,
+    // which may be 0, is not the force's).  Both halves: rounded once, it would
+    // put its error on every sum alike.
+    static __device__ __forceinline__ void factor(const ForceArgs& A, const InterRef& r, const GridInst& G, int k,
+                                                  double& f, double& lo) {
+        f = G.kq;
+        lo = G.kq_lo;
+        if (!FLUID && !CAUCHY) return;
+        const double m = r.btype == BT_SELF || r.btype == BT_DYNAMIC ? A.a_mass[k] : G.bmass, t = f * m;
+        lo = fma(f, m, -t) + lo * m;
+        f = t;
+        if (r.btype == BT_STATIC) {
+            f = 1.0;
+            lo = 0.0;
+        }
+    }
+    static __device__ __forceinline__ void store(const ForceArgs& A, const InterRef& r, const GridInst& G, int k,
+                                                 const Par&, int64_t gi, const Acc& acc) {
         const int64_t N = A.aN;
+        double f, lo;
+        factor(A, r, G, k, f, lo);
         // (reductions, as in the FP32 policy)
-        auto put = [&](double* to, int q, double x) { atomicAdd(to + q * N + gi, f * x); };
+        auto put = [&](double* to, int q, double x) { atomicAdd(to + q * N + gi, fma(f, x, lo * x)); };
         auto m = [&](int a, int b) { return acc.s[(a * ND + b) % NSUM]; };
         if (FLUID || CAUCHY) {
 #pragma unroll
@@ -323,9 +342,10 @@ struct PhysF64 {
                     // xx yy zz xy xz yz
                     constexpr int Y = NSA > 1 ? 1 : 0, Z = NSA > 2 ? 2 : 0, XY = NSA > 3 ? 3 : 0, XZ = NSA > 4 ? 4 : 0,
                                   YZ = NSA > 5 ? 5 : 0;
-                    acc.s[0] = fma(a[0] - pi, w[0], fma(a[XY], w[1], fma(a[XZ], w[ND - 1], acc.s[0])));
-                    acc.s[1] = fma(a[XY], w[0], fma(a[Y] - pi, w[1], fma(a[YZ], w[ND - 1], acc.s[1])));
-                    acc.s[ND - 1] = fma(a[XZ], w[0], fma(a[YZ], w[1], fma(a[Z] - pi, w[ND - 1], acc.s[ND - 1])));
+                    // (a term is rounded to the sum's precision once, not product by product)
+                    acc.s[0] += fma(a[0] - pi, w[0], fma(a[XY], w[1], a[XZ] * w[ND - 1]));
+                    acc.s[1] += fma(a[XY], w[0], fma(a[Y] - pi, w[1], a[YZ] * w[ND - 1]));
+                    acc.s[ND - 1] += fma(a[XZ], w[0], fma(a[YZ], w[1], (a[Z] - pi) * w[ND - 1]));
                 }
                 *dr = fma(g, q, *dr);
             }

@@ -409,7 +409,7 @@ __global__ void __launch_bounds__(WIN_TPB, MINB) k_sweep_win(ForceArgs A) {
                         }
                     }
                 }
-                if (active) Phys::store(A, gi, acc, par.kf);
+                if (active) Phys::store(A, r, G, k, par, gi, acc);
             }
             __syncwarp();
             if (active && r.counts) r.counts[gi] = accepted;
