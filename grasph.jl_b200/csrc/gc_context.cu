@@ -333,6 +333,11 @@ struct gc_ctx {
     int64_t* d_need_cap = nullptr;  // per plan entry, the cells capacity mode sizes for
     PlanItem* d_plans = nullptr;  // the steps' plans, one per entry of d_need
     unsigned long long* d_gscratch = nullptr;  // launch_groups' scratch
+    // what FP32 positions count from (launch_plan_all)
+    double* d_origin = nullptr;
+    double2* d_spacing = nullptr;
+    OriginSlot* d_origin_slots = nullptr;
+    std::vector<OriginSlot> origin_slots;
     std::vector<Snapshot> snaps;    // per slot (moving slots only)
     int64_t graph_steps = 0, rollbacks = 0;
     int64_t pack_epoch = 0;  // bumps at the start of every issued step and single sweep (never rolled back)
@@ -1091,6 +1096,19 @@ int finalize(gc_ctx* ctx) {
         TRY(hcopy(ctx, ctx->d_plans, items.data(), items.size() * sizeof(PlanItem), cudaMemcpyHostToDevice));
         TRY(dalloc(ctx, &ctx->d_gscratch, 2));
         CU(cudaMemsetAsync(ctx->d_gscratch, 0, 2 * sizeof(unsigned long long), ctx->stream));
+        std::vector<double2> spacing(ctx->inst.size());
+        for (size_t k = 0; k < spacing.size(); ++k) {
+            double cell = 0.0;
+            for (auto& it : ctx->inst[k].inters) cell = std::max(cell, 2.0 * it.H);
+            int e = 0;
+            frexp(cell, &e);  // cell < 2^e
+            spacing[k].x = ldexp(1.0, e + ORIGIN_CELLS_LOG2);
+            spacing[k].y = ldexp(1.0, -e - ORIGIN_CELLS_LOG2);
+        }
+        TRY(dalloc(ctx, &ctx->d_spacing, spacing.size()));
+        TRY(hcopy(ctx, ctx->d_spacing, spacing.data(), spacing.size() * sizeof(double2), cudaMemcpyHostToDevice));
+        TRY(dalloc(ctx, &ctx->d_origin, spacing.size() * MAXD));
+        TRY(dalloc(ctx, &ctx->d_origin_slots, ctx->slots.size()));
     }
     ctx->finalized = true;
     return GC_OK;
@@ -1444,8 +1462,12 @@ int prepare(gc_ctx* ctx, const std::vector<char>& sort_mask, bool half) {
             const size_t s = (size_t)(i0 + i);  // ghosts follow the slots
             if (s >= ctx->slots.size() || sort_mask[s]) mask.w[i >> 6] |= 1ull << (i & 63);
         }
+        OriginArgs org{};
+        if (i0 == 0)
+            org = OriginArgs{ctx->d_origin_slots, (int)ctx->origin_slots.size(), ctx->slots[0].nd, ctx->d_spacing,
+                             ctx->d_origin};
         launch_plan_all(ctx->d_plans + i0, n, ni, mask, ctx->d_need + i0, ctx->capmode ? ctx->d_need_max + i0 : nullptr,
-                        ctx->d_need_cap + i0, ctx->d_err, ctx->stream);
+                        ctx->d_need_cap + i0, ctx->d_err, org, ctx->stream);
     }
     TRY(check_launch(ctx, "plan"));
     std::vector<int64_t> need(ctx->nneed);
@@ -1866,7 +1888,7 @@ int sweep_group(gc_ctx* ctx, int a, const std::vector<int>& ids, int stage, bool
                           S.pack_done_mode == mode && S.pack_done_ns == pk_ns && S.pack_done_fp32 == fp32;
         if (!done) {
             launch_pack(fp32, mode, S.N, nullptr, S.nd, pk_ns, S.F(F_X), S.F(F_V), S.F(F_RHO), S.F(F_P),
-                        S.F(F_STRESS), S.inst_of, S.d_mass, hpos_of(S.fpk), nullptr, rec_of(S.fpk, S.N, S.nd),
+                        S.F(F_STRESS), S.inst_of, S.d_mass, ctx->d_origin, hpos_of(S.fpk), nullptr, rec_of(S.fpk, S.N, S.nd),
                         ctx->stream);
             S.pack_done_epoch = -1;  // no longer the half step's: a later functor of its mode packs again
         }
@@ -1899,6 +1921,7 @@ int sweep_group(gc_ctx* ctx, int a, const std::vector<int>& ids, int stage, bool
     A.a_mass = S.d_mass;
     A.a_cf = S.d_cf;
     A.arec = records ? rec_of(S.fpk, S.N, S.nd) : nullptr;
+    A.origin = ctx->d_origin;
     A.prec = fp32 ? GC_PRECISION_FP32_COMPENSATED : GC_PRECISION_FP64;
     A.err = ctx->d_err;
     A.num_sms = ctx->num_sms;
@@ -1956,7 +1979,7 @@ int sweep_group(gc_ctx* ctx, int a, const std::vector<int>& ids, int stage, bool
             if (records) {
                 TRY(ensure_fpk(ctx, G, G.CAP, G.nd, mode, fp32));
                 launch_pack(fp32, mode, G.CAP, G.d_count, G.nd, pk_ns, G.x[G.cur], G.v, G.rho, G.p, G.stress,
-                            G.ginst[G.cur], G.d_mass, hpos_of(G.fpk), nullptr, rec_of(G.fpk, G.CAP, G.nd),
+                            G.ginst[G.cur], G.d_mass, ctx->d_origin, hpos_of(G.fpk), nullptr, rec_of(G.fpk, G.CAP, G.nd),
                             ctx->stream);
                 r.bh = hpos_of(G.fpk);
                 r.brec = rec_of(G.fpk, G.CAP, G.nd);
@@ -1983,7 +2006,7 @@ int sweep_group(gc_ctx* ctx, int a, const std::vector<int>& ids, int stage, bool
                 const bool pos = !rec && (B.xpk_fp32 != fp32 ||
                                           (B.xmoves() ? B.xpk_epoch != ctx->pack_epoch : !B.xpk_static));
                 launch_pack(fp32, mode, B.N, nullptr, B.nd, pk_ns, B.F(F_X), B.F(F_V), B.F(F_RHO), B.F(F_P),
-                            B.kind >= GC_SYS_STRESS ? B.F(F_STRESS) : nullptr, B.inst_of, B.d_mass, hpos_of(B.fpk),
+                            B.kind >= GC_SYS_STRESS ? B.F(F_STRESS) : nullptr, B.inst_of, B.d_mass, ctx->d_origin, hpos_of(B.fpk),
                             pos ? pos_of(B.fpk, B.N, B.nd) : nullptr, rec ? rec_of(B.fpk, B.N, B.nd) : nullptr,
                             ctx->stream);
                 r.bh = hpos_of(B.fpk);
@@ -2248,7 +2271,7 @@ int gather_halfstep(gc_ctx* ctx, DSlot& S) {
             if (pl.records) {
                 TRY(ensure_fpk(ctx, S, S.N, S.nd, pl.mode, pl.fp32));
                 pk = PackArgs{pl.fp32, pl.mode, S.nd, pl.pk_ns, S.N, S.F(F_X), S.F(F_V), S.F(F_RHO), S.F(F_P),
-                              S.F(F_STRESS), S.inst_of, S.d_mass, hpos_of(S.fpk), nullptr,
+                              S.F(F_STRESS), S.inst_of, S.d_mass, ctx->d_origin, hpos_of(S.fpk), nullptr,
                               rec_of(S.fpk, S.N, S.nd)};
                 S.pack_done_epoch = ctx->pack_epoch;
                 S.pack_done_stage = 1;
@@ -2403,6 +2426,19 @@ void drop_graphs(gc_ctx* ctx) {
 void invalidate_steps(gc_ctx* ctx) {
     drop_graphs(ctx);
     ctx->exact_done = false;
+    for (auto& S : ctx->slots) S.xpk_static = false;  // may count from another point
+}
+
+// The systems at rest, for the steps' plans.
+int push_motion(gc_ctx* ctx) {
+    std::vector<OriginSlot> now;
+    for (auto& S : ctx->slots)
+        if (!S.probe) now.push_back(OriginSlot{S.d_inst, !S.xmoves()});
+    bool same = now.size() == ctx->origin_slots.size();
+    for (size_t i = 0; same && i < now.size(); ++i) same = now[i].still == ctx->origin_slots[i].still;
+    if (same) return GC_OK;
+    ctx->origin_slots = now;
+    return hcopy(ctx, ctx->d_origin_slots, now.data(), now.size() * sizeof(OriginSlot), cudaMemcpyHostToDevice);
 }
 
 std::vector<char> parity(gc_ctx* ctx) {
@@ -2876,6 +2912,9 @@ int gc_ctx_destroy(gc_ctx* ctx) {
     dev_free(ctx, ctx->d_need_cap);
     dev_free(ctx, ctx->d_plans);
     dev_free(ctx, ctx->d_gscratch);
+    dev_free(ctx, ctx->d_origin);
+    dev_free(ctx, ctx->d_spacing);
+    dev_free(ctx, ctx->d_origin_slots);
     if (ctx->h_need_max) cudaFreeHost(ctx->h_need_max);
     drop_graphs(ctx);
     for (auto& sn : ctx->snaps) {
@@ -3687,6 +3726,7 @@ int gc_step(gc_ctx* ctx, int nsteps, double cfl) {
         ctx->params_dirty = false;
     }
     if (decide_motion(ctx)) invalidate_steps(ctx);
+    TRY(push_motion(ctx));
     CU(cudaMemsetAsync(ctx->d_err, 0, sizeof(int), ctx->stream));
     TRY(run_steps(ctx, nsteps));
     return finish_status(ctx);

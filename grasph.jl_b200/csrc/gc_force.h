@@ -64,6 +64,7 @@ struct ForceArgs {
     const double* a_mass;  // per-instance particle mass
     const float* a_cf;     // FP32 copy of the sound speed
     const float4* arec;    // sweep records of system_a
+    const double* origin;  // per instance, the point that FP32 positions count from
     int prec;              // GC_PRECISION_*
     int* err;
     const int2* groups;        // warp groups of system_a particles (group_of)
@@ -119,11 +120,15 @@ __host__ __device__ constexpr int rec_quads(int nd, int mode, bool fp32) {
                 : nd + (mode == AUX_INV_RHO2 ? (nd == 2 ? 3 : 4) : mode == AUX_MASS_OVER_RHO ? 1 : 2);
 }
 __host__ __device__ constexpr int pos_quads(int nd, bool) { return nd == 2 ? 1 : 2; }
+// The FP32-compensated sweep's positions (h, l and hpos) count from a point of
+// their instance, origin[instance·MAXD + d] (launch_plan_all): FP32 is as good
+// in a domain far from the origin as next to it.  FP64 records and their hpos
+// hold the positions themselves.
 // hpos: the positions rounded to FP32, planar (the candidate test reads
 // these).  Nothing is written without pos or rec, either of which may be
 // nullptr; p and stress may be nullptr (zeros).
 void launch_pack(bool fp32, int mode, int64_t N, const int64_t* count, int nd, int ns, const double* x,
                  const double* v, const double* rho, const double* p, const double* stress, const int32_t* inst_of,
-                 const double* mass, float* hpos, float4* pos, float4* rec, cudaStream_t s);
+                 const double* mass, const double* origin, float* hpos, float4* pos, float4* rec, cudaStream_t s);
 
 }  // namespace gc

@@ -109,9 +109,24 @@ constexpr int PLAN_MAX = 256;  // entries per launch
 struct PlanMask {
     uint64_t w[PLAN_MAX / 64];  // which sorts to plan
 };
+// The point of each instance that its FP32 positions count from: the multiple
+// of a spacing (spacing[k].x, .y its inverse; powers of two) nearest to the
+// middle of its systems at rest, or of all where none is.  It follows from the
+// step's state alone, and records of a system at rest stay good.
+struct OriginSlot {
+    const SysInst* inst;  // boxes
+    int still;
+};
+struct OriginArgs {
+    const OriginSlot* slots;  // nullptr: not computed
+    int nslots, nd;
+    const double2* spacing;
+    double* origin;  // MAXD an instance
+};
+constexpr int ORIGIN_CELLS_LOG2 = 12;  // the spacing in cells, at least
 // need_max, need_cap: capacity mode (nullptr otherwise).
 void launch_plan_all(const PlanItem* items, int n, int ninst, const PlanMask& mask, int64_t* need, int64_t* need_max,
-                     const int64_t* need_cap, int* err, cudaStream_t s);
+                     const int64_t* need_cap, int* err, const OriginArgs& org, cudaStream_t s);
 // cell histogram of the particles of one slot on an interaction's grid
 // (skip: optional device flag; when set, the launch returns at once).
 void launch_grid_count(const double* x, int64_t N, int nd, const int32_t* inst_of, const int64_t* count,

@@ -86,6 +86,7 @@ __device__ __forceinline__ void pack_one(const PackArgs& a, int64_t g) {
 #pragma unroll
     for (int d = 0; d < MAXD; ++d) {
         x[d] = d < a.nd ? a.x[d * N + g] : 0.0;
+        if (a.fp32) x[d] -= a.origin[a.inst_of[g] * MAXD + d];
         h[d] = (float)x[d];
         l[d] = (float)(x[d] - (double)h[d]);
     }

@@ -38,7 +38,7 @@ struct PackArgs {
     int64_t N;
     const double *x, *v, *rho, *p, *stress;
     const int32_t* inst_of;
-    const double* mass;
+    const double *mass, *origin;
     float* hpos;
     float4 *pos, *rec;
 };

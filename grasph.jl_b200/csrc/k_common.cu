@@ -935,10 +935,38 @@ __device__ void ghost_bound_block(const GhostBound& g, int ninst) {
 // largest plan so far and the check against the capacity.  One launch in
 // place of a clear, a launch per sorted system and ghost set, the grids' and
 // the check's: each took about 2 us of the step's chain.
-__global__ void k_plan_all(const PlanItem* __restrict__ items, int ninst, PlanMask mask, int64_t* need,
-                           int64_t* need_max, const int64_t* need_cap, int* err) {
+__device__ void origin_block(const OriginArgs& a, int ninst) {
+    for (int k = threadIdx.x; k < ninst; k += blockDim.x) {
+        double lo[MAXD], hi[MAXD];
+        bool any = false;
+        for (int all = 0; all < 2 && !any; ++all) {
+            for (int s = 0; s < a.nslots; ++s) {
+                const SysInst& S = a.slots[s].inst[k];
+                if (S.n == 0 || !(all || a.slots[s].still)) continue;
+#pragma unroll
+                for (int d = 0; d < MAXD; ++d) {
+                    lo[d] = any ? fmin(lo[d], S.bbmin[d]) : S.bbmin[d];
+                    hi[d] = any ? fmax(hi[d], S.bbmax[d]) : S.bbmax[d];
+                }
+                any = true;
+            }
+        }
+#pragma unroll
+        for (int d = 0; d < MAXD; ++d) {
+            const double c = any && d < a.nd ? rint(0.5 * (lo[d] + hi[d]) * a.spacing[k].y) * a.spacing[k].x : 0.0;
+            a.origin[k * MAXD + d] = isfinite(c) ? c : 0.0;
+        }
+    }
+}
+
+__global__ void k_plan_all(const PlanItem* __restrict__ items, int n, int ninst, PlanMask mask, int64_t* need,
+                           int64_t* need_max, const int64_t* need_cap, int* err, OriginArgs org) {
     pdl_enter();
     const int i = blockIdx.x;
+    if (i == n) {
+        origin_block(org, ninst);
+        return;
+    }
     const PlanItem& it = items[i];
     if (threadIdx.x == 0) need[i] = 0;
     __syncthreads();
@@ -953,9 +981,10 @@ __global__ void k_plan_all(const PlanItem* __restrict__ items, int ninst, PlanMa
 }
 
 void launch_plan_all(const PlanItem* items, int n, int ninst, const PlanMask& mask, int64_t* need, int64_t* need_max,
-                     const int64_t* need_cap, int* err, cudaStream_t s) {
+                     const int64_t* need_cap, int* err, const OriginArgs& org, cudaStream_t s) {
     if (n <= 0) return;
-    k_plan_all<<<n, plan_threads(ninst), 0, s>>>(items, ninst, mask, need, need_max, need_cap, err);
+    k_plan_all<<<n + (org.slots ? 1 : 0), plan_threads(ninst), 0, s>>>(items, n, ninst, mask, need, need_max, need_cap,
+                                                                       err, org);
     COUNTED(1);
 }
 

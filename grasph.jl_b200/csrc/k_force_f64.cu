@@ -110,11 +110,11 @@ __global__ void k_pack(PackArgs a, const int64_t* count) {
 
 void launch_pack(bool fp32, int mode, int64_t N, const int64_t* count, int nd, int ns, const double* x, const double* v,
                    const double* rho, const double* p, const double* stress, const int32_t* inst_of,
-                   const double* mass, float* hpos, float4* pos, float4* rec, cudaStream_t s) {
+                   const double* mass, const double* origin, float* hpos, float4* pos, float4* rec, cudaStream_t s) {
     if (N <= 0 || (!pos && !rec)) return;
     int64_t blocks = (N + 255) / 256;
     if (blocks > 148 * 64) blocks = 148 * 64;
-    PackArgs a{fp32, mode, nd, ns, N, x, v, rho, p, stress, inst_of, mass, hpos, pos, rec};
+    PackArgs a{fp32, mode, nd, ns, N, x, v, rho, p, stress, inst_of, mass, origin, hpos, pos, rec};
     k_pack<<<(int)blocks, 256, 0, s>>>(a, count);
     g_launches.fetch_add(1, std::memory_order_relaxed);
 }

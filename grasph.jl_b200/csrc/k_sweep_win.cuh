@@ -154,8 +154,10 @@ __global__ void __launch_bounds__(WIN_TPB, MINB) k_sweep_win(ForceArgs A) {
                 const double m = 1.001 * A.ref[lane].gi[k].cell + 2.4e-7 * xmax;
                 reach = B.n > 0;
 #pragma unroll
-                for (int d = 0; d < ND; ++d)
-                    reach = reach & ((double)ghi[d] >= B.bbmin[d] - m) & ((double)glo[d] <= B.bbmax[d] + m);
+                for (int d = 0; d < ND; ++d) {
+                    const double x0 = Phys::EXACT ? 0.0 : A.origin[k * MAXD + d];
+                    reach = reach & (x0 + (double)ghi[d] >= B.bbmin[d] - m) & (x0 + (double)glo[d] <= B.bbmax[d] + m);
+                }
             }
             visit = __ballot_sync(FULL, reach);
         }
@@ -191,8 +193,8 @@ __global__ void __launch_bounds__(WIN_TPB, MINB) k_sweep_win(ForceArgs A) {
                 if (active && !ok) atomicOr(A.err, ERR_CAPACITY);
                 const int32_t c0 = __shfl_sync(FULL, c[0], 0), c1 = ND == 3 ? __shfl_sync(FULL, c[1], 0) : 0;
                 const bool same = ok && c[0] == c0 && (ND == 2 || c[1] == c1);
-                // positions over 2^20 cells from the origin, of which an FP32 pair
-                // would lose more than FP32 arithmetic does, take FP64 differences
+                // positions over 2^20 cells from their instance's point, of which an FP32
+                // pair would lose more than FP32 arithmetic does, take FP64 differences
                 const bool far = !Phys::EXACT && xmax * (float)G.inv_cell > 1048576.f;
                 const bool coop = !far && __all_sync(FULL, !active || same);
                 const bool self = r.btype == BT_SELF;

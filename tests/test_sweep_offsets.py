@@ -15,7 +15,7 @@ pytestmark = pytest.mark.gpu
 DX = 0.02
 
 
-def _build(nd, functor, cells, wall):
+def _build(nd, functor, cells, wall, spread=False):
     h, c = 1.3 * DX, 40.0
     n = (16, 30) if nd == 2 else (7, 8, 10)
     rng = np.random.default_rng(3)
@@ -35,6 +35,10 @@ def _build(nd, functor, cells, wall):
     ps.v[:] = rng.uniform(-1.0, 1.0, x.shape)
     ps.rho[:] = rng.uniform(990.0, 1010.0, ps.n)
     ps.x[:] = x + off
+    if spread:  # every other particle as far on the other side of the middle, along x
+        ps.x[:] = x
+        ps.x[::2, 0] += off[0]
+        ps.x[1::2, 0] -= off[0]
     systems, inters = [ps], [G.SystemInteraction(k, pfn, ps)]
     if wall:
         w = x[x[:, -1] < 3 * DX] * np.array([1.0] * (nd - 1) + [-1.0])
@@ -47,9 +51,9 @@ def _build(nd, functor, cells, wall):
     return G.LeapFrogTimeIntegrator(systems, inters)
 
 
-def _pairs(nd, functor, cells, wall):
+def _pairs(*args):
     """Accepted pairs, from the counting sweep."""
-    lf = _build(nd, functor, cells, wall)
+    lf = _build(*args)
     s = G.Session([lf], backend=make_backend("cuda"))
     s.push()
     for ps in lf.systems:
@@ -65,9 +69,20 @@ def _pairs(nd, functor, cells, wall):
 @pytest.mark.parametrize("nd,functor,wall", [(2, "fluid", True), (2, "stress", False), (3, "fluid", False),
                                              (3, "stress", True)])
 def test_offset(nd, functor, wall, cells):
+    _check(nd, functor, cells, wall)
+
+
+@pytest.mark.parametrize("cells", [1e4, 1e5, 4e5, 1.2e6])
+@pytest.mark.parametrize("functor", ["fluid", "stress"])
+def test_spread(functor, cells):
+    """Two halves of one system, as far from the point that both count from."""
+    _check(2, functor, cells, False, True)
+
+
+def _check(nd, functor, *rest):
     runs = {}
     for name in ("oracle", "fp64", "fp32c"):
-        lf = _build(nd, functor, cells, wall)
+        lf = _build(nd, functor, *rest)
         prec = G.PRECISION_FP32_COMPENSATED if name == "fp32c" else G.PRECISION_FP64
         be = make_backend("oracle", track=parity.INPUTS) if name == "oracle" else make_backend("cuda")
         s = G.Session([lf], backend=be, precision=prec)
@@ -78,7 +93,7 @@ def test_offset(nd, functor, wall, cells):
     ref, so = runs["oracle"]
     ps = ref.systems[0]
     scales = parity.particle_scales(ps, parity.oracle_magnitudes(so, ref)[id(ps)])
-    pairs, most = _pairs(nd, functor, cells, wall)
+    pairs, most = _pairs(nd, functor, *rest)
     for name in ("fp64", "fp32c"):
         got = runs[name][0].systems[0]
         assert runs[name][1].stats()["pairs_last_step"] == pairs
@@ -89,3 +104,25 @@ def test_offset(nd, functor, wall, cells):
             scale = np.max(np.asarray(scales[f]).reshape(ps.n, -1), axis=1, keepdims=True)
             worst = np.max(np.abs(a - b) / np.maximum(scale, 1e-300))
             assert np.all(np.abs(a - b) <= tol * scale), f"{name} {f}: {worst:.2e} against {tol:.2e}"
+
+
+@pytest.mark.parametrize("cells", [0, 7e3, 3e6])
+@pytest.mark.parametrize("wall", [False, True])
+def test_steps_far_out_depend_on_the_state_alone(wall, cells):
+    """Captured steps in one call, and one step a call with the state pulled
+    and pushed in between (FP32-compensated: the same bits)."""
+    steps, cfl = 24, 0.05
+    got, want = (_build(2, "fluid", cells, wall) for _ in range(2))
+    s = G.Session([got], precision=G.PRECISION_FP32_COMPENSATED)
+    s.push()
+    s.step(steps, cfl)
+    assert s.stats()["graph_steps"] > 0
+    s.pull()
+    t = G.Session([want], precision=G.PRECISION_FP32_COMPENSATED)
+    for _ in range(steps):
+        t.push()
+        t.step(1, cfl)
+        t.pull()
+    for a, b in zip(got.systems, want.systems):
+        for f, _ in a.particle_fields():
+            assert np.isfinite(getattr(a, f)).all() and np.array_equal(getattr(a, f), getattr(b, f)), f"{a.name} {f}"
