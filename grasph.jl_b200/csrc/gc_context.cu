@@ -120,6 +120,7 @@ struct DSlot {
     int64_t xpk_epoch = -1;    // pack_epoch the position records were made in
     bool xpk_static = false;   // position records of a system that does not move are current
     bool xpk_fp32 = false;     // their precision
+    bool lends = false, recs = false;  // which it holds: a dynamic boundary's positions, sweep records
     bool box_fresh = false;    // the boxes are those of the current positions (kept by the full step)
     bool written = false;      // some functor writes this system
     bool moving = true;        // sorted and integrated every step
@@ -175,6 +176,7 @@ struct DGhost {
     int64_t xpk_epoch = -1;
     bool xpk_static = false;  // never set: ghosts are regenerated every step
     int64_t pack_done_epoch = -1;  // never set: packed for every sweep
+    bool lends = false, recs = true;
     std::vector<std::vector<std::pair<int, int>>> copiers;
     bool ex_p = false, ex_stress = false;
     int64_t need_slot = -1;  // index into need[] for its sort cells
@@ -912,6 +914,11 @@ int finalize(gc_ctx* ctx) {
                 D.bslot = hh.idx;
             }
         }
+        if (!h0.probe) {
+            ctx->slots[D.a].recs = true;
+            if (D.btype == BT_DYNAMIC) ctx->slots[D.bslot].lends = true;
+            else if (D.bslot >= 0) ctx->slots[D.bslot].recs = true;
+        }
         D.two_fluid = D.btype == BT_SYSTEM && I0.sys[h0.a].kind == GC_SYS_FLUID &&
                       I0.sys[D.bslot].kind == GC_SYS_FLUID;
         for (int s = 0; s < (int)D.pk.size(); ++s)
@@ -1628,16 +1635,21 @@ int ghost_copy(gc_ctx* ctx, DGhost& G, int stage) {
     return check_launch(ctx, "ghost copy");
 }
 
-// Sweep buffers of a slot or ghost set: the planar FP32 positions (padded to
-// whole quads), N position-only records (pos_quads each), then N sweep
-// records (rec_quads of the mode and precision each).
+// Sweep buffers of a slot or ghost set X: the planar FP32 positions (padded to
+// whole quads), where it lends positions N position-only records (pos_quads
+// each), then N sweep records (rec_quads of the mode and precision each) where
+// it has those.
 float* hpos_of(float* fpk) { return fpk; }
 float4* pos_of(float* fpk, int64_t N, int nd) { return reinterpret_cast<float4*>(fpk) + (N * nd + 3) / 4; }
-float4* rec_of(float* fpk, int64_t N, int nd) { return pos_of(fpk, N, nd) + N * pos_quads(nd, true); }
+template <class T>
+float4* rec_of(const T& X, int64_t N, int nd) {
+    return pos_of(X.fpk, N, nd) + (X.lends ? N * pos_quads(nd, true) : 0);
+}
 
 template <class T>
 int ensure_fpk(gc_ctx* ctx, T& X, int64_t N, int nd, int mode, bool fp32) {
-    int64_t need = 4 * ((N * nd + 3) / 4 + N * (pos_quads(nd, fp32) + rec_quads(nd, mode, fp32)));
+    const int64_t quads = (X.lends ? pos_quads(nd, fp32) : 0) + (X.recs ? rec_quads(nd, mode, fp32) : 0);
+    const int64_t need = 4 * ((N * nd + 3) / 4 + N * quads);
     if (need > X.cap_fpk) {
         CU(cudaStreamSynchronize(ctx->stream));
         X.cap_fpk = 0;     // until the new buffer is there,
@@ -1888,7 +1900,7 @@ int sweep_group(gc_ctx* ctx, int a, const std::vector<int>& ids, int stage, bool
                           S.pack_done_mode == mode && S.pack_done_ns == pk_ns && S.pack_done_fp32 == fp32;
         if (!done) {
             launch_pack(fp32, mode, S.N, nullptr, S.nd, pk_ns, S.F(F_X), S.F(F_V), S.F(F_RHO), S.F(F_P),
-                        S.F(F_STRESS), S.inst_of, S.d_mass, ctx->d_origin, hpos_of(S.fpk), nullptr, rec_of(S.fpk, S.N, S.nd),
+                        S.F(F_STRESS), S.inst_of, S.d_mass, ctx->d_origin, hpos_of(S.fpk), nullptr, rec_of(S, S.N, S.nd),
                         ctx->stream);
             S.pack_done_epoch = -1;  // no longer the half step's: a later functor of its mode packs again
         }
@@ -1920,7 +1932,7 @@ int sweep_group(gc_ctx* ctx, int a, const std::vector<int>& ids, int stage, bool
     A.a_c = S.d_c;
     A.a_mass = S.d_mass;
     A.a_cf = S.d_cf;
-    A.arec = records ? rec_of(S.fpk, S.N, S.nd) : nullptr;
+    A.arec = records ? rec_of(S, S.N, S.nd) : nullptr;
     A.origin = ctx->d_origin;
     A.prec = fp32 ? GC_PRECISION_FP32_COMPENSATED : GC_PRECISION_FP64;
     A.err = ctx->d_err;
@@ -1979,10 +1991,10 @@ int sweep_group(gc_ctx* ctx, int a, const std::vector<int>& ids, int stage, bool
             if (records) {
                 TRY(ensure_fpk(ctx, G, G.CAP, G.nd, mode, fp32));
                 launch_pack(fp32, mode, G.CAP, G.d_count, G.nd, pk_ns, G.x[G.cur], G.v, G.rho, G.p, G.stress,
-                            G.ginst[G.cur], G.d_mass, ctx->d_origin, hpos_of(G.fpk), nullptr, rec_of(G.fpk, G.CAP, G.nd),
+                            G.ginst[G.cur], G.d_mass, ctx->d_origin, hpos_of(G.fpk), nullptr, rec_of(G, G.CAP, G.nd),
                             ctx->stream);
                 r.bh = hpos_of(G.fpk);
-                r.brec = rec_of(G.fpk, G.CAP, G.nd);
+                r.brec = rec_of(G, G.CAP, G.nd);
                 r.brq = rec_quads(G.nd, mode, fp32);
             }
         } else {
@@ -1996,7 +2008,7 @@ int sweep_group(gc_ctx* ctx, int a, const std::vector<int>& ids, int stage, bool
             r.brec = nullptr;
             if (records && D.btype == BT_SELF) {
                 r.bh = hpos_of(S.fpk);
-                r.brec = rec_of(S.fpk, S.N, S.nd);
+                r.brec = rec_of(S, S.N, S.nd);
                 r.brq = rec_quads(S.nd, mode, fp32);
             } else if (records) {
                 // dynamic walls lend only their positions; other systems their records
@@ -2007,11 +2019,11 @@ int sweep_group(gc_ctx* ctx, int a, const std::vector<int>& ids, int stage, bool
                                           (B.xmoves() ? B.xpk_epoch != ctx->pack_epoch : !B.xpk_static));
                 launch_pack(fp32, mode, B.N, nullptr, B.nd, pk_ns, B.F(F_X), B.F(F_V), B.F(F_RHO), B.F(F_P),
                             B.kind >= GC_SYS_STRESS ? B.F(F_STRESS) : nullptr, B.inst_of, B.d_mass, ctx->d_origin, hpos_of(B.fpk),
-                            pos ? pos_of(B.fpk, B.N, B.nd) : nullptr, rec ? rec_of(B.fpk, B.N, B.nd) : nullptr,
+                            pos ? pos_of(B.fpk, B.N, B.nd) : nullptr, rec ? rec_of(B, B.N, B.nd) : nullptr,
                             ctx->stream);
                 r.bh = hpos_of(B.fpk);
                 if (rec) {
-                    r.brec = rec_of(B.fpk, B.N, B.nd);
+                    r.brec = rec_of(B, B.N, B.nd);
                     r.brq = rec_quads(B.nd, mode, fp32);
                     B.pack_done_epoch = -1;  // packed in this sweep's mode: B's own sweep packs again
                 } else {
@@ -2077,7 +2089,7 @@ int sweep_group(gc_ctx* ctx, int a, const std::vector<int>& ids, int stage, bool
         R.a_c = B.d_c;
         R.a_mass = B.d_mass;
         R.a_cf = B.d_cf;
-        R.arec = records ? rec_of(B.fpk, B.N, B.nd) : nullptr;
+        R.arec = records ? rec_of(B, B.N, B.nd) : nullptr;
         R.nref = 1;
         InterRef& r = R.ref[0];
         r.btype = BT_SYSTEM;
@@ -2093,7 +2105,7 @@ int sweep_group(gc_ctx* ctx, int a, const std::vector<int>& ids, int stage, bool
         r.bstress = S.F(F_STRESS);
         r.bN = S.N;
         r.bh = records ? hpos_of(S.fpk) : nullptr;
-        r.brec = records ? rec_of(S.fpk, S.N, S.nd) : nullptr;
+        r.brec = records ? rec_of(S, S.N, S.nd) : nullptr;
         r.brq = rec_quads(S.nd, mode, fp32);
         st = launch_force_f64(R, false, ctx->stream);
         if (st == GC_ERR_CUDA) return check_launch(ctx, "sweep (system_b side)");
@@ -2272,7 +2284,7 @@ int gather_halfstep(gc_ctx* ctx, DSlot& S) {
                 TRY(ensure_fpk(ctx, S, S.N, S.nd, pl.mode, pl.fp32));
                 pk = PackArgs{pl.fp32, pl.mode, S.nd, pl.pk_ns, S.N, S.F(F_X), S.F(F_V), S.F(F_RHO), S.F(F_P),
                               S.F(F_STRESS), S.inst_of, S.d_mass, ctx->d_origin, hpos_of(S.fpk), nullptr,
-                              rec_of(S.fpk, S.N, S.nd)};
+                              rec_of(S, S.N, S.nd)};
                 S.pack_done_epoch = ctx->pack_epoch;
                 S.pack_done_stage = 1;
                 S.pack_done_mode = pl.mode;
@@ -4132,10 +4144,21 @@ int64_t ctx_moving_particles(gc_ctx* c, int inst) {
 int64_t ctx_estimate_bytes(gc_ctx* m, int inst) {
     const HInst& I = m->inst[inst];
     int64_t b = 0;
-    auto record_bytes = [](int nd, int ns) {  // a particle's sweep buffers (ensure_fpk), in the wider precision
+    // a particle's sweep buffers (ensure_fpk), in the model's precision (FP64, the wider, unless set)
+    auto record_bytes = [&](int nd, int ns, bool lends, bool recs) {
+        const bool fp32 = m->precision == GC_PRECISION_FP32_COMPENSATED;
         const int mode = ns ? AUX_INV_RHO2 : AUX_P_OVER_RHO2;
-        return 4 * nd + 16 * (pos_quads(nd, false) + rec_quads(nd, mode, false));
+        return 4 * nd + 16 * ((lends ? pos_quads(nd, fp32) : 0) + (recs ? rec_quads(nd, mode, fp32) : 0));
     };
+    std::vector<char> lends(I.sys.size()), recs(I.sys.size());
+    for (auto& it : I.inters) {
+        recs[it.a] = 1;
+        if (it.b < 0) continue;
+        const HHandle& h = I.handles[it.b];
+        if (h.type == H_DYN) lends[h.idx] = 1;
+        else if (h.type == H_VIRT) recs[I.virts[h.idx].src] = 1;
+        else if (h.type != H_GHOST) recs[h.idx] = 1;
+    }
     for (auto& s : I.sys) {
         int comps = 0;
         for (int f = 0; f < GC_NFIELDS; ++f) {
@@ -4143,12 +4166,12 @@ int64_t ctx_estimate_bytes(gc_ctx* m, int inst) {
             const int c = sys_comps(s, f);
             if (c > 0) comps += c;
         }
-        b += s.n * (comps * 8 * 3 + (s.nd + 2) * 8 + 4 * 4 + record_bytes(s.nd, s.ns) + 8 + 4 * 4);
+        b += s.n * (comps * 8 * 3 + (s.nd + 2) * 8 + 4 * 4 + record_bytes(s.nd, s.ns, lends[&s - I.sys.data()], recs[&s - I.sys.data()]) + 8 + 4 * 4);
     }
     for (auto& g : I.ghosts) {
         const HSys& src = I.sys[g.src];
         const int64_t cap = src.n * g.nplanes;
-        b += cap * (src.nd * 8 * 4 + 4 * 8 + 8 * 3 + src.ns * 8 + record_bytes(src.nd, src.ns));
+        b += cap * (src.nd * 8 * 4 + 4 * 8 + 8 * 3 + src.ns * 8 + record_bytes(src.nd, src.ns, false, true));
     }
     // grid cells from the staged positions' bounding box
     double lo[3] = {1e300, 1e300, 1e300}, hi[3] = {-1e300, -1e300, -1e300};
