@@ -1796,7 +1796,7 @@ int interp_sweeps(gc_ctx* ctx, int a, const std::vector<int>& ids, int stage) {
             r.bx = S.F(F_X);
             r.bv = S.F(F_V);
             r.brho = S.F(F_RHO);
-                r.bstress = S.F(F_STRESS);
+            r.bstress = S.F(F_STRESS);
             r.bN = S.N;
         }
         int st = launch_force_f64(R, false, ctx->stream);

@@ -94,51 +94,12 @@ __device__ __forceinline__ double kernel_w(double norm, double q) {
         return (norm * (a2 * a2)) * (2.0 * q + 1.0);
     }
 }
-template <int KK>
-__device__ __forceinline__ double kernel_dw_dq(double norm, double q) {
-    if (KK == GC_KERNEL_CUBIC_SPLINE) {
-        double a = jmax(0.0, 2.0 - q), b = jmax(0.0, 1.0 - q);
-        return norm * (-3.0 * (0.25 * (a * a) - (b * b)));
-    } else {
-        double a = jmax(0.0, 2.0 - q);
-        return ((-norm * 10.0) * q) * (a * a * a);
-    }
-}
-
 template <int ND>
 __device__ __forceinline__ double dotv(const double* a, const double* b) {
     double s = a[0] * b[0];
 #pragma unroll
     for (int d = 1; d < ND; ++d) s = s + a[d] * b[d];
     return s;
-}
-
-// src/PairwisePhysics.jl:29-34.  When dot(dx,dv) >= 0 the result is -0.0
-// exactly (muv == 0), so the divisions are skipped.
-template <int ND>
-__device__ __forceinline__ double art_visc(const double* dx, const double* dv, double rr, double h, double ri,
-                                           double rj, double alpha, double beta, double ci, double cj) {
-    double vr = jmin(dotv<ND>(dx, dv), 0.0);
-    if (vr == 0.0 && !signbit(vr) && h > 0.0) {
-        // muv = (h*0)/(positive) = +0 exactly; the quotient of a signed zero
-        // by a positive finite denominator is that signed zero.
-        double mc = 0.5 * (ci + cj);
-        double t = (beta * 0.0 - alpha * mc) * 0.0;
-        double den = (0.5 * ri) * rj;
-        return den > 0.0 ? t : t / den;
-    }
-    double muv = (h * vr) / (rr + (h * h) * 0.01);
-    double mc = 0.5 * (ci + cj);
-    return ((beta * muv - alpha * mc) * muv) / ((0.5 * ri) * rj);
-}
-
-// src/PairwisePhysics.jl:238-243
-template <int ND>
-__device__ __forceinline__ double diffusion(const double* dx, double rr, double ri, double rj, double ci,
-                                            double cj, double hi, double hj, const double* gx, double delta) {
-    double c = 0.5 * (ci + cj);
-    double h = 0.5 * (hi + hj);
-    return (((((2.0 * delta) * c) * h) * (ri - rj)) * dotv<ND>(dx, gx)) / rr;
 }
 
 // src/PairwisePhysics.jl:258-263

@@ -1,20 +1,21 @@
-// k_force_impl.cuh — the fused pair sweep in FP64, and what it shares with the
-// FP32-compensated one (k_sweep_f32.cuh).
+// k_force_impl.cuh — the buffered sweep of the counting, interpolation and
+// velocity-adjust (XSPH) functors in FP64, and what it shares with the window
+// sweep of the others (k_sweep_win.cuh).
 //
 // Gather formulation of src/Interaction.jl:393-732: one thread owns one
 // system_a particle and sums its side of every accepted pair of every
 // interaction of the current stage, in registers, then writes once.  The
-// reference's coloured half-shell writes both endpoints; every functor on
-// this path is exactly antisymmetric (or symmetric) under i↔j, so each
-// side's term is bit-identical to the one the reference adds — only the
-// order of the additions differs.
+// reference's coloured half-shell writes both endpoints; the functors here are
+// exactly antisymmetric (or symmetric) under i↔j and their terms the
+// reference's own expressions, so each side's term is bit-identical to the one
+// the reference adds — only the order of the additions differs.
 //
 // Candidate enumeration walks the same 3-cell strips of the CSR grid as the
 // reference (3 strips in 2-D, 9 in 3-D) and applies the same acceptance
 // test r² < (2h)² on the same FP64 dx, so the neighbour sets are
 // bit-identical.  Accepted neighbour indices are staged in a per-thread
-// column of shared memory and processed in batches: the expensive pair
-// physics runs with every lane busy instead of diverging on rejections.
+// column of shared memory and processed in batches, so that the pair terms
+// run with every lane busy instead of diverging on rejections.
 //
 // The arithmetic relies on -fmad=false.
 #pragma once
@@ -31,7 +32,7 @@ namespace gc {
 template <int ND>
 struct OwnState {
     double x[ND], v[ND];
-    double rho, aux;
+    double rho;
 };
 
 // ------------------------------------------------------- pair physics
@@ -282,9 +283,8 @@ __device__ __forceinline__ void warp_zrange(const int32_t* c, bool active, int32
 // starts from −cut, so it ends at r² − cut and its sign bit is the hit: one
 // funnel shift per candidate moves it into the mask (candidates pushed from
 // last to first).  A NaN result is not guaranteed a clear sign bit, so the
-// callers mask out inactive lanes.  V4: 16-byte loads of four candidates'
-// coordinates (rows and the base 16-byte aligned).
-template <int ND, bool V4 = false>
+// callers mask out inactive lanes.
+template <int ND>
 __device__ __forceinline__ unsigned batch_hits(const float* cb, int stride, int mb, const float* xi, float cut_f) {
     const float2 neg1 = make_float2(-1.0f, -1.0f);
     const float2 ncut = make_float2(-cut_f, -cut_f);
@@ -299,15 +299,7 @@ __device__ __forceinline__ unsigned batch_hits(const float* cb, int stride, int 
 #pragma unroll
             for (int d = 0; d < ND; ++d) {
                 const float* row = cb + d * stride + t0 + t;
-                float2 xa, xb;
-                if (V4) {
-                    const float4 q = *reinterpret_cast<const float4*>(row);
-                    xa = make_float2(q.x, q.y);
-                    xb = make_float2(q.z, q.w);
-                } else {
-                    xa = *reinterpret_cast<const float2*>(row);
-                    xb = *reinterpret_cast<const float2*>(row + 2);
-                }
+                const float2 xa = *reinterpret_cast<const float2*>(row), xb = *reinterpret_cast<const float2*>(row + 2);
                 const float2 xo = make_float2(xi[d], xi[d]);
                 const float2 da = __ffma2_rn(xa, neg1, xo), db = __ffma2_rn(xb, neg1, xo);
                 ra = __ffma2_rn(da, da, ra);
@@ -373,28 +365,21 @@ __host__ __device__ constexpr int sweep_smem_bytes(int buf) {
 // to the lane's shared-memory column; when any column is nearly full the
 // whole warp evaluates its staged pairs, so the pair physics runs on
 // converged warps.
-template <class Phys, bool COUNT_ONLY, int UNROLL, int PFN>
+template <class Phys, bool COUNT_ONLY, int PFN>
 __device__ __forceinline__ int flush_all(const ForceArgs& A, const InterRef& r, const GridInst& G,
                                          const PfnInst& P, int k, const typename Phys::Own& w, int nbuf,
                                          const int32_t* col, int BT, typename Phys::AccT& acc) {
     constexpr int P2 = COUNT_ONLY ? GC_PFN_COUNT : PFN;
     int acc_n = 0;
-    int t = 0;
-    if (UNROLL == 2) {
-        for (; t + 1 < nbuf; t += 2) {
-            const int32_t j0 = col[t * BT], j1 = col[(t + 1) * BT];
-            acc_n += Phys::template pair<P2>(A, r, G, P, k, w, j0, acc);
-            acc_n += Phys::template pair<P2>(A, r, G, P, k, w, j1, acc);
-        }
-    }
-    for (; t < nbuf; ++t) acc_n += Phys::template pair<P2>(A, r, G, P, k, w, col[t * BT], acc);
+    for (int t = 0; t < nbuf; ++t) acc_n += Phys::template pair<P2>(A, r, G, P, k, w, col[t * BT], acc);
     return acc_n;
 }
 
-template <class Phys, int ND, int PFN, bool COUNT_ONLY, int MINB, int BUF, int UNROLL>
-__global__ void __launch_bounds__(FORCE_TPB, MINB) k_sweep(ForceArgs A) {
+template <class Phys, int ND, int PFN, bool COUNT_ONLY>
+__global__ void __launch_bounds__(FORCE_TPB, 4) k_sweep(ForceArgs A) {
     pdl_enter();
     extern __shared__ int32_t sbuf[];
+    constexpr int BUF = FORCE_BUF;
     const unsigned FULL = 0xffffffffu;
     const int lane = threadIdx.x & 31;
     const int tid = threadIdx.x;
@@ -467,7 +452,7 @@ __global__ void __launch_bounds__(FORCE_TPB, MINB) k_sweep(ForceArgs A) {
                     const int32_t lo = active ? r.cs[base + c[L] - 1] : 0, hi = active ? r.cs[base + c[L] + 2] : 0;
                     for (int32_t ch = u0; ch < u1; ch += 32) {
                         if (__any_sync(FULL, nbuf > BUF - 32)) {
-                            accepted += flush_all<Phys, COUNT_ONLY, UNROLL, PFN>(A, r, Gs, Ps, k, w, nbuf, col, BT, acc);
+                            accepted += flush_all<Phys, COUNT_ONLY, PFN>(A, r, Gs, Ps, k, w, nbuf, col, BT, acc);
                             nbuf = 0;
                             __syncwarp();
                         }
@@ -488,7 +473,7 @@ __global__ void __launch_bounds__(FORCE_TPB, MINB) k_sweep(ForceArgs A) {
                         __syncwarp();
                     }
                 }
-                accepted += flush_all<Phys, COUNT_ONLY, UNROLL, PFN>(A, r, Gs, Ps, k, w, nbuf, col, BT, acc);
+                accepted += flush_all<Phys, COUNT_ONLY, PFN>(A, r, Gs, Ps, k, w, nbuf, col, BT, acc);
                 nbuf = 0;
                 __syncwarp();
             } else if (active && ok) {
@@ -503,12 +488,12 @@ __global__ void __launch_bounds__(FORCE_TPB, MINB) k_sweep(ForceArgs A) {
                         if (self && j == gi) continue;
                         col[(nbuf++) * BT] = j;
                         if (nbuf == BUF) {
-                            accepted += flush_all<Phys, COUNT_ONLY, UNROLL, PFN>(A, r, Gs, Ps, k, w, nbuf, col, BT, acc);
+                            accepted += flush_all<Phys, COUNT_ONLY, PFN>(A, r, Gs, Ps, k, w, nbuf, col, BT, acc);
                             nbuf = 0;
                         }
                     }
                 }
-                accepted += flush_all<Phys, COUNT_ONLY, UNROLL, PFN>(A, r, Gs, Ps, k, w, nbuf, col, BT, acc);
+                accepted += flush_all<Phys, COUNT_ONLY, PFN>(A, r, Gs, Ps, k, w, nbuf, col, BT, acc);
                 nbuf = 0;
             }
             __syncwarp();
@@ -528,7 +513,7 @@ static void launch_t(const ForceArgs& A, cudaStream_t s) {
     if (blocks > (int64_t)A.num_sms * 16) blocks = (int64_t)A.num_sms * 16;
     if (blocks < 1) blocks = 1;
     const size_t smem = (size_t)sweep_smem_bytes<ND>(FORCE_BUF);
-    k_sweep<PhysGather<ND, NS, P2, KK>, ND, P2, COUNT_ONLY, 4, FORCE_BUF, 1><<<(int)blocks, FORCE_TPB, smem, s>>>(A);
+    k_sweep<PhysGather<ND, NS, P2, KK>, ND, P2, COUNT_ONLY><<<(int)blocks, FORCE_TPB, smem, s>>>(A);
     g_launches.fetch_add(1, std::memory_order_relaxed);
 }
 

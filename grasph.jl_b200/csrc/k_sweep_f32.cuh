@@ -11,10 +11,10 @@
 //   * dv·∇W is W'·(dv·dx), so ∇W itself is never formed; the kernel's constant
 //     factor multiplies the sums, not the terms;
 //   * components go through packed FP32x2 arithmetic.
-// Three-dimensional dam break of a million jittered particles: 894 us a launch
-// with strips staged one at a time and FP64 differences, 700 us with this
-// kernel; 64 batched columns (1.07 M particles) 292 to 230 us; a
-// Lennard-Jones box of 18 k particles 72 to 45 us.  Sixteen warps per SM (128
+// Three-dimensional dam break of a million jittered particles: 920 us a launch
+// with strips staged one at a time and FP64 differences, 709 us with this
+// kernel; 64 batched columns (1.07 M particles) 292 to 230 us; a Lennard-Jones
+// box of 30 k particles 82 to 51 us.  Sixteen warps per SM (128
 // registers, chunks of 192) beat eighteen to twenty-four at 80-96 registers,
 // whose spills cost more than the occupancy gives.
 //
@@ -449,7 +449,7 @@ struct PhysF32 {
 
 // One translation unit per dimension: defines launch_force_<ND>d_f32.
 #define GC_DEFINE_FORCE_F32_TU(NDIM, NAME)                                                                       \
-    int NAME(const ForceArgs& A, bool, cudaStream_t s) {                                                         \
+    int NAME(const ForceArgs& A, cudaStream_t s) {                                                         \
         if (A.kk == GC_KERNEL_CUBIC_SPLINE) return launch_win_nd<PhysF32, NDIM, GC_KERNEL_CUBIC_SPLINE>(A, s);   \
         return launch_win_nd<PhysF32, NDIM, GC_KERNEL_WENDLAND_C2>(A, s);                                        \
     }

@@ -8,9 +8,11 @@
 // what is left), with fused multiply-adds, dv·∇W as W'·(dv·dx), and the
 // kernel's constant factor on the sums.  Every quantity stays FP64; a term
 // differs from the reference's expression by a few units in the last place.
-// Sweep of a 224 k particle 3-D dam break 847 -> 246 us, 5,000 particles in 2-D
-// 61 -> 22.5 us, an 80 k column 79 -> 42 us a launch.  Blocks few enough that
-// nothing spills (168 registers, twelve warps per SM) are the fastest.
+// Sweep of 224 k particles of 3-D water 885 -> 261 us, of 5,000 in 2-D 63.5 ->
+// 24.5 us, of an 80 k column 81 -> 44 us a launch (jittered starts).  The first
+// configuration (twelve warps per SM) is mostly the fastest: up to 168
+// registers, and only the 3-D Cauchy terms spill (92 bytes; every
+// configuration of theirs does).
 // The acceptance test keeps the reference's unfused r² < (2h)², so the
 // neighbour sets are bit-identical.
 #pragma once

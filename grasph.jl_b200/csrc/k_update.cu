@@ -92,7 +92,7 @@ __global__ void k_gather_halfstep(StepArgs a, StepSrc src, const __grid_constant
 }
 
 // src/TimeIntegration.jl:673-682: damping, full step, zero XSPH pass, x += dt·v
-// (every load before the first store, as in halfstep_one).
+// (every load before the first store, as in halfstep_from).
 // BOX: the moved positions' bounding boxes too (gc_box.cuh), which the next
 // step's plan would otherwise read all positions for (16 us of a million
 // particles' step, and a launch).
@@ -101,7 +101,8 @@ __global__ void k_gather_halfstep(StepArgs a, StepSrc src, const __grid_constant
 // wave; 31 us without the boxes).
 constexpr int FULL_PER_SM = 4;
 template <bool BOX>
-__global__ void __launch_bounds__(UTPB, FULL_PER_SM) k_fullstep(StepArgs a, unsigned long long* scratch, SysInst* box, int ninst, int64_t tiles_per_block) {
+__global__ void __launch_bounds__(UTPB, FULL_PER_SM)
+    k_fullstep(StepArgs a, unsigned long long* scratch, SysInst* box, int ninst, int64_t tiles_per_block) {
     pdl_enter();
     BoxRun run;
     for (int64_t tile = (int64_t)blockIdx.x * tiles_per_block;
