@@ -120,6 +120,7 @@ struct DSlot {
     int64_t xpk_epoch = -1;    // pack_epoch the position records were made in
     bool xpk_static = false;   // position records of a system that does not move are current
     bool xpk_fp32 = false;     // their precision
+    bool hpos_fp32 = false;    // the precision that packed the buffer's FP32 positions last
     bool lends = false, recs = false;  // which it holds: a dynamic boundary's positions, sweep records
     bool box_fresh = false;    // the boxes are those of the current positions (kept by the full step)
     bool written = false;      // some functor writes this system
@@ -1897,11 +1898,13 @@ int sweep_group(gc_ctx* ctx, int a, const std::vector<int>& ids, int stage, bool
         TRY(ensure_fpk(ctx, S, S.N, S.nd, mode, fp32));
         // the fused half step of this step may have packed these records
         const bool done = S.pack_done_epoch == ctx->pack_epoch && S.pack_done_stage == stage &&
-                          S.pack_done_mode == mode && S.pack_done_ns == pk_ns && S.pack_done_fp32 == fp32;
+                          S.pack_done_mode == mode && S.pack_done_ns == pk_ns && S.pack_done_fp32 == fp32 &&
+                          S.hpos_fp32 == fp32;
         if (!done) {
             launch_pack(fp32, mode, S.N, nullptr, S.nd, pk_ns, S.F(F_X), S.F(F_V), S.F(F_RHO), S.F(F_P),
                         S.F(F_STRESS), S.inst_of, S.d_mass, ctx->d_origin, hpos_of(S.fpk), nullptr, rec_of(S, S.N, S.nd),
                         ctx->stream);
+            S.hpos_fp32 = fp32;
             S.pack_done_epoch = -1;  // no longer the half step's: a later functor of its mode packs again
         }
     }
@@ -2015,12 +2018,13 @@ int sweep_group(gc_ctx* ctx, int a, const std::vector<int>& ids, int stage, bool
                 const bool rec = D.btype == BT_SYSTEM || D.btype == BT_STATIC || D.btype == BT_VIRTUAL;
                 TRY(ensure_fpk(ctx, B, B.N, B.nd, mode, fp32));
                 // positions: once per step, once for good for a system that does not move
-                const bool pos = !rec && (B.xpk_fp32 != fp32 ||
+                const bool pos = !rec && (B.xpk_fp32 != fp32 || B.hpos_fp32 != fp32 ||
                                           (B.xmoves() ? B.xpk_epoch != ctx->pack_epoch : !B.xpk_static));
                 launch_pack(fp32, mode, B.N, nullptr, B.nd, pk_ns, B.F(F_X), B.F(F_V), B.F(F_RHO), B.F(F_P),
                             B.kind >= GC_SYS_STRESS ? B.F(F_STRESS) : nullptr, B.inst_of, B.d_mass, ctx->d_origin, hpos_of(B.fpk),
                             pos ? pos_of(B.fpk, B.N, B.nd) : nullptr, rec ? rec_of(B, B.N, B.nd) : nullptr,
                             ctx->stream);
+                if (rec || pos) B.hpos_fp32 = fp32;
                 r.bh = hpos_of(B.fpk);
                 if (rec) {
                     r.brec = rec_of(B, B.N, B.nd);
@@ -2289,7 +2293,7 @@ int gather_halfstep(gc_ctx* ctx, DSlot& S) {
                 S.pack_done_stage = 1;
                 S.pack_done_mode = pl.mode;
                 S.pack_done_ns = pl.pk_ns;
-                S.pack_done_fp32 = pl.fp32;
+                S.pack_done_fp32 = S.hpos_fp32 = pl.fp32;
             }
         }
     }

@@ -51,9 +51,8 @@ def _build(nd, functor, cells, wall, spread=False):
     return G.LeapFrogTimeIntegrator(systems, inters)
 
 
-def _pairs(*args):
-    """Accepted pairs, from the counting sweep."""
-    lf = _build(*args)
+def _pairs(lf):
+    """Accepted pairs, from the counting sweep, and the most of a particle."""
     s = G.Session([lf], backend=make_backend("cuda"))
     s.push()
     for ps in lf.systems:
@@ -62,7 +61,8 @@ def _pairs(*args):
     for si in lf.interactions:
         s.create_grid(si)
         counts.append(s.neighbor_counts(si))
-    return counts[0].sum() // 2 + sum(int(c.sum()) for c in counts[1:]), max(c.max() for c in counts)
+    pairs = sum(int(c.sum()) // (1 if si.is_coupled() else 2) for c, si in zip(counts, lf.interactions))
+    return pairs, max(c.max() for c in counts)
 
 
 @pytest.mark.parametrize("cells", [0, 5e3, 1e4, 1e5, 9e5, 1.5e6])
@@ -93,7 +93,7 @@ def _check(nd, functor, *rest):
     ref, so = runs["oracle"]
     ps = ref.systems[0]
     scales = parity.particle_scales(ps, parity.oracle_magnitudes(so, ref)[id(ps)])
-    pairs, most = _pairs(nd, functor, *rest)
+    pairs, most = _pairs(_build(nd, functor, *rest))
     for name in ("fp64", "fp32c"):
         got = runs[name][0].systems[0]
         assert runs[name][1].stats()["pairs_last_step"] == pairs
@@ -126,3 +126,47 @@ def test_steps_far_out_depend_on_the_state_alone(wall, cells):
     for a, b in zip(got.systems, want.systems):
         for f, _ in a.particle_fields():
             assert np.isfinite(getattr(a, f)).all() and np.array_equal(getattr(a, f), getattr(b, f)), f"{a.name} {f}"
+
+
+@pytest.mark.parametrize("cells", [0, 3e6])
+def test_both_precisions_in_one_step(cells):
+    """A system swept in FP64 (the S = 1 pressure form always is) that lends
+    its positions to an FP32-compensated sweep in between."""
+    def build():
+        rng = np.random.default_rng(6)
+        h = 1.3 * DX
+        off = 2.0 * h * cells
+        k = G.CubicSplineKernel(h, ndims=2)
+        systems = []
+        for name, y in (("a", 0.0), ("b", -12 * DX)):
+            i, j = np.meshgrid(np.arange(14), np.arange(12), indexing="ij")
+            ps = G.FluidParticleSystem(name, i.size, 2, 0.4, 40.0)
+            ps.x[:] = np.stack([i.ravel(), j.ravel()], axis=1) * DX + [0.0, y] + off
+            ps.x[:] += rng.uniform(-2e-3, 2e-3, ps.x.shape)
+            ps.v[:] = rng.uniform(-1.0, 1.0, ps.x.shape)
+            ps.rho[:] = rng.uniform(990.0, 1010.0, ps.n)
+            ps.p[:] = rng.uniform(-50.0, 500.0, ps.n)
+            systems.append(ps)
+        a, b = systems
+        wall = G.DynamicBoundarySystem(b, [0.0, 1.0], [off, off - DX / 2], 1.5)
+        return G.LeapFrogTimeIntegrator(systems, [
+            G.SystemInteraction(k, G.FluidPfn(0.1, 0.1, h), a),
+            G.SystemInteraction(k, G.FluidPfn(0.1, 0.1, h), a, wall),
+            G.SystemInteraction(k, G.FluidPfn(0.1, 0.1, h, sigma=1), b)])
+
+    ref, lf = build(), build()
+    so = G.Session([ref], backend=make_backend("oracle", track=parity.INPUTS))
+    s = G.Session([lf], precision=G.PRECISION_FP32_COMPENSATED)
+    for q in (so, s):
+        q.push()
+        q.step(1, 0.01)
+        q.pull()
+    pairs, most = _pairs(build())
+    assert s.stats()["pairs_last_step"] == pairs
+    got, ps = lf.systems[1], ref.systems[1]
+    scales = parity.particle_scales(ps, parity.oracle_magnitudes(so, ref)[id(ps)])
+    assert np.array_equal(got.id, ps.id)
+    for f in ("dvdt", "drhodt"):
+        a, b = (np.asarray(getattr(q, f), float).reshape(ps.n, -1) for q in (got, ps))
+        scale = np.max(np.asarray(scales[f]).reshape(ps.n, -1), axis=1, keepdims=True)
+        assert np.all(np.abs(a - b) <= 2.0 * (40 + most) * 2.0 ** -53 * scale), f
