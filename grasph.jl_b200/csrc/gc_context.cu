@@ -340,7 +340,8 @@ struct gc_ctx {
     double* d_origin = nullptr;
     double2* d_spacing = nullptr;
     OriginSlot* d_origin_slots = nullptr;
-    std::vector<OriginSlot> origin_slots;
+    int norigin_slots = 0;
+    bool walls_rest = false;  // no system that no functor writes moves
     std::vector<Snapshot> snaps;    // per slot (moving slots only)
     int64_t graph_steps = 0, rollbacks = 0;
     int64_t pack_epoch = 0;  // bumps at the start of every issued step and single sweep (never rolled back)
@@ -1116,7 +1117,12 @@ int finalize(gc_ctx* ctx) {
         TRY(dalloc(ctx, &ctx->d_spacing, spacing.size()));
         TRY(hcopy(ctx, ctx->d_spacing, spacing.data(), spacing.size() * sizeof(double2), cudaMemcpyHostToDevice));
         TRY(dalloc(ctx, &ctx->d_origin, spacing.size() * MAXD));
-        TRY(dalloc(ctx, &ctx->d_origin_slots, ctx->slots.size()));
+        std::vector<OriginSlot> org;
+        for (auto& S : ctx->slots)
+            if (!S.probe) org.push_back(OriginSlot{S.d_inst, !S.written});
+        TRY(dalloc(ctx, &ctx->d_origin_slots, org.size()));
+        TRY(hcopy(ctx, ctx->d_origin_slots, org.data(), org.size() * sizeof(OriginSlot), cudaMemcpyHostToDevice));
+        ctx->norigin_slots = (int)org.size();
     }
     ctx->finalized = true;
     return GC_OK;
@@ -1472,7 +1478,7 @@ int prepare(gc_ctx* ctx, const std::vector<char>& sort_mask, bool half) {
         }
         OriginArgs org{};
         if (i0 == 0)
-            org = OriginArgs{ctx->d_origin_slots, (int)ctx->origin_slots.size(), ctx->slots[0].nd, ctx->d_spacing,
+            org = OriginArgs{ctx->d_origin_slots, ctx->norigin_slots, ctx->slots[0].nd, ctx->d_spacing,
                              ctx->d_origin};
         launch_plan_all(ctx->d_plans + i0, n, ni, mask, ctx->d_need + i0, ctx->capmode ? ctx->d_need_max + i0 : nullptr,
                         ctx->d_need_cap + i0, ctx->d_err, org, ctx->stream);
@@ -2017,9 +2023,10 @@ int sweep_group(gc_ctx* ctx, int a, const std::vector<int>& ids, int stage, bool
                 // dynamic walls lend only their positions; other systems their records
                 const bool rec = D.btype == BT_SYSTEM || D.btype == BT_STATIC || D.btype == BT_VIRTUAL;
                 TRY(ensure_fpk(ctx, B, B.N, B.nd, mode, fp32));
-                // positions: once per step, once for good for a system that does not move
+                // positions: once per step, once for good for a wall while none moves
+                const bool kept = !B.written && !B.xmoves() && ctx->walls_rest;
                 const bool pos = !rec && (B.xpk_fp32 != fp32 || B.hpos_fp32 != fp32 ||
-                                          (B.xmoves() ? B.xpk_epoch != ctx->pack_epoch : !B.xpk_static));
+                                          (kept ? !B.xpk_static : B.xpk_epoch != ctx->pack_epoch));
                 launch_pack(fp32, mode, B.N, nullptr, B.nd, pk_ns, B.F(F_X), B.F(F_V), B.F(F_RHO), B.F(F_P),
                             B.kind >= GC_SYS_STRESS ? B.F(F_STRESS) : nullptr, B.inst_of, B.d_mass, ctx->d_origin, hpos_of(B.fpk),
                             pos ? pos_of(B.fpk, B.N, B.nd) : nullptr, rec ? rec_of(B, B.N, B.nd) : nullptr,
@@ -2033,7 +2040,7 @@ int sweep_group(gc_ctx* ctx, int a, const std::vector<int>& ids, int stage, bool
                 } else {
                     B.xpk_epoch = ctx->pack_epoch;
                     B.xpk_fp32 = fp32;
-                    if (!B.xmoves()) B.xpk_static = true;
+                    if (kept) B.xpk_static = true;
                     r.brec = pos_of(B.fpk, B.N, B.nd);
                     r.brq = pos_quads(B.nd, fp32);
                 }
@@ -2443,18 +2450,6 @@ void invalidate_steps(gc_ctx* ctx) {
     drop_graphs(ctx);
     ctx->exact_done = false;
     for (auto& S : ctx->slots) S.xpk_static = false;  // may count from another point
-}
-
-// The systems at rest, for the steps' plans.
-int push_motion(gc_ctx* ctx) {
-    std::vector<OriginSlot> now;
-    for (auto& S : ctx->slots)
-        if (!S.probe) now.push_back(OriginSlot{S.d_inst, !S.xmoves()});
-    bool same = now.size() == ctx->origin_slots.size();
-    for (size_t i = 0; same && i < now.size(); ++i) same = now[i].still == ctx->origin_slots[i].still;
-    if (same) return GC_OK;
-    ctx->origin_slots = now;
-    return hcopy(ctx, ctx->d_origin_slots, now.data(), now.size() * sizeof(OriginSlot), cudaMemcpyHostToDevice);
 }
 
 std::vector<char> parity(gc_ctx* ctx) {
@@ -3742,7 +3737,9 @@ int gc_step(gc_ctx* ctx, int nsteps, double cfl) {
         ctx->params_dirty = false;
     }
     if (decide_motion(ctx)) invalidate_steps(ctx);
-    TRY(push_motion(ctx));
+    // (what a wall's kept records count from follows from these systems)
+    ctx->walls_rest = true;
+    for (auto& S : ctx->slots) ctx->walls_rest &= S.probe || S.written || !S.xmoves();
     CU(cudaMemsetAsync(ctx->d_err, 0, sizeof(int), ctx->stream));
     TRY(run_steps(ctx, nsteps));
     return finish_status(ctx);

@@ -111,11 +111,12 @@ struct PlanMask {
 };
 // The point of each instance that its FP32 positions count from: the multiple
 // of a spacing (spacing[k].x, .y its inverse; powers of two) nearest to the
-// middle of its systems at rest, or of all where none is.  It follows from the
-// step's state alone, and records of a system at rest stay good.
+// middle of its walls (the systems that no functor writes), or of all its
+// systems where it has none.  It follows from the instance's state in the step
+// alone, and records of walls at rest stay good.
 struct OriginSlot {
     const SysInst* inst;  // boxes
-    int still;
+    int wall;
 };
 struct OriginArgs {
     const OriginSlot* slots;  // nullptr: not computed

@@ -942,7 +942,7 @@ __device__ void origin_block(const OriginArgs& a, int ninst) {
         for (int all = 0; all < 2 && !any; ++all) {
             for (int s = 0; s < a.nslots; ++s) {
                 const SysInst& S = a.slots[s].inst[k];
-                if (S.n == 0 || !(all || a.slots[s].still)) continue;
+                if (S.n == 0 || !(all || a.slots[s].wall)) continue;
 #pragma unroll
                 for (int d = 0; d < MAXD; ++d) {
                     lo[d] = any ? fmin(lo[d], S.bbmin[d]) : S.bbmin[d];

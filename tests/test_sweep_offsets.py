@@ -170,3 +170,24 @@ def test_both_precisions_in_one_step(cells):
         a, b = (np.asarray(getattr(q, f), float).reshape(ps.n, -1) for q in (got, ps))
         scale = np.max(np.asarray(scales[f]).reshape(ps.n, -1), axis=1, keepdims=True)
         assert np.all(np.abs(a - b) <= 2.0 * (40 + most) * 2.0 ** -53 * scale), f
+
+
+def test_instance_far_out_in_a_mix_equals_alone():
+    """(FP32-compensated; a wall at rest in one instance moves in the other)"""
+    def build(k):
+        lf = _build(2, "fluid", 3e6 + 1e4 * k, True)
+        lf.systems[1].v[:] = [0.3 * k, 0.0]
+        return lf
+    mix, alone = [build(k) for k in range(2)], [build(k) for k in range(2)]
+    s = G.Session(mix, precision=G.PRECISION_FP32_COMPENSATED)
+    s.push()
+    s.step(20, 0.05)
+    s.pull()
+    for a, b in zip(mix, alone):
+        t = G.Session([b], precision=G.PRECISION_FP32_COMPENSATED)
+        t.push()
+        t.step(20, 0.05)
+        t.pull()
+        for p, q in zip(a.systems, b.systems):
+            for f, _ in p.particle_fields():
+                assert np.isfinite(getattr(p, f)).all() and np.array_equal(getattr(p, f), getattr(q, f)), f"{p.name} {f}"
