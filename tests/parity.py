@@ -1,7 +1,8 @@
 """The per-particle error metric of the parity tests.
 
-The device and the oracle evaluate the same pair terms (bit-identical in
-FP64; FP32 in the compensated mode) but sum each particle's terms in a
+The device and the oracle evaluate the same pair terms (in FP64 to a few
+units in the last place, the counting, interpolation and XSPH functors' bit
+by bit; FP32 in the compensated mode) but sum each particle's terms in a
 different order: the device gathers them per particle, the reference
 scatters them in colour order.  A rate field that cancels to near zero
 (dv/dt of a particle in hydrostatic balance starts at gravity and loses it
@@ -43,8 +44,8 @@ comparisons after many steps do not depend on both sides sorting alike.
 Two kinds of shadow (the oracle's magnitude modes):
 
 * TERMS (mode 1), for one step from identical inputs: Σ|term| as above.
-  The two sides evaluate bit-identical FP64 terms and differ only in the
-  order of the sums.
+  The two sides differ in the order of the sums and, for the fluid and stress
+  functors, by a few units in the last place of each FP64 term.
 * INPUTS (mode 2), for comparisons whose inputs differ: after many steps
   (the trajectories drifted by a few ulps) and for the FP32-compensated
   mode (its records round v, ρ, p/ρ² and σ to FP32).  Each term's
