@@ -12,15 +12,18 @@ constexpr int FORCE_TPB = 128;  // threads per block of the sweep
 constexpr int WIN_TPB = 64;     // threads per block of the window sweep
 constexpr int FORCE_BUF = 64;   // staged-neighbour column of the counting sweep (shared memory)
 
-// Launch configurations of the window sweep: resident blocks per SM and
-// candidates per chunk, chosen per (system, stage) by the tuner in
-// gc_context.cu.  Every one gives the same bits.
+// Launch configurations of the window sweep: resident blocks per SM, candidates
+// per chunk and, FP32-compensated, whether the pair loop lists the candidates
+// that it does not add (for particles at rest on a lattice with pairs at the
+// cutoff), chosen per (system, stage) by the tuner in gc_context.cu.  Every one
+// gives the same bits.
 struct WinCfg {
     int minb, chunk;
+    bool list;
 };
 constexpr int NUM_FORCE_CFG = GC_NUM_SWEEP_CONFIGS;
-constexpr WinCfg WIN_CFGS32[NUM_FORCE_CFG] = {{8, 192}, {7, 192}, {6, 224}, {10, 160}};
-constexpr WinCfg WIN_CFGS64[NUM_FORCE_CFG] = {{6, 192}, {5, 192}, {7, 160}, {8, 128}};
+constexpr WinCfg WIN_CFGS32[NUM_FORCE_CFG] = {{8, 192, false}, {8, 192, true}, {6, 224, false}, {10, 160, false}};
+constexpr WinCfg WIN_CFGS64[NUM_FORCE_CFG] = {{6, 192, false}, {5, 192, false}, {7, 160, false}, {8, 128, false}};
 constexpr int WIN_SM_BLOCKS = 10;  // no configuration holds more blocks on an SM
 constexpr int MAX_REFS = 8;     // interactions fused into one launch
 

@@ -298,6 +298,14 @@ struct PhysF32 {
 #pragma unroll
         for (int q = 0; q < NP; ++q) a.s[q] = bc2(CUDART_NAN_F);
     }
+    template <class Q>
+    static __device__ __forceinline__ bool at_no_distance(const Rec& o, const Q& quad) {
+        Rec b;
+        float2 d;
+        float dz;
+        pos_read(quad, b);
+        return delta(o, b, d, dz) <= FLT_MIN;
+    }
     // whether pair() left this candidate to the FP64 test
     template <class Q>
     static __device__ __forceinline__ bool in_band(const Par& p, const Rec& o, const Q& quad, Acc& a) {
@@ -318,7 +326,9 @@ struct PhysF32 {
     // force need not, has exact() decide them here.  o: own record; da: own
     // distance to a dynamic boundary's plane.  BTK: the system_b kind when
     // known at compile time (BT_SELF then has no density diffusion).
-    template <int BTK, class Q, class Exact>
+    // LIST: the caller keeps a list of what is not added, so a pair at no distance
+    // is not, and `nearest` is not kept.
+    template <int BTK, bool LIST, class Q, class Exact>
     static __device__ __forceinline__ int pair(const Par& p, const GridInst& G, const PfnInst& P, const Rec& o,
                                                float da, const Q& quad, const Exact& exact, float& nearest,
                                                Acc& acc) {
@@ -335,6 +345,8 @@ struct PhysF32 {
         bool in = off < -p.band;
         if (lj_wall(bt)) {
             if (fabsf(off) <= p.band) in = exact();
+        } else if (LIST) {
+            in = in && rr > FLT_MIN;
         } else {
             nearest = min3(nearest, fabsf(off), rr);
         }

@@ -234,7 +234,7 @@ struct PhysF64 {
     // (returns 1 when accepted).  exact(): the candidate lies in this lane's
     // own strip; asked next to the cutoff only, as one further off is two
     // cells away otherwise.
-    template <int BTK, class Q, class Exact>
+    template <int BTK, bool, class Q, class Exact>
     static __device__ __forceinline__ int pair(const Par& p, const GridInst& G, const PfnInst& P, const Rec& o,
                                                double da, const Q& quad, const Exact& exact, float& nearest,
                                                Acc& acc) {

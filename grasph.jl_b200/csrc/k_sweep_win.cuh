@@ -103,7 +103,7 @@ __host__ __device__ constexpr int win_warp_bytes() {
     return NQ * CH * 16 + ND * CH * 4 + (CH / 32 + 1) * 128;
 }
 
-template <class Phys, int ND, int PFN, int MINB, int CH>
+template <class Phys, int ND, int PFN, int MINB, int CH, bool LIST>
 __global__ void __launch_bounds__(WIN_TPB, MINB) k_sweep_win(ForceArgs A) {
     pdl_enter();
     static_assert(CH % 32 == 0 && CH / 32 <= 8, "a lane's masks are numbered by batch, four bits each in a word");
@@ -213,9 +213,10 @@ __global__ void __launch_bounds__(WIN_TPB, MINB) k_sweep_win(ForceArgs A) {
                 };
                 if (coop) {
                     const int nq = r.btype == BT_DYNAMIC ? Phys::NQP : NQ;  // quads staged per candidate
-                    // conservative cutoff of the candidate test: 0.1% plus the coordinates' rounding
+                    // conservative cutoff of the candidate test: the coordinates' rounding, and
+                    // 1e-5 for the arithmetic's, below 1e-6
                     const float ce = (float)G.cell + 4.8e-7f * (xmax + 2.f * (float)G.cell);
-                    const float cut_f = 1.001f * ce * ce;
+                    const float cut_f = 1.00001f * ce * ce;
                     // every strip's warp-wide candidate range, lane s holding strip s's
                     int32_t su0 = 0, sn = 0, zlo, zhi;
                     warp_zrange<ND>(c, active, zlo, zhi);
@@ -328,6 +329,10 @@ __global__ void __launch_bounds__(WIN_TPB, MINB) k_sweep_win(ForceArgs A) {
                         // the accepted candidates, from the copies, in increasing order; the
                         // next mask is loaded while the current one is worked through
                         float nearest = FLT_MAX;
+                        // LIST: the last four candidates that were not added, their slots' numbers
+                        // + 1 a byte each
+                        unsigned left = 0;
+                        const int32_t before = accepted;
                         auto pairs = [&](auto btk) {
                             uint32_t mp = masks_s, batch = slots_s;
                             unsigned cur = 0, nxt = lds32(mp), bq = bn;
@@ -354,9 +359,11 @@ __global__ void __launch_bounds__(WIN_TPB, MINB) k_sweep_win(ForceArgs A) {
                                 const int t = __clz(cur);
                                 cur ^= 0x80000000u >> t;
                                 const uint32_t slot = batch + t * 16;
-                                accepted += Phys::template pair<decltype(btk)::value>(
+                                const int in = Phys::template pair<decltype(btk)::value, LIST>(
                                     par, G, P, o, da, [&](int q) { return lds128(slot + q * CH * 16); },
                                     [&]() { return exact_slot(wc, cc, (int)(slot - slots_s) >> 4); }, nearest, acc);
+                                accepted += in;
+                                if (LIST) left = in ? left : __byte_perm(left, ((slot - slots_s) >> 4) + 1, 0x2104);
                             }
                         };
                         if (self && !Phys::diffuses(par)) pairs(std::integral_constant<int, BT_SELF>{});
@@ -366,8 +373,32 @@ __global__ void __launch_bounds__(WIN_TPB, MINB) k_sweep_win(ForceArgs A) {
                         // them).  The masks are cut down to these first, so that the lanes wait
                         // for their FP64 positions together: the resting 80 k column's sweep
                         // 61 -> 40 us, the others unchanged.  And pairs at no distance, for
-                        // which the reference's kernel gradient is 0/0.
-                        if (nearest <= Phys::band(par)) {
+                        // which the reference's kernel gradient is 0/0.  LIST: the candidates to
+                        // look at again are listed already (four, if the others were added).
+                        if constexpr (LIST) {
+                            if (left && !Phys::lj_wall(r.btype)) {
+                                auto again = [&](int t) {
+                                    auto quad = [&](int q) { return slots[q * CH + t]; };
+                                    const bool near = Phys::in_band(par, o, quad, acc);
+                                    if (Phys::at_no_distance(o, quad) || (near && exact_slot(wc, cc, t))) ++accepted;
+                                };
+                                int32_t others = before - accepted;
+                                if (left >> 24)
+                                    for (int mi = 0; mi < nm; ++mi) others += __popc(masks[mi * 32]);
+                                if (!(left >> 24) || others == 4) {
+                                    for (; left; left >>= 8) again((int)(left & 255u) - 1);
+                                } else {
+                                    for (int mi = 0; mi < nm; ++mi) {
+                                        const int b = (bn >> (4 * mi) & 15u) * 32;
+                                        for (unsigned cur = masks[mi * 32]; cur;) {
+                                            const int t = __clz(cur);
+                                            cur ^= 0x80000000u >> t;
+                                            again(b + t);
+                                        }
+                                    }
+                                }
+                            }
+                        } else if (nearest <= Phys::band(par)) {
                             for (int mi = 0; mi < nm; ++mi) {
                                 const int b = (bn >> (4 * mi) & 15u) * 32;
                                 unsigned near = 0;
@@ -431,7 +462,7 @@ static int launch_win(const ForceArgs& A, cudaStream_t s) {
     if (blocks > (int64_t)A.num_sms * cf.minb * 4) blocks = (int64_t)A.num_sms * cf.minb * 4;
     if (blocks < 1) blocks = 1;
     constexpr size_t need = (size_t)(WIN_TPB / 32) * win_warp_bytes<ND, Phys::NQ, cf.chunk>();
-    auto kern = k_sweep_win<Phys, ND, PFN, cf.minb, cf.chunk>;
+    auto kern = k_sweep_win<Phys, ND, PFN, cf.minb, cf.chunk, cf.list>;
     // Few groups: a sweep launched while the kernel before it still runs
     // (programmatic dependent launch) finds free the SMs that finished first
     // and piles its blocks on those; with shared memory asked for beyond what
