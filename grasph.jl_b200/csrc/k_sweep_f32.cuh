@@ -298,14 +298,6 @@ struct PhysF32 {
 #pragma unroll
         for (int q = 0; q < NP; ++q) a.s[q] = bc2(CUDART_NAN_F);
     }
-    template <class Q>
-    static __device__ __forceinline__ bool at_no_distance(const Rec& o, const Q& quad) {
-        Rec b;
-        float2 d;
-        float dz;
-        pos_read(quad, b);
-        return delta(o, b, d, dz) <= FLT_MIN;
-    }
     // whether pair() left this candidate to the FP64 test
     template <class Q>
     static __device__ __forceinline__ bool in_band(const Par& p, const Rec& o, const Q& quad, Acc& a) {

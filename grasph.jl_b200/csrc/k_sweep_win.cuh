@@ -87,6 +87,10 @@ __device__ __forceinline__ unsigned lds32(uint32_t a) {
     return *reinterpret_cast<const unsigned*>(__cvta_shared_to_generic(a));
 }
 
+__device__ __forceinline__ void sts32(uint32_t a, unsigned x) {
+    *reinterpret_cast<unsigned*>(__cvta_shared_to_generic(a)) = x;
+}
+
 // Min and max over the warp of a finite float.
 __device__ __forceinline__ void warp_minmax(float v, float& lo, float& hi) {
     const int b = __float_as_int(v), key = b ^ ((b >> 31) & 0x7fffffff);
@@ -97,10 +101,10 @@ __device__ __forceinline__ void warp_minmax(float v, float& lo, float& hi) {
 
 // Shared memory of one warp: the chunk's records ([NQ][CH] quads), the
 // candidates' FP32 positions ([ND][CH]) and each lane's non-empty hit masks
-// with the empty one that ends them.
-template <int ND, int NQ, int CH>
+// with the empty one that ends them (LIST: and a word before them).
+template <int ND, int NQ, int CH, bool LIST>
 __host__ __device__ constexpr int win_warp_bytes() {
-    return NQ * CH * 16 + ND * CH * 4 + (CH / 32 + 1) * 128;
+    return NQ * CH * 16 + ND * CH * 4 + (CH / 32 + 1 + LIST) * 128;
 }
 
 template <class Phys, int ND, int PFN, int MINB, int CH, bool LIST>
@@ -109,7 +113,7 @@ __global__ void __launch_bounds__(WIN_TPB, MINB) k_sweep_win(ForceArgs A) {
     static_assert(CH % 32 == 0 && CH / 32 <= 8, "a lane's masks are numbered by batch, four bits each in a word");
     constexpr int NQ = Phys::NQ;
     constexpr int NSTR = 3, NWIN = ND == 2 ? 1 : 3;  // strips per window, windows
-    constexpr int WB = win_warp_bytes<ND, NQ, CH>();
+    constexpr int WB = win_warp_bytes<ND, NQ, CH, LIST>();
     constexpr int L = ND - 1;
     extern __shared__ float4 sstg[];
     const unsigned FULL = 0xffffffffu;
@@ -117,7 +121,7 @@ __global__ void __launch_bounds__(WIN_TPB, MINB) k_sweep_win(ForceArgs A) {
     char* wbase = reinterpret_cast<char*>(sstg) + (threadIdx.x >> 5) * WB;
     float4* slots = reinterpret_cast<float4*>(wbase);
     float* cand = reinterpret_cast<float*>(wbase + NQ * CH * 16);
-    unsigned* masks = reinterpret_cast<unsigned*>(wbase + NQ * CH * 16 + ND * CH * 4) + lane;
+    unsigned* masks = reinterpret_cast<unsigned*>(wbase + NQ * CH * 16 + ND * CH * 4 + LIST * 128) + lane;
     const uint32_t slots_s = (uint32_t)__cvta_generic_to_shared(slots);
     const uint32_t masks_s = (uint32_t)__cvta_generic_to_shared(masks);
     const int64_t ngroups = *A.ngroups;
@@ -329,10 +333,9 @@ __global__ void __launch_bounds__(WIN_TPB, MINB) k_sweep_win(ForceArgs A) {
                         // the accepted candidates, from the copies, in increasing order; the
                         // next mask is loaded while the current one is worked through
                         float nearest = FLT_MAX;
-                        // LIST: the last four candidates that were not added, their slots' numbers
-                        // + 1 a byte each
+                        // LIST: the current mask's candidates that were not added, which take
+                        // its place when the next one comes
                         unsigned left = 0;
-                        const int32_t before = accepted;
                         auto pairs = [&](auto btk) {
                             uint32_t mp = masks_s, batch = slots_s;
                             unsigned cur = 0, nxt = lds32(mp), bq = bn;
@@ -350,6 +353,10 @@ __global__ void __launch_bounds__(WIN_TPB, MINB) k_sweep_win(ForceArgs A) {
                                     // which the FP32 terms do not hide (699 against 690 us on the
                                     // million-particle dam break; FP64 prefers the branch)
                                     const bool pop = cur == 0;
+                                    if (LIST) {
+                                        if (pop) sts32(mp - 128, left);
+                                        left = pop ? 0u : left;
+                                    }
                                     cur = pop ? nxt : cur;
                                     batch = pop ? slots_s + (bq & 15u) * (32 * 16) : batch;
                                     bq = pop ? bq >> 4 : bq;
@@ -363,8 +370,9 @@ __global__ void __launch_bounds__(WIN_TPB, MINB) k_sweep_win(ForceArgs A) {
                                     par, G, P, o, da, [&](int q) { return lds128(slot + q * CH * 16); },
                                     [&]() { return exact_slot(wc, cc, (int)(slot - slots_s) >> 4); }, nearest, acc);
                                 accepted += in;
-                                if (LIST) left = in ? left : __byte_perm(left, ((slot - slots_s) >> 4) + 1, 0x2104);
+                                if (LIST) left = in ? left : left | 0x80000000u >> t;
                             }
+                            if (LIST) sts32(mp - 128, left);
                         };
                         if (self && !Phys::diffuses(par)) pairs(std::integral_constant<int, BT_SELF>{});
                         else pairs(std::integral_constant<int, -1>{});
@@ -373,29 +381,24 @@ __global__ void __launch_bounds__(WIN_TPB, MINB) k_sweep_win(ForceArgs A) {
                         // them).  The masks are cut down to these first, so that the lanes wait
                         // for their FP64 positions together: the resting 80 k column's sweep
                         // 61 -> 40 us, the others unchanged.  And pairs at no distance, for
-                        // which the reference's kernel gradient is 0/0.  LIST: the candidates to
-                        // look at again are listed already (four, if the others were added).
+                        // which the reference's kernel gradient is 0/0.  LIST: the masks hold
+                        // what was not added, and FP64 decides about all of it.
                         if constexpr (LIST) {
-                            if (left && !Phys::lj_wall(r.btype)) {
-                                auto again = [&](int t) {
-                                    auto quad = [&](int q) { return slots[q * CH + t]; };
-                                    const bool near = Phys::in_band(par, o, quad, acc);
-                                    if (Phys::at_no_distance(o, quad) || (near && exact_slot(wc, cc, t))) ++accepted;
-                                };
-                                int32_t others = before - accepted;
-                                if (left >> 24)
-                                    for (int mi = 0; mi < nm; ++mi) others += __popc(masks[mi * 32]);
-                                if (!(left >> 24) || others == 4) {
-                                    for (; left; left >>= 8) again((int)(left & 255u) - 1);
-                                } else {
-                                    for (int mi = 0; mi < nm; ++mi) {
-                                        const int b = (bn >> (4 * mi) & 15u) * 32;
-                                        for (unsigned cur = masks[mi * 32]; cur;) {
-                                            const int t = __clz(cur);
-                                            cur ^= 0x80000000u >> t;
-                                            again(b + t);
-                                        }
-                                    }
+                            int32_t u2[NSTR], e2[NSTR + 1];
+                            window(wc, u2, e2);
+                            for (int mi = 0; mi < nm && !Phys::lj_wall(r.btype); ++mi) {
+                                const int b = (bn >> (4 * mi) & 15u) * 32;
+                                for (unsigned cur = masks[mi * 32]; cur;) {
+                                    const int t = b + __clz(cur);
+                                    cur ^= 0x80000000u >> (t - b);
+                                    const int32_t tt = cc + t;
+                                    const int32_t j = tt + (tt < e2[1] ? u2[0] : tt < e2[2] ? u2[1] : u2[2]);
+                                    double y[ND], r2;
+                                    if (!exact_test(j, y, r2)) continue;
+                                    // (the strip's range matters along its own direction alone)
+                                    if (fabs(y[L]) > G.cell * (1.0 - strip_doubt<ND>(G)) && !exact_slot(wc, cc, t)) continue;
+                                    ++accepted;
+                                    if (r2 < 1e-30) Phys::in_band(par, o, [&](int q) { return slots[q * CH + t]; }, acc);
                                 }
                             }
                         } else if (nearest <= Phys::band(par)) {
@@ -461,7 +464,7 @@ static int launch_win(const ForceArgs& A, cudaStream_t s) {
     int64_t blocks = (A.aN * 32 + WIN_TPB - 1) / WIN_TPB;
     if (blocks > (int64_t)A.num_sms * cf.minb * 4) blocks = (int64_t)A.num_sms * cf.minb * 4;
     if (blocks < 1) blocks = 1;
-    constexpr size_t need = (size_t)(WIN_TPB / 32) * win_warp_bytes<ND, Phys::NQ, cf.chunk>();
+    constexpr size_t need = (size_t)(WIN_TPB / 32) * win_warp_bytes<ND, Phys::NQ, cf.chunk, cf.list>();
     auto kern = k_sweep_win<Phys, ND, PFN, cf.minb, cf.chunk, cf.list>;
     // Few groups: a sweep launched while the kernel before it still runs
     // (programmatic dependent launch) finds free the SMs that finished first

@@ -161,9 +161,8 @@ typedef struct gc_stats {
                                     (src/Sorting.jl:176-186)                     */
 } gc_stats;
 
-/* Launch configurations of the pair sweep (block residency, staged
- * neighbours per thread, prefetch of the next neighbour's data); all give
- * bit-identical results.                                                  */
+/* Launch configurations of the pair sweep (block residency, candidates per
+ * chunk, a list of the pairs at the cutoff); all give bit-identical results. */
 #define GC_NUM_SWEEP_CONFIGS 4
 
 /* ============================================================ lifecycle */
