@@ -298,6 +298,16 @@ struct PhysF32 {
 #pragma unroll
         for (int q = 0; q < NP; ++q) a.s[q] = bc2(CUDART_NAN_F);
     }
+    // whether pair<.., LIST>() did not add this candidate
+    template <class Q>
+    static __device__ __forceinline__ bool not_added(const Par& p, const Rec& o, const Q& quad) {
+        Rec b;
+        float2 d;
+        float dz;
+        pos_read(quad, b);
+        const float rr = delta(o, b, d, dz);
+        return !(rr - p.cut < -p.band && rr > FLT_MIN);
+    }
     // whether pair() left this candidate to the FP64 test
     template <class Q>
     static __device__ __forceinline__ bool in_band(const Par& p, const Rec& o, const Q& quad, Acc& a) {

@@ -333,9 +333,12 @@ __global__ void __launch_bounds__(WIN_TPB, MINB) k_sweep_win(ForceArgs A) {
                         // the accepted candidates, from the copies, in increasing order; the
                         // next mask is loaded while the current one is worked through
                         float nearest = FLT_MAX;
-                        // LIST: the current mask's candidates that were not added, which take
-                        // its place when the next one comes
+                        // LIST: the candidates that were not added.  In 2-D (few) the last four
+                        // of the chunk, their slots' numbers + 1 a byte each; in 3-D those of the
+                        // current mask, which take its place when the next one comes.
+                        constexpr bool BYTES = LIST && ND == 2, MASKS = LIST && ND == 3;
                         unsigned left = 0;
+                        const int32_t before = accepted;
                         auto pairs = [&](auto btk) {
                             uint32_t mp = masks_s, batch = slots_s;
                             unsigned cur = 0, nxt = lds32(mp), bq = bn;
@@ -353,7 +356,7 @@ __global__ void __launch_bounds__(WIN_TPB, MINB) k_sweep_win(ForceArgs A) {
                                     // which the FP32 terms do not hide (699 against 690 us on the
                                     // million-particle dam break; FP64 prefers the branch)
                                     const bool pop = cur == 0;
-                                    if (LIST) {
+                                    if (MASKS) {
                                         if (pop) sts32(mp - 128, left);
                                         left = pop ? 0u : left;
                                     }
@@ -370,9 +373,10 @@ __global__ void __launch_bounds__(WIN_TPB, MINB) k_sweep_win(ForceArgs A) {
                                     par, G, P, o, da, [&](int q) { return lds128(slot + q * CH * 16); },
                                     [&]() { return exact_slot(wc, cc, (int)(slot - slots_s) >> 4); }, nearest, acc);
                                 accepted += in;
-                                if (LIST) left = in ? left : left | 0x80000000u >> t;
+                                if (BYTES) left = in ? left : __byte_perm(left, ((slot - slots_s) >> 4) + 1, 0x2104);
+                                if (MASKS) left = in ? left : left | 0x80000000u >> t;
                             }
-                            if (LIST) sts32(mp - 128, left);
+                            if (MASKS) sts32(mp - 128, left);
                         };
                         if (self && !Phys::diffuses(par)) pairs(std::integral_constant<int, BT_SELF>{});
                         else pairs(std::integral_constant<int, -1>{});
@@ -381,24 +385,58 @@ __global__ void __launch_bounds__(WIN_TPB, MINB) k_sweep_win(ForceArgs A) {
                         // them).  The masks are cut down to these first, so that the lanes wait
                         // for their FP64 positions together: the resting 80 k column's sweep
                         // 61 -> 40 us, the others unchanged.  And pairs at no distance, for
-                        // which the reference's kernel gradient is 0/0.  LIST: the masks hold
-                        // what was not added, and FP64 decides about all of it.
+                        // which the reference's kernel gradient is 0/0.  LIST: FP64 decides about
+                        // all that was not added, two candidates at a time for the latency.
                         if constexpr (LIST) {
                             int32_t u2[NSTR], e2[NSTR + 1];
                             window(wc, u2, e2);
-                            for (int mi = 0; mi < nm && !Phys::lj_wall(r.btype); ++mi) {
-                                const int b = (bn >> (4 * mi) & 15u) * 32;
-                                for (unsigned cur = masks[mi * 32]; cur;) {
-                                    const int t = b + __clz(cur);
-                                    cur ^= 0x80000000u >> (t - b);
-                                    const int32_t tt = cc + t;
+                            auto decide = [&](int t0, int t1) {  // (t1 < 0: none)
+                                int t[2] = {t0, t1 < 0 ? t0 : t1};
+                                double y[2][ND], r2[2];
+                                bool in[2];
+#pragma unroll
+                                for (int q = 0; q < 2; ++q) {
+                                    const int32_t tt = cc + t[q];
                                     const int32_t j = tt + (tt < e2[1] ? u2[0] : tt < e2[2] ? u2[1] : u2[2]);
-                                    double y[ND], r2;
-                                    if (!exact_test(j, y, r2)) continue;
+                                    in[q] = exact_test(j, y[q], r2[q]);
+                                }
+                                in[1] = in[1] && t1 >= 0;
+#pragma unroll
+                                for (int q = 0; q < 2; ++q) {
                                     // (the strip's range matters along its own direction alone)
-                                    if (fabs(y[L]) > G.cell * (1.0 - strip_doubt<ND>(G)) && !exact_slot(wc, cc, t)) continue;
-                                    ++accepted;
-                                    if (r2 < 1e-30) Phys::in_band(par, o, [&](int q) { return slots[q * CH + t]; }, acc);
+                                    if (in[q] && fabs(y[q][L]) > G.cell * (1.0 - strip_doubt<ND>(G)))
+                                        in[q] = exact_slot(wc, cc, t[q]);
+                                    accepted += in[q];
+                                    if (in[q] && r2[q] < 1e-30)
+                                        Phys::in_band(par, o, [&](int c) { return slots[c * CH + t[q]]; }, acc);
+                                }
+                            };
+                            const bool some = !Phys::lj_wall(r.btype) && (MASKS || left);
+                            bool listed = BYTES;
+                            if (BYTES && some && left >> 24) {
+                                // four are all of them if the others were added
+                                int32_t others = before - accepted;
+                                for (int mi = 0; mi < nm; ++mi) others += __popc(masks[mi * 32]);
+                                listed = others == 4;
+                            }
+                            if (some && listed) {
+                                for (; left; left >>= 16) decide((int)(left & 255u) - 1, (int)(left >> 8 & 255u) - 1);
+                            } else if (some) {
+                                for (int mi = 0; mi < nm; ++mi) {
+                                    const int b = (bn >> (4 * mi) & 15u) * 32;
+                                    for (unsigned cur = masks[mi * 32]; cur;) {
+                                        const int t0 = __clz(cur);
+                                        cur ^= 0x80000000u >> t0;
+                                        int t1 = -1;
+                                        if (MASKS && cur) {
+                                            t1 = __clz(cur);
+                                            cur ^= 0x80000000u >> t1;
+                                            t1 += b;
+                                        }
+                                        // (2-D: all the accepted candidates, of which some were added)
+                                        if (MASKS || Phys::not_added(par, o, [&](int c) { return slots[c * CH + b + t0]; }))
+                                            decide(b + t0, t1);
+                                    }
                                 }
                             }
                         } else if (nearest <= Phys::band(par)) {
