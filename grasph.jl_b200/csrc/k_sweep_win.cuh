@@ -390,6 +390,11 @@ __global__ void __launch_bounds__(WIN_TPB, MINB) k_sweep_win(ForceArgs A) {
                         if constexpr (LIST) {
                             int32_t u2[NSTR], e2[NSTR + 1];
                             window(wc, u2, e2);
+                            // (the strip's range matters along its own direction alone)
+                            const double edge = G.cell * (1.0 - strip_doubt<ND>(G)), cut = G.cutoff_sq;
+                            double xo[ND];
+#pragma unroll
+                            for (int d = 0; d < ND; ++d) xo[d] = A.ax[d * A.aN + gi];
                             auto decide = [&](int t0, int t1) {  // (t1 < 0: none)
                                 int t[2] = {t0, t1 < 0 ? t0 : t1};
                                 double y[2][ND], r2[2];
@@ -398,14 +403,15 @@ __global__ void __launch_bounds__(WIN_TPB, MINB) k_sweep_win(ForceArgs A) {
                                 for (int q = 0; q < 2; ++q) {
                                     const int32_t tt = cc + t[q];
                                     const int32_t j = tt + (tt < e2[1] ? u2[0] : tt < e2[2] ? u2[1] : u2[2]);
-                                    in[q] = exact_test(j, y[q], r2[q]);
+#pragma unroll
+                                    for (int d = 0; d < ND; ++d) y[q][d] = __dsub_rn(xo[d], r.bx[d * r.bN + j]);
+                                    r2[q] = dot_exact<ND>(y[q], y[q]);
+                                    in[q] = r2[q] < cut;
                                 }
                                 in[1] = in[1] && t1 >= 0;
 #pragma unroll
                                 for (int q = 0; q < 2; ++q) {
-                                    // (the strip's range matters along its own direction alone)
-                                    if (in[q] && fabs(y[q][L]) > G.cell * (1.0 - strip_doubt<ND>(G)))
-                                        in[q] = exact_slot(wc, cc, t[q]);
+                                    if (in[q] && fabs(y[q][L]) > edge) in[q] = exact_slot(wc, cc, t[q]);
                                     accepted += in[q];
                                     if (in[q] && r2[q] < 1e-30)
                                         Phys::in_band(par, o, [&](int c) { return slots[c * CH + t[q]]; }, acc);
