@@ -324,10 +324,11 @@ struct PhysF32 {
     // lies below the band around the cutoff (returns 1); `nearest` keeps how
     // near to the cutoff, or to 0, an r² came (one three-input minimum).  The
     // pairs inside the band are left to the caller to count: the kernel's
-    // gradient there is below 1e-11 of its peak, so their terms vanish in FP32.  Only a Lennard-Jones wall, whose
-    // force need not, has exact() decide them here.  o: own record; da: own
-    // distance to a dynamic boundary's plane.  BTK: the system_b kind when
-    // known at compile time (BT_SELF then has no density diffusion).
+    // gradient there is below 1e-11 of its peak, so their terms vanish in FP32.
+    // Only a Lennard-Jones wall, whose force need not, has exact() decide them
+    // here.  o: own record; da: own distance to a dynamic boundary's plane.  BTK:
+    // the system_b kind when known at compile time (BT_SELF then has no density
+    // diffusion).
     // LIST: the caller keeps a list of what is not added, so a pair at no distance
     // is not, and `nearest` is not kept.
     template <int BTK, bool LIST, class Q, class Exact>
