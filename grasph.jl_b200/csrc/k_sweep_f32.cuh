@@ -298,9 +298,9 @@ struct PhysF32 {
 #pragma unroll
         for (int q = 0; q < NP; ++q) a.s[q] = bc2(CUDART_NAN_F);
     }
-    // whether pair<.., LIST>() did not add this candidate
+    // whether pair<.., LIST>() did not count this candidate
     template <class Q>
-    static __device__ __forceinline__ bool not_added(const Par& p, const Rec& o, const Q& quad) {
+    static __device__ __forceinline__ bool not_counted(const Par& p, const Rec& o, const Q& quad) {
         Rec b;
         float2 d;
         float dz;
@@ -308,16 +308,16 @@ struct PhysF32 {
         const float rr = delta(o, b, d, dz);
         return !(rr - p.cut < -p.band && rr > FLT_MIN);
     }
-    // whether pair() left this candidate to the FP64 test
+    // whether pair() left this candidate to the FP64 test, next to the cutoff or
+    // where the FP32 pairs of the two positions are equal
     template <class Q>
-    static __device__ __forceinline__ bool in_band(const Par& p, const Rec& o, const Q& quad, Acc& a) {
+    static __device__ __forceinline__ bool left_over(const Par& p, const Rec& o, const Q& quad, Acc&) {
         Rec b;
         float2 d;
         float dz;
         pos_read(quad, b);
         const float rr = delta(o, b, d, dz);
-        if (rr <= FLT_MIN) spoil(p, a);
-        return fabsf(rr - p.cut) <= p.band;
+        return fabsf(rr - p.cut) <= p.band || rr <= FLT_MIN;
     }
 
     // One candidate: r² from the FP32 pairs, then the functor's term when it
@@ -329,8 +329,8 @@ struct PhysF32 {
     // here.  o: own record; da: own distance to a dynamic boundary's plane.  BTK:
     // the system_b kind when known at compile time (BT_SELF then has no density
     // diffusion).
-    // LIST: the caller keeps a list of what is not added, so a pair at no distance
-    // is not, and `nearest` is not kept.
+    // LIST: the caller keeps a list of what this does not count, which a pair at
+    // no distance is among, and `nearest` is not kept.
     template <int BTK, bool LIST, class Q, class Exact>
     static __device__ __forceinline__ int pair(const Par& p, const GridInst& G, const PfnInst& P, const Rec& o,
                                                float da, const Q& quad, const Exact& exact, float& nearest,
@@ -348,13 +348,11 @@ struct PhysF32 {
         bool in = off < -p.band;
         if (lj_wall(bt)) {
             if (fabsf(off) <= p.band) in = exact();
-        } else if (LIST) {
-            in = in && rr > FLT_MIN;
-        } else {
+        } else if (!LIST) {
             nearest = min3(nearest, fabsf(off), rr);
         }
         term<BTK>(p, G, P, o, da, b, d, dz, rr, in, acc);
-        return in ? 1 : 0;
+        return LIST && !lj_wall(bt) ? in && rr > FLT_MIN : in;
     }
 
     // The term of an accepted pair from its FP64 differences.
@@ -363,7 +361,7 @@ struct PhysF32 {
         const float rr = lj_wall(p.bt) ? (float)r2 : fmaxf((float)r2, FLT_MIN);
         term<-1>(p, G, P, o, da, b, make_float2((float)y[0], (float)y[1]), ND == 3 ? (float)y[ND - 1] : 0.f, rr, true,
                  acc);
-        if (r2 == 0.0) spoil(p, acc);
+        if ((float)r2 == 0.f) spoil(p, acc);
     }
 
     // The functor's term of a pair at distance (d, dz), r² = rr, onto the

@@ -173,7 +173,7 @@ struct PhysF64 {
         for (int q = 0; q < NSUM; ++q) a.s[q] = CUDART_NAN;
     }
     template <class Q>
-    static __device__ __forceinline__ bool in_band(const Par& p, const Rec& o, const Q& quad, Acc& a) {
+    static __device__ __forceinline__ bool left_over(const Par& p, const Rec& o, const Q& quad, Acc& a) {
         Rec b;
         pos_read(quad, b);
         double d[ND];

@@ -241,7 +241,7 @@ __global__ void __launch_bounds__(WIN_TPB, MINB) k_sweep_win(ForceArgs A) {
                     };
                     // the reference's test of slot t of window wi's chunk at ch, which has
                     // to lie in this lane's own strip [cs[z-1], cs[z+2])
-                    auto exact_slot = [&](int wi, int32_t ch, int32_t t) {
+                    auto exact_slot = [&](int wi, int32_t ch, int32_t t, double& r2) {
                         t += ch;
                         int32_t lo = 0, hi = 0, j = 0, e = 0;
 #pragma unroll 1
@@ -256,7 +256,7 @@ __global__ void __launch_bounds__(WIN_TPB, MINB) k_sweep_win(ForceArgs A) {
                             }
                             e += n;
                         }
-                        double y[ND], r2;
+                        double y[ND];
                         return j >= lo && j < hi && exact_test(j, y, r2);
                     };
                     // f(slot, candidate) for this lane's share of the chunk at ch
@@ -333,7 +333,7 @@ __global__ void __launch_bounds__(WIN_TPB, MINB) k_sweep_win(ForceArgs A) {
                         // the accepted candidates, from the copies, in increasing order; the
                         // next mask is loaded while the current one is worked through
                         float nearest = FLT_MAX;
-                        // LIST: the candidates that were not added.  In 2-D (few) the last four
+                        // LIST: the candidates that were not counted.  In 2-D (few) the last four
                         // of the chunk, their slots' numbers + 1 a byte each; in 3-D those of the
                         // current mask, which take its place when the next one comes.
                         constexpr bool BYTES = LIST && ND == 2, MASKS = LIST && ND == 3;
@@ -371,7 +371,11 @@ __global__ void __launch_bounds__(WIN_TPB, MINB) k_sweep_win(ForceArgs A) {
                                 const uint32_t slot = batch + t * 16;
                                 const int in = Phys::template pair<decltype(btk)::value, LIST>(
                                     par, G, P, o, da, [&](int q) { return lds128(slot + q * CH * 16); },
-                                    [&]() { return exact_slot(wc, cc, (int)(slot - slots_s) >> 4); }, nearest, acc);
+                                    [&]() {
+                                        double r2;
+                                        return exact_slot(wc, cc, (int)(slot - slots_s) >> 4, r2);
+                                    },
+                                    nearest, acc);
                                 accepted += in;
                                 if (BYTES) left = in ? left : __byte_perm(left, ((slot - slots_s) >> 4) + 1, 0x2104);
                                 if (MASKS) left = in ? left : left | 0x80000000u >> t;
@@ -385,8 +389,10 @@ __global__ void __launch_bounds__(WIN_TPB, MINB) k_sweep_win(ForceArgs A) {
                         // them).  The masks are cut down to these first, so that the lanes wait
                         // for their FP64 positions together: the resting 80 k column's sweep
                         // 61 -> 40 us, the others unchanged.  And pairs at no distance, for
-                        // which the reference's kernel gradient is 0/0.  LIST: FP64 decides about
-                        // all that was not added, two candidates at a time for the latency.
+                        // which the reference's kernel gradient is 0/0: by their FP64 r², as
+                        // FP32 pairs are equal an ulp apart too (709 us at 1 M particles with
+                        // and without; decided in the first of the two loops, 724).  LIST: FP64 decides about
+                        // all that was not counted, two candidates at a time for the latency.
                         if constexpr (LIST) {
                             int32_t u2[NSTR], e2[NSTR + 1];
                             window(wc, u2, e2);
@@ -411,16 +417,15 @@ __global__ void __launch_bounds__(WIN_TPB, MINB) k_sweep_win(ForceArgs A) {
                                 in[1] = in[1] && t1 >= 0;
 #pragma unroll
                                 for (int q = 0; q < 2; ++q) {
-                                    if (in[q] && fabs(y[q][L]) > edge) in[q] = exact_slot(wc, cc, t[q]);
+                                    if (in[q] && fabs(y[q][L]) > edge) in[q] = exact_slot(wc, cc, t[q], r2[q]);
                                     accepted += in[q];
-                                    if (in[q] && r2[q] < 1e-30)
-                                        Phys::in_band(par, o, [&](int c) { return slots[c * CH + t[q]]; }, acc);
+                                    if (in[q] && (float)r2[q] == 0.f) Phys::spoil(par, acc);
                                 }
                             };
                             const bool some = !Phys::lj_wall(r.btype) && (MASKS || left);
                             bool listed = BYTES;
                             if (BYTES && some && left >> 24) {
-                                // four are all of them if the others were added
+                                // four are all of them if the others were counted
                                 int32_t others = before - accepted;
                                 for (int mi = 0; mi < nm; ++mi) others += __popc(masks[mi * 32]);
                                 listed = others == 4;
@@ -439,8 +444,8 @@ __global__ void __launch_bounds__(WIN_TPB, MINB) k_sweep_win(ForceArgs A) {
                                             cur ^= 0x80000000u >> t1;
                                             t1 += b;
                                         }
-                                        // (2-D: all the accepted candidates, of which some were added)
-                                        if (MASKS || Phys::not_added(par, o, [&](int c) { return slots[c * CH + b + t0]; }))
+                                        // (2-D: all the accepted candidates, of which some were counted)
+                                        if (MASKS || Phys::not_counted(par, o, [&](int c) { return slots[c * CH + b + t0]; }))
                                             decide(b + t0, t1);
                                     }
                                 }
@@ -452,8 +457,8 @@ __global__ void __launch_bounds__(WIN_TPB, MINB) k_sweep_win(ForceArgs A) {
                                 for (unsigned cur = masks[mi * 32]; cur;) {
                                     const int t = __clz(cur);
                                     cur ^= 0x80000000u >> t;
-                                    if (Phys::in_band(par, o, [&](int q) { return slots[q * CH + b + t]; }, acc))
-                                        near |= 0x80000000u >> t;
+                                    auto quad = [&](int q) { return slots[q * CH + b + t]; };
+                                    if (Phys::left_over(par, o, quad, acc)) near |= 0x80000000u >> t;
                                 }
                                 masks[mi * 32] = near;
                             }
@@ -464,7 +469,11 @@ __global__ void __launch_bounds__(WIN_TPB, MINB) k_sweep_win(ForceArgs A) {
                                     if (!near) break;
                                     const int t = __clz(near);
                                     near ^= 0x80000000u >> t;
-                                    if (exact_slot(wc, cc, (int)(bn >> (4 * mi) & 15u) * 32 + t)) ++accepted;
+                                    double r2;
+                                    if (!exact_slot(wc, cc, (int)(bn >> (4 * mi) & 15u) * 32 + t, r2)) continue;
+                                    // (at no distance: counted already)
+                                    if (r2 > 1e-9 * G.cutoff_sq) ++accepted;
+                                    else if ((float)r2 == 0.f) Phys::spoil(par, acc);
                                 }
                             }
                         }

@@ -43,12 +43,14 @@ def _build(nd, functor, kernel, spoil, wall=None):
     return G.LeapFrogTimeIntegrator(systems, [G.SystemInteraction(k, pfn, ps, b)])
 
 
-def _check(build, precision, tol, fields):
+def _check(build, precision, tol, fields, config=-1):
     """One sweep of every stage (a step would integrate what is not finite)."""
     runs = {}
     for name in ("oracle", "cuda"):
         lf = build()
         s = G.Session([lf], backend=make_backend(name), precision=precision if name == "cuda" else G.PRECISION_FP64)
+        if name == "cuda" and config >= 0:
+            s.backend.set_sweep_config(config)
         s.push()
         ps, si = lf.systems[0], lf.interactions[0]
         for q in lf.systems:
@@ -123,3 +125,16 @@ def test_coincident_far_out(precision):
     ps = _check(lambda: _build(2, "stress", "wendland", spoil), precision,
                 1e-12 if precision == G.PRECISION_FP64 else 1e-5, FIELDS["stress"])
     assert np.isnan(ps.drhodt).sum() == 2
+
+
+@pytest.mark.parametrize("config", range(4))
+@pytest.mark.parametrize("kernel", ["spline", "wendland"])
+@pytest.mark.parametrize("nd,functor", [(2, "fluid"), (3, "stress")])
+def test_an_ulp_apart(nd, functor, kernel, config):
+    """Positions that differ, but by less than an FP32 pair holds: no NaN."""
+    def spoil(ps):
+        ps.x[7] = ps.x[8]
+        ps.x[7, 0] = np.nextafter(ps.x[8, 0], 1.0)
+    ps = _check(lambda: _build(nd, functor, kernel, spoil), G.PRECISION_FP32_COMPENSATED, 1e-5, FIELDS[functor],
+                config)
+    assert np.isfinite(ps.dvdt).all() and np.isfinite(ps.drhodt).all()
